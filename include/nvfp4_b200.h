@@ -83,7 +83,7 @@ NVFP4_API int nvfp4_quantize_weight(const void* w, int w_dtype, int E, int N, in
  * image: it calls no cudaMalloc, no cudaFree and no allocating library routine.
  *
  *   - At most NVFP4_STATIC_MAX_EXPERTS experts per call; more is NVFP4_E_INVALID_ARGUMENT.
- *   - The array (4 KB) exists once per GPU per process for as long as the library is loaded.
+ *   - The array (128 KB) exists once per GPU per process for as long as the library is loaded.
  *   - The first call made on a device looks the array's device address up (one
  *     cudaGetSymbolAddress); make that first call outside any stream capture.
  *   - All calls on a device share the array, which is cleared at the start of each call on

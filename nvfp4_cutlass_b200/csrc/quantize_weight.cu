@@ -4,13 +4,21 @@
 // torch implementation (python/nvfp4_gemm/layout.py:68-127): the same three true
 // FP32 divisions, the same clamps, RNE everywhere.
 //
-// HBM-bound: 2 or 4 bytes read per element, 9/16 byte written.  One thread owns one
-// 64-element scale atom of one weight row (a 128-byte line of BF16 input, a 32-byte
-// sector of packed output); consecutive threads take consecutive rows, so the scale
-// words, which the kernel wants transposed to (K/64, N), are written coalesced.
+// HBM-bound: 2 or 4 bytes read per element, 9/16 byte written.  G needs the maximum of a whole expert before any of its
+// blocks can be quantised, so the weights are read twice; the second read should come out of L2.  The experts are
+// therefore taken in batches (one expert, or several small ones, kBatchBytes) and one kernel walks a list of tiles in
+// which the quantisation of batch i - 1, which sits in L2, is interleaved with the maxima of batch i, which streams in
+// from HBM.  Blocks draw tiles from a counter in list order and a quantisation tile waits only for tiles ahead of it,
+// so whatever number of blocks runs at a time, the ones that are waited for are running or done.
+// Measured (BF16): 8 experts of 4096 x 7168 (58 MB each, too large for two of them to share L2) 176 us = 1.07 GB of traffic at
+// 6.1 TB/s, before 1000 us (a scalar load per element, 40 instructions per element, an atomic per warp on one word);
+// 32 of 4096 x 1536: 128 us = 4.1 TB/s of 400 MB read and 113 MB written once, the rest is the warps' latency.
+#include <climits>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "host_common.hpp"
 #include "launchers.hpp"
@@ -19,26 +27,11 @@
 namespace nvfp4 {
 namespace {
 
-template <typename T> __device__ __forceinline__ float load_f32(const T* p);
-template <> __device__ __forceinline__ float load_f32<float>(const float* p) { return __ldg(p); }
-template <> __device__ __forceinline__ float load_f32<__nv_bfloat16>(const __nv_bfloat16* p)
-{
-    return __uint_as_float(static_cast<uint32_t>(__ldg(reinterpret_cast<const unsigned short*>(p))) << 16);
-}
-
-template <typename T>
-__global__ void expert_amax_kernel(const T* __restrict__ w, int64_t per_expert, uint32_t* __restrict__ amax_bits)
-{
-    const int e = blockIdx.y;
-    const T* we = w + static_cast<int64_t>(e) * per_expert;
-    float m = 0.0f;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < per_expert;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        m = fmaxf(m, fabsf(load_f32(we + i)));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(amax_bits + e, __float_as_uint(m));   // non-negative floats order as integers
-}
+constexpr int kThreads = 256, kWarps = kThreads / 32, kBlocksPerSm = 3;
+constexpr int kUnitRows = 8, kUnitK = 512, kStep = 2;      // a warp's share of a quantisation tile: 8 weight rows x 512 K,
+constexpr int kTileRows = kWarps * kUnitRows;              // two rows at a time; the tile: 64 rows
+constexpr int kAmaxUnroll = 8, kAmaxSteps = 2;             // a maximum tile: two times eight 32-byte loads per thread
+constexpr int64_t kBatchBytes = 24ll << 20;
 
 __device__ __forceinline__ float e4m3_to_f32(uint32_t code)
 {
@@ -47,65 +40,334 @@ __device__ __forceinline__ float e4m3_to_f32(uint32_t code)
     return __half2float(__ushort_as_half(static_cast<unsigned short>(h2 & 0xffffu)));
 }
 
-template <typename T>
-__global__ void quantize_weight_kernel(const T* __restrict__ w, int N, int K, const uint32_t* __restrict__ amax_bits,
-                                       uint8_t* __restrict__ b, int32_t* __restrict__ sfb, float* __restrict__ gw)
+// 32 bytes of weights.  kLast: the last use of the line, which may leave L2 before the lines that are still to be read.
+// kAligned = false: a tensor that starts off a 32-byte boundary, read element by element.
+struct Vec { uint32_t w[8]; };
+template <typename T, bool kAligned, bool kLast>
+__device__ __forceinline__ Vec load32(const T* p)
 {
-    const int atoms = K / 64;
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const int at = blockIdx.y, e = blockIdx.z;
-    const float tiny = 1.17549435e-38f;
-    const float g = fmaxf(__fdiv_rn(__uint_as_float(amax_bits[e]), 2688.0f), tiny);
-    if (n == 0 && at == 0) gw[e] = g;
-    if (n >= N) return;
-    const T* src = w + (static_cast<int64_t>(e) * N + n) * K + at * 64;
-    uint32_t word = 0;
-    uint32_t packed[8];
+    Vec v;
+    if constexpr (!kAligned) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        float x[16];
-        float bmax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { x[i] = load_f32(src + j * 16 + i); bmax = fmaxf(bmax, fabsf(x[i])); }
-        const float s_pre = fmaxf(__fdiv_rn(__fdiv_rn(bmax, 6.0f), g), 0.001953125f);
-        const uint32_t sc = ptx::cvt_e4m3(s_pre);
-        word |= sc << (8 * j);
-        const float denom = fmaxf(__fmul_rn(e4m3_to_f32(sc), g), tiny);
-        float q[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) q[i] = __fdiv_rn(x[i], denom);
-        packed[2 * j] = ptx::cvt_e2m1x8(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
-        packed[2 * j + 1] = ptx::cvt_e2m1x8(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
+        for (int i = 0; i < 8; ++i) {
+            if constexpr (std::is_same_v<T, float>) v.w[i] = __float_as_uint(p[i]);
+            else v.w[i] = __bfloat16_as_ushort(p[2 * i]) | static_cast<uint32_t>(__bfloat16_as_ushort(p[2 * i + 1])) << 16;
+        }
+    } else if constexpr (kLast) {
+        asm volatile("ld.global.nc.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p));
+    } else {
+        asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p));
     }
-    uint4* dst = reinterpret_cast<uint4*>(b + (static_cast<int64_t>(e) * N + n) * (K / 2) + at * 32);
-    dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-    dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-    sfb[(static_cast<int64_t>(e) * atoms + at) * N + n] = static_cast<int32_t>(word);
+    return v;
 }
 
-// The two kernels (G needs the whole expert's maximum first) with the per-expert maxima staged in `amax_bits`,
-// E words the caller provides; they are cleared here, on the call's stream.
-int run_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw, uint32_t* amax_bits,
+// max(m, largest magnitude of the vector)
+template <typename T>
+__device__ __forceinline__ float amax_of(float m, const Vec& v)
+{
+    if constexpr (std::is_same_v<T, float>) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(__uint_as_float(v.w[i])));
+        return m;
+    } else {
+        uint32_t h = v.w[0];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) h = ptx::max_abs_bf16x2(h, v.w[i]);
+        h = ptx::max_abs_bf16x2(h, h >> 16);
+        return fmaxf(m, __uint_as_float((h & 0x7fffu) << 16));
+    }
+}
+
+// One tile of the maximum pass: 128 KB of one expert; the result is valid in thread 0.
+template <typename T, bool kAligned>
+__device__ __forceinline__ uint32_t amax_tile(const T* __restrict__ expert, int64_t per_expert, uint32_t tile, uint32_t (&warp_max)[kWarps])
+{
+    constexpr int kElems = 32 / sizeof(T);
+    const int64_t vecs = per_expert / kElems;
+    float m = 0.0f;
+#pragma unroll 1
+    for (int step = 0; step < kAmaxSteps; ++step) {
+        const int64_t first = (static_cast<int64_t>(tile) * kAmaxSteps + step) * (kThreads * kAmaxUnroll) + threadIdx.x;
+        Vec v[kAmaxUnroll];
+#pragma unroll
+        for (int u = 0; u < kAmaxUnroll; ++u)
+            v[u] = first + u * kThreads < vecs ? load32<T, kAligned, false>(expert + (first + u * kThreads) * kElems) : Vec{};
+#pragma unroll
+        for (int u = 0; u < kAmaxUnroll; ++u) m = amax_of<T>(m, v[u]);
+    }
+    uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));  // non-negative floats order as integers
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = bits;
+    __syncthreads();
+    return threadIdx.x < 32 ? __reduce_max_sync(0xffffffffu, threadIdx.x < kWarps ? warp_max[threadIdx.x] : 0u) : 0u;
+}
+
+// Two FP32 operations per instruction: b * c and a * b + c on pairs, each half rounded on its own.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 r;
+    asm("{\n .reg .b64 x, y, z, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 w, x, y, z;\n"
+        " mov.b64 {%0, %1}, w;\n}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+
+// Quotients are rounded to FP32 before they are coded (the torch code divides), so they have to be the correctly rounded
+// ones wherever a code depends on it.  With y = 1 / d and an approximate quotient q, the remainder r = x - d * q is exact
+// in one FMA and q + r * y, rounded once, is the next approximation; when y is the rounded reciprocal and q is within one
+// ulp, it is the correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34, 1990).  x * y is within 1.5 ulp, so one step
+// gets q there and a second one finishes.  Nothing underflows as long as d is of ordinary size, which the caller sees
+// to (kOrdinary); the other instantiation divides.  -q is what is computed, so that a zero keeps its sign: q itself would
+// be -0 + 0.
+template <bool kOrdinary>
+__device__ __forceinline__ float divide(float x, float d, float y)
+{
+    if constexpr (!kOrdinary) return __fdiv_rn(x, d);
+    float q = __fmul_rn(x, -y);
+    q = __fmaf_rn(__fmaf_rn(d, q, x), -y, q);
+    return -__fmaf_rn(__fmaf_rn(d, q, x), -y, q);
+}
+
+// E2M1 codes of the 16 quotients x / d.
+//
+// A BF16 numerator needs one step less, and y may be a few ulp^2 off the rounded reciprocal.  The result is then rounded
+// from a value within 2^-47 of x / d, and its code can only be wrong if x / d is that close to a rounding boundary next
+// to a threshold t of the E2M1 grid.  With x = X 2^a (X < 2^8), d = D (2^23 <= D < 2^24) and t = T 2^j
+// (T in {1, 3, 5, 7}) that asks for X 2^a = D (T 2^b +- 1) + eps with |eps| <= 4, a >= 41 and b in {22, 23, 24}; modulo
+// 2^41 the only solution below 2^24 is D = 2^24 - 1 with T = 1 and X a power of two.  For that D the reciprocal
+// (1 + 2^-24 + 2^-48 times a power of two) is rounded up by hand; the remainder step then lands above the boundary.
+template <typename T, bool kOrdinary>
+__device__ __forceinline__ void quantize_block(const float (&x)[16], float d, uint32_t (&packed)[2])
+{
+    float q[16];
+    if constexpr (kOrdinary && !std::is_same_v<T, float>) {
+        const float r = ptx::rcp_approx(d);
+        float y = __fmaf_rn(r, __fmaf_rn(-d, r, 1.0f), r);
+        if ((__float_as_uint(d) & 0x7fffffu) == 0x7fffffu) y = __uint_as_float(__float_as_uint(y) | 1u);
+        const float2 ny = make_float2(-y, -y), dd = make_float2(d, d);
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+            const float2 xx = make_float2(x[i], x[i + 1]), u = mul2(xx, ny);
+            const float2 v = fma2(fma2(dd, u, xx), ny, u);
+            q[i] = v.x;
+            q[i + 1] = v.y;
+        }
+    } else {
+        const float y = kOrdinary ? __frcp_rn(d) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) q[i] = divide<kOrdinary>(x[i], d, y);
+    }
+    packed[0] = ptx::cvt_e2m1x8(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
+    packed[1] = ptx::cvt_e2m1x8(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
+    if constexpr (kOrdinary && !std::is_same_v<T, float>) {              // these are the codes of -x / d
+        packed[0] ^= 0x88888888u;
+        packed[1] ^= 0x88888888u;
+    }
+}
+
+// A warp's share of a quantisation tile: 8 weight rows x 512 K of one expert, a row at a time, a lane one 16-element block of
+// it, so that reads and code stores are contiguous; four neighbouring lanes make one scale word, and the eight rows' words
+// of a K atom are one 32-byte sector of the transposed (K/64, N) array.  The next two rows are on their way while the warp
+// computes on the current two; `v` holds the first two at the start.  kFull: the tile lies inside the matrix, nothing
+// needs a bounds check.
+template <typename T>
+using Rows = Vec[kStep][16 * sizeof(T) / 32];
+template <typename T, bool kAligned, bool kFull>
+__device__ __forceinline__ void request_rows(const T* __restrict__ w, int N, int K, int e, int n0, int k0, Rows<T>& to)
+{
+    constexpr int kElems = 32 / sizeof(T), kVecs = 16 / kElems;          // 32-byte vectors of a block: 1 or 2
+    const int k = k0 + (threadIdx.x & 31) * 16;
+    const T* src = w + (static_cast<int64_t>(e) * N + n0) * K + k;
+#pragma unroll
+    for (int r = 0; r < kStep; ++r)
+#pragma unroll
+        for (int c = 0; c < kVecs; ++c)
+            to[r][c] = kFull || (n0 + r < N && k < K) ? load32<T, kAligned, true>(src + static_cast<int64_t>(r) * K + c * kElems) : Vec{};
+}
+
+template <typename T, bool kAligned, bool kFull, bool kOrdinary>
+__device__ __forceinline__ void quantize_unit(const T* __restrict__ w, int N, int K, int e, int n0, int k0, uint8_t* __restrict__ b,
+                                              int32_t* __restrict__ sfb, Rows<T>& first, float g, float rg)
+{
+    constexpr int kVecs = 16 * sizeof(T) / 32;
+    const float tiny = 1.17549435e-38f;
+    const int lane = threadIdx.x & 31, k = k0 + lane * 16;
+    uint8_t* dst = b + (static_cast<int64_t>(e) * N + n0) * (K / 2) + k / 2;
+    Rows<T> second;
+    uint32_t word = 0;                                                   // lane 4 i + j ends up with rows j and j + 4 of K atom i
+    uint32_t word_hi = 0;
+#pragma unroll
+    for (int step = 0; step < kUnitRows / kStep; ++step) {
+        Rows<T>& now = step & 1 ? second : first;
+        if (step + 1 < kUnitRows / kStep) request_rows<T, kAligned, kFull>(w, N, K, e, n0 + (step + 1) * kStep, k0, step & 1 ? first : second);
+#pragma unroll
+        for (int r = 0; r < kStep; ++r) {
+            const int n = step * kStep + r;
+            float m = 0.0f;
+            float x[16];
+#pragma unroll
+            for (int c = 0; c < kVecs; ++c) {
+                const Vec& q = now[r][c];
+                m = amax_of<T>(m, q);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if constexpr (std::is_same_v<T, float>) {
+                        x[8 * c + i] = __uint_as_float(q.w[i]);
+                    } else {
+                        x[2 * i] = __uint_as_float(q.w[i] << 16);
+                        x[2 * i + 1] = __uint_as_float(q.w[i] & 0xffff0000u);
+                    }
+                }
+            }
+            // m / 6 is at least 1/6 of a unit away from every rounding boundary: the product with 1/6 (to 2^-49) decides
+            const float m6 = kOrdinary ? __fmaf_rn(m, 0x1.555556p-3f, __fmul_rn(m, -0x1.555556p-28f)) : __fdiv_rn(m, 6.0f);
+            const uint32_t sc = ptx::cvt_e4m3(fmaxf(divide<kOrdinary>(m6, g, rg), 0.001953125f));
+            uint32_t packed[2];
+            quantize_block<T, kOrdinary>(x, fmaxf(__fmul_rn(e4m3_to_f32(sc), g), tiny), packed);
+            if (kFull || (n0 + n < N && k < K))
+                *reinterpret_cast<uint2*>(dst + static_cast<int64_t>(n) * (K / 2)) = make_uint2(packed[0], packed[1]);
+            uint32_t s4 = sc << (8 * (lane & 3));
+            s4 |= __shfl_xor_sync(0xffffffffu, s4, 1);
+            s4 |= __shfl_xor_sync(0xffffffffu, s4, 2);
+            if ((lane & 3) == (n & 3)) { if (n < 4) word = s4; else word_hi = s4; }
+        }
+    }
+    const int at = k0 / 64 + (lane >> 2), n = n0 + (lane & 3);
+    int32_t* out = sfb + (static_cast<int64_t>(e) * (K / 64) + at) * N + n;
+    if (kFull || (at < K / 64 && n < N)) out[0] = static_cast<int32_t>(word);
+    if (kFull || (at < K / 64 && n + 4 < N)) out[4] = static_cast<int32_t>(word_hi);
+}
+
+// The scratch words of a call, zero at its start: the next tile to draw, and per expert the maximum (FP32 bits) and the
+// number of its maximum tiles that are done, each spread over kSlots words.  (An atomic per warp on one word of either
+// kind was what the kernel waited for: some 7 ns each on one address.)
+constexpr int kSlots = 16;
+struct Scratch {
+    uint32_t* amax_bits;
+    uint32_t* done;
+    uint32_t* ticket;
+};
+constexpr int64_t scratch_words(int64_t experts) { return 2 * kSlots * experts + 1; }
+constexpr long long kDoneBudget = 2000000000ll;      // cycles, about a second; maxima are taken in microseconds
+
+// List position i: stage 0 is the maxima of batch 0; stage s the quantisation of batch s - 1 and the maxima of batch s
+// in proportion; the last stage the quantisation of the last batch.  A stage opens with as many maxima tiles as there are
+// blocks: while they are read, the maxima that its quantisation tiles need, drawn just before them, are finished.
+template <typename T, bool kAligned>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm)
+quantize_weight_kernel(const T* __restrict__ w, int E, int N, int K, int batch, uint32_t qt, uint32_t at, Scratch scratch,
+                       uint8_t* __restrict__ b, int32_t* __restrict__ sfb, float* __restrict__ gw)
+{
+    __shared__ uint32_t warp_max[kWarps];
+    __shared__ uint32_t drawn;
+    const uint32_t kt = static_cast<uint32_t>((K + kUnitK - 1) / kUnitK), lane = threadIdx.x & 31;
+    const uint32_t total = static_cast<uint32_t>(E) * (at + qt);
+    uint32_t next = 0;
+    if (threadIdx.x == 0) next = atomicAdd(scratch.ticket, 1u);
+    int known = -1;                                  // expert whose global scale this thread holds
+    float g = 0.0f, rg = 0.0f;
+    for (;;) {
+        if (threadIdx.x == 0) drawn = next;
+        __syncthreads();
+        uint32_t i = drawn;
+        __syncthreads();
+        if (i >= total) return;
+        if (threadIdx.x == 0) next = atomicAdd(scratch.ticket, 1u);      // arrives while this tile is worked on
+        int first_a = 0;                             // first expert of the stage's maxima
+        uint32_t na = min(batch, E) * at, nq = 0;    // tiles of either kind in the stage
+        while (i >= na + nq) {
+            i -= na + nq;
+            nq = min(batch, E - first_a) * qt;
+            first_a += batch;
+            na = first_a < E ? min(batch, E - first_a) * at : 0u;
+        }
+        const uint32_t lead = min(na, gridDim.x);
+        const uint64_t here = static_cast<uint64_t>(na - lead) + nq, at_mix = i < lead ? 0 : i - lead;
+        const uint32_t q_before = here ? static_cast<uint32_t>(at_mix * nq / here) : 0u;
+        const uint32_t q_after = here && i >= lead ? static_cast<uint32_t>((at_mix + 1) * nq / here) : q_before;
+        if (q_after > q_before) {
+            const int e = first_a - batch + static_cast<int>(q_before / qt);
+            const uint32_t r = q_before % qt;
+            const int n0 = static_cast<int>(r / kt) * kTileRows, k0 = static_cast<int>(r % kt) * kUnitK;
+            const int nw = n0 + static_cast<int>(threadIdx.x >> 5) * kUnitRows;
+            const bool full = n0 + kTileRows <= N && k0 + kUnitK <= K;
+            Rows<T> rows;
+            if (full) request_rows<T, kAligned, true>(w, N, K, e, nw, k0, rows);
+            else request_rows<T, kAligned, false>(w, N, K, e, nw, k0, rows);
+            if (known != e) {
+                const long long t0 = clock64();
+                const uint32_t slot = static_cast<uint32_t>(e) * kSlots + lane % kSlots;
+                uint32_t n = 0;
+                for (;;) {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(scratch.done + slot) : "memory");
+                    n = __reduce_add_sync(0xffffffffu, lane < kSlots ? n : 0u);
+                    // (running out of time does not happen in a healthy run: go on with what there is rather than wait for ever)
+                    if (n >= at || __any_sync(0xffffffffu, clock64() - t0 > kDoneBudget)) break;
+                    __nanosleep(100);
+                }
+                const uint32_t bits = __reduce_max_sync(0xffffffffu, *reinterpret_cast<const volatile uint32_t*>(scratch.amax_bits + slot));
+                g = fmaxf(__fdiv_rn(__uint_as_float(bits), 2688.0f), 1.17549435e-38f);
+                rg = __frcp_rn(g);
+                known = e;
+            }
+            // block scales lie between 2^-9 g and 448 g
+            const bool ordinary = g > 0x1p-60f && g < 0x1p60f;
+            if (full && ordinary) quantize_unit<T, kAligned, true, true>(w, N, K, e, nw, k0, b, sfb, rows, g, rg);
+            else if (ordinary) quantize_unit<T, kAligned, false, true>(w, N, K, e, nw, k0, b, sfb, rows, g, rg);
+            else quantize_unit<T, kAligned, false, false>(w, N, K, e, nw, k0, b, sfb, rows, g, rg);
+            if (r == 0 && threadIdx.x == 0) gw[e] = g;
+        } else {
+            const uint32_t t = i - q_before;
+            const int e = first_a + static_cast<int>(t / at);
+            const int64_t per_expert = static_cast<int64_t>(N) * K;
+            const uint32_t bits = amax_tile<T, kAligned>(w + e * per_expert, per_expert, t % at, warp_max);
+            if (threadIdx.x == 0) {
+                const uint32_t slot = static_cast<uint32_t>(e) * kSlots + t % kSlots;
+                atomicMax(scratch.amax_bits + slot, bits);
+                __threadfence();
+                atomicAdd(scratch.done + slot, 1u);
+            }
+        }
+    }
+}
+
+template <typename T>
+int run_batches(const T* w, int E, int N, int K, void* b, void* sfb, float* gw, const Scratch& scratch, cudaStream_t stream)
+{
+    const int64_t per_expert = static_cast<int64_t>(N) * K;
+    const int64_t fit = kBatchBytes / (per_expert * static_cast<int64_t>(sizeof(T)));
+    const int batch = fit < 1 ? 1 : (fit > E ? E : static_cast<int>(fit));
+    const int64_t per_tile = static_cast<int64_t>(kThreads) * kAmaxUnroll * kAmaxSteps * 32 / static_cast<int64_t>(sizeof(T));
+    const int64_t at = (per_expert + per_tile - 1) / per_tile;
+    const int64_t qt = static_cast<int64_t>((K + kUnitK - 1) / kUnitK) * ((N + kTileRows - 1) / kTileRows);
+    NVFP4_REQUIRE((at + qt) * E <= INT32_MAX, "weights too large for one call (E=%d, N=%d, K=%d)", E, N, K);
+    host::DeviceInfo* dev;
+    if (int rc = host::device_info(-1, &dev)) return rc;
+    const int64_t blocks = static_cast<int64_t>(dev->hw_sms) * kBlocksPerSm, tiles = (at + qt) * E;
+    const bool aligned = (reinterpret_cast<uintptr_t>(w) & 31u) == 0;
+    auto kernel = aligned ? quantize_weight_kernel<T, true> : quantize_weight_kernel<T, false>;
+    return host::launch_kernel(kernel, dim3(static_cast<unsigned>(blocks < tiles ? blocks : tiles)), dim3(kThreads), 0, stream, false, w, E, N, K,
+                               batch, static_cast<uint32_t>(qt), static_cast<uint32_t>(at), scratch, static_cast<uint8_t*>(b),
+                               static_cast<int32_t*>(sfb), gw);
+}
+
+// `words`: scratch_words(E) words the caller provides; they are cleared here, on the call's stream.
+int run_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw, uint32_t* words,
                         cudaStream_t stream)
 {
-    NVFP4_CUDA_CHECK(cudaMemsetAsync(amax_bits, 0, sizeof(uint32_t) * E, stream));
-    const int64_t per_expert = static_cast<int64_t>(N) * K;
-    int blocks = static_cast<int>((per_expert + 256 * 16 - 1) / (256 * 16));
-    blocks = blocks < 1 ? 1 : (blocks > 1024 ? 1024 : blocks);
-    const dim3 qgrid((N + 127) / 128, K / 64, E);
-    if (w_dtype == NVFP4_DTYPE_BF16) {
-        auto* wt = static_cast<const __nv_bfloat16*>(w);
-        expert_amax_kernel<<<dim3(blocks, E), 256, 0, stream>>>(wt, per_expert, amax_bits);
-        quantize_weight_kernel<<<qgrid, 128, 0, stream>>>(wt, N, K, amax_bits, static_cast<uint8_t*>(b),
-                                                          static_cast<int32_t*>(sfb), gw);
-    } else {
-        auto* wt = static_cast<const float*>(w);
-        expert_amax_kernel<<<dim3(blocks, E), 256, 0, stream>>>(wt, per_expert, amax_bits);
-        quantize_weight_kernel<<<qgrid, 128, 0, stream>>>(wt, N, K, amax_bits, static_cast<uint8_t*>(b),
-                                                          static_cast<int32_t*>(sfb), gw);
-    }
-    NVFP4_CUDA_CHECK(cudaGetLastError());
-    return NVFP4_OK;
+    NVFP4_CUDA_CHECK(cudaMemsetAsync(words, 0, sizeof(uint32_t) * scratch_words(E), stream));
+    const int64_t slots = static_cast<int64_t>(kSlots) * E;
+    const Scratch scratch{words, words + slots, words + 2 * slots};
+    return w_dtype == NVFP4_DTYPE_BF16 ? run_batches(static_cast<const __nv_bfloat16*>(w), E, N, K, b, sfb, gw, scratch, stream)
+                                       : run_batches(static_cast<const float*>(w), E, N, K, b, sfb, gw, scratch, stream);
 }
 
 }  // namespace
@@ -121,7 +383,7 @@ int launch_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void
     cudaMemPool_t pool;
     if (int rc = host::workspace_pool(dev, &pool)) return rc;
     uint32_t* amax_bits = nullptr;
-    NVFP4_CUDA_CHECK(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&amax_bits), sizeof(uint32_t) * E, pool, stream));
+    NVFP4_CUDA_CHECK(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&amax_bits), sizeof(uint32_t) * scratch_words(E), pool, stream));
     const int rc = run_quantize_weight(w, w_dtype, E, N, K, b, sfb, gw, amax_bits, stream);
     cudaFreeAsync(amax_bits, stream);
     return rc;
@@ -130,9 +392,9 @@ int launch_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void
 // ---- allocation-free variant ----------------------------------------------------------
 // Same two kernels, but the per-expert maxima are staged in a fixed array that is part of
 // the library image instead of an allocation.  Every process that loads the library holds
-// NVFP4_STATIC_MAX_EXPERTS words of it on every GPU it uses, until it exits.
+// scratch_words(NVFP4_STATIC_MAX_EXPERTS) words of it on every GPU it uses, until it exits.
 namespace {
-static __device__ __align__(256) uint32_t g_static_amax[NVFP4_STATIC_MAX_EXPERTS];
+static __device__ __align__(256) uint32_t g_static_amax[scratch_words(NVFP4_STATIC_MAX_EXPERTS)];
 std::mutex g_static_mutex;
 }  // namespace
 

@@ -1,0 +1,36 @@
+"""Weight quantiser at the edges of its tiles (64 rows x 512 K, 128 KB of maxima) and of its arithmetic (kept-reciprocal
+quotients instead of divisions): byte for byte against the oracle, which divides."""
+import pytest
+import torch
+
+import nvfp4_gemm
+
+pytestmark = pytest.mark.gpu
+
+
+def check(oracle, w, wd):
+    got, want = nvfp4_gemm.quantize_weight_nvfp4(wd), oracle.quantize_weight(w.contiguous())
+    for name, x, y in zip(("b", "sfb", "gw"), got, want):
+        assert torch.equal(x.cpu(), y), name
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape,offset", [((1, 1, 64), 0), ((3, 63, 576), 0), ((2, 65, 448), 1), ((40, 64, 512), 0), ((2, 200, 4160), 3)])
+def test_tile_edges_and_unaligned_views(oracle, dtype, shape, offset):
+    g = torch.Generator().manual_seed(sum(shape) + offset)
+    flat = torch.randn(shape[0] * shape[1] * shape[2] + offset, generator=g) * 0.02
+    flat[::5] *= 0.0                                         # zeros of both signs: the sign bit is part of the code
+    flat = flat.to(dtype)
+    check(oracle, flat[offset:].view(shape), flat.cuda()[offset:].view(shape))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -70, 2.0 ** 70, 2.0 ** -120])
+def test_every_global_scale_mantissa(oracle, dtype, scale):
+    g = torch.Generator().manual_seed(7)
+    w = torch.randint(-128, 128, (128, 16, 128), generator=g).to(torch.float32) * 2.0 ** torch.randint(-12, -7, (128, 16, 1), generator=g)
+    if dtype == torch.float32:
+        w = w * (1 + torch.rand(w.shape, generator=g))
+    w[:, 0, 0] = 1.0 + torch.arange(128) / 128.0             # one expert per BF16 mantissa of the largest magnitude
+    w = (w * scale).to(dtype)
+    check(oracle, w, w.cuda())
