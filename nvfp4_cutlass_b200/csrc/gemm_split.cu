@@ -713,6 +713,12 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
                 }
             }
             ptx::grid_launch_dependents();
+            // neither CTA leaves before the leader's commits of the last ring positions have arrived (nobody else waits
+            // for them, and a barrier must not be signalled in a CTA that no longer exists)
+            for (uint32_t i = 0; i < C::kDepth && ok; ++i) {
+                if (!ptx::mbar_wait_sleep<false>(empty + r.slot, r.phase ^ 1, abort_flag, PAIR_SLEEP_TMA, pa, 0)) give_up(1);
+                r.advance<C::kDepth>();
+            }
         }
     } else if (warp == kWarpMma) {
         // ================= MMA issue (leader only) =================
