@@ -93,8 +93,7 @@ struct Cfg {
     static constexpr uint32_t kOffB = kOffCodes + kDepthP * kSlotCodes;
     static constexpr uint32_t kOffScales = kOffB + kDepthB * kSlotB;
     static constexpr uint32_t kOffSFB = kOffScales + kDepthP * kSlotScales;
-    static constexpr uint32_t kOffStage = kOffSFB + kDepthB * kSlotSFB;
-    static constexpr uint32_t kOffBars = kOffStage + kNumEpiWarps * gemm::kStageWarp;
+    static constexpr uint32_t kOffBars = kOffSFB + kDepthB * kSlotSFB;
     static constexpr uint32_t kNumBars = 2 * kDepthA + 4 * kDepthP + kDepthB + 2;
     // what one CTA sends to one peer per K block: its rows of the packed codes, its block of scale words
     static constexpr uint32_t kShareCodes = kSlotCodes / CL, kShareScales = kSlotScales / CL;
@@ -394,8 +393,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             ptx::tcgen05_fence_after_sync();
             const long long epi0 = ptx::probe_clock();
             const uint32_t taddr = tmem_base + ((quad * 32) << 16) + kColAcc + part * kEpiCols;
-            const uint32_t stage = smem + C::kOffStage + (warp - kWarpEpi0) * gemm::kStageWarp;
-            __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(m_blk * BM + quad * 32 + (lane >> 3)) * p.ldd + n_blk * BN +
+            __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(m_blk * BM + quad * 32 + (lane & 24u)) * p.ldd + n_blk * BN +
                                     part * kEpiCols + (lane & 7u) * 8;
 #pragma unroll
             for (uint32_t hh = 0; hh < kEpiCols / 64; ++hh) {
@@ -418,7 +416,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                     }
                     gemm::scale_pack_bf16(v, g, o + 16);
                 }
-                gemm::store_rows_staged(o, stage, d_lane + hh * 64, p.ldd, lane);
+                gemm::store_rows(o, d_lane + hh * 64, p.ldd, lane);
             }
             acc_phase ^= 1;
         }

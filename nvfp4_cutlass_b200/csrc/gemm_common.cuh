@@ -93,27 +93,35 @@ struct TileWalker {
 // Epilogue stores of one warp: `o` holds this lane's output row as 32 BF16 pairs (64 columns; in tensor memory
 // a lane is a row).  A store instruction should write whole 128-byte lines, and with one row per lane every
 // 16-byte store of the warp would land in a different line -- 4096 partial-line requests per 128 x 256 tile,
-// measured to hold up the operand loads and the tensor pipe of the next tile for thousands of cycles.  So four
-// rows at a time go through a 576-byte staging area (`stage`, this warp's own): four lanes write their 128
-// bytes, then the whole warp reads 16 bytes per lane and stores four full lines.  `d_lane` points at the first
-// of the eight 16-byte pieces this lane stores: row (lane / 8) of the warp's 32, column piece (lane % 8).
-constexpr uint32_t kStageRow = 144, kStageWarp = 4 * kStageRow;   // 128-byte rows padded against bank conflicts
-__device__ __forceinline__ void store_rows_staged(const uint32_t (&o)[32], uint32_t stage, __nv_bfloat16* d_lane, int64_t ldd,
-                                                  uint32_t lane)
+// measured to hold up the operand loads and the tensor pipe of the next tile for thousands of cycles.  So the
+// eight lanes of a group first transpose their 8 x 8 pieces of 16 bytes in registers, three butterfly steps, after
+// which lane j of the group holds piece j of each of the group's eight rows and a store writes four full lines.
+// (Going through shared memory, four rows at a time, was a chain of 24 dependent accesses; under the tensor core's
+// operand reads each takes some 300 cycles, and a tile's stores took 7500 -- longer than the MMAs of a tile of
+// K = 512: 48.5 us against 39.8 for 32 experts, 16k ragged rows, N = 2048, K = 512.  A 32-byte store per lane straight
+// from the row-per-lane layout, which needs d and ldd aligned to 32 bytes: 43.4 us.)
+// `d_lane` points at row (lane & 24), column piece (lane & 7) of the warp's 32 rows x 64 columns.
+__device__ __forceinline__ void store_rows(uint32_t (&o)[32], __nv_bfloat16* d_lane, int64_t ldd, uint32_t lane)
 {
-    const uint32_t rd = stage + (lane >> 3) * kStageRow + (lane & 7u) * 16;
-#pragma unroll 1
-    for (uint32_t pass = 0; pass < 8; ++pass) {
-        if ((lane >> 2) == pass) {
-            const uint32_t wr = stage + (lane & 3u) * kStageRow;
 #pragma unroll
-            for (uint32_t c = 0; c < 8; ++c) ptx::sts128(wr + c * 16, o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+    for (uint32_t s = 1; s < 8; s <<= 1) {
+        const bool up = (lane & s) != 0;
+#pragma unroll
+        for (uint32_t c = 0; c < 8; ++c) {
+            if ((c & s) != 0) continue;
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                uint32_t& lo = o[4 * c + i];
+                uint32_t& hi = o[4 * (c | s) + i];
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, s);
+                if (up) lo = got;
+                else hi = got;
+            }
         }
-        __syncwarp();
-        const uint4 q = ptx::lds128(rd);
-        *reinterpret_cast<uint4*>(d_lane + static_cast<int64_t>(pass * 4) * ldd) = q;
-        __syncwarp();
     }
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c)
+        *reinterpret_cast<uint4*>(d_lane + static_cast<int64_t>(c) * ldd) = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
 }
 
 // 32 FP32 accumulator values x gw -> 16 BF16 pairs

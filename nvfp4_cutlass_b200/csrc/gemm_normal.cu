@@ -56,8 +56,7 @@ struct Cfg {
     static constexpr uint32_t kOffSFA0 = kOffB + kDepthB * kSlotB;
     static constexpr uint32_t kOffSFA1 = kOffSFA0 + kDepthP * kSlotSFA;
     static constexpr uint32_t kOffSFB = kOffSFA1 + kDepthP * kSlotSFA;
-    static constexpr uint32_t kOffStage = kOffSFB + kDepthB * kSlotSFB;     // epilogue staging (gemm::store_rows_staged)
-    static constexpr uint32_t kOffBars = kOffStage + 4 * gemm::kStageWarp;
+    static constexpr uint32_t kOffBars = kOffSFB + kDepthB * kSlotSFB;
     static constexpr uint32_t kNumBars = 2 * 3 + 2 * kDepthP + 3 * kDepthB + 2;
     static constexpr uint32_t kSmemBytes = kOffBars + kNumBars * 8 + 16;
     static constexpr uint32_t kSmemAlloc = kSmemBytes + 1024;            // slack to align the base to 1024 B
@@ -288,8 +287,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             // 64 columns at a time: tensor memory -> registers -> x G_W -> BF16 -> four whole 128-byte lines per store
             // instruction through the warp's staging area; the accumulator goes back to the MMA warp as soon as this
             // warp's last columns are in registers, so the stores of the tail run under the next tile's main loop
-            const uint32_t stage = smem + C::kOffStage + (warp - kWarpEpi0) * gemm::kStageWarp;
-            __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(m_blk * BM + quad * 32 + (lane >> 3)) * p.ldd + n_blk * BN + (lane & 7u) * 8;
+            __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(m_blk * BM + quad * 32 + (lane & 24u)) * p.ldd + n_blk * BN + (lane & 7u) * 8;
 #pragma unroll 1
             for (uint32_t c = 0; c < BN; c += 64) {
                 uint32_t o[32];
@@ -306,7 +304,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
                     gemm::scale_pack_bf16(va, g, o);
                     gemm::scale_pack_bf16(vb, g, o + 16);
                 }
-                gemm::store_rows_staged(o, stage, d_lane + c, p.ldd, lane);
+                gemm::store_rows(o, d_lane + c, p.ldd, lane);
             }
             acc_phase ^= 1;
         }

@@ -139,7 +139,7 @@ struct Cfg {
     // (8 columns per atom: two 128-row groups)
     static constexpr uint32_t kTmemCols = 512, kColAcc = 0, kColSF = 256;
     static constexpr uint32_t kSfA = 0, kSfB = 4 * kAtoms * kPass, kSfCols = kSfB + 8 * kAtoms;
-    static constexpr uint32_t kDepthSmem = (kSmemBudget - 1024 - kNumEpiWarps * 4 * 144) / kStage, kDepthTmem = (kTmemCols - kColSF) / kSfCols;
+    static constexpr uint32_t kDepthSmem = (kSmemBudget - 1024) / kStage, kDepthTmem = (kTmemCols - kColSF) / kSfCols;
     static constexpr uint32_t kDepthRaw = kDepthSmem < kDepthTmem ? kDepthSmem : kDepthTmem;
     static constexpr uint32_t kDepthCap = kDepthRaw > 8 ? 8 : kDepthRaw;
     static constexpr uint32_t kDepth = kDepthCap / kGroup * kGroup;           // whole groups
@@ -149,9 +149,7 @@ struct Cfg {
     static constexpr uint32_t kOffB = kOffA + kDepth * kPass * kSlotA;
     static constexpr uint32_t kOffSFA = kOffB + kDepth * kSlotB;
     static constexpr uint32_t kOffSFB = kOffSFA + kDepth * kSlotSFA;
-    // epilogue staging: per warp four output rows of 64 BF16 (gemm::store_rows_staged)
-    static constexpr uint32_t kOffStage = kOffSFB + kDepth * kSlotSFB;
-    static constexpr uint32_t kOffBars = kOffStage + kNumEpiWarps * gemm::kStageWarp;
+    static constexpr uint32_t kOffBars = kOffSFB + kDepth * kSlotSFB;
     static constexpr uint32_t kNumBars = 4 * kDepth + 2;
     static constexpr uint32_t kSmemAlloc = kOffBars + kNumBars * 8 + 16 + 1024;
     static_assert(kSmemAlloc <= 232448, "shared memory budget");
@@ -430,10 +428,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
             if constexpr (kSwigluOut) {
                 store_swiglu_quantized(o, p, t.row0 + quad * 32 + lane, t.n_blk * (BN / 2) + group * 32);
             } else {
-                const uint32_t stage = smem + C::kOffStage + (warp - kWarpEpi0) * gemm::kStageWarp;
-                __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(t.row0 + quad * 32 + (lane >> 3)) * p.ldd + t.n_blk * BN +
+                __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(t.row0 + quad * 32 + (lane & 24u)) * p.ldd + t.n_blk * BN +
                                         group * 64 + (lane & 7u) * 8;
-                gemm::store_rows_staged(o, stage, d_lane, p.ldd, lane);
+                gemm::store_rows(o, d_lane, p.ldd, lane);
             }
             if (warp == kWarpEpi0) NVFP4_TRACE(8, (tile - blockIdx.x) / gridDim.x);
             acc_phase ^= 1;
@@ -497,8 +494,7 @@ struct PairCfg {
     static_assert(kColSF + kDepth * kSfCols <= kTmemCols, "scale columns");
     static constexpr uint32_t kOffA = 0;                                       // [kDepth][A0, A1, B]
     static constexpr uint32_t kOffSf = kDepth * kStage;                        // [kDepthSf][SFA, SFB]
-    static constexpr uint32_t kOffStage = kOffSf + kDepthSf * kSfStage;
-    static constexpr uint32_t kOffUnits = kOffStage + kNumEpiWarps * gemm::kStageWarp;
+    static constexpr uint32_t kOffUnits = kOffSf + kDepthSf * kSfStage;
     static constexpr uint32_t kOffBars = kOffUnits + kMaxUnitBlocks * 2;
     static constexpr uint32_t kNumBars = 3 * kDepth + 2 * kDepthSf + 2;
     static constexpr uint32_t kSmemAlloc = kOffBars + kNumBars * 8 + 16 + 1024;
@@ -843,10 +839,9 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
             if constexpr (kSwigluOut) {
                 store_swiglu_quantized(o, p, my_row0(t) + quad * 32 + lane, t.n_blk * (BN / 2) + group * 32);
             } else {
-                const uint32_t stage = smem + C::kOffStage + (warp - kWarpEpi0) * gemm::kStageWarp;
-                __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(my_row0(t) + quad * 32 + (lane >> 3)) * p.ldd + t.n_blk * BN +
+                __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(my_row0(t) + quad * 32 + (lane & 24u)) * p.ldd + t.n_blk * BN +
                                         group * 64 + (lane & 7u) * 8;
-                gemm::store_rows_staged(o, stage, d_lane, p.ldd, lane);
+                gemm::store_rows(o, d_lane, p.ldd, lane);
             }
             if (warp == kWarpEpi0) NVFP4_TRACE(8, (tile - pair_id) / num_pairs);
         }
