@@ -9,6 +9,7 @@ any kind: without the compiled library, or without a CUDA tensor, calls raise.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 
@@ -90,7 +91,26 @@ def _check(rc: int) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the handle alone: building a torch.cuda.Stream object around it costs a launch-bound call a microsecond
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+_ALREADY_CURRENT = contextlib.nullcontext()
+
+
+def _on(device):
+    """Context in which `device` (a torch.device or its index) is current; entering and leaving ``torch.cuda.device`` costs
+    about as much as a launch, so nothing is done when it is current already."""
+    index = device if isinstance(device, int) else device.index
+    return _ALREADY_CURRENT if index == torch.cuda.current_device() else torch.cuda.device(index)
+
+
+def _tune_array(tune: dict):
+    """The tune_* arguments as the library takes them, None if they are all zero (tune_swap_ab travels on its own)."""
+    given = {key: int(value) for key, value in tune.items()}
+    if not any(value for key, value in given.items() if key != "tune_swap_ab"):
+        return None
+    return (ctypes.c_int32 * len(TUNE_KEYS))(*[given.get(key, 0) for key in TUNE_KEYS])
 
 
 def _require(cond: bool, what: str) -> None:
@@ -100,7 +120,7 @@ def _require(cond: bool, what: str) -> None:
 
 def _one_device(*tensors) -> torch.device:
     """All tensors are CUDA tensors of ONE device; returns it.  The library launches on the current device and
-    stream, so every wrapper below makes that device current for the call (``with torch.cuda.device(...)``): stream,
+    stream, so every wrapper below makes that device current for the call (``with _on(...)``): stream,
     memory pool, SM count and tensor maps then belong to the GPU that holds the operands."""
     dev = None
     for t in tensors:
@@ -133,15 +153,20 @@ def set_probe_buffer(t=None) -> None:
     """The reference's in-kernel clock probe has no counterpart; accepted and ignored."""
 
 
-def m_grouped_bf16_dual_nvfp4_gemm_contiguous(a, b, sfb, gw, d, m_indices, scale_policy: str = "derived_div8",
-                                              enable_residual_pass: bool = True, *, device_status=None,
-                                              m_alignment: int = 0, **tune) -> None:
-    """d = (A0 + A1) @ W^T * gw per expert group; same contract as the reference entry
-    (src/api.hpp:26-144): dtype / shape assertions first, then a silent return for
-    M == 0 or N == 0, then an asynchronous launch on the current stream."""
-    for key in tune:
-        if key not in TUNE_KEYS:
-            raise TypeError(f"m_grouped_bf16_dual_nvfp4_gemm_contiguous() got an unexpected keyword argument {key!r}")
+def _contiguous_device(a, b, sfb, gw, d, m_indices, device_status) -> int:
+    """Index of the operands' device; raises if they do not fit together.  The first expression is the whole list of
+    conditions for an ordinary call (a launch-bound one spends a third of its time here); whatever fails it goes through
+    the conditions one by one, which accept a little more and name the one that does not hold."""
+    index = a.get_device()
+    if a.dtype == d.dtype == torch.bfloat16 and b.dtype == torch.int8 and sfb.dtype == m_indices.dtype == torch.int32 and \
+            gw.dtype == torch.float32 and a.dim() == d.dim() == b.dim() == sfb.dim() == 2 and m_indices.dim() == 1 and \
+            device_status is None and \
+            index == b.get_device() == sfb.get_device() == gw.get_device() == d.get_device() == m_indices.get_device() >= 0 and \
+            b.is_contiguous() and sfb.is_contiguous() and gw.is_contiguous() and m_indices.is_contiguous() and \
+            a.stride(1) == d.stride(1) == 1 and a.is_cuda:
+        (m, k), (rows, n), e = a.shape, d.shape, gw.numel()
+        if rows == m and m_indices.shape[0] == m and b.shape == (e * n, k // 2) and sfb.shape == (e * (k // 64), n):
+            return index
     _require(a.dtype == torch.bfloat16, "a.dtype == bfloat16")
     _require(d.dtype == torch.bfloat16, "d.dtype == bfloat16")
     _require(b.dtype == torch.int8, "b.dtype == int8")
@@ -164,17 +189,31 @@ def m_grouped_bf16_dual_nvfp4_gemm_contiguous(a, b, sfb, gw, d, m_indices, scale
     _require(a.stride(1) == 1 and d.stride(1) == 1, "a and d are contiguous along their last dimension")
     _require(b.is_contiguous() and sfb.is_contiguous() and gw.is_contiguous() and m_indices.is_contiguous(),
              "b, sfb, gw, m_indices are contiguous")
+    return dev.index
+
+
+def m_grouped_bf16_dual_nvfp4_gemm_contiguous(a, b, sfb, gw, d, m_indices, scale_policy: str = "derived_div8",
+                                              enable_residual_pass: bool = True, *, device_status=None,
+                                              m_alignment: int = 0, **tune) -> None:
+    """d = (A0 + A1) @ W^T * gw per expert group; same contract as the reference entry
+    (src/api.hpp:26-144): dtype / shape assertions first, then a silent return for
+    M == 0 or N == 0, then an asynchronous launch on the current stream."""
+    for key in tune:
+        if key not in TUNE_KEYS:
+            raise TypeError(f"m_grouped_bf16_dual_nvfp4_gemm_contiguous() got an unexpected keyword argument {key!r}")
+    dev = _contiguous_device(a, b, sfb, gw, d, m_indices, device_status)
+    (m, k), n, e = a.shape, d.shape[1], gw.numel()
     if scale_policy not in POLICY_CODES:
         raise RuntimeError("scale_policy must be 'derived_div8', 'derived_div4', 'div4_radix8' or 'residual_amax'")
     swap = int(tune.get("tune_swap_ab", 0)) != 0
-    tune_arr = (ctypes.c_int32 * len(TUNE_KEYS))(*[int(tune.get(key, 0)) for key in TUNE_KEYS])
+    tune_arr = _tune_array(tune)
     lda = a.stride(0) if m > 1 else max(a.stride(0), k)
     ldd = d.stride(0) if m > 1 else max(d.stride(0), n)
-    with torch.cuda.device(dev):
+    with _on(dev):
         _check(lib().nvfp4_grouped_gemm_contiguous(
             a.data_ptr(), lda, b.data_ptr(), sfb.data_ptr(), gw.data_ptr(), d.data_ptr(), ldd,
             m_indices.data_ptr(), m, n, k, e, POLICY_CODES[scale_policy], 1 if enable_residual_pass else 0,
-            1 if swap else 0, int(m_alignment), ctypes.cast(tune_arr, ctypes.c_void_p),
+            1 if swap else 0, int(m_alignment), tune_arr,
             device_status.data_ptr() if device_status is not None else None, _stream()))
 
 
@@ -203,12 +242,12 @@ def m_grouped_bf16_dual_nvfp4_gemm_masked(a, b, sfb, gw, d, masked_m, scale_poli
              "b, sfb, gw, masked_m are contiguous")
     if scale_policy not in POLICY_CODES:
         raise RuntimeError("scale_policy must be 'derived_div8', 'derived_div4', 'div4_radix8' or 'residual_amax'")
-    tune_arr = (ctypes.c_int32 * len(TUNE_KEYS))(*[int(tune.get(key, 0)) for key in TUNE_KEYS])
-    with torch.cuda.device(dev):
+    tune_arr = _tune_array(tune)
+    with _on(dev):
         _check(lib().nvfp4_grouped_gemm_masked(
             a.data_ptr(), a.stride(1), b.data_ptr(), sfb.data_ptr(), gw.data_ptr(), d.data_ptr(), d.stride(1),
             masked_m.data_ptr(), e, max_m, n, k, POLICY_CODES[scale_policy], 1 if enable_residual_pass else 0,
-            1 if fold_swiglu else 0, ctypes.cast(tune_arr, ctypes.c_void_p),
+            1 if fold_swiglu else 0, tune_arr,
             device_status.data_ptr() if device_status is not None else None, _stream()))
 
 
@@ -241,7 +280,7 @@ def load_checkpoint_weights(parts, global_scale_is_divisor: bool = True):
     gw = torch.empty(e, dtype=torch.float32, device=dev)
     ptrs = lambda ts: (ctypes.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
     rows = (ctypes.c_int32 * len(packed))(*[wp.shape[1] for wp in packed])
-    with torch.cuda.device(dev):
+    with _on(dev):
         _check(lib().nvfp4_load_checkpoint_weights(len(packed), ctypes.cast(ptrs(packed), ctypes.c_void_p),
                                                    ctypes.cast(ptrs(scale), ctypes.c_void_p), ctypes.cast(ptrs(glob), ctypes.c_void_p),
                                                    ctypes.cast(rows, ctypes.c_void_p), 1 if global_scale_is_divisor else 0, e, k,
@@ -254,14 +293,14 @@ def read_status(device_status: torch.Tensor) -> int:
     NVFP4_E_DEVICE_TIMEOUT if a bounded in-kernel wait had expired, else returns 0."""
     _require(device_status.is_cuda and device_status.dtype == torch.int32 and device_status.numel() >= 1, "an int32 CUDA tensor")
     value = ctypes.c_int32(0)
-    with torch.cuda.device(device_status.device):
+    with _on(device_status.device):
         _check(lib().nvfp4_read_status(device_status.data_ptr(), ctypes.byref(value), _stream()))
     return value.value
 
 
 def debug_wait_timeout(budget_cycles: int, device_status: torch.Tensor) -> None:
     """Launches the kernel whose bounded wait runs out (test hook of the unwind path)."""
-    with torch.cuda.device(device_status.device):
+    with _on(device_status.device):
         _check(lib().nvfp4_debug_wait_timeout(int(budget_cycles), device_status.data_ptr(), _stream()))
 
 
@@ -276,7 +315,7 @@ def debug_split_workspace(a: torch.Tensor, scale_policy: str = "derived_div8", e
     a0 = torch.zeros(m, k // 2, dtype=torch.uint8, device=a.device)
     a1 = torch.zeros_like(a0)
     sfa = torch.zeros(m // 128, k // 64, passes, 512, dtype=torch.uint8, device=a.device)
-    with torch.cuda.device(a.device):
+    with _on(a.device):
         _check(lib().nvfp4_debug_split_workspace(a.data_ptr(), a.stride(0), m, k, POLICY_CODES[scale_policy],
                                                  1 if enable_residual_pass else 0, 1 if fold_swiglu else 0,
                                                  a0.data_ptr(), a1.data_ptr(), sfa.data_ptr(), _stream()))
@@ -293,7 +332,7 @@ def quantize_weight(w: torch.Tensor):
     b = torch.empty(e * n, k // 2, dtype=torch.int8, device=w.device)
     sfb = torch.empty(e * k // 64, n, dtype=torch.int32, device=w.device)
     gw = torch.empty(e, dtype=torch.float32, device=w.device)
-    with torch.cuda.device(w.device):
+    with _on(w.device):
         _check(lib().nvfp4_quantize_weight(w.data_ptr(), 0 if w.dtype == torch.bfloat16 else 1, e, n, k,
                                            b.data_ptr(), sfb.data_ptr(), gw.data_ptr(), _stream()))
     return b, sfb, gw
@@ -310,7 +349,7 @@ def permute_rows(src: torch.Tensor, n_rows: int, dst: torch.Tensor, src_idx: tor
     for idx in (src_idx, dst_idx):
         _require(idx is None or (idx.is_cuda and idx.dtype == torch.int64 and idx.is_contiguous() and idx.numel() >= n_rows),
                  "indices are contiguous int64 CUDA tensors with at least n_rows entries")
-    with torch.cuda.device(_one_device(src, dst, src_idx, dst_idx)):
+    with _on(_one_device(src, dst, src_idx, dst_idx)):
         _check(lib().nvfp4_permute_rows(src.data_ptr(), src.stride(0) * 2, src_idx.data_ptr() if src_idx is not None else None,
                                         src_div, dst_idx.data_ptr() if dst_idx is not None else None, n_rows, src.shape[1] * 2,
                                         dst.data_ptr(), dst.stride(0) * 2, _stream()))
@@ -321,7 +360,7 @@ def swiglu(h: torch.Tensor) -> torch.Tensor:
     _require(_rows_ok(h) and h.shape[1] % 16 == 0, "h is a 2-D BF16 CUDA tensor whose width is a multiple of 16")
     inter = h.shape[1] // 2
     out = torch.empty(h.shape[0], inter, dtype=torch.bfloat16, device=h.device)
-    with torch.cuda.device(_one_device(h)):
+    with _on(_one_device(h)):
         _check(lib().nvfp4_swiglu(h.data_ptr(), h.stride(0), h.shape[0], inter, out.data_ptr(), out.stride(0), _stream()))
     return out
 
@@ -334,7 +373,7 @@ def combine_rows(rows: torch.Tensor, pos: torch.Tensor, w: torch.Tensor, tokens:
              "pos (int64) and w (float32) are contiguous CUDA tensors of tokens * k entries")
     y = torch.empty(tokens, rows.shape[1], dtype=torch.bfloat16, device=rows.device)
     k = pos.numel() // tokens if tokens else 1
-    with torch.cuda.device(_one_device(rows, pos, w)):
+    with _on(_one_device(rows, pos, w)):
         _check(lib().nvfp4_combine_rows(rows.data_ptr(), rows.stride(0), pos.data_ptr(), w.data_ptr(), tokens, k, rows.shape[1],
                                         y.data_ptr(), y.stride(0), _stream()))
     return y
@@ -355,7 +394,7 @@ def m_grouped_swiglu_dual_nvfp4_gemm_contiguous(h, b, sfb, gw, d, m_indices, ena
              "operand shapes do not fit together")
     _require(b.is_contiguous() and sfb.is_contiguous() and gw.is_contiguous() and m_indices.is_contiguous(),
              "b, sfb, gw and m_indices are contiguous")
-    with torch.cuda.device(_one_device(h, b, sfb, gw, d, m_indices, device_status)):
+    with _on(_one_device(h, b, sfb, gw, d, m_indices, device_status)):
         _check(lib().nvfp4_grouped_gemm_swiglu_contiguous(
             h.data_ptr(), h.stride(0), b.data_ptr(), sfb.data_ptr(), gw.data_ptr(), d.data_ptr(), d.stride(0),
             m_indices.data_ptr(), m, n, k, e, 1 if enable_residual_pass else 0, None,
@@ -366,7 +405,7 @@ def expert_histogram(ids: torch.Tensor, num_experts: int) -> torch.Tensor:
     """counts[e] = number of entries of ids equal to e (int64 CUDA tensors)."""
     _require(_i64_ok(ids, ids.numel()), "ids is a contiguous int64 CUDA tensor")
     counts = torch.empty(num_experts, dtype=torch.int64, device=ids.device)
-    with torch.cuda.device(_one_device(ids)):
+    with _on(_one_device(ids)):
         _check(lib().nvfp4_expert_histogram(ids.data_ptr(), ids.numel(), num_experts, counts.data_ptr(), _stream()))
     return counts
 
@@ -381,7 +420,7 @@ def plan_peer_masked(all_counts: torch.Tensor, ids: torch.Tensor, world: int, ra
     limit = torch.empty(num_experts, dtype=torch.int64, device=dev)
     masked_m = torch.empty(num_experts // world, dtype=torch.int32, device=dev)
     dst_row = torch.empty(ids.numel(), dtype=torch.int64, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         _check(lib().nvfp4_plan_peer_masked(all_counts.data_ptr(), world, num_experts, rank, cap_m, ids.data_ptr(), ids.numel(),
                                             base.data_ptr(), limit.data_ptr(), masked_m.data_ptr(), dst_row.data_ptr(),
                                             status.data_ptr(), _stream()))
@@ -391,7 +430,7 @@ def plan_peer_masked(all_counts: torch.Tensor, ids: torch.Tensor, world: int, ra
 def peer_barrier(flag_peers: torch.Tensor, rank: int, world: int, slot: int, epoch: int, status: torch.Tensor,
                  budget_cycles: int = 2_000_000_000) -> None:
     """Bounded barrier over the ranks whose flag arrays ``flag_peers`` lists (see the header)."""
-    with torch.cuda.device(_one_device(flag_peers, status)):
+    with _on(_one_device(flag_peers, status)):
         _check(lib().nvfp4_peer_barrier(flag_peers.data_ptr(), rank, world, slot, epoch, budget_cycles, status.data_ptr(), _stream()))
 
 
@@ -403,7 +442,7 @@ def dispatch_rows_peer(src: torch.Tensor, src_idx, src_div: int, peers: torch.Te
     _require(_rows_ok(src), "src is a 2-D BF16 CUDA tensor")
     _require((src_idx is None or _i64_ok(src_idx, n)) and _i64_ok(dst_rank, n) and _i64_ok(dst_row, n) and _i64_ok(peers, 1),
              "indices and peer addresses are contiguous int64 CUDA tensors")
-    with torch.cuda.device(_one_device(src, src_idx, peers, dst_rank, dst_row, status)):
+    with _on(_one_device(src, src_idx, peers, dst_rank, dst_row, status)):
         _check(lib().nvfp4_dispatch_rows_peer(src.data_ptr(), src.stride(0) * 2, src_idx.data_ptr() if src_idx is not None else None,
                                               src_div, peers.data_ptr(), dst_rank.data_ptr(), dst_row.data_ptr(), n, src.shape[1] * 2,
                                               dst_ld_elems * 2, peers.numel(), rows_cap, int(sm_budget),
@@ -434,7 +473,7 @@ def dispatch_quantized_peer(x: torch.Tensor, k_choices: int, peers: torch.Tensor
     _require(_rows_ok(x) and x.shape[1] == rows.k, "x is a (tokens, K) BF16 CUDA tensor")
     _require(_i64_ok(dst_rank, n) and _i64_ok(dst_row, n) and _i64_ok(peers, 1) and n == x.shape[0] * k_choices,
              "indices and peer addresses are contiguous int64 CUDA tensors, one entry per (token, choice)")
-    with torch.cuda.device(_one_device(x, peers, dst_rank, dst_row, status)):
+    with _on(_one_device(x, peers, dst_rank, dst_row, status)):
         _check(lib().nvfp4_dispatch_quantized_peer(x.data_ptr(), x.stride(0), x.shape[0], int(k_choices), rows.k, peers.data_ptr(),
                                                    rows.a1_offset, rows.scale_offset, dst_rank.data_ptr(), dst_row.data_ptr(),
                                                    peers.numel(), rows.e * rows.max_m, int(sm_budget),
@@ -443,7 +482,7 @@ def dispatch_quantized_peer(x: torch.Tensor, k_choices: int, peers: torch.Tensor
 
 def relayout_scales(rows: "QuantizedRows", masked_m: torch.Tensor = None) -> None:
     """rows.scale_rows -> rows.scale_atoms for the live row blocks of every group."""
-    with torch.cuda.device(_one_device(rows.store, rows.scale_atoms, masked_m)):
+    with _on(_one_device(rows.store, rows.scale_atoms, masked_m)):
         _check(lib().nvfp4_relayout_scales(rows.scale_rows.data_ptr(), masked_m.data_ptr() if masked_m is not None else None,
                                            rows.e, rows.max_m, rows.k, rows.scale_atoms.data_ptr(), _stream()))
 
@@ -464,12 +503,12 @@ def m_grouped_quantized_dual_nvfp4_gemm_masked(rows: "QuantizedRows", b, sfb, gw
              "weight shapes do not fit")
     _require(b.is_contiguous() and sfb.is_contiguous() and gw.is_contiguous() and masked_m.is_contiguous(),
              "b, sfb, gw, masked_m are contiguous")
-    tune_arr = (ctypes.c_int32 * len(TUNE_KEYS))(*[int(tune.get(key, 0)) for key in TUNE_KEYS])
-    with torch.cuda.device(_one_device(rows.store, rows.scale_atoms, b, sfb, gw, d, masked_m, device_status)):
+    tune_arr = _tune_array(tune)
+    with _on(_one_device(rows.store, rows.scale_atoms, b, sfb, gw, d, masked_m, device_status)):
         _check(lib().nvfp4_grouped_gemm_masked_quantized(
             rows.a0.data_ptr(), rows.a1.data_ptr(), rows.scale_atoms.data_ptr(), b.data_ptr(), sfb.data_ptr(), gw.data_ptr(),
             d.data_ptr(), d.stride(1), masked_m.data_ptr(), e, max_m, n, k, 1 if enable_residual_pass else 0,
-            ctypes.cast(tune_arr, ctypes.c_void_p), device_status.data_ptr() if device_status is not None else None, _stream()))
+            tune_arr, device_status.data_ptr() if device_status is not None else None, _stream()))
 
 
 def interleave_gate_up(b: torch.Tensor, sfb: torch.Tensor, num_experts: int, inter: int):
@@ -501,12 +540,12 @@ def m_grouped_quantized_swiglu_dual_nvfp4_gemm_masked(rows: "QuantizedRows", b, 
              "weight shapes do not fit")
     _require(b.is_contiguous() and sfb.is_contiguous() and gw.is_contiguous() and masked_m.is_contiguous(),
              "b, sfb, gw, masked_m are contiguous")
-    tune_arr = (ctypes.c_int32 * len(TUNE_KEYS))(*[int(tune.get(key, 0)) for key in TUNE_KEYS])
-    with torch.cuda.device(_one_device(rows.store, rows.scale_atoms, out.store, out.scale_atoms, b, sfb, gw, masked_m, device_status)):
+    tune_arr = _tune_array(tune)
+    with _on(_one_device(rows.store, rows.scale_atoms, out.store, out.scale_atoms, b, sfb, gw, masked_m, device_status)):
         _check(lib().nvfp4_grouped_gemm_masked_quantized_swiglu(
             rows.a0.data_ptr(), rows.a1.data_ptr(), rows.scale_atoms.data_ptr(), b.data_ptr(), sfb.data_ptr(), gw.data_ptr(),
             out.a0.data_ptr(), out.a1.data_ptr(), out.scale_atoms.data_ptr(), masked_m.data_ptr(), e, max_m, n, k,
-            ctypes.cast(tune_arr, ctypes.c_void_p), device_status.data_ptr() if device_status is not None else None, _stream()))
+            tune_arr, device_status.data_ptr() if device_status is not None else None, _stream()))
 
 
 def combine_rows_peer(peers: torch.Tensor, rows_ld_elems: int, src_rank: torch.Tensor, src_row: torch.Tensor, w: torch.Tensor,
@@ -520,7 +559,7 @@ def combine_rows_peer(peers: torch.Tensor, rows_ld_elems: int, src_rank: torch.T
     _require(out is None or (_rows_ok(out) and out.shape == (tokens, hidden)), "out is a (tokens, hidden) BF16 CUDA tensor")
     y = out if out is not None else torch.empty(tokens, hidden, dtype=torch.bfloat16, device=w.device)
     k = n // tokens if tokens else 1
-    with torch.cuda.device(_one_device(peers, src_rank, src_row, w, status)):
+    with _on(_one_device(peers, src_rank, src_row, w, status)):
         _check(lib().nvfp4_combine_rows_peer(peers.data_ptr(), rows_ld_elems, src_rank.data_ptr(), src_row.data_ptr(), w.data_ptr(),
                                              tokens, k, hidden, y.data_ptr(), y.stride(0), peers.numel(), rows_cap, int(sm_budget),
                                              1 if bulk else 0, status.data_ptr() if status is not None else None, _stream()))
@@ -536,7 +575,7 @@ def debug_decompose(a: torch.Tensor, scale_policy: str = "derived_div8"):
     q1 = torch.empty_like(q0)
     s0 = torch.empty(m, k // 16, dtype=torch.uint8, device=a.device)
     s1 = torch.empty_like(s0)
-    with torch.cuda.device(_one_device(a)):
+    with _on(_one_device(a)):
         _check(lib().nvfp4_debug_decompose(a.data_ptr(), a.stride(0), m, k, POLICY_CODES[scale_policy],
                                            q0.data_ptr(), q1.data_ptr(), s0.data_ptr(), s1.data_ptr(), _stream()))
     return q0, q1, s0, s1
