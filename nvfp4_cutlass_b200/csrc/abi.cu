@@ -240,7 +240,7 @@ int nvfp4_grouped_gemm_contiguous(const void* a, int64_t lda_elems, const void* 
     NVFP4_REQUIRE(lda_elems >= K && ldd_elems >= N, "row strides too small (lda=%lld, ldd=%lld)",
                   static_cast<long long>(lda_elems), static_cast<long long>(ldd_elems));
     NVFP4_REQUIRE(lda_elems % 8 == 0 && ldd_elems % 8 == 0, "row strides must be multiples of 8 elements (16 bytes)");
-    NVFP4_REQUIRE((reinterpret_cast<uintptr_t>(d) & 15u) == 0, "d must be 16-byte aligned");
+    NVFP4_REQUIRE(((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(d)) & 15u) == 0, "a and d must be 16-byte aligned");
     NVFP4_REQUIRE(scale_policy >= NVFP4_POLICY_DERIVED_DIV8 && scale_policy <= NVFP4_POLICY_DIV4_RADIX8,
                   "unknown scale policy %d", scale_policy);
 

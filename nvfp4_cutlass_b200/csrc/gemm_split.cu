@@ -41,78 +41,89 @@ constexpr uint32_t kSmemBudget = 232448 - 1024;
 //   a0, a1  (M, K/2) bytes, two E2M1 codes per byte, even element in the low nibble
 //   sfa     (M/128, K/64, passes, 512) bytes: one scale atom per 128 rows x 64 K x pass; inside an atom the
 //           four scale bytes of row r sit at (r % 32) * 16 + (r / 32) * 4 (the tensor-memory image)
-// One thread per 16-element block; the four threads of a 64-K atom row combine their scale bytes into one
-// 32-bit store.
-// ---------------------------------------------------------------------------------------------------
+// A block takes one tile of 128 rows x 128 K: a thread the same 16-element block of rows r, r + 32, r + 64 and r + 96, so
+// that its four loads are in flight together and, after a 4 x 4 transposition of bytes between the four threads of a K
+// atom, the words they store are one 16-byte unit of the atom and a warp's stores 64 contiguous bytes of it.  (One thread per
+// block over the flat index had a 64-bit division per thread, half as long as Algorithm 1 itself, and stored every scale
+// word into a sector of its own.)
+// Bound by instruction issue, then HBM.  32 experts of 1024 reserved rows, 16k of them live, N = 3072, K = 4096: the call 282 us
+// before, 263 now (of which this kernel had 62); 256 experts, 32k zipf rows, N = 4096, K = 7168: 1840 and 1780.
 // With kSwiglu the activation is not read but made: `a` is the (M, 2 K) output of a fused gate+up projection and
 // element (row, j) is bf16(silu(a[row, j]) * a[row, K + j]) -- the same arithmetic and the same BF16 rounding as
 // the stand-alone SwiGLU kernel (moe_glue.cu), so the codes are those of the unfused sequence, bit for bit.
-// Masked layout (masked_m != nullptr): the rows are `m / max_m` groups of max_m rows of which only the first
+// Masked layout (masked_m != nullptr): the rows are groups of max_m rows of which only the first
 // masked_m[g], rounded up to the 128-row tile, are quantised; the others are never read by the GEMM.
+constexpr uint32_t kQuantK = 128, kQuantRows = 4;      // K of a tile; rows of a thread
+
+// 16 BF16.  `wide`: base and row stride are multiples of 32 bytes, and one load brings the sector.
+__device__ __forceinline__ void load_block16(const __nv_bfloat16* p, bool wide, uint32_t (&w)[8])
+{
+    if (wide) {
+        asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p));
+    } else {
+        asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(p));
+        asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p + 8));
+    }
+}
+
+// Byte i of thread t (of four neighbours) -> byte t of thread i.
+__device__ __forceinline__ uint32_t transpose_bytes(uint32_t v, uint32_t t)
+{
+    v = __byte_perm(v, __shfl_xor_sync(0xffffffffu, v, 2), (t & 2u) ? 0x3276u : 0x5410u);
+    return __byte_perm(v, __shfl_xor_sync(0xffffffffu, v, 1), (t & 1u) ? 0x3715u : 0x6240u);
+}
+
 template <bool kResidual, int kPolicy, bool kSwiglu = false>
-__global__ void __launch_bounds__(256)
-quantize_activation_kernel(const __nv_bfloat16* __restrict__ a, int64_t lda, uint32_t m, uint32_t k,
-                           uint8_t* __restrict__ a0, uint8_t* __restrict__ a1, uint8_t* __restrict__ sfa,
-                           const int32_t* __restrict__ masked_m, uint32_t max_m)
+__global__ void __launch_bounds__(256, kSwiglu ? 2 : 3)
+quantize_activation_kernel(const __nv_bfloat16* __restrict__ a, int64_t lda, uint32_t k, bool wide, uint8_t* __restrict__ a0,
+                           uint8_t* __restrict__ a1, uint8_t* __restrict__ sfa, const int32_t* __restrict__ masked_m, uint32_t max_m)
 {
     constexpr uint32_t kPass = kResidual ? 2 : 1;
-    const uint32_t k16 = k / 16;
-    const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const uint64_t total = static_cast<uint64_t>(m) * k16;
+    const uint32_t chunks = k / kQuantK, tile = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
+    const uint32_t row0 = tile * BM, r = threadIdx.x / 8, blk = threadIdx.x % 8;
     // the activations (and the row counts) may be the previous kernel's output
     ptx::grid_dependency_wait();
-    // the grid is padded to whole warps of valid work: m * k16 is a multiple of 128 * 4
-    if (idx >= total) { ptx::grid_launch_dependents(); return; }
-    const uint32_t row = static_cast<uint32_t>(idx / k16), blk16 = static_cast<uint32_t>(idx % k16);
-    if (masked_m != nullptr) {      // whole warps leave together: a 128-row tile is 128 * k16 blocks, a multiple of 32, so
-                                    // the 32 blocks of a warp never straddle a tile boundary
-        const uint32_t rows = min(static_cast<uint32_t>(max(0, __ldg(masked_m + row / max_m))), max_m);
-        if (row % max_m >= (rows + BM - 1) / BM * BM) { ptx::grid_launch_dependents(); return; }
+    if (masked_m != nullptr) {
+        const uint32_t rows = min(static_cast<uint32_t>(max(0, __ldg(masked_m + row0 / max_m))), max_m);
+        if (row0 % max_m >= rows) { ptx::grid_launch_dependents(); return; }
     }
-    const uint4* src = reinterpret_cast<const uint4*>(a + static_cast<int64_t>(row) * lda + blk16 * 16);
-    uint32_t w[8];
-    {
-        uint4 lo, hi;
-        asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w) : "l"(src));
-        asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "l"(src + 1));
-        w[0] = lo.x; w[1] = lo.y; w[2] = lo.z; w[3] = lo.w;
-        w[4] = hi.x; w[5] = hi.y; w[6] = hi.z; w[7] = hi.w;
-    }
-    if constexpr (kSwiglu) {
-        const uint4* up = reinterpret_cast<const uint4*>(a + static_cast<int64_t>(row) * lda + k + blk16 * 16);
-        uint4 lo, hi;
-        asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w) : "l"(up));
-        asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "l"(up + 1));
-        const uint32_t u[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    const uint32_t col = chunk * kQuantK + blk * 16;
+    const __nv_bfloat16* src = a + static_cast<int64_t>(row0 + r) * lda + col;
+    uint32_t w[kQuantRows][8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float2 gf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
-            const float2 uf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[i]));
-            const __nv_bfloat162 p = __floats2bfloat162_rn(gf.x / (1.0f + __expf(-gf.x)) * uf.x, gf.y / (1.0f + __expf(-gf.y)) * uf.y);
-            w[i] = *reinterpret_cast<const uint32_t*>(&p);
-        }
+    for (uint32_t i = 0; i < kQuantRows; ++i) load_block16(src + static_cast<int64_t>(i * 32) * lda, wide, w[i]);
+    if constexpr (kSwiglu) {
+        uint32_t u[kQuantRows][8];
+#pragma unroll
+        for (uint32_t i = 0; i < kQuantRows; ++i) load_block16(src + static_cast<int64_t>(i * 32) * lda + k, wide, u[i]);
+#pragma unroll
+        for (uint32_t i = 0; i < kQuantRows; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float2 gf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i][j]));
+                const float2 uf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[i][j]));
+                const __nv_bfloat162 p = __floats2bfloat162_rn(gf.x / (1.0f + __expf(-gf.x)) * uf.x, gf.y / (1.0f + __expf(-gf.y)) * uf.y);
+                w[i][j] = *reinterpret_cast<const uint32_t*>(&p);
+            }
     }
-    xform::Block16 out;
-    xform::decompose_block16<kResidual, kPolicy>(w, out);
-    const uint64_t code_off = static_cast<uint64_t>(row) * (k / 2) + blk16 * 8;
-    *reinterpret_cast<uint2*>(a0 + code_off) = make_uint2(out.q0[0], out.q0[1]);
-    if constexpr (kResidual) *reinterpret_cast<uint2*>(a1 + code_off) = make_uint2(out.q1[0], out.q1[1]);
-    // scale bytes of the four blocks of a K atom -> one word (the four threads are neighbours in a warp)
-    const uint32_t sh = (threadIdx.x & 3u) * 8u;
-    uint32_t s0 = static_cast<uint32_t>(out.s0) << sh, s1 = static_cast<uint32_t>(out.s1) << sh;
-    s0 |= __shfl_xor_sync(0xffffffffu, s0, 1); s0 |= __shfl_xor_sync(0xffffffffu, s0, 2);
-    if constexpr (kResidual) { s1 |= __shfl_xor_sync(0xffffffffu, s1, 1); s1 |= __shfl_xor_sync(0xffffffffu, s1, 2); }
-    if ((threadIdx.x & 3u) == 0) {
-        const uint32_t r = row % BM;
-        const uint64_t atom = (static_cast<uint64_t>(row / BM) * (k / 64) + blk16 / 4) * kPass;
-        uint8_t* dst = sfa + atom * 512 + (r % 32) * 16 + (r / 32) * 4;
-        *reinterpret_cast<uint32_t*>(dst) = s0;
-        if constexpr (kResidual) *reinterpret_cast<uint32_t*>(dst + 512) = s1;
+    uint64_t code_off = static_cast<uint64_t>(row0 + r) * (k / 2) + col / 2;
+    uint32_t s0 = 0, s1 = 0;                           // scale bytes of the thread's four rows
+#pragma unroll
+    for (uint32_t i = 0; i < kQuantRows; ++i) {
+        xform::Block16 out;
+        xform::decompose_block16<kResidual, kPolicy>(w[i], out);
+        *reinterpret_cast<uint2*>(a0 + code_off) = make_uint2(out.q0[0], out.q0[1]);
+        if constexpr (kResidual) *reinterpret_cast<uint2*>(a1 + code_off) = make_uint2(out.q1[0], out.q1[1]);
+        code_off += static_cast<uint64_t>(32) * (k / 2);
+        s0 |= out.s0 << (8 * i);
+        s1 |= out.s1 << (8 * i);
     }
+    // thread j of an atom ends up with the word of row r + 32 j: bytes = the atom's four blocks
+    const uint64_t atom = (static_cast<uint64_t>(tile) * (k / 64) + col / 64) * kPass;
+    uint8_t* dst = sfa + atom * 512 + r * 16 + (blk & 3u) * 4;
+    *reinterpret_cast<uint32_t*>(dst) = transpose_bytes(s0, blk);
+    if constexpr (kResidual) *reinterpret_cast<uint32_t*>(dst + 512) = transpose_bytes(s1, blk);
     // the GEMM may be scheduled once every block has come this far (its prologue then overlaps our tail; it waits
     // for the completion of this grid before it reads the workspace)
     ptx::grid_launch_dependents();
@@ -884,10 +895,10 @@ int launch_quantize(const Call& c, uint8_t* a0, uint8_t* a1, uint8_t* sfa)
             quantize = quantize_activation_kernel<kResidual, decltype(pol)::value, false>;
             return 0;
         });
-    const uint64_t blocks16 = static_cast<uint64_t>(c.M) * (c.K / 16);
-    return host::launch_kernel(quantize, dim3(static_cast<unsigned>((blocks16 + 255) / 256)), dim3(256), 0, c.stream, c.pdl,
-                               static_cast<const __nv_bfloat16*>(c.a), c.lda, static_cast<uint32_t>(c.M),
-                               static_cast<uint32_t>(c.K), a0, a1, sfa, c.masked_m, static_cast<uint32_t>(c.max_m > 0 ? c.max_m : 1));
+    const bool wide = ((reinterpret_cast<uintptr_t>(c.a) | static_cast<uintptr_t>(c.lda * 2)) & 31u) == 0;
+    return host::launch_kernel(quantize, dim3(static_cast<unsigned>(c.M / static_cast<int>(BM)) * (c.K / kQuantK)), dim3(256), 0, c.stream, c.pdl,
+                               static_cast<const __nv_bfloat16*>(c.a), c.lda, static_cast<uint32_t>(c.K), wide, a0, a1, sfa, c.masked_m,
+                               static_cast<uint32_t>(c.max_m > 0 ? c.max_m : 1));
 }
 
 template <uint32_t BK, bool kResidual, uint32_t kGroup, bool kMasked, bool kPair = false, bool kSwigluOut = false>

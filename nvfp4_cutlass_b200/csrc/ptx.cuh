@@ -358,6 +358,22 @@ NVFP4_DEVICE float fma_f32_f16(unsigned short a, unsigned short b, float c)
     asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"(a), "h"(b), "f"(c));
     return d;
 }
+// Two FP32 operations per instruction: a * b and a * b + c on pairs, each half rounded on its own.
+NVFP4_DEVICE float2 mul_f32x2(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+NVFP4_DEVICE float2 fma_f32x2(float2 a, float2 b, float2 c)
+{
+    float2 r;
+    asm("{\n .reg .b64 x, y, z, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 w, x, y, z;\n"
+        " mov.b64 {%0, %1}, w;\n}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
 // max(|a|, |b|) per BF16 lane; the sign of the result is the xor of the signs.
 NVFP4_DEVICE uint32_t max_abs_bf16x2(uint32_t a, uint32_t b)
 {

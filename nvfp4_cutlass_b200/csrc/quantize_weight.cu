@@ -103,23 +103,6 @@ __device__ __forceinline__ uint32_t amax_tile(const T* __restrict__ expert, int6
     return threadIdx.x < 32 ? __reduce_max_sync(0xffffffffu, threadIdx.x < kWarps ? warp_max[threadIdx.x] : 0u) : 0u;
 }
 
-// Two FP32 operations per instruction: b * c and a * b + c on pairs, each half rounded on its own.
-__device__ __forceinline__ float2 mul2(float2 a, float2 b)
-{
-    float2 r;
-    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
-{
-    float2 r;
-    asm("{\n .reg .b64 x, y, z, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 w, x, y, z;\n"
-        " mov.b64 {%0, %1}, w;\n}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return r;
-}
-
 // Quotients are rounded to FP32 before they are coded (the torch code divides), so they have to be the correctly rounded
 // ones wherever a code depends on it.  With y = 1 / d and an approximate quotient q, the remainder r = x - d * q is exact
 // in one FMA and q + r * y, rounded once, is the next approximation; when y is the rounded reciprocal and q is within one
@@ -155,8 +138,8 @@ __device__ __forceinline__ void quantize_block(const float (&x)[16], float d, ui
         const float2 ny = make_float2(-y, -y), dd = make_float2(d, d);
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
-            const float2 xx = make_float2(x[i], x[i + 1]), u = mul2(xx, ny);
-            const float2 v = fma2(fma2(dd, u, xx), ny, u);
+            const float2 xx = make_float2(x[i], x[i + 1]), u = ptx::mul_f32x2(xx, ny);
+            const float2 v = ptx::fma_f32x2(ptx::fma_f32x2(dd, u, xx), ny, u);
             q[i] = v.x;
             q[i + 1] = v.y;
         }

@@ -123,12 +123,13 @@ NVFP4_DEVICE void decompose_block16(const uint32_t (&w)[8], Block16& out)
     const float r_lo = __fmul_rn(__fmaf_rn(-s0, r_hi, 1.0f), r_hi);
 
     float u[16];
+    const float2 r_hi2 = make_float2(r_hi, r_hi), r_lo2 = make_float2(r_lo, r_lo);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const float x0 = __uint_as_float(w[i] << 16);
-        const float x1 = __uint_as_float(w[i] & 0xffff0000u);
-        u[2 * i] = __fmaf_rn(x0, r_hi, __fmul_rn(x0, r_lo));
-        u[2 * i + 1] = __fmaf_rn(x1, r_hi, __fmul_rn(x1, r_lo));
+        const float2 x = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+        const float2 v = ptx::fma_f32x2(x, r_hi2, ptx::mul_f32x2(x, r_lo2));
+        u[2 * i] = v.x;
+        u[2 * i + 1] = v.y;
     }
     out.q0[0] = ptx::cvt_e2m1x8(u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7]);
     out.q0[1] = ptx::cvt_e2m1x8(u[8], u[9], u[10], u[11], u[12], u[13], u[14], u[15]);
@@ -164,8 +165,9 @@ NVFP4_DEVICE void decompose_block16(const uint32_t (&w)[8], Block16& out)
         for (int i = 0; i < 8; ++i) {
             const uint32_t byte = (out.q0[i >> 2] >> (8 * (i & 3))) & 0xffu;
             const uint32_t d = ptx::cvt_e2m1x2_to_f16x2(byte);
-            r[2 * i] = ptx::fma_f32_f16(static_cast<unsigned short>(d & 0xffffu), kNegRadixF16, __fmul_rn(u[2 * i], kRadix));
-            r[2 * i + 1] = ptx::fma_f32_f16(static_cast<unsigned short>(d >> 16), kNegRadixF16, __fmul_rn(u[2 * i + 1], kRadix));
+            const float2 v = ptx::mul_f32x2(make_float2(u[2 * i], u[2 * i + 1]), make_float2(kRadix, kRadix));
+            r[2 * i] = ptx::fma_f32_f16(static_cast<unsigned short>(d & 0xffffu), kNegRadixF16, v.x);
+            r[2 * i + 1] = ptx::fma_f32_f16(static_cast<unsigned short>(d >> 16), kNegRadixF16, v.y);
         }
         out.q1[0] = ptx::cvt_e2m1x8(r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7]);
         out.q1[1] = ptx::cvt_e2m1x8(r[8], r[9], r[10], r[11], r[12], r[13], r[14], r[15]);
