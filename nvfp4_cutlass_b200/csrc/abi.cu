@@ -560,7 +560,8 @@ int nvfp4_relayout_scales(const void* scale_rows, const int32_t* masked_m, int E
                   "max_m must be a multiple of 128 and K of 64 (E=%d, max_m=%d, K=%d)", E, max_m, K);
     if (E == 0 || max_m == 0) return NVFP4_OK;
     NVFP4_REQUIRE(scale_rows && scale_atoms, "null pointer argument");
-    NVFP4_REQUIRE(((reinterpret_cast<uintptr_t>(scale_rows) | reinterpret_cast<uintptr_t>(scale_atoms)) & 3u) == 0, "scale buffers must be 4-byte aligned");
+    NVFP4_REQUIRE((reinterpret_cast<uintptr_t>(scale_rows) & 3u) == 0 && (reinterpret_cast<uintptr_t>(scale_atoms) & 15u) == 0,
+                  "scale rows must be 4-byte and scale atoms 16-byte aligned");
     return launch_relayout_scales(scale_rows, masked_m, max_m, static_cast<int64_t>(E) * max_m, K, scale_atoms, true,
                                   static_cast<cudaStream_t>(stream));
 }

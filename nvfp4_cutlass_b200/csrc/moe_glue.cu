@@ -141,111 +141,89 @@ dispatch_rows_peer_kernel(const uint4* __restrict__ src, int64_t src_ld16, const
 // the first two are what the split path's GEMM reads through its tensor maps; the scale rows are re-laid into
 // 512-byte tensor-memory atoms by relayout_scales_kernel on the owner (scattering 4-byte words over NVLink instead
 // would cost more than the BF16 rows did).
-// One warp per token.  In step j lane l owns the block pair j * 32 + l (32 elements): its loads are 64-byte pieces of
-// one row, its code stores 16 bytes next to its neighbours' (512 contiguous bytes per warp instruction).  Scale bytes
-// are gathered by shuffles so that every lane stores 8 consecutive bytes per pass.  K % 1024 == 0.
-template <int kRounds>
+// A warp takes 1024 elements of one token (K % 1024 == 0), lane l the 32 elements at 32 l: its loads are 64-byte pieces of
+// one row, its code stores 16 bytes next to its neighbours' (512 contiguous bytes per warp instruction), and the scale bytes
+// are gathered by shuffles so that eight lanes store the 64 of a pass.  Consecutive pieces go to different blocks, so that
+// a few hundred tokens still reach every SM (a warp per token: 256 tokens of K = 4096 ran on eight SMs, 29 us against
+// 5.6; 8192 tokens: 71 us against 69, 370 MB).
 __global__ void __launch_bounds__(kPeerThreads, 1)
-dispatch_quantized_peer_kernel(const uint4* __restrict__ x, int64_t x_ld16, int64_t tokens, int k,
+dispatch_quantized_peer_kernel(const uint4* __restrict__ x, int64_t x_ld16, uint32_t pieces, uint32_t rounds, int k,
                                const int64_t* __restrict__ peers, int64_t a1_off, int64_t sf_off,
                                const int64_t* __restrict__ dst_rank, const int64_t* __restrict__ dst_row, int world,
                                int64_t rows_cap, int32_t* __restrict__ status)
 {
-    constexpr int kMaxRounds = kRounds, rounds = kRounds, kdim = kRounds * 1024;
-    const int lane = threadIdx.x & 31, warps = kPeerThreads / 32;
-    for (int64_t t = static_cast<int64_t>(blockIdx.x) * warps + (threadIdx.x >> 5); t < tokens; t += static_cast<int64_t>(gridDim.x) * warps) {
-        const uint4* row = x + t * x_ld16;
-        uint4 q0[kMaxRounds], q1[kMaxRounds];
-        uint32_t s0[kMaxRounds], s1[kMaxRounds];         // two scale bytes each
+    const uint32_t lane = threadIdx.x & 31, warps = kPeerThreads / 32;
+    const int64_t kdim = static_cast<int64_t>(rounds) * 1024;
+    for (uint32_t piece = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; piece < pieces; piece += gridDim.x * warps) {
+        const uint32_t t = piece / rounds, j = piece % rounds;
+        const uint4* src = x + t * x_ld16 + (j * 32 + lane) * 4;
+        const uint4 v0 = __ldg(src), v1 = __ldg(src + 1), v2 = __ldg(src + 2), v3 = __ldg(src + 3);
+        const uint32_t wa[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        const uint32_t wb[8] = {v2.x, v2.y, v2.z, v2.w, v3.x, v3.y, v3.z, v3.w};
+        xform::Block16 a, b;
+        xform::decompose_block16<true, 0>(wa, a);
+        xform::decompose_block16<true, 0>(wb, b);
+        // scale bytes [8 i, 8 i + 8) of the piece come from lanes 4 i ... 4 i + 3; lanes 0-7 store the first pass, 8-15 the second
+        const uint32_t mine = a.s0 | b.s0 << 8 | a.s1 << 16 | b.s1 << 24, half = lane & 8u ? 0x7632u : 0x5410u;
+        uint32_t g[4];
 #pragma unroll
-        for (int j = 0; j < kMaxRounds; ++j) {
-            if (j >= rounds) break;
-            const uint4* src = row + (j * 32 + lane) * 4;
-            const uint4 v0 = __ldg(src), v1 = __ldg(src + 1), v2 = __ldg(src + 2), v3 = __ldg(src + 3);
-            const uint32_t wa[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-            const uint32_t wb[8] = {v2.x, v2.y, v2.z, v2.w, v3.x, v3.y, v3.z, v3.w};
-            xform::Block16 a, b;
-            xform::decompose_block16<true, 0>(wa, a);
-            xform::decompose_block16<true, 0>(wb, b);
-            q0[j] = make_uint4(a.q0[0], a.q0[1], b.q0[0], b.q0[1]);
-            q1[j] = make_uint4(a.q1[0], a.q1[1], b.q1[0], b.q1[1]);
-            s0[j] = static_cast<uint32_t>(a.s0) | (static_cast<uint32_t>(b.s0) << 8);
-            s1[j] = static_cast<uint32_t>(a.s1) | (static_cast<uint32_t>(b.s1) << 8);
-        }
-        // scale bytes [8 l, 8 l + 8) of the row belong to round l / 8, lanes 4 (l % 8) ... + 3
-        uint32_t s0w[2] = {0, 0}, s1w[2] = {0, 0};
-#pragma unroll
-        for (int j = 0; j < kMaxRounds; ++j) {
-            if (j >= rounds) break;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint32_t g0 = __shfl_sync(0xffffffffu, s0[j], 4 * (lane & 7) + i);
-                const uint32_t g1 = __shfl_sync(0xffffffffu, s1[j], 4 * (lane & 7) + i);
-                if (j == (lane >> 3)) {
-                    s0w[i >> 1] |= g0 << (16 * (i & 1));
-                    s1w[i >> 1] |= g1 << (16 * (i & 1));
-                }
+        for (uint32_t i = 0; i < 4; ++i) g[i] = __shfl_sync(0xffffffffu, mine, 4 * (lane & 7u) + i);
+        const uint2 scales = make_uint2(__byte_perm(g[0], g[1], half), __byte_perm(g[2], g[3], half));
+        const uint4 q0 = make_uint4(a.q0[0], a.q0[1], b.q0[0], b.q0[1]), q1 = make_uint4(a.q1[0], a.q1[1], b.q1[0], b.q1[1]);
+        const int64_t code_off = j * 512 + lane * 16, scale_off = sf_off + (lane & 8u ? kdim / 16 : 0) + j * 64 + (lane & 7u) * 8;
+        for (int c0 = 0; c0 < k; c0 += 32) {             // lane c looks up pair c
+            int64_t base = 0, row = -1;
+            bool valid = false;
+            if (c0 + static_cast<int>(lane) < k) {
+                const int64_t at = static_cast<int64_t>(t) * k + c0 + lane, r = dst_rank[at];
+                row = dst_row[at];
+                valid = r >= 0 && r < world && row >= 0 && row < rows_cap;
+                if (valid) base = peers[r];
+                else if (row != -1 && j == 0 && status != nullptr) atomicOr(status, 8);
             }
-        }
-        for (int c = 0; c < k; ++c) {
-            const int64_t r = dst_rank[t * k + c], dr = dst_row[t * k + c];
-            if (r < 0 || r >= world || dr < 0 || dr >= rows_cap) {
-                if (dr != -1 && lane == 0 && status != nullptr) atomicOr(status, 8);
-                continue;
-            }
-            uint8_t* base = reinterpret_cast<uint8_t*>(peers[r]);
-            uint4* d0 = reinterpret_cast<uint4*>(base + dr * (kdim / 2));
-            uint4* d1 = reinterpret_cast<uint4*>(base + a1_off + dr * (kdim / 2));
-#pragma unroll
-            for (int j = 0; j < kMaxRounds; ++j) {
-                if (j >= rounds) break;
-                d0[j * 32 + lane] = q0[j];
-                d1[j * 32 + lane] = q1[j];
-            }
-            // a row's scale bytes: K / 16 per pass; the lanes of rounds that exist cover them 8 bytes each
-            if (lane < rounds * 8) {
-                uint2* ds = reinterpret_cast<uint2*>(base + sf_off + dr * (kdim / 8));
-                ds[lane] = make_uint2(s0w[0], s0w[1]);
-                ds[kdim / 128 + lane] = make_uint2(s1w[0], s1w[1]);
+            for (unsigned todo = __ballot_sync(0xffffffffu, valid); todo != 0; todo &= todo - 1) {
+                const int c = __ffs(todo) - 1;
+                uint8_t* to = reinterpret_cast<uint8_t*>(__shfl_sync(0xffffffffu, base, c));
+                const int64_t dr = __shfl_sync(0xffffffffu, row, c);
+                *reinterpret_cast<uint4*>(to + dr * (kdim / 2) + code_off) = q0;
+                *reinterpret_cast<uint4*>(to + a1_off + dr * (kdim / 2) + code_off) = q1;
+                if (lane < 16) *reinterpret_cast<uint2*>(to + dr * (kdim / 8) + scale_off) = scales;
             }
         }
     }
 }
 
 // Scale rows (rows, 2, K/16) as the quantised dispatch delivers them -> the (rows/128, K/64, 2, 512) atoms the GEMM's
-// scale warps read (inside an atom the four bytes of row r at (r % 32) * 16 + (r / 32) * 4).  One block per 128-row block,
-// one warp per atom at a time: lane l gathers the words of rows l, l + 32, l + 64, l + 96 (a row's consecutive K atoms are
-// consecutive words, so neighbouring warps share the sectors they read) and the warp writes the atom as 512 contiguous
-// bytes per pass.  Masked layout: groups of max_m rows of which the first masked_m[g], rounded up to the 128-row tile,
-// are converted.  Runs on the owner, on local memory.  (One thread per row and atom, with its two scattered 4-byte stores,
-// took three times as long.)
+// scale warps read (inside an atom the four bytes of row r at (r % 32) * 16 + (r / 32) * 4).  One block per 128 rows x 8 K
+// atoms: a thread brings the 32 bytes of one row and pass, a whole sector, through shared memory the 8 KB of atoms leave as
+// one run.  Masked layout: groups of max_m rows of which the first masked_m[g], rounded up to the 128-row tile, are
+// converted.  Runs on the owner, on local memory.  (A warp per atom, gathering 4-byte words of 128 rows: 24 us for 128 row blocks of K = 4096 where
+// this takes 9, 51 us for some 550 of them where this takes 20.)
+constexpr uint32_t kRelayoutAtoms = 8;
 __global__ void __launch_bounds__(256)
-relayout_scales_kernel(const uint8_t* __restrict__ sf_rows, const int32_t* __restrict__ masked_m, uint32_t max_m, uint64_t rows,
-                       uint32_t kdim, uint8_t* __restrict__ atoms)
+relayout_scales_kernel(const uint8_t* __restrict__ sf_rows, const int32_t* __restrict__ masked_m, uint32_t max_m, uint32_t kdim, bool wide,
+                       uint8_t* __restrict__ atoms)
 {
+    __shared__ __align__(16) uint32_t staged[kRelayoutAtoms][2][128];
+    const uint32_t k64 = kdim / 64, chunks = (k64 + kRelayoutAtoms - 1) / kRelayoutAtoms;
+    const uint32_t first = blockIdx.x % chunks * kRelayoutAtoms, here = min(kRelayoutAtoms, k64 - first);
+    const uint64_t row0 = static_cast<uint64_t>(blockIdx.x / chunks) * 128;
     ptx::grid_dependency_wait();
-    const uint32_t k64 = kdim / 64, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t row0 = static_cast<uint64_t>(blockIdx.x) * 128;
-    bool live = row0 < rows;
-    if (live && masked_m != nullptr) {
-        const uint32_t count = min(static_cast<uint32_t>(max(0, __ldg(masked_m + row0 / max_m))), max_m);
-        live = row0 % max_m < (count + 127) / 128 * 128;
-    }
-    if (live) {
-        const uint8_t* src = sf_rows + (row0 + lane) * (kdim / 8);
-        const uint64_t row_step = static_cast<uint64_t>(32) * (kdim / 8);
-        for (uint32_t katom = warp; katom < k64; katom += 8) {
-            uint32_t w0[4], w1[4];
+    if (masked_m == nullptr || row0 % max_m < min(static_cast<uint32_t>(max(0, __ldg(masked_m + row0 / max_m))), max_m)) {
+        const uint32_t r = threadIdx.x / 2, pass = threadIdx.x % 2, word = (r % 32) * 4 + r / 32;
+        const uint8_t* src = sf_rows + (row0 + r) * (kdim / 8) + pass * (kdim / 16) + first * 4;
+        if (wide) {
+            const uint4 lo = *reinterpret_cast<const uint4*>(src), hi = *reinterpret_cast<const uint4*>(src + 16);
+            const uint32_t v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint8_t* p = src + j * row_step + katom * 4;
-                w0[j] = *reinterpret_cast<const uint32_t*>(p);
-                w1[j] = *reinterpret_cast<const uint32_t*>(p + kdim / 16);
-            }
-            uint4* dst = reinterpret_cast<uint4*>(atoms + ((row0 / 128) * k64 + katom) * 1024) + lane;
-            dst[0] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
-            dst[32] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+            for (uint32_t i = 0; i < kRelayoutAtoms; ++i) staged[i][pass][word] = v[i];
+        } else {
+            for (uint32_t i = 0; i < here; ++i) staged[i][pass][word] = *reinterpret_cast<const uint32_t*>(src + i * 4);
         }
+        __syncthreads();
+        uint4* dst = reinterpret_cast<uint4*>(atoms + ((row0 / 128) * k64 + first) * 1024);
+        const uint4* out = reinterpret_cast<const uint4*>(staged);
+        for (uint32_t i = threadIdx.x; i < here * 64; i += 256) dst[i] = out[i];
     }
     ptx::grid_launch_dependents();
 }
@@ -306,13 +284,18 @@ combine_rows_peer_kernel(const int64_t* __restrict__ peers, int64_t rows_ld16, c
 // instead of per-thread loads: a bulk copy is one request for a whole row, and a CTA can have its entire shared memory
 // in flight, where a thread's loads over NVLink are bounded by what the SM's load path keeps outstanding (sixteen SMs of
 // the kernel above pull ~250 GB/s, all 148 about 600).
-// One CTA per granted SM.  Shared memory is a ring of slots, a slot = the k rows of one token.  Thread 0 walks the CTA's
-// tokens, waits for a slot to be free and requests the rows of every valid pair; the other warps wait for the slot's
-// bytes, form y[t] = sum_j w[t, j] * row_j in FP32 in ascending j (the order of the kernel above and of the all-to-all
-// path: the same bits), store the BF16 row and free the slot.  No multicast; every wait is bounded.
-// Measured (2 GPUs, 16384 tokens x 8 rows of 8 KB per rank): on the whole GPU 0.85 ms against 0.88 ms for the kernel
-// above; on 8 SMs the eight arithmetic warps, not NVLink, set the pace (2.5 ms for half the tokens).
-constexpr int kBulkThreads = 288;                       // warp 0: requests; warps 1-8: arithmetic
+// One CTA per granted SM.  Shared memory is a ring of slots, a slot = the k rows of one token.  Warp 0 walks the CTA's
+// tokens, a lane per pair: it waits for a slot to be free, leaves the weights and the mask of valid pairs beside it and
+// requests the valid rows; the other sixteen warps wait for the slot's bytes, form y[t] = sum_j w[t, j] * row_j in FP32 in
+// ascending j (the order of the kernel above and of the all-to-all path: the same bits), store the BF16 row and free the
+// slot.  No multicast; every wait is bounded.
+// Bound by HBM (NVLink for peers' rows) as long as the arithmetic keeps up: with eight warps, each thread looking up the k
+// pairs of every token itself, 8192 tokens x 8 rows of 8 KB on one GPU took 132 us (4.1 TB/s), now 103 (5.2 TB/s).
+constexpr int kBulkThreads = 544, kBulkPairs = 16;      // warp 0: requests; warps 1-16: arithmetic
+struct BulkSlot {                                       // beside every slot's rows
+    float w[kBulkPairs];
+    uint32_t valid;                                     // bit j: pair j exists and its bytes were requested
+};
 __global__ void __launch_bounds__(kBulkThreads, 1)
 combine_rows_bulk_kernel(const int64_t* __restrict__ peers, int64_t rows_ld_bytes, const int64_t* __restrict__ src_rank,
                          const int64_t* __restrict__ src_row, const float* __restrict__ w, int64_t tokens, int k, int row_bytes,
@@ -324,7 +307,8 @@ combine_rows_bulk_kernel(const int64_t* __restrict__ peers, int64_t rows_ld_byte
     const uint32_t slot_bytes = static_cast<uint32_t>(k) * row_bytes;
     uint64_t* full = reinterpret_cast<uint64_t*>(gen + static_cast<size_t>(slots) * slot_bytes);
     uint64_t* empty = full + slots;
-    volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(empty + slots);
+    BulkSlot* info = reinterpret_cast<BulkSlot*>(empty + slots);
+    volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(info + slots);
     constexpr int kWorkers = kBulkThreads / 32 - 1;
     if (threadIdx.x == 0) {
         for (int i = 0; i < slots; ++i) { ptx::mbar_init(full + i, 1); ptx::mbar_init(empty + i, kWorkers); }
@@ -333,55 +317,68 @@ combine_rows_bulk_kernel(const int64_t* __restrict__ peers, int64_t rows_ld_byte
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    auto valid_pair = [&](int64_t p) {
-        const int64_t pr = src_rank[p], prow = src_row[p];
-        return pr >= 0 && pr < world && prow >= 0 && prow < rows_cap;
-    };
+    uint32_t slot = 0, phase = 0;
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t slot = 0, phase = 0;
-            for (int64_t t = blockIdx.x; t < tokens; t += gridDim.x) {
-                if (!ptx::mbar_wait_impl(empty + slot, phase ^ 1, abort_flag)) {
-                    *abort_flag = 1;
-                    if (status != nullptr) atomicOr(status, 1);
-                    break;
-                }
-                uint32_t bytes = 0;
-                for (int j = 0; j < k; ++j) bytes += valid_pair(t * k + j) ? row_bytes : 0;
-                ptx::mbar_arrive_expect_tx(full + slot, bytes);
-                for (int j = 0; j < k; ++j) {
-                    const int64_t p = t * k + j;
-                    if (!valid_pair(p)) continue;
-                    const uint8_t* row = reinterpret_cast<const uint8_t*>(peers[src_rank[p]]) + src_row[p] * rows_ld_bytes;
-                    ptx::bulk_load(gen + static_cast<size_t>(slot) * slot_bytes + static_cast<size_t>(j) * row_bytes, row, row_bytes, full + slot);
-                }
-                if (++slot == static_cast<uint32_t>(slots)) { slot = 0; phase ^= 1; }
+        // the pair of this lane in the CTA's next token, looked up one token ahead
+        int64_t row = 0, base = 0;
+        float weight = 0.0f;
+        bool valid = false;
+        auto look_up = [&](int64_t t) {
+            valid = false;
+            if (t >= tokens || lane >= k) return;
+            const int64_t rank = src_rank[t * k + lane];
+            row = src_row[t * k + lane];
+            weight = w[t * k + lane];
+            valid = rank >= 0 && rank < world && row >= 0 && row < rows_cap;
+            if (valid) base = peers[rank];
+        };
+        look_up(blockIdx.x);
+        for (int64_t t = blockIdx.x; t < tokens; t += gridDim.x) {
+            const bool free_again = ptx::mbar_wait_impl(empty + slot, phase ^ 1, abort_flag);
+            if (!__all_sync(0xffffffffu, free_again)) {
+                *abort_flag = 1;
+                if (lane == 0 && status != nullptr) atomicOr(status, 1);
+                break;
             }
+            const unsigned mask = __ballot_sync(0xffffffffu, valid);
+            if (lane < k) info[slot].w[lane] = weight;
+            if (lane == 0) info[slot].valid = mask;
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive_expect_tx(full + slot, __popc(mask) * row_bytes);
+            __syncwarp();
+            if (valid)
+                ptx::bulk_load(gen + static_cast<size_t>(slot) * slot_bytes + static_cast<size_t>(lane) * row_bytes,
+                               reinterpret_cast<const uint8_t*>(base) + row * rows_ld_bytes, row_bytes, full + slot);
+            look_up(t + gridDim.x);
+            if (++slot == static_cast<uint32_t>(slots)) { slot = 0; phase ^= 1; }
         }
     } else {
-        uint32_t slot = 0, phase = 0;
         const int worker = threadIdx.x - 32, row16 = row_bytes / 16;
         for (int64_t t = blockIdx.x; t < tokens; t += gridDim.x) {
-            float wj[16];
-            bool live[16];
-            for (int j = 0; j < k; ++j) { live[j] = valid_pair(t * k + j); wj[j] = live[j] ? w[t * k + j] : 0.0f; }
             if (!ptx::mbar_wait_impl(full + slot, phase, abort_flag)) {
                 *abort_flag = 1;
                 if (status != nullptr) atomicOr(status, 1);
                 break;
             }
-            const uint32_t base = smem + slot * slot_bytes;
+            const uint32_t base = smem + slot * slot_bytes, valid = info[slot].valid;
             for (int c = worker; c < row16; c += kWorkers * 32) {
                 float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                for (int j = 0; j < k; ++j) {
-                    if (!live[j]) continue;                     // contributes nothing (its bytes were never requested)
-                    const uint4 v = ptx::lds128(base + j * row_bytes + c * 16);
-                    const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+                for (int j0 = 0; j0 < k; j0 += 8) {
+                    uint4 v[8];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&vw[i]));
-                        acc[2 * i] = fmaf(wj[j], f.x, acc[2 * i]);
-                        acc[2 * i + 1] = fmaf(wj[j], f.y, acc[2 * i + 1]);
+                    for (int u = 0; u < 8; ++u)                  // a pair that is not valid contributes nothing
+                        if (valid >> (j0 + u) & 1u) v[u] = ptx::lds128(base + (j0 + u) * row_bytes + c * 16);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        if (!(valid >> (j0 + u) & 1u)) continue;
+                        const float wj = info[slot].w[j0 + u];
+                        const uint32_t vw[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&vw[i]));
+                            acc[2 * i] = fmaf(wj, f.x, acc[2 * i]);
+                            acc[2 * i + 1] = fmaf(wj, f.y, acc[2 * i + 1]);
+                        }
                     }
                 }
                 uint32_t ow[4];
@@ -636,10 +633,10 @@ int launch_combine_rows_peer(const int64_t* peers, int64_t rows_ld_elems, const 
     // bulk copies: a slot holds the k rows of a token; at least two slots must fit beside the barriers
     const size_t slot_bytes = static_cast<size_t>(k) * hidden * 2;
     constexpr size_t kSmemMax = 232448 - 1024;
-    const int slots = slot_bytes ? static_cast<int>((kSmemMax - 256) / slot_bytes) : 0;
-    if (bulk && slots >= 2 && k <= 16 && (hidden * 2) % 16 == 0) {
+    const int slots = slot_bytes ? static_cast<int>((kSmemMax - 1024) / slot_bytes) : 0;
+    if (bulk && slots >= 2 && k <= kBulkPairs && (hidden * 2) % 16 == 0) {
         const int use = slots > 8 ? 8 : slots;
-        const size_t smem = use * slot_bytes + 2 * use * 8 + 16 + 128;
+        const size_t smem = use * (slot_bytes + 2 * sizeof(uint64_t) + sizeof(BulkSlot)) + 16 + 128;
         static bool attr_set[host::kMaxDevices] = {};
         int dev = 0;
         NVFP4_CUDA_CHECK(cudaGetDevice(&dev));
@@ -664,21 +661,13 @@ int launch_dispatch_quantized_peer(const void* x, int64_t x_ld_bytes, int64_t to
                                    int64_t a1_off, int64_t sf_off, const int64_t* dst_rank, const int64_t* dst_row, int world,
                                    int64_t rows_cap, int32_t* status, int num_sms, cudaStream_t stream)
 {
-    auto go = [&](auto kernel) {
-        kernel<<<static_cast<unsigned>(num_sms), kPeerThreads, 0, stream>>>(static_cast<const uint4*>(x), x_ld_bytes / 16, tokens, k, peers,
-                                                                           a1_off, sf_off, dst_rank, dst_row, world, rows_cap, status);
-    };
-    switch (kdim / 1024) {
-        case 1: go(dispatch_quantized_peer_kernel<1>); break;
-        case 2: go(dispatch_quantized_peer_kernel<2>); break;
-        case 3: go(dispatch_quantized_peer_kernel<3>); break;
-        case 4: go(dispatch_quantized_peer_kernel<4>); break;
-        case 5: go(dispatch_quantized_peer_kernel<5>); break;
-        case 6: go(dispatch_quantized_peer_kernel<6>); break;
-        case 7: go(dispatch_quantized_peer_kernel<7>); break;
-        case 8: go(dispatch_quantized_peer_kernel<8>); break;
-        default: return host::fail(NVFP4_E_UNSUPPORTED, "quantised dispatch is built for K = 1024 ... 8192 in steps of 1024 (K=%d)", kdim);
-    }
+    if (kdim % 1024 != 0 || kdim < 1024 || kdim > 8192)
+        return host::fail(NVFP4_E_UNSUPPORTED, "quantised dispatch is built for K = 1024 ... 8192 in steps of 1024 (K=%d)", kdim);
+    const int64_t pieces = tokens * (kdim / 1024);
+    NVFP4_REQUIRE(pieces <= INT32_MAX, "too many tokens (%lld)", static_cast<long long>(tokens));
+    dispatch_quantized_peer_kernel<<<static_cast<unsigned>(num_sms), kPeerThreads, 0, stream>>>(
+        static_cast<const uint4*>(x), x_ld_bytes / 16, static_cast<uint32_t>(pieces), static_cast<uint32_t>(kdim / 1024), k, peers, a1_off, sf_off,
+        dst_rank, dst_row, world, rows_cap, status);
     NVFP4_CUDA_CHECK(cudaGetLastError());
     return NVFP4_OK;
 }
@@ -687,9 +676,12 @@ int launch_relayout_scales(const void* sf_rows, const int32_t* masked_m, int max
                            cudaStream_t stream)
 {
     if (rows == 0) return NVFP4_OK;
-    return host::launch_kernel(relayout_scales_kernel, dim3(static_cast<unsigned>((rows + 127) / 128)), dim3(256), 0, stream, pdl,
+    // whole chunks of atoms, every row piece on a 16-byte boundary
+    const bool wide = kdim % 512 == 0 && (reinterpret_cast<uintptr_t>(sf_rows) & 15u) == 0;
+    const int64_t blocks = rows / 128 * ((kdim / 64 + kRelayoutAtoms - 1) / kRelayoutAtoms);
+    return host::launch_kernel(relayout_scales_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, pdl,
                                static_cast<const uint8_t*>(sf_rows), masked_m, static_cast<uint32_t>(max_m > 0 ? max_m : 1),
-                               static_cast<uint64_t>(rows), static_cast<uint32_t>(kdim), static_cast<uint8_t*>(atoms));
+                               static_cast<uint32_t>(kdim), wide, static_cast<uint8_t*>(atoms));
 }
 
 }  // namespace nvfp4
