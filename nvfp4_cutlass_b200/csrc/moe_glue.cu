@@ -197,8 +197,8 @@ dispatch_quantized_peer_kernel(const uint4* __restrict__ x, int64_t x_ld16, uint
 // scale warps read (inside an atom the four bytes of row r at (r % 32) * 16 + (r / 32) * 4).  One block per 128 rows x 8 K
 // atoms: a thread brings the 32 bytes of one row and pass, a whole sector, through shared memory the 8 KB of atoms leave as
 // one run.  Masked layout: groups of max_m rows of which the first masked_m[g], rounded up to the 128-row tile, are
-// converted.  Runs on the owner, on local memory.  (A warp per atom, gathering 4-byte words of 128 rows: 24 us for 128 row blocks of K = 4096 where
-// this takes 9, 51 us for some 550 of them where this takes 20.)
+// converted.  Runs on the owner, on local memory.  (A warp per atom, gathering 4-byte
+// words of 128 rows: 24 us for 128 row blocks of K = 4096 where this takes 9, 51 us for some 550 of them where this takes 20.)
 constexpr uint32_t kRelayoutAtoms = 8;
 __global__ void __launch_bounds__(256)
 relayout_scales_kernel(const uint8_t* __restrict__ sf_rows, const int32_t* __restrict__ masked_m, uint32_t max_m, uint32_t kdim, bool wide,
@@ -396,8 +396,9 @@ combine_rows_bulk_kernel(const int64_t* __restrict__ peers, int64_t rows_ld_byte
     }
 }
 
-// counts[e] += number of ids equal to e (counts zeroed by the caller); per-block histogram in shared memory first, so
-// that the global atomics are one per expert and block instead of one per pair on a handful of addresses
+// counts[e] += number of ids equal to e (counts zeroed by the caller; a grid of one block stores them instead);
+// per-block histogram in shared memory first, so that the global atomics are one per expert and block instead of one per
+// pair on a handful of addresses
 __global__ void __launch_bounds__(1024)
 expert_histogram_kernel(const int64_t* __restrict__ ids, int64_t n, int num_experts, unsigned long long* __restrict__ counts)
 {
@@ -409,8 +410,10 @@ expert_histogram_kernel(const int64_t* __restrict__ ids, int64_t n, int num_expe
         if (e >= 0 && e < num_experts) atomicAdd(&hist[e], 1u);
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < num_experts; e += blockDim.x)
-        if (hist[e] != 0) atomicAdd(&counts[e], static_cast<unsigned long long>(hist[e]));
+    for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
+        if (gridDim.x == 1) counts[e] = hist[e];
+        else if (hist[e] != 0) atomicAdd(&counts[e], static_cast<unsigned long long>(hist[e]));
+    }
 }
 
 // Routing plan of the peer-memory path, from the gathered (source rank, expert) count matrix (plan_offsets_masked_kernel
@@ -418,10 +421,10 @@ expert_histogram_kernel(const int64_t* __restrict__ ids, int64_t n, int num_expe
 // -- a stable counting sort without the sort: pairs keep their order inside an expert's group.  With `limit`
 // (fixed-capacity plan) a pair whose row would reach limit[e] does not fit and gets row -1.
 // Two passes over the pairs, each block on its own chunk: plan_chunk_hist_kernel counts every chunk's pairs per expert;
-// plan_rows_kernel starts each expert's counter at base[e] + (pairs of e in earlier chunks) and hands out rows chunk-locally:
-// 1024 pairs at a time, the warps take turns in order (inside a warp __match_any_sync ranks the lanes of one expert), so
-// the order of the pairs is kept.  (The first version gave every expert a block that scanned ALL pairs: 128 experts x
-// 131072 pairs took 0.2 ms.)
+// plan_rows_kernel starts each expert's counter at base[e] + (pairs of e in earlier chunks) and hands out rows chunk-locally.
+// Up to kPlanOnePass pairs one block does all of it, offsets included (plan_small_kernel): the three launches were 14 us of a
+// layer of 256 tokens, this one under 8.  (The first version gave every expert a block that scanned ALL pairs: 128
+// experts x 131072 pairs took 0.2 ms.)
 constexpr int kPlanThreads = 1024;
 __global__ void __launch_bounds__(kPlanThreads)
 plan_chunk_hist_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t chunk, int num_experts, int32_t* __restrict__ chunk_hist)
@@ -438,20 +441,21 @@ plan_chunk_hist_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t chunk
     for (int e = threadIdx.x; e < num_experts; e += blockDim.x) chunk_hist[static_cast<int64_t>(blockIdx.x) * num_experts + e] = hist_s[e];
 }
 
-__global__ void __launch_bounds__(kPlanThreads)
-plan_rows_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t chunk, int num_experts, const int32_t* __restrict__ chunk_hist,
-                 const int64_t* __restrict__ base, const int64_t* __restrict__ limit, int64_t* __restrict__ dst_row)
+constexpr int64_t kPlanOnePass = 8192;               // eight rounds of 1024: about where a second pass over chunks is cheaper
+
+// Rows for pairs [lo, hi) in their order, 1024 at a time, from the counters next_row[e] (shared memory): inside a warp
+// __match_any_sync ranks the lanes of one expert, `before` ([32 warps][num_experts], shared memory) gives what lower warps
+// of the round take.  With more than kPlanTable experts there is no room for that table and the warps take turns instead
+// (32 block barriers a round in place of four).
+constexpr int kPlanTable = 512;
+__device__ __forceinline__ void hand_out_rows(const int64_t* __restrict__ ids, int64_t lo, int64_t hi, int num_experts, long long* next_row,
+                                              unsigned short* before, const int64_t* limit, int64_t* __restrict__ dst_row)
 {
-    extern __shared__ long long next_row[];          // [num_experts] next free row of every expert, for this chunk onwards
-    for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
-        long long r = base[e];
-        for (int c = 0; c < static_cast<int>(blockIdx.x); ++c) r += chunk_hist[static_cast<int64_t>(c) * num_experts + e];
-        next_row[e] = r;
-    }
-    __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int64_t lo = blockIdx.x * chunk, hi = min(lo + chunk, n);
-    for (int64_t p0 = lo; p0 < hi; p0 += blockDim.x) {
+    const bool table = num_experts <= kPlanTable;
+    if (table) for (int i = threadIdx.x; i < 32 * num_experts; i += kPlanThreads) before[i] = 0;
+    __syncthreads();
+    for (int64_t p0 = lo; p0 < hi; p0 += kPlanThreads) {
         const int64_t p = p0 + threadIdx.x;
         const int64_t e = p < hi ? ids[p] : -1;
         const bool valid = e >= 0 && e < num_experts;
@@ -459,6 +463,30 @@ plan_rows_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t chunk, int 
         const unsigned same = __match_any_sync(0xffffffffu, valid ? static_cast<int>(e) : -1 - lane);
         const int rank_in_warp = __popc(same & ((1u << lane) - 1u));
         const int leader = __ffs(same) - 1;
+        if (table) {
+            if (valid && lane == leader) before[wid * num_experts + e] = static_cast<unsigned short>(__popc(same));
+            __syncthreads();
+            int taken = 0;                           // rows of expert threadIdx.x handed out in this round
+            if (static_cast<int>(threadIdx.x) < num_experts)
+                for (int w = 0; w < 32; ++w) {
+                    unsigned short& b = before[w * num_experts + threadIdx.x];
+                    const int c = b;
+                    b = static_cast<unsigned short>(taken);
+                    taken += c;
+                }
+            __syncthreads();
+            if (valid) {
+                const long long row = next_row[e] + before[wid * num_experts + e] + rank_in_warp;
+                dst_row[p] = (limit == nullptr || row < limit[e]) ? row : -1;
+            }
+            __syncthreads();
+            if (static_cast<int>(threadIdx.x) < num_experts) {
+                next_row[threadIdx.x] += taken;
+                for (int w = 0; w < 32; ++w) before[w * num_experts + threadIdx.x] = 0;
+            }
+            __syncthreads();
+            continue;
+        }
         for (int w = 0; w < kPlanThreads / 32; ++w) {
             if (w == wid) {
                 long long first = 0;
@@ -476,16 +504,33 @@ plan_rows_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t chunk, int 
         }
     }
 }
+size_t plan_smem(int num_experts)
+{
+    return num_experts * (sizeof(long long) + (num_experts <= kPlanTable ? 32 * sizeof(unsigned short) : 0));
+}
+
+__global__ void __launch_bounds__(kPlanThreads)
+plan_rows_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t chunk, int num_experts, const int32_t* __restrict__ chunk_hist,
+                 const int64_t* __restrict__ base, const int64_t* __restrict__ limit, int64_t* __restrict__ dst_row)
+{
+    extern __shared__ long long next_row[];          // [num_experts] next free row of every expert, for this chunk onwards
+    for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
+        long long r = base[e];
+        for (int c = 0; c < static_cast<int>(blockIdx.x); ++c) r += chunk_hist[static_cast<int64_t>(c) * num_experts + e];
+        next_row[e] = r;
+    }
+    const int64_t lo = blockIdx.x * chunk;
+    hand_out_rows(ids, lo, min(lo + chunk, n), num_experts, next_row, reinterpret_cast<unsigned short*>(next_row + num_experts), limit, dst_row);
+}
 
 // Fixed-capacity plan: every local expert owns `cap_m` rows of its rank's buffer (the masked layout of the GEMM),
 // so a pair's row depends only on the gathered counts, never on a host-side prefix sum of padded group sizes.
 //   base[e]  = (e % e_local) * cap_m + rows of e from lower ranks      limit[e] = (e % e_local + 1) * cap_m
 //   masked_m[j] = min(rows of local expert j, cap_m)                   status |= 4 if some expert anywhere overflows
 // Every rank sees the same gathered counts, hence the same overflow verdict.
-__global__ void __launch_bounds__(1024)
-plan_offsets_masked_kernel(const int64_t* __restrict__ all_counts, int world, int num_experts, int rank, int cap_m,
-                           int64_t* __restrict__ base, int64_t* __restrict__ limit, int32_t* __restrict__ masked_m,
-                           int32_t* __restrict__ status)
+__device__ __forceinline__ void plan_offsets(const int64_t* __restrict__ all_counts, int world, int num_experts, int rank, int cap_m,
+                                             int64_t* base, int64_t* limit, int32_t* __restrict__ masked_m,
+                                             int32_t* __restrict__ status, long long* next_row)
 {
     const int e_local = num_experts / world;
     for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
@@ -498,9 +543,28 @@ plan_offsets_masked_kernel(const int64_t* __restrict__ all_counts, int world, in
         const int64_t group = static_cast<int64_t>(e % e_local) * cap_m;
         base[e] = group + before;
         limit[e] = group + cap_m;
+        if (next_row != nullptr) next_row[e] = group + before;
         if (e / e_local == rank) masked_m[e % e_local] = static_cast<int32_t>(total < cap_m ? total : cap_m);
         if (total > cap_m && status != nullptr) atomicOr(status, 4);
     }
+}
+__global__ void __launch_bounds__(1024)
+plan_offsets_masked_kernel(const int64_t* __restrict__ all_counts, int world, int num_experts, int rank, int cap_m,
+                           int64_t* __restrict__ base, int64_t* __restrict__ limit, int32_t* __restrict__ masked_m,
+                           int32_t* __restrict__ status)
+{
+    plan_offsets(all_counts, world, num_experts, rank, cap_m, base, limit, masked_m, status, nullptr);
+}
+// `limit` is written and read here: no __restrict__ on what hand_out_rows reads back
+__global__ void __launch_bounds__(kPlanThreads)
+plan_small_kernel(const int64_t* __restrict__ all_counts, int world, int num_experts, int rank, int cap_m, const int64_t* __restrict__ ids,
+                  int64_t n, int64_t* base, int64_t* limit, int32_t* __restrict__ masked_m, int64_t* __restrict__ dst_row,
+                  int32_t* __restrict__ status)
+{
+    extern __shared__ long long next_row[];
+    plan_offsets(all_counts, world, num_experts, rank, cap_m, base, limit, masked_m, status, next_row);
+    __syncthreads();
+    hand_out_rows(ids, 0, n, num_experts, next_row, reinterpret_cast<unsigned short*>(next_row + num_experts), limit, dst_row);
 }
 
 // Barrier over the GPUs of one NVLink domain with a bounded wait.  `flag_peers[r]` is the address, in this process,
@@ -571,9 +635,9 @@ int launch_combine_rows(const void* rows, int64_t rows_ld_elems, const int64_t* 
 
 int launch_expert_histogram(const int64_t* ids, int64_t n, int num_experts, int64_t* counts, cudaStream_t stream)
 {
-    NVFP4_CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(int64_t) * num_experts, stream));
-    if (n == 0) return NVFP4_OK;
     const unsigned blocks = static_cast<unsigned>((n + 8191) / 8192 < 64 ? (n + 8191) / 8192 : 64);
+    if (blocks != 1) NVFP4_CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(int64_t) * num_experts, stream));
+    if (n == 0) return NVFP4_OK;
     expert_histogram_kernel<<<blocks, 1024, num_experts * sizeof(unsigned int), stream>>>(
         ids, n, num_experts, reinterpret_cast<unsigned long long*>(counts));
     NVFP4_CUDA_CHECK(cudaGetLastError());
@@ -584,6 +648,12 @@ int launch_plan_peer_masked(const int64_t* all_counts, int world, int num_expert
                             int64_t n, int64_t* base, int64_t* limit, int32_t* masked_m, int64_t* dst_row, int32_t* status,
                             cudaStream_t stream)
 {
+    if (n > 0 && n <= kPlanOnePass) {
+        plan_small_kernel<<<1, kPlanThreads, plan_smem(num_experts), stream>>>(all_counts, world, num_experts, rank, cap_m, ids, n, base, limit,
+                                                                               masked_m, dst_row, status);
+        NVFP4_CUDA_CHECK(cudaGetLastError());
+        return NVFP4_OK;
+    }
     plan_offsets_masked_kernel<<<1, 1024, 0, stream>>>(all_counts, world, num_experts, rank, cap_m, base, limit, masked_m, status);
     NVFP4_CUDA_CHECK(cudaGetLastError());
     if (n == 0) return NVFP4_OK;
@@ -598,7 +668,7 @@ int launch_plan_peer_masked(const int64_t* all_counts, int world, int num_expert
     int32_t* chunk_hist = nullptr;
     NVFP4_CUDA_CHECK(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&chunk_hist), sizeof(int32_t) * blocks * num_experts, pool, stream));
     plan_chunk_hist_kernel<<<blocks, kPlanThreads, num_experts * sizeof(int), stream>>>(ids, n, chunk, num_experts, chunk_hist);
-    plan_rows_kernel<<<blocks, kPlanThreads, num_experts * sizeof(long long), stream>>>(ids, n, chunk, num_experts, chunk_hist, base, limit,
+    plan_rows_kernel<<<blocks, kPlanThreads, plan_smem(num_experts), stream>>>(ids, n, chunk, num_experts, chunk_hist, base, limit,
                                                                                       dst_row);
     const cudaError_t err = cudaGetLastError();
     cudaFreeAsync(chunk_hist, stream);

@@ -447,8 +447,10 @@ class ExpertParallelMoE:
         routing entry out of range.  Bits 0, 1 and 3 raise; the overflow bit is returned for the caller to act on."""
         bits = 0
         for buf in self.peer or []:
-            bits |= int(buf.status.item())
-            buf.status.zero_()
+            found = int(buf.status.item())
+            if found:
+                buf.status.zero_()
+            bits |= found
         if bits & 0b1011:
             raise RuntimeError(f"expert-parallel step failed on the device (status {bits:#x}: "
                                f"{'GEMM wait expired; ' if bits & 1 else ''}{'a peer never reached a barrier; ' if bits & 2 else ''}"
