@@ -115,7 +115,7 @@ NVFP4_API int nvfp4_quantize_weight_static(const void* w, int w_dtype, int E, in
  *              [13] split_transform.  NOTE [13] means something else than in the reference (there:
  *              signal A0 early inside its one kernel): here 1 = quantise the activations once in a
  *              kernel of their own ahead of the GEMM, 2 = Algorithm 1 inside the GEMM main loop,
- *              0 = the library's choice.  All other knobs (epilogue_threads, num_stages,
+ *              0 = the library's choice; both orientations.  All other knobs (epilogue_threads, num_stages,
  *              swizzle_cd, epilogue_stages, l2_pin_weights, timing_probe, tail_split,
  *              shallow_stages, produced_stages, a token tile of 128) are accepted and ignored.
  *   device_status optional device int32 the kernel ORs error bits into (bit 0 =
@@ -237,6 +237,17 @@ NVFP4_API int nvfp4_grouped_gemm_masked_quantized_swiglu(const void* a0, const v
                                                          const void* sfb, const float* gw, void* out_a0, void* out_a1,
                                                          void* out_scale_atoms, const int32_t* masked_m, int E, int max_m, int N, int K,
                                                          const int32_t* tune, int32_t* device_status, void* stream);
+
+/* Both forms above for a few rows per expert: the decode kernel (128 weight rows x token_tile = 32 or 64 rows) over quantised rows whose
+ * scales stay in rows, scale_rows (E * max_m, 2, K / 16), as nvfp4_dispatch_quantized_peer leaves them.  Output: BF16 rows in
+ * d (out_* NULL), or, with gate/up-interleaved weights (d NULL), the quantised SwiGLU activation: out_a0, out_a1
+ * (E * max_m, N / 4) and out_scale_rows (E * max_m, 2, N / 32).  Any row counts; an expert's weights are streamed once per
+ * token tile.  The two passes are summed apart and added at the end, so the last bits may differ from the forms
+ * above.  N % 256 == 0, K % 256 == 0.  No counterpart in the reference. */
+NVFP4_API int nvfp4_grouped_gemm_masked_quantized_rows(const void* a0, const void* a1, const void* scale_rows, const void* b,
+                                                       const void* sfb, const float* gw, void* d, int64_t ldd_elems, void* out_a0,
+                                                       void* out_a1, void* out_scale_rows, const int32_t* masked_m, int E, int max_m,
+                                                       int N, int K, int token_tile, int32_t* device_status, void* stream);
 
 /* The same two steps over peer memory, for ranks on the GPUs of one NVLink domain.  `peers` is a device array
  * with one int64 per rank: the address, in THIS process, of that rank's copy of a symmetric buffer (rows of

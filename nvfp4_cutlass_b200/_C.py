@@ -31,7 +31,7 @@ EXPORTS = ("nvfp4_last_error", "nvfp4_version", "nvfp4_get_num_sms", "nvfp4_set_
            "nvfp4_quantize_weight", "nvfp4_quantize_weight_static", "nvfp4_grouped_gemm_contiguous", "nvfp4_debug_decompose",
            "nvfp4_debug_mma_peak", "nvfp4_debug_mma_peak_pair", "nvfp4_debug_mma_pattern", "nvfp4_permute_rows", "nvfp4_swiglu", "nvfp4_combine_rows",
            "nvfp4_dispatch_rows_peer", "nvfp4_dispatch_quantized_peer", "nvfp4_relayout_scales",
-           "nvfp4_grouped_gemm_masked_quantized", "nvfp4_grouped_gemm_masked_quantized_swiglu", "nvfp4_combine_rows_peer", "nvfp4_expert_histogram",
+           "nvfp4_grouped_gemm_masked_quantized", "nvfp4_grouped_gemm_masked_quantized_swiglu", "nvfp4_grouped_gemm_masked_quantized_rows", "nvfp4_combine_rows_peer", "nvfp4_expert_histogram",
            "nvfp4_grouped_gemm_swiglu_contiguous", "nvfp4_grouped_gemm_masked", "nvfp4_load_checkpoint_weights",
            "nvfp4_read_status", "nvfp4_debug_split_workspace", "nvfp4_debug_wait_timeout", "nvfp4_plan_peer_masked",
            "nvfp4_peer_barrier")
@@ -73,6 +73,7 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_relayout_scales.argtypes = [vp, vp, i32, i32, i32, vp, vp]
         L.nvfp4_grouped_gemm_masked_quantized.argtypes = [vp, vp, vp, vp, vp, vp, vp, i64, vp, i32, i32, i32, i32, i32, vp, vp, vp]
         L.nvfp4_grouped_gemm_masked_quantized_swiglu.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp]
+        L.nvfp4_grouped_gemm_masked_quantized_rows.argtypes = [vp, vp, vp, vp, vp, vp, vp, i64, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp]
         L.nvfp4_grouped_gemm_masked.argtypes = [vp, i64, vp, vp, vp, vp, i64, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp]
         L.nvfp4_load_checkpoint_weights.argtypes = [i32, vp, vp, vp, vp, i32, i32, i32, vp, vp, vp, vp]
         L.nvfp4_read_status.argtypes = [vp, ctypes.POINTER(ctypes.c_int32), vp]
@@ -546,6 +547,33 @@ def m_grouped_quantized_swiglu_dual_nvfp4_gemm_masked(rows: "QuantizedRows", b, 
             rows.a0.data_ptr(), rows.a1.data_ptr(), rows.scale_atoms.data_ptr(), b.data_ptr(), sfb.data_ptr(), gw.data_ptr(),
             out.a0.data_ptr(), out.a1.data_ptr(), out.scale_atoms.data_ptr(), masked_m.data_ptr(), e, max_m, n, k,
             tune_arr, device_status.data_ptr() if device_status is not None else None, _stream()))
+
+
+def m_grouped_few_quantized_rows_gemm_masked(rows: "QuantizedRows", b, sfb, gw, out, masked_m, *, token_tile: int = 32,
+                                               device_status=None) -> None:
+    """The two masked GEMMs above for a few rows per expert (the decode kernel): reads ``rows.scale_rows``, no
+    relayout_scales.  ``out``: a BF16 tensor (E, max_m, N), or a QuantizedRows (E, max_m, N / 2) that receives silu(gate) * up
+    with its scales in ``scale_rows`` (weights interleaved by interleave_gate_up).  K and N multiples of 256; token_tile 32 or 64."""
+    e, max_m, k = rows.e, rows.max_m, rows.k
+    quantized = isinstance(out, QuantizedRows)
+    if quantized:
+        n, planes = 2 * out.k, (out.a0.data_ptr(), out.a1.data_ptr(), out.scale_rows.data_ptr())
+        _require(out.e == e and out.max_m == max_m, "out is (E, max_m, I)")
+    else:
+        _require(out.dtype == torch.bfloat16 and out.dim() == 3 and out.shape[:2] == (e, max_m) and out.stride(2) == 1 and
+                 out.stride(0) == max_m * out.stride(1), "out is (E, max_m, N) BF16, last dimension contiguous, groups max_m rows apart")
+        n, planes = out.shape[2], (None, None, None)
+    _require(b.dtype == torch.int8 and sfb.dtype == torch.int32 and gw.dtype == torch.float32 and masked_m.dtype == torch.int32,
+             "b int8, sfb int32, gw float32, masked_m int32")
+    _require(gw.numel() == e and masked_m.numel() == e and b.shape == (e * n, k // 2) and sfb.shape == (e * (k // 64), n),
+             "weight shapes do not fit")
+    _require(b.is_contiguous() and sfb.is_contiguous() and gw.is_contiguous() and masked_m.is_contiguous(),
+             "b, sfb, gw, masked_m are contiguous")
+    with _on(_one_device(rows.store, out.store if quantized else out, b, sfb, gw, masked_m, device_status)):
+        _check(lib().nvfp4_grouped_gemm_masked_quantized_rows(
+            rows.a0.data_ptr(), rows.a1.data_ptr(), rows.scale_rows.data_ptr(), b.data_ptr(), sfb.data_ptr(), gw.data_ptr(),
+            None if quantized else out.data_ptr(), 0 if quantized else out.stride(1), *planes, masked_m.data_ptr(), e, max_m, n, k, int(token_tile),
+            device_status.data_ptr() if device_status is not None else None, _stream()))
 
 
 def combine_rows_peer(peers: torch.Tensor, rows_ld_elems: int, src_rank: torch.Tensor, src_row: torch.Tensor, w: torch.Tensor,

@@ -214,6 +214,12 @@ static bool split_gemm_as_pair(const int32_t* tune, int64_t rows, int experts, b
     return groups_of_256 || (experts > 0 && rows / experts >= 2048);
 }
 
+// Bytes of weights per decode call (each token tile streams N x K of them) from which its activations get a pass of their own.
+// The pass costs a launch, some 3 us; what it saves is Algorithm 1 on a token tile once per 128 weight rows, which is the
+// more the larger the tile.  Measured, in the main loop / in a pass of its own: 64-token tiles, 151 MB: 79 / 40 us; 32-token
+// tiles, 302 MB: 76 / 58 us, 19 MB: 22 / 25; 16-token tiles, 264 MB: 54 / 57 us, 3.7 GB: 675 / 582.
+static double stream_weight_bytes(int token_tile) { return token_tile == 16 ? 1e9 : (token_tile == 32 ? 64e6 : 32e6); }
+
 int nvfp4_grouped_gemm_contiguous(const void* a, int64_t lda_elems, const void* b, const void* sfb, const float* gw,
                                   void* d, int64_t ldd_elems, const int32_t* m_indices, int M, int N, int K, int E,
                                   int scale_policy, int enable_residual_pass, int orientation, int m_alignment,
@@ -261,6 +267,13 @@ int nvfp4_grouped_gemm_contiguous(const void* a, int64_t lda_elems, const void* 
         const int tune_block_k = tune ? tune[5] : 0;   // 0 = the largest of 512 / 256 / 128 that divides K and fits
         NVFP4_REQUIRE(tune_block_k == 0 || tune_block_k == 128 || tune_block_k == 256 || tune_block_k == 512,
                       "tune_block_k must be 0, 128, 256 or 512");
+        // tune_split_transform as in the normal orientation: 1 = activations quantised in a pass of their own, 2 = in the
+        // main loop, 0 = the library's choice
+        const int tune_split = tune ? tune[13] : 0;
+        const double weight_bytes = static_cast<double>(M / tile) * N * K * (9.0 / 16.0);
+        if (K % 256 == 0 && tune_block_k == 0 && tune_split != 2 && (tune_split == 1 || weight_bytes >= stream_weight_bytes(tile)))
+            return launch_gemm_stream(a, lda_elems, b, sfb, gw, d, ldd_elems, m_indices, M, N, K, E, enable_residual_pass != 0, tile,
+                                      scale_policy, !(tune && tune[11]), dev->num_sms, device_status, s);
         return launch_gemm_swap(a, lda_elems, b, sfb, gw, d, ldd_elems, m_indices, M, N, K, E, enable_residual_pass != 0,
                                 tile, tune_block_k, scale_policy, !(tune && tune[11]), dev->num_sms, device_status, s);
     }
@@ -615,6 +628,35 @@ int nvfp4_grouped_gemm_masked_quantized_swiglu(const void* a0, const void* a1, c
                                        tune ? tune[12] : 0, !(tune && tune[11]), dev->num_sms,
                                        split_gemm_as_pair(tune, static_cast<int64_t>(E) * (max_m / 2), E, false), out_a0, out_a1,
                                        out_scale_atoms, device_status, static_cast<cudaStream_t>(stream));
+}
+
+int nvfp4_grouped_gemm_masked_quantized_rows(const void* a0, const void* a1, const void* scale_rows, const void* b, const void* sfb,
+                                             const float* gw, void* d, int64_t ldd_elems, void* out_a0, void* out_a1, void* out_scale_rows,
+                                             const int32_t* masked_m, int E, int max_m, int N, int K, int token_tile,
+                                             int32_t* device_status, void* stream)
+{
+    host::clear_error();
+    NVFP4_REQUIRE(E >= 0 && max_m >= 0 && N >= 0 && K >= 0, "negative size (E=%d, max_m=%d, N=%d, K=%d)", E, max_m, N, K);
+    NVFP4_REQUIRE(token_tile == 32 || token_tile == 64, "token tile %d must be 32 or 64", token_tile);
+    NVFP4_REQUIRE(N % 256 == 0 && K % 256 == 0, "N and K must be multiples of 256 (N=%d, K=%d)", N, K);
+    NVFP4_REQUIRE(max_m % 128 == 0, "max_m must be a multiple of 128 (max_m=%d)", max_m);
+    NVFP4_REQUIRE(static_cast<int64_t>(E) * max_m <= INT32_MAX, "E * max_m = %lld rows exceed the 32-bit row index",
+                  static_cast<long long>(E) * max_m);
+    if (E == 0 || max_m == 0 || N == 0) return NVFP4_OK;
+    NVFP4_REQUIRE(K > 0, "empty weights (K=%d)", K);
+    NVFP4_REQUIRE(a0 && a1 && scale_rows && b && sfb && gw && masked_m, "null pointer argument");
+    const bool quantized_out = out_a0 != nullptr || out_a1 != nullptr || out_scale_rows != nullptr;
+    NVFP4_REQUIRE(quantized_out ? out_a0 && out_a1 && out_scale_rows && d == nullptr : d != nullptr,
+                  "the output is either d or the three planes of quantised rows");
+    NVFP4_REQUIRE(quantized_out || (ldd_elems >= N && ldd_elems % 8 == 0), "bad row stride %lld", static_cast<long long>(ldd_elems));
+    NVFP4_REQUIRE(((reinterpret_cast<uintptr_t>(a0) | reinterpret_cast<uintptr_t>(a1) | reinterpret_cast<uintptr_t>(scale_rows) |
+                    reinterpret_cast<uintptr_t>(d) | reinterpret_cast<uintptr_t>(out_a0) | reinterpret_cast<uintptr_t>(out_a1) |
+                    reinterpret_cast<uintptr_t>(out_scale_rows)) & 15u) == 0, "all activation buffers must be 16-byte aligned");
+    host::DeviceInfo* dev;
+    if (int rc = host::device_info(-1, &dev)) return rc;
+    if (dev->cc_major != 10) return host::fail(NVFP4_E_UNSUPPORTED, "needs an sm_100 GPU, found sm_%d%d", dev->cc_major, dev->cc_minor);
+    return launch_gemm_stream_quantized(a0, a1, scale_rows, b, sfb, gw, d, ldd_elems, masked_m, max_m, N, K, E, token_tile, out_a0, out_a1,
+                                        out_scale_rows, true, dev->num_sms, device_status, static_cast<cudaStream_t>(stream));
 }
 
 int nvfp4_combine_rows_peer(const int64_t* peers, int64_t rows_ld_elems, const int64_t* src_rank, const int64_t* src_row,

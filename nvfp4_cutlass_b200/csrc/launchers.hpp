@@ -58,6 +58,13 @@ int launch_gemm_swap(const void* a, int64_t lda, const void* b, const void* sfb,
                      int64_t ldd, const int32_t* m_indices, int M, int N, int K, int E, bool residual,
                      int token_tile, int block_k, int policy, bool pdl, int num_sms, int32_t* status, cudaStream_t stream);
 
+int launch_gemm_stream(const void* a, int64_t lda, const void* b, const void* sfb, const float* gw, void* d, int64_t ldd,
+                       const int32_t* m_indices, int M, int N, int K, int E, bool residual, int token_tile, int policy, bool pdl, int num_sms,
+                       int32_t* status, cudaStream_t stream);
+int launch_gemm_stream_quantized(const void* a0, const void* a1, const void* scale_rows, const void* b, const void* sfb, const float* gw,
+                                 void* d, int64_t ldd, const int32_t* masked_m, int max_m, int N, int K, int E, int token_tile, void* out_a0,
+                                 void* out_a1, void* out_sf, bool pdl, int num_sms, int32_t* status, cudaStream_t stream);
+
 int launch_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,
                            cudaStream_t stream);
 

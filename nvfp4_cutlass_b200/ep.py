@@ -264,11 +264,13 @@ class ExpertParallelMoE:
         masked_ok = self.gemm_masked is not None and (2 * inter) % 256 == 0 and hidden % 256 == 0
         # Quantised dispatch: the sender runs Algorithm 1 once per token and the rows cross NVLink as NVFP4 codes and
         # scales (1.125 instead of 2 bytes per element); the owners' up-projection then starts from the codes.  Same
-        # codes as quantising the BF16 rows on arrival, so the layer's output does not change by a bit.
+        # codes as quantising the BF16 rows on arrival, so the layer's output does not change by a bit (but
+        # for steps with few rows per expert, whose GEMMs add in another order: see _few_rows_tile).
         self.quantized_dispatch = bool(quantized_dispatch) and hidden % 1024 == 0 and hidden <= 8192
         self.bulk_combine = bool(bulk_combine)   # combine fetches rows by bulk copies into shared memory (see combine_rows_bulk_kernel)
         # SwiGLU and the down-projection's activation quantisation in the up-projection's epilogue (needs the quantised
-        # dispatch's GEMM entry and gate/up-interleaved weights; same bits as the separate kernels)
+        # dispatch's GEMM entry and gate/up-interleaved weights; same bits as the separate kernels, with the same
+        # exception)
         self.fused_swiglu = bool(fused_swiglu) and self.quantized_dispatch and inter % 128 == 0 and self.gemm_masked is not None
         self.up_interleaved = None
         if peer_rows_cap > 0 and torch.cuda.is_available() and masked_ok:
@@ -350,7 +352,24 @@ class ExpertParallelMoE:
         y.index_add_(0, plan.order // k, back.float() * topk_w.reshape(-1)[plan.order].unsqueeze(1))
         return y.to(torch.bfloat16)
 
-    def _peer_step(self, buf: "PeerBuffers", x, topk_ids, topk_w, y, marks: Optional[list] = None, gemm_gate=None) -> None:
+    def _few_rows_tile(self, pairs: int) -> int:
+        """Token tile of the decode kernel for this step, 0 for the 128-row kernels.  With a few rows per expert the weights
+        set the pace and most of a 128-row tile would be empty.  Only the average is known here, the real counts are on the
+        device; an expert with more rows than a tile has its weights read again, out of L2.  Measured on 128 experts,
+        4096 / 1536, per step: up to 24 rows on average 330 us with tiles of 32 against 437 with 128 rows, at
+        48 rows 384 us with tiles of 64 against 444, at 64 rows 540 against 447."""
+        if self.inter % 256 != 0:
+            return 0
+        rows = pairs * self.world
+        for average, tile in self.FEW_ROWS:
+            if rows <= self.num_experts * average:
+                return tile
+        return 0
+
+    FEW_ROWS = ((26, 32), (52, 64))        # (rows per expert on average up to which the tile is taken, tile)
+
+    def _peer_step(self, buf: "PeerBuffers", x, topk_ids, topk_w, y, marks: Optional[list] = None, gemm_gate=None,
+                   pairs: Optional[int] = None) -> None:
         """One (micro-)step over peer memory on the current stream, into `y`.  Nothing here reads anything back to the
         host.  Everything that can fail on this rank alone -- argument checks, allocations -- happens before the first
         barrier; if a call between the barriers raises all the same, the remaining barriers are still enqueued before
@@ -388,7 +407,14 @@ class ExpertParallelMoE:
             # choice the parts' GEMM kernels alternate, every part finishes late and the combines pile up at the end.
             if gemm_gate is not None and gemm_gate[0] is not None:
                 torch.cuda.current_stream().wait_event(gemm_gate[0])
-            if buf.hq is not None:
+            # `pairs`: one size for all parts of a step, so that all of them run the same kernels
+            tile = self._few_rows_tile(topk_ids.numel() if pairs is None else pairs) if buf.hq is not None else 0
+            if tile:
+                _C.m_grouped_few_quantized_rows_gemm_masked(buf.q, *self.up_interleaved, buf.hq, plan.masked_m, token_tile=tile,
+                                                            device_status=buf.status)
+                _C.m_grouped_few_quantized_rows_gemm_masked(buf.hq, *self.down, buf.out, plan.masked_m, token_tile=tile,
+                                                            device_status=buf.status)
+            elif buf.hq is not None:
                 _C.relayout_scales(buf.q, plan.masked_m)
                 _C.m_grouped_quantized_swiglu_dual_nvfp4_gemm_masked(buf.q, *self.up_interleaved, buf.hq, plan.masked_m,
                                                                      device_status=buf.status)
@@ -434,7 +460,8 @@ class ExpertParallelMoE:
                 lo, hi = bounds[i], bounds[i + 1]
                 stream.wait_stream(cur)
                 with torch.cuda.stream(stream):
-                    self._peer_step(self.peer[i], x[lo:hi], topk_ids[lo:hi], topk_w[lo:hi], y[lo:hi], marks if i == 0 else None, gate)
+                    self._peer_step(self.peer[i], x[lo:hi], topk_ids[lo:hi], topk_w[lo:hi], y[lo:hi], marks if i == 0 else None, gate,
+                                    tokens // self.micro * topk_ids.shape[1])
             for stream in self.streams:
                 cur.wait_stream(stream)
         finally:

@@ -1,0 +1,93 @@
+"""The decode GEMM over quantised rows (gemm_stream.cu): every token tile and K block against the oracle, the masked form
+and the layer that uses it against the 128-row kernels, which differ from it in the order of the FP32 sums only."""
+import pytest
+import torch
+
+import nvfp4_gemm
+from nvfp4_cutlass_b200 import _C
+from nvfp4_cutlass_b200.ep import ExpertParallelMoE, route_topk
+
+pytestmark = pytest.mark.gpu
+
+
+def rel_l2(a, b):
+    a, b = a.float().cpu(), b.float().cpu()
+    return float((a - b).norm() / b.norm().clamp_min(1e-30))
+
+
+def weights(e, n, k, seed):
+    g = torch.Generator().manual_seed(seed)
+    return nvfp4_gemm.quantize_weight_nvfp4((torch.randn(e, n, k, generator=g) * 0.05).to(torch.bfloat16).cuda())
+
+
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("align,n,k", [(16, 128, 256), (16, 640, 1536), (32, 256, 512), (32, 128, 768), (64, 384, 1024), (128, 128, 256)])
+def test_contiguous_matches_oracle(oracle, align, n, k, residual):
+    sizes = [align, 0, 3 * align, align, 2 * align]
+    b, sfb, gw = weights(len(sizes), n, k, n + k)
+    mi = nvfp4_gemm.make_m_indices(sizes, alignment=align)
+    a = torch.randn(sum(sizes), k, generator=torch.Generator().manual_seed(k)).to(torch.bfloat16)
+    d = torch.full((sum(sizes), n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(a.cuda(), b, sfb, gw, d, mi.cuda(), enable_residual_pass=residual, m_alignment=align,
+                                                         tune_swap_ab=1, tune_split_transform=1, device_status=status)
+    assert _C.read_status(status) == 0
+    want = oracle.grouped_gemm(a, b.cpu(), sfb.cpu(), gw.cpu(), mi, n, mode="dual" if residual else "single")
+    # FP32 sums in another order move a BF16 output by one ulp (2^-8) where it sits at a tie: far less than one in ten
+    assert rel_l2(d, want) < 2.5e-3
+
+
+@pytest.mark.parametrize("k,inter,tile", [(1024, 256, 32), (256, 512, 32), (512, 256, 64)])
+def test_masked_rows_match_the_128_row_kernels(k, inter, tile):
+    e, max_m, hidden, counts = 5, 256, 512, [1, 0, tile - 1, tile + 1, 256]
+    up, down = weights(e, 2 * inter, k, 1), weights(e, hidden, inter, 2)
+    up = (*_C.interleave_gate_up(up[0], up[1], e, inter), up[2])
+    a = torch.randn(e * max_m, k, generator=torch.Generator().manual_seed(3)).to(torch.bfloat16).cuda()
+    masked_m = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def planes(width):
+        return _C.QuantizedRows(torch.zeros(e * max_m * (width + width // 8), dtype=torch.uint8, device="cuda"), e, max_m, width)
+
+    rows = planes(k)
+    a0, a1, sfa = _C.debug_split_workspace(a)
+    rows.a0.copy_(a0), rows.a1.copy_(a1), rows.scale_atoms.copy_(sfa)
+    rows.scale_rows.copy_(sfa.view(e * max_m // 128, k // 64, 2, 32, 4, 4).permute(0, 4, 3, 2, 1, 5).reshape(rows.scale_rows.shape))
+    live = torch.cat([torch.arange(c) + i * max_m for i, c in enumerate(counts)]).cuda()
+    # one GEMM, BF16 out
+    got, want = (torch.zeros(e, max_m, 2 * inter, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    _C.m_grouped_few_quantized_rows_gemm_masked(rows, *up, got, masked_m, token_tile=tile, device_status=status)
+    _C.m_grouped_quantized_dual_nvfp4_gemm_masked(rows, *up, want, masked_m, device_status=status)
+    assert _C.read_status(status) == 0
+    assert rel_l2(got.view(-1, 2 * inter)[live], want.view(-1, 2 * inter)[live]) < 2.5e-3
+    assert float(got[1].abs().max()) == 0.0 and float(got[0, tile:].abs().max()) == 0.0        # past the token tiles: untouched
+    # SwiGLU and quantisation in the epilogue, then the down-projection
+    hq, hw = planes(inter), planes(inter)
+    _C.m_grouped_few_quantized_rows_gemm_masked(rows, *up, hq, masked_m, token_tile=tile, device_status=status)
+    _C.m_grouped_quantized_swiglu_dual_nvfp4_gemm_masked(rows, *up, hw, masked_m, device_status=status)
+    assert _C.read_status(status) == 0
+    atoms = hw.scale_atoms.view(e * max_m // 128, inter // 64, 2, 32, 4, 4).permute(0, 4, 3, 2, 1, 5).reshape(hq.scale_rows.shape)
+    for x, y in ((hq.a0, hw.a0), (hq.a1, hw.a1), (hq.scale_rows, atoms)):
+        # a gate or up value at a BF16 tie moves its product by an ulp and perhaps a code; residual codes see every ulp
+        assert float((x[live] != y[live]).float().mean()) < 0.02
+    out, ref = (torch.zeros(e, max_m, hidden, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    _C.m_grouped_few_quantized_rows_gemm_masked(hq, *down, out, masked_m, token_tile=tile, device_status=status)
+    _C.m_grouped_quantized_dual_nvfp4_gemm_masked(hw, *down, ref, masked_m, device_status=status)
+    assert _C.read_status(status) == 0
+    assert rel_l2(out.view(-1, hidden)[live], ref.view(-1, hidden)[live]) < 4e-3
+
+
+def test_layer_of_few_tokens_matches_the_bf16_dispatch():
+    e, hidden, inter, tokens, k = 16, 1024, 256, 40, 4
+    up, down = weights(e, 2 * inter, hidden, 5), weights(e, hidden, inter, 6)
+    g = torch.Generator().manual_seed(7)
+    x = torch.randn(tokens, hidden, generator=g).to(torch.bfloat16).cuda()
+    logits = torch.randn(tokens, e, generator=g)
+    logits[:, 3] += 4.0                                                    # one expert gets nearly every token
+    ids, w = route_topk(logits.cuda(), k)
+    few = ExpertParallelMoE(e, hidden, inter, up, down, peer_rows_cap=128)
+    assert few._few_rows_tile(ids.numel()) == 32 and few.peer[0].hq is not None
+    y = [few(x, ids, w) for _ in range(2)]
+    want = ExpertParallelMoE(e, hidden, inter, up, down, peer_rows_cap=128, quantized_dispatch=False)(x, ids, w)
+    halves = ExpertParallelMoE(e, hidden, inter, up, down, peer_rows_cap=128, micro_batches=2)(x, ids, w)
+    assert few.steps_repeated == 0 and torch.equal(y[0], y[1]) and torch.equal(y[0], halves) and rel_l2(y[0], want) < 4e-3
