@@ -293,7 +293,10 @@ int nvfp4_grouped_gemm_contiguous(const void* a, int64_t lda_elems, const void* 
     // K = 2048); on wider layers the fused kernel repeats Algorithm 1 per column span and the separate pass wins.
     // Explicit fused-kernel knobs (cluster, transform warps, direct A) keep the fused kernels.
     const bool fused_knobs = tune && (tune[8] != 0 || tune[1] != 0 || tune[9] != 0);
-    if (tune_split == 1 || (tune_split == 0 && !fused_knobs && N % 256 == 0 && N > 1024)) {
+    // Where no cluster fits (N % 512 != 0) the single-CTA fused kernel transforms an activation tile per 128 or 256 columns
+    // and the separate pass wins from N = 640 on, even with half a column tile of padding: 32 experts x 256
+    // rows, K = 2048: N = 640 56 / 31 us, N = 768 53 / 37; 8 x 512 rows, N = 14464, K = 4096: 939 / 207.
+    if (tune_split == 1 || (tune_split == 0 && !fused_knobs && (N > 1024 || (N % 512 != 0 && N > 512)))) {
         const int tune_block_k = tune ? tune[5] : 0;
         return launch_gemm_split(a, lda_elems, b, sfb, gw, d, ldd_elems, m_indices, nullptr, 0, M, N, K, E,
                                  enable_residual_pass != 0, tune_block_k, tune_sched_group, pdl, scale_policy, false,

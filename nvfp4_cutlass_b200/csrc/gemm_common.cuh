@@ -53,7 +53,7 @@ struct TileWalker {
 
     __device__ __forceinline__ TileWalker(const int32_t* layout_, uint32_t m_rows, uint32_t n_cols, uint32_t bn,
                                           uint32_t group_m_, uint32_t groups_, uint32_t max_m_)
-        : layout(layout_), num_m(m_rows / kBM), num_n(n_cols / bn), group_m(group_m_), groups(groups_), max_m(max_m_)
+        : layout(layout_), num_m(m_rows / kBM), num_n((n_cols + bn - 1) / bn), group_m(group_m_), groups(groups_), max_m(max_m_)
     {
     }
 

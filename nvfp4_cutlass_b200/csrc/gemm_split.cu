@@ -438,7 +438,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
             }
             if constexpr (kSwigluOut) {
                 store_swiglu_quantized(o, p, t.row0 + quad * 32 + lane, t.n_blk * (BN / 2) + group * 32);
-            } else {
+            } else if (t.n_blk * BN + group * 64 < p.n) {          // N an odd multiple of 128: the last tile is half a tile
                 __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(t.row0 + quad * 32 + (lane & 24u)) * p.ldd + t.n_blk * BN +
                                         group * 64 + (lane & 7u) * 8;
                 gemm::store_rows(o, d_lane, p.ldd, lane);
@@ -677,7 +677,7 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         build_units(p.layout, p.m / BM, reinterpret_cast<int32_t*>(smem_gen + C::kOffA), units, num_units_slot);
 
     const uint32_t num_kb = p.k / BK;
-    PairWalker<kMasked> walk{p.layout, units, *num_units_slot, p.n / BN, p.group_m, p.groups, p.max_m};
+    PairWalker<kMasked> walk{p.layout, units, *num_units_slot, (p.n + BN - 1) / BN, p.group_m, p.groups, p.max_m};
     PairTile t;
     bool ok = true;
     ptx::ProbeAcc pa;
@@ -849,7 +849,7 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
             }
             if constexpr (kSwigluOut) {
                 store_swiglu_quantized(o, p, my_row0(t) + quad * 32 + lane, t.n_blk * (BN / 2) + group * 32);
-            } else {
+            } else if (t.n_blk * BN + group * 64 < p.n) {
                 __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(my_row0(t) + quad * 32 + (lane & 24u)) * p.ldd + t.n_blk * BN +
                                         group * 64 + (lane & 7u) * 8;
                 gemm::store_rows(o, d_lane, p.ldd, lane);
@@ -959,7 +959,7 @@ int launch_variant(const Call& c, Params p)
         attr_set[dev] = true;
     }
     // masked layout: the number of tiles is only known on the device; surplus CTAs find no tile and leave
-    const int num_tiles = (M / static_cast<int>(BM)) * (N / static_cast<int>(BN));
+    const int num_tiles = (M / static_cast<int>(BM)) * ((N + static_cast<int>(BN) - 1) / static_cast<int>(BN));
     if constexpr (kPair) {
         // one cluster of two CTAs per pair of SMs; a unit is at most two row blocks, so there are at least num_tiles / 2
         // and at most num_tiles pair tiles
@@ -1002,7 +1002,9 @@ int launch_for_layout(const Call& c, const Params& p, bool residual, int block_k
 
 }  // namespace
 
-// Two launches: activations -> NVFP4 workspace, then the block-scaled GEMM over it.  N % 256 == 0.
+// Two launches: activations -> NVFP4 workspace, then the block-scaled GEMM over it.  N % 128 == 0: when N is an odd multiple
+// of 128 the last column tile loads 128 rows too many (the next expert's weights, or zeros past the last one) and stores
+// nothing of them.
 // masked_m == nullptr: contiguous layout (layout = m_indices, M rows).  Otherwise the masked layout: E groups of
 // max_m rows (M = E * max_m), masked_m[g] of them real.
 int launch_gemm_split(const void* a, int64_t lda, const void* b, const void* sfb, const float* gw, void* d,
