@@ -302,7 +302,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         Ring rp;
         for (uint32_t st = cid; st < num_super && ok; st += ncl) {
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                if (!ptx::mbar_wait(share_full + rp.slot, rp.phase, abort_flag, pa, 0)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait(share_full + rp.slot, rp.phase, abort_flag, pa, 0))) { give_up(1); break; }
                 NVFP4_CTRACE(4, (st - cid) / ncl * num_kb + kb);
                 if (lane < kCopies) {
                     const uint32_t peer = (rank + 1 + lane / 2) % CL;
@@ -333,10 +333,10 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 const uint32_t sf = tmem_base + ((quad * 32) << 16) + kColSF + rp.slot * kSfBufCols;
                 // the columns of this ring position are free once its previous MMAs have retired
-                if (!ptx::mbar_wait_sleep<true>(p_empty + rp.slot, rp.phase ^ 1, abort_flag, 32, pa, 2)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait_sleep<true>(p_empty + rp.slot, rp.phase ^ 1, abort_flag, 32, pa, 2))) { give_up(1); break; }
                 if (warp == kWarpSf0 + 4) NVFP4_CTRACE(6, (st - cid) / ncl * num_kb + kb);
                 if (kind == 0) {
-                    if (!ptx::mbar_wait_sleep<false>(b_full + rp.slot, rp.phase, abort_flag, 32, pa, 1)) { give_up(1); break; }
+                    if (!ptx::all_lanes(ptx::mbar_wait_sleep<false>(b_full + rp.slot, rp.phase, abort_flag, 32, pa, 1))) { give_up(1); break; }
                     if (warp == kWarpSf0) NVFP4_CTRACE(7, (st - cid) / ncl * num_kb + kb);
                     ptx::tcgen05_fence_after_sync();
                     const uint32_t sfb = smem + C::kOffSFB + rp.slot * kSlotSFB + lane * 4;
@@ -347,7 +347,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                         for (uint32_t j = 0; j < 4; ++j) v[4 * i + j] = ptx::lds32(sfb + i * 512 + j * 128);
                     ptx::tmem_st_32x32b(sf + kSfB, v);
                 } else {
-                    if (!ptx::mbar_wait_cluster(p_full + rp.slot, rp.phase, abort_flag, pa, 1)) { give_up(1); break; }
+                    if (!ptx::all_lanes(ptx::mbar_wait_cluster(p_full + rp.slot, rp.phase, abort_flag, pa, 1))) { give_up(1); break; }
                     if (warp == kWarpSf0 + 4) NVFP4_CTRACE(8, (st - cid) / ncl * num_kb + kb);
                     ptx::tcgen05_fence_after_sync();
                     // staging layout [source CTA][pass][K atom][row of that CTA]; lane r wants rows r, r + 32, r + 64, r + 96
@@ -389,7 +389,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             const uint32_t n_blk = ns * CL + rank;
             const int32_t e = max(0, __ldg(p.m_indices + m_blk * BM));
             const float g = __ldg(p.gw + e);
-            if (!ptx::mbar_wait_relaxed(tmem_full, acc_phase, abort_flag, 100)) { give_up(1); break; }
+            if (!ptx::all_lanes(ptx::mbar_wait_relaxed(tmem_full, acc_phase, abort_flag, 100))) { give_up(1); break; }
             ptx::tcgen05_fence_after_sync();
             const long long epi0 = ptx::probe_clock();
             const uint32_t taddr = tmem_base + ((quad * 32) << 16) + kColAcc + part * kEpiCols;
@@ -442,7 +442,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++it) {
                 if (C::kGroups > 1 && it % C::kGroups != gid) continue;            // another group's K block
                 const Ring ra{it % C::kDepthA, (it / C::kDepthA) & 1u}, rp{it % C::kDepthP, (it / C::kDepthP) & 1u};
-                if (!ptx::mbar_wait_sleep<false>(a_full + ra.slot, ra.phase, abort_flag, 32, pa, 0)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait_sleep<false>(a_full + ra.slot, ra.phase, abort_flag, 32, pa, 0))) { give_up(1); break; }
                 const long long xt0 = ptx::probe_clock();
                 const bool leader = (warp - kWarpXform0) % C::kGroupWarps == 0;
                 if (leader) NVFP4_CTRACE(0, it);
@@ -480,7 +480,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                 ptx::probe_count(pa, 3, xt2 - xt1);
                 if (leader) NVFP4_CTRACE(1, it);
                 // every tensor core of the cluster must be done with this slot before anyone rewrites it
-                if (!ptx::mbar_wait_sleep<true>(p_empty + rp.slot, rp.phase ^ 1, abort_flag, 32, pa, 1)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait_sleep<true>(p_empty + rp.slot, rp.phase ^ 1, abort_flag, 32, pa, 1))) { give_up(1); break; }
                 const long long xt3 = ptx::probe_clock();
                 if (leader) NVFP4_CTRACE(2, it);
                 const uint32_t codes = smem + C::kOffCodes + rp.slot * C::kSlotCodes + code_off;

@@ -192,7 +192,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
                 }
             }
         }
-    } else if (warp == kWarpMma) {
+    } else if (warp == kWarpMma && lane == 0) {
         // ================= MMA issue (one lane) =================
         Ring rp, rb;
         uint32_t acc_phase = 0;
@@ -205,44 +205,41 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
                     !ptx::mbar_wait(b_ready + rb.slot, rb.phase, abort_flag, pa, 2) ||
                     !ptx::mbar_wait(b_full + rb.slot, rb.phase, abort_flag, pa, 3)) { give_up(1); break; }
                 ptx::tcgen05_fence_after_sync();
-                if (lane == 0) {
-                    const uint32_t sfa0 = smem + kOffSFA0 + rp.slot * kSlotSFA;
-                    const uint32_t sfa1 = smem + kOffSFA1 + rp.slot * kSlotSFA;
-                    const uint32_t sfb = smem + kOffSFB + rb.slot * kSlotSFB;
+                const uint32_t sfa0 = smem + kOffSFA0 + rp.slot * kSlotSFA;
+                const uint32_t sfa1 = smem + kOffSFA1 + rp.slot * kSlotSFA;
+                const uint32_t sfb = smem + kOffSFB + rb.slot * kSlotSFB;
 #pragma unroll
-                    for (uint32_t a = 0; a < kKAtoms; ++a) {
-                        ptx::tcgen05_cp_32x128b_warpx4(tmem_base + kColSFA0 + 4 * a,
-                                                       ptx::make_smem_desc(sfa0 + a * 512, 128, ptx::kSwizzleNone));
-                        if constexpr (kResidual)
-                            ptx::tcgen05_cp_32x128b_warpx4(tmem_base + kColSFA1 + 4 * a,
-                                                           ptx::make_smem_desc(sfa1 + a * 512, 128, ptx::kSwizzleNone));
+                for (uint32_t a = 0; a < kKAtoms; ++a) {
+                    ptx::tcgen05_cp_32x128b_warpx4(tmem_base + kColSFA0 + 4 * a,
+                                                   ptx::make_smem_desc(sfa0 + a * 512, 128, ptx::kSwizzleNone));
+                    if constexpr (kResidual)
+                        ptx::tcgen05_cp_32x128b_warpx4(tmem_base + kColSFA1 + 4 * a,
+                                                       ptx::make_smem_desc(sfa1 + a * 512, 128, ptx::kSwizzleNone));
 #pragma unroll
-                        for (uint32_t i = 0; i < BN / 128; ++i)
-                            ptx::tcgen05_cp_32x128b_warpx4(
-                                tmem_base + kColSFB + 4 * (a * (BN / 128) + i),
-                                ptx::make_smem_desc(sfb + (a * (BN / 128) + i) * 512, 128, ptx::kSwizzleNone));
-                    }
-                    const uint32_t a0 = smem + kOffA0 + rp.slot * kSlotA0;
-                    const uint32_t a1 = smem + kOffA1 + rp.slot * kSlotA0;
-                    const uint32_t b = smem + kOffB + rb.slot * kSlotB;
-#pragma unroll
-                    for (uint32_t a = 0; a < kKAtoms; ++a) {
-                        // 64 K elements = 32 bytes further along each 64-byte swizzled row
-                        const uint64_t desc_b = ptx::make_smem_desc(b + a * 32, 512, ptx::kSwizzle64B);
-                        ptx::tcgen05_mma_nvf4(tmem_base + kColAcc, ptx::make_smem_desc(a0 + a * 32, 512, ptx::kSwizzle64B),
-                                              desc_b, idesc, tmem_base + kColSFA0 + 4 * a,
-                                              tmem_base + kColSFB + 4 * a * (BN / 128), (kb | a) != 0 ? 1u : 0u);
-                        if constexpr (kResidual)
-                            ptx::tcgen05_mma_nvf4(tmem_base + kColAcc,
-                                                  ptx::make_smem_desc(a1 + a * 32, 512, ptx::kSwizzle64B), desc_b, idesc,
-                                                  tmem_base + kColSFA1 + 4 * a,
-                                                  tmem_base + kColSFB + 4 * a * (BN / 128), 1u);
-                    }
-                    ptx::tcgen05_commit(p_empty + rp.slot);
-                    ptx::tcgen05_commit(b_empty + rb.slot);
-                    if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full);
+                    for (uint32_t i = 0; i < BN / 128; ++i)
+                        ptx::tcgen05_cp_32x128b_warpx4(
+                            tmem_base + kColSFB + 4 * (a * (BN / 128) + i),
+                            ptx::make_smem_desc(sfb + (a * (BN / 128) + i) * 512, 128, ptx::kSwizzleNone));
                 }
-                __syncwarp();
+                const uint32_t a0 = smem + kOffA0 + rp.slot * kSlotA0;
+                const uint32_t a1 = smem + kOffA1 + rp.slot * kSlotA0;
+                const uint32_t b = smem + kOffB + rb.slot * kSlotB;
+#pragma unroll
+                for (uint32_t a = 0; a < kKAtoms; ++a) {
+                    // 64 K elements = 32 bytes further along each 64-byte swizzled row
+                    const uint64_t desc_b = ptx::make_smem_desc(b + a * 32, 512, ptx::kSwizzle64B);
+                    ptx::tcgen05_mma_nvf4(tmem_base + kColAcc, ptx::make_smem_desc(a0 + a * 32, 512, ptx::kSwizzle64B),
+                                          desc_b, idesc, tmem_base + kColSFA0 + 4 * a,
+                                          tmem_base + kColSFB + 4 * a * (BN / 128), (kb | a) != 0 ? 1u : 0u);
+                    if constexpr (kResidual)
+                        ptx::tcgen05_mma_nvf4(tmem_base + kColAcc,
+                                              ptx::make_smem_desc(a1 + a * 32, 512, ptx::kSwizzle64B), desc_b, idesc,
+                                              tmem_base + kColSFA1 + 4 * a,
+                                              tmem_base + kColSFB + 4 * a * (BN / 128), 1u);
+                }
+                ptx::tcgen05_commit(p_empty + rp.slot);
+                ptx::tcgen05_commit(b_empty + rb.slot);
+                if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full);
                 rp.advance<kDepthP>();
                 rb.advance<kDepthB>();
             }
@@ -255,7 +252,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         Ring rb;
         for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                if (!ptx::mbar_wait(b_full + rb.slot, rb.phase, abort_flag, pa, 0)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait(b_full + rb.slot, rb.phase, abort_flag, pa, 0))) { give_up(1); break; }
                 const uint32_t base = smem + kOffSFB + rb.slot * kSlotSFB;
 #pragma unroll
                 for (uint32_t i = 0; i < kKAtoms * (BN / 128); ++i) {
@@ -282,7 +279,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             tile_coords(tile, num_m, num_n, p.group_m, m_blk, n_blk);
             const int32_t e = max(0, __ldg(p.m_indices + m_blk * BM));
             const float g = __ldg(p.gw + e);
-            if (!ptx::mbar_wait(tmem_full, acc_phase, abort_flag, pa, 0)) { give_up(1); break; }
+            if (!ptx::all_lanes(ptx::mbar_wait(tmem_full, acc_phase, abort_flag, pa, 0))) { give_up(1); break; }
             ptx::tcgen05_fence_after_sync();
             // 64 columns at a time: tensor memory -> registers -> x G_W -> BF16 -> four whole 128-byte lines per store
             // instruction through the warp's staging area; the accumulator goes back to the MMA warp as soon as this
@@ -332,7 +329,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
                     if (ntile < num_tiles) tile_coords(ntile, num_m, num_n, p.group_m, nm, n_blk);
                 }
                 if (ntile < num_tiles) xform::load_tile_global(nxt, tile_ptr(nm, nkb), p.lda, t);
-                if (!ptx::mbar_wait(p_empty + rp.slot, rp.phase ^ 1, abort_flag, pa, 1)) { give_up(1); return; }
+                if (!ptx::all_lanes(ptx::mbar_wait(p_empty + rp.slot, rp.phase ^ 1, abort_flag, pa, 1))) { give_up(1); return; }
                 xform::emit_tile<BM, BK, kXformThreads, kResidual, 4, 0, kPolicy>(
                     cur, smem + kOffA0 + rp.slot * kSlotA0, smem + kOffA1 + rp.slot * kSlotA0,
                     smem + kOffSFA0 + rp.slot * kSlotSFA, smem + kOffSFA1 + rp.slot * kSlotSFA, t);
@@ -350,7 +347,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         } else {
             for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
                 for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                    if (!ptx::mbar_wait(a_full + ra.slot, ra.phase, abort_flag, pa, 0)) { give_up(1); break; }
+                    if (!ptx::all_lanes(ptx::mbar_wait(a_full + ra.slot, ra.phase, abort_flag, pa, 0))) { give_up(1); break; }
                     bool p_ok = true;
                     xform::transform_tile<BM, BK, kXformThreads, kResidual, 4, 0, kPolicy>(
                         smem + kOffA + ra.slot * kSlotA, smem + kOffA0 + rp.slot * kSlotA0, smem + kOffA1 + rp.slot * kSlotA0,
@@ -358,7 +355,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
                             // the tile now lives in registers: hand the BF16 slot back before the arithmetic
                             __syncwarp();
                             if (lane == 0) ptx::mbar_arrive(a_empty + ra.slot);
-                            p_ok = ptx::mbar_wait(p_empty + rp.slot, rp.phase ^ 1, abort_flag, pa, 1);
+                            p_ok = ptx::all_lanes(ptx::mbar_wait(p_empty + rp.slot, rp.phase ^ 1, abort_flag, pa, 1));
                         });
                     if (!p_ok) { give_up(1); break; }
                     ptx::fence_proxy_async_smem();

@@ -315,7 +315,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
         }
-    } else if (warp == kWarpMma) {
+    } else if (warp == kWarpMma && lane == 0) {
         // ================= MMA issue: one wait, 2 x kAtoms (x passes) MMAs, one commit per K block =================
         Ring r;
         uint32_t acc_phase = 0;
@@ -330,37 +330,34 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
                 NVFP4_TRACE(3, (tile - blockIdx.x) / gridDim.x * num_kb + kb);
                 ptx::tcgen05_fence_after_sync();
                 const long long pt1 = ptx::probe_clock();
-                if (lane == 0) {
-                    const uint32_t a0 = smem + C::kOffA + r.slot * C::kPass * C::kSlotA, a1 = a0 + C::kSlotA;
-                    const uint32_t b = smem + C::kOffB + r.slot * C::kSlotB;
-                    const uint32_t sf = tmem_base + C::kColSF + r.slot * C::kSfCols;
+                const uint32_t a0 = smem + C::kOffA + r.slot * C::kPass * C::kSlotA, a1 = a0 + C::kSlotA;
+                const uint32_t b = smem + C::kOffB + r.slot * C::kSlotB;
+                const uint32_t sf = tmem_base + C::kColSF + r.slot * C::kSfCols;
 #pragma unroll
-                    for (uint32_t a = 0; a < C::kAtoms; ++a) {
-                        const uint64_t desc_b = ptx::make_smem_desc(b + a * 32, C::kSBO, C::kSwizzle);
-                        ptx::tcgen05_mma_nvf4(tmem_base + C::kColAcc, ptx::make_smem_desc(a0 + a * 32, C::kSBO, C::kSwizzle),
-                                              desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass), sf + C::kSfB + 8 * a,
-                                              (kb | a) != 0 ? 1u : 0u);
-                        if constexpr (kResidual)
-                            ptx::tcgen05_mma_nvf4(tmem_base + C::kColAcc, ptx::make_smem_desc(a1 + a * 32, C::kSBO, C::kSwizzle),
-                                                  desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass + 1), sf + C::kSfB + 8 * a, 1u);
-                        // A commit holds this thread until the MMAs before it have been handed to the tensor pipe.
-                        // Issued at the end of a K block it would leave the pipe with nothing queued while this
-                        // thread finds the next K block; issued after the first atom of the NEXT block it costs the
-                        // ring positions a few hundred cycles but the pipe keeps its queue.
-                        if (a == 0 && pending >= 0) ptx::tcgen05_commit(empty + pending);
-                    }
-                    const long long pt2 = ptx::probe_clock();
-                    ptx::probe_count(pa, 5, pt2 - pt1);
-                    if (kb == num_kb - 1) {
-                        if (r.slot % kGroup == kGroup - 1) ptx::tcgen05_commit(empty + r.slot / kGroup);
-                        ptx::tcgen05_commit(tmem_full);
-                    }
-                    ptx::probe_count(pa, 6, ptx::probe_clock() - pt2);
+                for (uint32_t a = 0; a < C::kAtoms; ++a) {
+                    const uint64_t desc_b = ptx::make_smem_desc(b + a * 32, C::kSBO, C::kSwizzle);
+                    ptx::tcgen05_mma_nvf4(tmem_base + C::kColAcc, ptx::make_smem_desc(a0 + a * 32, C::kSBO, C::kSwizzle),
+                                          desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass), sf + C::kSfB + 8 * a,
+                                          (kb | a) != 0 ? 1u : 0u);
+                    if constexpr (kResidual)
+                        ptx::tcgen05_mma_nvf4(tmem_base + C::kColAcc, ptx::make_smem_desc(a1 + a * 32, C::kSBO, C::kSwizzle),
+                                              desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass + 1), sf + C::kSfB + 8 * a, 1u);
+                    // A commit holds this thread until the MMAs before it have been handed to the tensor pipe.
+                    // Issued at the end of a K block it would leave the pipe with nothing queued while this
+                    // thread finds the next K block; issued after the first atom of the NEXT block it costs the
+                    // ring positions a few hundred cycles but the pipe keeps its queue.
+                    if (a == 0 && pending >= 0) ptx::tcgen05_commit(empty + pending);
                 }
+                const long long pt2 = ptx::probe_clock();
+                ptx::probe_count(pa, 5, pt2 - pt1);
+                if (kb == num_kb - 1) {
+                    if (r.slot % kGroup == kGroup - 1) ptx::tcgen05_commit(empty + r.slot / kGroup);
+                    ptx::tcgen05_commit(tmem_full);
+                }
+                ptx::probe_count(pa, 6, ptx::probe_clock() - pt2);
                 // a group is complete with its last ring position; at a tile end it has been committed above
                 pending = (r.slot % kGroup == kGroup - 1 && kb != num_kb - 1) ? static_cast<int32_t>(r.slot / kGroup) : -1;
                 NVFP4_TRACE(4, (tile - blockIdx.x) / gridDim.x * num_kb + kb);
-                __syncwarp();
                 r.advance<C::kDepth>();
             }
             acc_phase ^= 1;
@@ -379,7 +376,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 // the scales of this phase were requested after the producer had seen the ring position free, so the
                 // MMAs that used its scale columns have retired
-                if (!ptx::mbar_wait(sf_in + r.slot, r.phase, abort_flag, pa, 2)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait(sf_in + r.slot, r.phase, abort_flag, pa, 2))) { give_up(1); break; }
                 if (warp == kWarpSf0) NVFP4_TRACE(1, (tile - blockIdx.x) / gridDim.x * num_kb + kb);
                 const uint32_t sf = tmem_base + ((quad * 32) << 16) + C::kColSF + r.slot * C::kSfCols;
                 const long long duty0 = ptx::probe_clock();
@@ -419,7 +416,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
         uint32_t acc_phase = 0;
         for (uint32_t tile = blockIdx.x; ok && walk.next(tile, t); tile += gridDim.x) {
             const float g = __ldg(p.gw + t.expert);
-            if (!ptx::mbar_wait_relaxed(tmem_full, acc_phase, abort_flag, 100)) { give_up(1); break; }
+            if (!ptx::all_lanes(ptx::mbar_wait_relaxed(tmem_full, acc_phase, abort_flag, 100))) { give_up(1); break; }
             if (warp == kWarpEpi0) NVFP4_TRACE(5, (tile - blockIdx.x) / gridDim.x);
             ptx::tcgen05_fence_after_sync();
             const uint32_t taddr = tmem_base + ((quad * 32) << 16) + C::kColAcc + group * 64;
@@ -729,7 +726,7 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         }
     } else if (warp == kWarpMma) {
         // ================= MMA issue (leader only) =================
-        if (rank == 0) {
+        if (rank == 0 && lane == 0) {
             Ring r;
             uint32_t acc_phase = 0;
             int32_t pending = -1;                   // ring position whose commit is still to be issued
@@ -743,31 +740,28 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
                         !ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 2)) { give_up(1); break; }
                     NVFP4_TRACE(3, (tile - pair_id) / num_pairs * num_kb + kb);
                     ptx::tcgen05_fence_after_sync();
-                    if (lane == 0) {
-                        const uint32_t a0 = smem + C::kOffA + r.slot * C::kStage, a1 = a0 + C::kSlotA;
-                        const uint32_t b = a0 + C::kPass * C::kSlotA;
-                        const uint32_t sf = tmem_base + C::kColSF + r.slot * C::kSfCols;
+                    const uint32_t a0 = smem + C::kOffA + r.slot * C::kStage, a1 = a0 + C::kSlotA;
+                    const uint32_t b = a0 + C::kPass * C::kSlotA;
+                    const uint32_t sf = tmem_base + C::kColSF + r.slot * C::kSfCols;
 #pragma unroll
-                        for (uint32_t a = 0; a < C::kAtoms; ++a) {
-                            const uint64_t desc_b = ptx::make_smem_desc(b + a * 32, C::kSBO, C::kSwizzle);
-                            ptx::tcgen05_mma_nvf4_pair(tmem_base + C::kColAcc, ptx::make_smem_desc(a0 + a * 32, C::kSBO, C::kSwizzle),
-                                                       desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass), sf + C::kSfB + 8 * a,
-                                                       (kb | a) != 0 ? 1u : 0u);
-                            if constexpr (kResidual)
-                                ptx::tcgen05_mma_nvf4_pair(tmem_base + C::kColAcc,
-                                                           ptx::make_smem_desc(a1 + a * 32, C::kSBO, C::kSwizzle), desc_b, idesc,
-                                                           sf + C::kSfA + 4 * (a * C::kPass + 1), sf + C::kSfB + 8 * a, 1u);
-                            // as in the single-CTA kernel: the commit of a K block goes out after the first atom of the next
-                            if (a == 0 && pending >= 0) ptx::tcgen05_commit_pair(empty + pending, kBoth);
-                        }
-                        if (kb == num_kb - 1) {
-                            ptx::tcgen05_commit_pair(empty + r.slot, kBoth);
-                            ptx::tcgen05_commit_pair(tmem_full, kBoth);
-                        }
+                    for (uint32_t a = 0; a < C::kAtoms; ++a) {
+                        const uint64_t desc_b = ptx::make_smem_desc(b + a * 32, C::kSBO, C::kSwizzle);
+                        ptx::tcgen05_mma_nvf4_pair(tmem_base + C::kColAcc, ptx::make_smem_desc(a0 + a * 32, C::kSBO, C::kSwizzle),
+                                                   desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass), sf + C::kSfB + 8 * a,
+                                                   (kb | a) != 0 ? 1u : 0u);
+                        if constexpr (kResidual)
+                            ptx::tcgen05_mma_nvf4_pair(tmem_base + C::kColAcc,
+                                                       ptx::make_smem_desc(a1 + a * 32, C::kSBO, C::kSwizzle), desc_b, idesc,
+                                                       sf + C::kSfA + 4 * (a * C::kPass + 1), sf + C::kSfB + 8 * a, 1u);
+                        // as in the single-CTA kernel: the commit of a K block goes out after the first atom of the next
+                        if (a == 0 && pending >= 0) ptx::tcgen05_commit_pair(empty + pending, kBoth);
+                    }
+                    if (kb == num_kb - 1) {
+                        ptx::tcgen05_commit_pair(empty + r.slot, kBoth);
+                        ptx::tcgen05_commit_pair(tmem_full, kBoth);
                     }
                     pending = kb != num_kb - 1 ? static_cast<int32_t>(r.slot) : -1;
                     NVFP4_TRACE(4, (tile - pair_id) / num_pairs * num_kb + kb);
-                    __syncwarp();
                     r.advance<C::kDepth>();
                 }
                 acc_phase ^= 1;
@@ -782,7 +776,7 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 // the scale columns of ring position r are free: the producer requested these scales only after it had
                 // seen the position's MMAs retire
-                if (!ptx::mbar_wait_sleep<false>(sf_in + rs.slot, rs.phase, abort_flag, PAIR_SLEEP_SF, pa, 2)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait_sleep<false>(sf_in + rs.slot, rs.phase, abort_flag, PAIR_SLEEP_SF, pa, 2))) { give_up(1); break; }
                 if (warp == kWarpSf0) NVFP4_TRACE(1, (tile - pair_id) / num_pairs * num_kb + kb);
                 const uint32_t sf = tmem_base + ((quad * 32) << 16) + C::kColSF + r.slot * C::kSfCols;
                 if (group == 0) {
@@ -825,7 +819,7 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         uint32_t acc_phase = 0;
         for (uint32_t tile = pair_id; ok && walk.next(tile, t); tile += num_pairs) {
             const float g = __ldg(p.gw + t.expert);
-            if (!ptx::mbar_wait_relaxed(tmem_full, acc_phase, abort_flag, 100)) { give_up(1); break; }
+            if (!ptx::all_lanes(ptx::mbar_wait_relaxed(tmem_full, acc_phase, abort_flag, 100))) { give_up(1); break; }
             if (warp == kWarpEpi0) NVFP4_TRACE(5, (tile - pair_id) / num_pairs);
             ptx::tcgen05_fence_after_sync();
             acc_phase ^= 1;

@@ -151,7 +151,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
         }
-    } else if (warp == kWarpMma) {
+    } else if (warp == kWarpMma && lane == 0) {
         Ring r;
         uint32_t it = 0, cnt = 0;
         constexpr uint32_t idesc = ptx::make_idesc_nvf4(BW, C::kRowsP);
@@ -165,18 +165,15 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
                 if (!ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 1) ||
                     !ptx::mbar_wait(sf_full + buf, (cnt >> 1) & 1u, abort_flag, pa, 2)) { give_up(1); break; }
                 ptx::tcgen05_fence_after_sync();
-                if (lane == 0) {
-                    const uint32_t w = smem + C::kOffW + r.slot * C::kSlotW, a = smem + C::kOffP + r.slot * C::kSlotP;
-                    const uint32_t sf = tmem_base + C::kColSF + buf * C::kSfBufCols;
+                const uint32_t w = smem + C::kOffW + r.slot * C::kSlotW, a = smem + C::kOffP + r.slot * C::kSlotP;
+                const uint32_t sf = tmem_base + C::kColSF + buf * C::kSfBufCols;
 #pragma unroll
-                    for (uint32_t i = 0; i < C::kAtoms; ++i)
-                        ptx::tcgen05_mma_nvf4(tmem_acc, ptx::make_smem_desc(w + (i / 4) * C::kSubW + (i % 4) * 32, C::kSBO, ptx::kSwizzle128B),
-                                              ptx::make_smem_desc(a + (i / 4) * C::kSubP + (i % 4) * 32, C::kSBO, ptx::kSwizzle128B), idesc,
-                                              sf + C::kSfW + 4 * i, sf + C::kSfT + 4 * i, (kb | i) != 0 ? 1u : 0u);
-                    ptx::tcgen05_commit(empty + r.slot);       // frees the ring position and the block's scale columns
-                    if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full + acc);
-                }
-                __syncwarp();
+                for (uint32_t i = 0; i < C::kAtoms; ++i)
+                    ptx::tcgen05_mma_nvf4(tmem_acc, ptx::make_smem_desc(w + (i / 4) * C::kSubW + (i % 4) * 32, C::kSBO, ptx::kSwizzle128B),
+                                          ptx::make_smem_desc(a + (i / 4) * C::kSubP + (i % 4) * 32, C::kSBO, ptx::kSwizzle128B), idesc,
+                                          sf + C::kSfW + 4 * i, sf + C::kSfT + 4 * i, (kb | i) != 0 ? 1u : 0u);
+                ptx::tcgen05_commit(empty + r.slot);       // frees the ring position and the block's scale columns
+                if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full + acc);
                 r.advance<C::kDepth>();
             }
         }
@@ -191,12 +188,12 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++cnt) {
                 const uint32_t buf = cnt & 1u;
                 const uint32_t sf = tmem_base + ((quad * 32) << 16) + C::kColSF + buf * C::kSfBufCols;
-                if (!ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 0)) { give_up(1); break; }
-                if (cnt >= 2 && !ptx::mbar_wait(empty + (cnt - 2) % C::kDepth, ((cnt - 2) / C::kDepth) & 1u, abort_flag, pa, 1)) {
+                if (!ptx::all_lanes(ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 0) &&
+                                    (cnt < 2 || ptx::mbar_wait(empty + (cnt - 2) % C::kDepth, ((cnt - 2) / C::kDepth) & 1u, abort_flag,
+                                                               pa, 1)))) {
                     give_up(1);
                     break;
                 }
-                __syncwarp();
                 ptx::tcgen05_fence_after_sync();
                 const uint32_t sfw = smem + C::kOffSFW + r.slot * C::kSlotSFW + lane * 4;
                 uint32_t v[4 * C::kAtoms];
@@ -236,7 +233,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
         for (uint32_t tile = blockIdx.x; ok && walk.next(tile, t); tile += gridDim.x, ++it) {
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
             const float g = __ldg(p.gw + t.expert);
-            bool mine = ptx::mbar_wait(tmem_full + acc, acc_phase, abort_flag, pa, 0);
+            bool mine = ptx::all_lanes(ptx::mbar_wait(tmem_full + acc, acc_phase, abort_flag, pa, 0));
             // the four warps stay together (they share barriers below): one that gave up takes the others along
             if constexpr (kSwigluOut) {
                 uint32_t all;
@@ -245,7 +242,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
                 mine = all != 0;
             }
             if (!mine) { give_up(1); break; }
-            __syncwarp();
             ptx::tcgen05_fence_after_sync();
             const uint32_t taddr = tmem_base + ((quad * 32) << 16) + acc * C::kAccStride;
             __nv_bfloat16* dcol = p.d + static_cast<int64_t>(t.row0) * p.ldd + t.n_blk * BW + quad * 32 + lane;

@@ -199,7 +199,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 }
             }
         }
-    } else if (warp == kWarpMma) {
+    } else if (warp == kWarpMma && lane == 0) {
         Ring rw, rp;
         uint32_t it = 0, cnt = 0;
         constexpr uint32_t idesc = ptx::make_idesc_nvf4(BW, C::kRowsP);
@@ -214,24 +214,21 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     !ptx::mbar_wait(w_full + rw.slot, rw.phase, abort_flag, pa, 2) ||
                     !ptx::mbar_wait(sf_full + buf, (cnt >> 1) & 1u, abort_flag, pa, 3)) { give_up(1); break; }
                 ptx::tcgen05_fence_after_sync();
-                if (lane == 0) {
-                    // the scales are already in tensor memory (scale warps, tcgen05.st): a tensor-memory copy per
-                    // scale atom cost this thread as much issue time as an MMA, and there were two per K atom
-                    const uint32_t w = smem + C::kOffW + rw.slot * C::kSlotW;
-                    const uint32_t pt = smem + C::kOffP + rp.slot * C::kSlotP;
-                    const uint32_t sf = tmem_base + C::kColSF + buf * C::kSfBufCols;
+                // the scales are already in tensor memory (scale warps, tcgen05.st): a tensor-memory copy per
+                // scale atom cost this thread as much issue time as an MMA, and there were two per K atom
+                const uint32_t w = smem + C::kOffW + rw.slot * C::kSlotW;
+                const uint32_t pt = smem + C::kOffP + rp.slot * C::kSlotP;
+                const uint32_t sf = tmem_base + C::kColSF + buf * C::kSfBufCols;
 #pragma unroll
-                    for (uint32_t a = 0; a < C::kAtoms; ++a)
-                        ptx::tcgen05_mma_nvf4(tmem_acc,
-                                              ptx::make_smem_desc(w + (a / 4) * C::kSubW + (a % 4) * 32, C::kSBO, C::kSwizzle),
-                                              ptx::make_smem_desc(pt + (a / 4) * C::kSubP + (a % 4) * 32, C::kSBO, C::kSwizzle), idesc,
-                                              sf + C::kSfW + 4 * a, sf + C::kSfT + 4 * a, (kb | a) != 0 ? 1u : 0u);
-                    // one commit per K block: the weight producer, the scale warps and the transform warps all
-                    // read "the MMAs of K block i have retired" from this barrier
-                    ptx::tcgen05_commit(w_empty + rw.slot);
-                    if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full + acc);
-                }
-                __syncwarp();
+                for (uint32_t a = 0; a < C::kAtoms; ++a)
+                    ptx::tcgen05_mma_nvf4(tmem_acc,
+                                          ptx::make_smem_desc(w + (a / 4) * C::kSubW + (a % 4) * 32, C::kSBO, C::kSwizzle),
+                                          ptx::make_smem_desc(pt + (a / 4) * C::kSubP + (a % 4) * 32, C::kSBO, C::kSwizzle), idesc,
+                                          sf + C::kSfW + 4 * a, sf + C::kSfT + 4 * a, (kb | a) != 0 ? 1u : 0u);
+                // one commit per K block: the weight producer, the scale warps and the transform warps all
+                // read "the MMAs of K block i have retired" from this barrier
+                ptx::tcgen05_commit(w_empty + rw.slot);
+                if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full + acc);
                 rp.advance<C::kDepthP>();
                 rw.advance<C::kDepthW>();
             }
@@ -250,9 +247,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++cnt) {
                 const uint32_t buf = cnt & 1u;
                 const uint32_t sf = tmem_base + ((quad * 32) << 16) + C::kColSF + buf * C::kSfBufCols;
-                if (!ptx::mbar_wait(w_full + rw.slot, rw.phase, abort_flag, pa, 0) ||
-                    !ptx::mbar_wait(p_full + rp.slot, rp.phase, abort_flag, pa, 1)) { give_up(1); break; }
-                if (cnt >= 2 && !ptx::mbar_wait(w_empty + (cnt - 2) % C::kDepthW, ((cnt - 2) / C::kDepthW) & 1u, abort_flag, pa, 2)) {
+                if (!ptx::all_lanes(ptx::mbar_wait(w_full + rw.slot, rw.phase, abort_flag, pa, 0) &&
+                                    ptx::mbar_wait(p_full + rp.slot, rp.phase, abort_flag, pa, 1) &&
+                                    (cnt < 2 || ptx::mbar_wait(w_empty + (cnt - 2) % C::kDepthW, ((cnt - 2) / C::kDepthW) & 1u,
+                                                               abort_flag, pa, 2)))) {
                     give_up(1);
                     break;
                 }
@@ -284,7 +282,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             const uint32_t m_blk = tile / num_n, n_blk = tile % num_n;
             const int32_t e = max(0, __ldg(p.m_indices + m_blk * T));
             const float g = __ldg(p.gw + e);
-            if (!ptx::mbar_wait(tmem_full + acc, acc_phase, abort_flag, pa, 0)) { give_up(1); break; }
+            if (!ptx::all_lanes(ptx::mbar_wait(tmem_full + acc, acc_phase, abort_flag, pa, 0))) { give_up(1); break; }
             ptx::tcgen05_fence_after_sync();
             __nv_bfloat16* dcol = p.d + static_cast<int64_t>(m_blk * T) * p.ldd + n_blk * BW + quad * 32 + lane;
             const uint32_t taddr = tmem_base + ((quad * 32) << 16) + acc * C::kAccStride;
@@ -333,7 +331,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         uint32_t cnt = 0;
         for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++cnt) {
-                if (!ptx::mbar_wait(a_full + ra.slot, ra.phase, abort_flag, pa, 0)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait(a_full + ra.slot, ra.phase, abort_flag, pa, 0))) { give_up(1); break; }
                 bool p_ok = true;
                 xform::transform_tile<T, BK, kXformThreads, kResidual, C::kSfCols, C::kRowsP, kPolicy>(
                     smem + C::kOffA + ra.slot * C::kSlotA, smem + C::kOffP + rp.slot * C::kSlotP,
@@ -342,9 +340,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                         __syncwarp();
                         if (lane == 0) ptx::mbar_arrive(a_empty + ra.slot);
                         // the slot is free once the MMAs of kDepthP K blocks ago have retired
-                        p_ok = cnt < C::kDepthP ||
-                               ptx::mbar_wait(w_empty + (cnt - C::kDepthP) % C::kDepthW, ((cnt - C::kDepthP) / C::kDepthW) & 1u,
-                                              abort_flag, pa, 1);
+                        p_ok = ptx::all_lanes(cnt < C::kDepthP ||
+                                              ptx::mbar_wait(w_empty + (cnt - C::kDepthP) % C::kDepthW,
+                                                             ((cnt - C::kDepthP) / C::kDepthW) & 1u, abort_flag, pa, 1));
                     });
                 if (!p_ok) { give_up(1); break; }
                 ptx::fence_proxy_async_smem();

@@ -334,8 +334,7 @@ combine_rows_bulk_kernel(const int64_t* __restrict__ peers, int64_t rows_ld_byte
         };
         look_up(blockIdx.x);
         for (int64_t t = blockIdx.x; t < tokens; t += gridDim.x) {
-            const bool free_again = ptx::mbar_wait_impl(empty + slot, phase ^ 1, abort_flag);
-            if (!__all_sync(0xffffffffu, free_again)) {
+            if (!ptx::all_lanes(ptx::mbar_wait_impl(empty + slot, phase ^ 1, abort_flag))) {
                 *abort_flag = 1;
                 if (lane == 0 && status != nullptr) atomicOr(status, 1);
                 break;
@@ -355,7 +354,7 @@ combine_rows_bulk_kernel(const int64_t* __restrict__ peers, int64_t rows_ld_byte
     } else {
         const int worker = threadIdx.x - 32, row16 = row_bytes / 16;
         for (int64_t t = blockIdx.x; t < tokens; t += gridDim.x) {
-            if (!ptx::mbar_wait_impl(full + slot, phase, abort_flag)) {
+            if (!ptx::all_lanes(ptx::mbar_wait_impl(full + slot, phase, abort_flag))) {
                 *abort_flag = 1;
                 if (status != nullptr) atomicOr(status, 1);
                 break;

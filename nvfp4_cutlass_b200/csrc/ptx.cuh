@@ -81,6 +81,13 @@ NVFP4_DEVICE bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, volatile uin
     }
 }
 
+// The outcome of a wait that all 32 lanes of a warp made, the same for every lane.  Each lane polls on its own and may
+// leave the poll at another time than its neighbours, while what usually follows is one of the warp-wide instructions
+// (tcgen05.ld / .st, aligned barriers), whose behaviour is undefined unless the lanes run them together; and a lane that
+// gave up while another went on would leave that one alone in the next warp barrier, for good.  The vote brings the
+// lanes back together and makes them go on, or give up, as one.
+NVFP4_DEVICE bool all_lanes(bool ok) { return __all_sync(0xffffffffu, ok); }
+
 // Optional per-site wait accounting for timing studies (NVFP4_PROBE is never defined in
 // the shipped build): waits add their duration to a thread-local counter that the role
 // flushes once, when it leaves its loop.
@@ -176,6 +183,7 @@ template <uint32_t kCols>
 NVFP4_DEVICE void tmem_alloc(uint32_t* smem_result)
 {
     static_assert(kCols >= 32 && kCols <= 512 && (kCols & (kCols - 1)) == 0, "TMEM columns: power of two in [32, 512]");
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
                  "n"(kCols)
                  : "memory");
@@ -184,6 +192,7 @@ NVFP4_DEVICE void tmem_alloc(uint32_t* smem_result)
 template <uint32_t kCols>
 NVFP4_DEVICE void tmem_dealloc(uint32_t taddr)
 {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(kCols) : "memory");
 }
 NVFP4_DEVICE void tcgen05_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -406,6 +415,7 @@ NVFP4_DEVICE uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank)
 }
 NVFP4_DEVICE void cluster_sync()
 {
+    __syncwarp();                                    // one lane may come from a role of its own
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Arrive on an mbarrier of another CTA of the cluster (address from map_to_cta) with the default, CTA-scope release:
@@ -491,6 +501,7 @@ template <uint32_t kCols>
 NVFP4_DEVICE void tmem_alloc_pair(uint32_t* smem_result)
 {
     static_assert(kCols >= 32 && kCols <= 512 && (kCols & (kCols - 1)) == 0, "TMEM columns: power of two in [32, 512]");
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
                  "n"(kCols)
                  : "memory");
@@ -499,6 +510,7 @@ NVFP4_DEVICE void tmem_alloc_pair(uint32_t* smem_result)
 template <uint32_t kCols>
 NVFP4_DEVICE void tmem_dealloc_pair(uint32_t taddr)
 {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(kCols) : "memory");
 }
 // Tiled load into this CTA's shared memory whose bytes complete on an mbarrier that may live in the other CTA
