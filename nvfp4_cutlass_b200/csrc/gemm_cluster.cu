@@ -205,12 +205,9 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                 }
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
-            // The commits of the last ring positions are still on their way here from every CTA of the cluster, and nobody
-            // else waits for them: a CTA that left before they arrived would be signalled when it no longer exists.
-            for (uint32_t i = 0; i < C::kDepthP && ok; ++i) {
-                if (!ptx::mbar_wait_sleep<true>(p_empty + rb.slot, rb.phase ^ 1, abort_flag, 64, pa, 0)) give_up(1);
-                rb.advance<C::kDepthB>();
-            }
+            // commits arrive here from every CTA of the cluster
+            if (ok && !gemm::drain_ring<C::kDepthP>(rb, [&](uint32_t i, uint32_t parity) {
+                    return ptx::mbar_wait_sleep<true>(p_empty + i, parity, abort_flag, 64, pa, 0); })) give_up(1);
         }
     } else if (warp == kWarpTmaA) {
         // ================= activation producer: this CTA's share of the rows =================

@@ -1,21 +1,12 @@
-// Pieces shared by the GEMM kernels of the normal orientation: the ring cursor, the persistent tile order
-// (contiguous and masked layouts) and the epilogue's staged, line-coalesced output stores.
+// Pieces shared by the GEMM kernels: the ring cursor (ring.cuh), the persistent tile order (contiguous and masked
+// layouts) and the epilogue's line-coalesced output stores.
 #pragma once
 #include <cuda_bf16.h>
 
 #include "ptx.cuh"
+#include "ring.cuh"
 
 namespace nvfp4::gemm {
-
-// Cursor of a ring of `kDepth` slots; the phase bit flips on every wrap.
-struct Ring {
-    uint32_t slot = 0, phase = 0;
-    template <uint32_t kDepth>
-    __device__ __forceinline__ void advance()
-    {
-        if (++slot == kDepth) { slot = 0; phase ^= 1; }
-    }
-};
 
 // Tiles are walked in groups of `group_m` row blocks: inside a group the row block changes fastest, so the
 // CTAs running at the same time share a few weight tiles and a few activation tiles in L2.

@@ -154,7 +154,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     if (warp == kWarpTma) {
         // ================= weight producer (one lane) =================
         if (lane == 0) {
-            Ring rb;
+            Ring rb, rp;
             for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
                 uint32_t m_blk, n_blk;
                 tile_coords(tile, num_m, num_n, p.group_m, m_blk, n_blk);
@@ -167,9 +167,14 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
                     ptx::tma_load_2d(smem_gen + kOffSFB + rb.slot * kSlotSFB, &tm_sfb, b_full + rb.slot, n_blk * BN,
                                      e * (p.k / 64) + kb * kKAtoms);
                     rb.advance<kDepthB>();
+                    rp.advance<kDepthP>();
                 }
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
+            if (ok && !(gemm::drain_ring<kDepthB>(rb, [&](uint32_t i, uint32_t parity) {
+                            return ptx::mbar_wait(b_empty + i, parity, abort_flag, pa, 0); }) &&
+                        gemm::drain_ring<kDepthP>(rp, [&](uint32_t i, uint32_t parity) {
+                            return ptx::mbar_wait(p_empty + i, parity, abort_flag, pa, 0); }))) give_up(1);
         }
     } else if (warp == kWarpTmaA) {
         // ================= activation producer of the staged variant (its own lane) =====

@@ -314,6 +314,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
                 }
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
+            if (ok && !gemm::drain_ring<C::kDepth, kGroup>(r, [&](uint32_t i, uint32_t parity) {
+                    return ptx::mbar_wait(empty + i, parity, abort_flag, pa, 0); })) give_up(1);
         }
     } else if (warp == kWarpMma && lane == 0) {
         // ================= MMA issue: one wait, 2 x kAtoms (x passes) MMAs, one commit per K block =================
@@ -717,12 +719,9 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
                 }
             }
             ptx::grid_launch_dependents();
-            // neither CTA leaves before the leader's commits of the last ring positions have arrived (nobody else waits
-            // for them, and a barrier must not be signalled in a CTA that no longer exists)
-            for (uint32_t i = 0; i < C::kDepth && ok; ++i) {
-                if (!ptx::mbar_wait_sleep<false>(empty + r.slot, r.phase ^ 1, abort_flag, PAIR_SLEEP_TMA, pa, 0)) give_up(1);
-                r.advance<C::kDepth>();
-            }
+            // the leader's commits arrive in both CTAs
+            if (ok && !gemm::drain_ring<C::kDepth>(r, [&](uint32_t i, uint32_t parity) {
+                    return ptx::mbar_wait_sleep<false>(empty + i, parity, abort_flag, PAIR_SLEEP_TMA, pa, 0); })) give_up(1);
         }
     } else if (warp == kWarpMma) {
         // ================= MMA issue (leader only) =================

@@ -150,6 +150,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
                 }
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
+            if (ok && !gemm::drain_ring<C::kDepth>(r, [&](uint32_t i, uint32_t parity) {
+                    return ptx::mbar_wait(empty + i, parity, abort_flag, pa, 0); })) give_up(1);
         }
     } else if (warp == kWarpMma && lane == 0) {
         Ring r;

@@ -19,6 +19,7 @@
 // epilogue/sm100_store_cd_swap_ab.cuh, src/kernels/sm100_bf16_dual_nvfp4_gemm.hpp:489-632.
 #include <cuda_bf16.h>
 
+#include "gemm_common.cuh"
 #include "host_common.hpp"
 #include "launchers.hpp"
 #include "transform.cuh"
@@ -88,14 +89,7 @@ struct Params {
     int32_t* status;
 };
 
-struct Ring {
-    uint32_t slot = 0, phase = 0;
-    template <uint32_t kDepth>
-    __device__ __forceinline__ void advance()
-    {
-        if (++slot == kDepth) { slot = 0; phase ^= 1; }
-    }
-};
+using gemm::Ring;
 
 template <uint32_t T, uint32_t BK, bool kResidual, int kPolicy>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -181,6 +175,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 }
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
+            if (ok && !gemm::drain_ring<C::kDepthW>(rw, [&](uint32_t i, uint32_t parity) {
+                    return ptx::mbar_wait(w_empty + i, parity, abort_flag, pa, 0); })) give_up(1);
         }
     } else if (warp == kWarpTmaA) {
         // activation producer (a separate thread, so a full A ring never holds the weights back)

@@ -2,6 +2,7 @@
 import glob
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -54,3 +55,69 @@ def test_warp_wide_instructions_start_converged():
         assert places
         for at in places:
             assert "__syncwarp();" in text[text.rfind("{", 0, text.rfind("asm", 0, at)):at], mnemonic
+
+
+RING_CHECK = r"""
+#include <cstdio>
+#include <cstdlib>
+#include "ring.cuh"
+using nvfp4::gemm::Ring;
+using nvfp4::gemm::drain_ring;
+
+// `blocks` K blocks through the ring: the producer waits for a group's last use before it opens it again, the tensor core
+// commits every group that is full.  Parity p of a barrier that has been opened u times stands for use u - 1 when
+// p == (u - 1) % 2; a barrier that was never opened passes for parity 1.
+template <uint32_t kDepth, uint32_t kGroup> bool check(uint32_t blocks)
+{
+    constexpr uint32_t kGroups = kDepth / kGroup;
+    uint32_t committed[kGroups] = {}, awaited[kGroups] = {};
+    for (uint32_t b = 0; b < blocks; ++b)
+        if (b % kGroup == kGroup - 1) ++committed[b / kGroup % kGroups];
+    Ring r;
+    // what the producer has waited for by the time of its last load: use u of a group before it opens use u + 1
+    uint32_t opened[kGroups] = {};
+    for (uint32_t b = 0; b < blocks; ++b) {
+        if (r.slot % kGroup == 0) awaited[r.slot / kGroup] = opened[r.slot / kGroup]++;
+        r.template advance<kDepth>();
+    }
+    bool fine = true;
+    drain_ring<kDepth, kGroup>(r, [&](uint32_t group, uint32_t parity) {
+        // the parity names the last use that was opened: it has to be one that will be committed
+        if (opened[group] == 0) { fine = fine && parity == 1; return true; }
+        fine = fine && ((opened[group] - 1) & 1u) == parity && committed[group] == opened[group];
+        awaited[group] = opened[group];
+        return true;
+    });
+    for (uint32_t g = 0; g < kGroups; ++g) fine = fine && awaited[g] == committed[g];
+    return fine;
+}
+template <uint32_t kDepth, uint32_t kGroup> void all()
+{
+    for (uint32_t blocks = 0; blocks <= 4 * kDepth + 3; ++blocks)
+        if (!check<kDepth, kGroup>(blocks)) { std::printf("depth %u group %u blocks %u\n", kDepth, kGroup, blocks); std::exit(1); }
+}
+int main()
+{
+    all<2, 1>(); all<3, 1>(); all<4, 1>(); all<5, 1>(); all<7, 1>(); all<10, 1>(); all<12, 1>();
+    all<4, 2>(); all<6, 2>(); all<8, 2>(); all<6, 3>(); all<12, 4>();
+    return 0;
+}
+"""
+
+
+def test_the_drain_awaits_every_commit_and_no_other(tmp_path):
+    program = tmp_path / "ring.cpp"
+    program.write_text(RING_CHECK)
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-I", CSRC, str(program), "-o", str(tmp_path / "ring")], check=True)
+    assert subprocess.run([str(tmp_path / "ring")], capture_output=True, text=True).stdout == ""
+
+
+@pytest.mark.parametrize("name", [k for k in KERNELS if "tcgen05_commit" in source(k) and k.startswith("gemm_")])
+def test_every_ring_freed_by_commits_is_drained(name):
+    """No block leaves before the commits to its ring barriers have arrived: each barrier array that a commit signals, the
+    accumulator's apart (the epilogue waits for all of those), has a drain in its kernel."""
+    text = source(name)
+    for kernel in text.split("__global__")[1:]:
+        signalled = set(re.findall(r"tcgen05_commit\w*\((\w+)", kernel)) - {"tmem_full"}
+        drained = set(re.findall(r"drain_ring<.*?mbar_wait[\w<>]*\((\w+)", kernel, re.S))
+        assert signalled <= drained, (name, signalled, drained)
