@@ -87,6 +87,7 @@ struct Cfg {
     // transform -> copy to the peers -> scale warps -> MMA -> commit back to every CTA is longer than four K blocks of
     // tensor work, so with four positions the tensor pipe idles a quarter of the time.
     static constexpr uint32_t kDepthP = CL == 4 ? 5 : 4, kDepthB = kDepthP, kDepthA = CL == 4 ? 5 : 4;
+    static_assert(kDepthA == kDepthP, "the transform groups take the end of a P slot's use for the end of the A slot's");
     static_assert(kColSF + kDepthP * kSfBufCols <= kTmemCols, "scale columns");
     static constexpr uint32_t kOffA = 0;
     static constexpr uint32_t kOffCodes = kOffA + kDepthA * kSlotA;
@@ -439,7 +440,12 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++it) {
                 if (C::kGroups > 1 && it % C::kGroups != gid) continue;            // another group's K block
                 const Ring ra{it % C::kDepthA, (it / C::kDepthA) & 1u}, rp{it % C::kDepthP, (it / C::kDepthP) & 1u};
-                if (!ptx::all_lanes(ptx::mbar_wait_sleep<false>(a_full + ra.slot, ra.phase, abort_flag, 32, pa, 0))) { give_up(1); break; }
+                // "done" for this CTA: its share of the slot's last use is written, for which the tile had landed and the P slot
+                // had been released before (so the P-empty wait below is unambiguous too)
+                const bool landed = ptx::all_lanes(gemm::wait_turn<C::kDepthA, C::kGroups>(
+                    it, [&](uint32_t i, uint32_t parity) { return ptx::mbar_wait_sleep<false>(share_full + i, parity, abort_flag, 32, pa, 0); },
+                    [&](uint32_t i, uint32_t parity) { return ptx::mbar_wait_sleep<false>(a_full + i, parity, abort_flag, 32, pa, 0); }));
+                if (!landed) { give_up(1); break; }
                 const long long xt0 = ptx::probe_clock();
                 const bool leader = (warp - kWarpXform0) % C::kGroupWarps == 0;
                 if (leader) NVFP4_CTRACE(0, it);

@@ -39,4 +39,18 @@ NVFP4_RING_FN bool drain_ring(Ring next, Wait&& wait)
     return true;
 }
 
+// The waits of one of `kGroups` groups that take the blocks of a ring in turn, ahead of block `it`.  A barrier's parity tells
+// a use from the one before it, no more: whoever waits for use u has to know that use u - 1 is over, or the parity of
+// u - 2 passes for it.  A group that takes every block knows, having waited for u - 1 itself; one that takes every third has
+// not, and a load that arrived later than its successors was enough to let it through early.  So it first waits
+// for the end of the slot's last use, done(slot, parity), a barrier that its own work moves on and that therefore cannot be
+// ahead; then for full(slot, parity).  Returns false when a wait gave up.
+template <uint32_t kDepth, uint32_t kGroups, typename Done, typename Full>
+NVFP4_RING_FN bool wait_turn(uint32_t it, Done&& done, Full&& full)
+{
+    const uint32_t slot = it % kDepth, phase = (it / kDepth) & 1u;
+    if (kGroups > 1 && it >= kDepth && !done(slot, phase ^ 1u)) return false;
+    return full(slot, phase);
+}
+
 }  // namespace nvfp4::gemm

@@ -121,3 +121,72 @@ def test_every_ring_freed_by_commits_is_drained(name):
         signalled = set(re.findall(r"tcgen05_commit\w*\((\w+)", kernel)) - {"tmem_full"}
         drained = set(re.findall(r"drain_ring<.*?mbar_wait[\w<>]*\((\w+)", kernel, re.S))
         assert signalled <= drained, (name, signalled, drained)
+
+
+TURN_CHECK = r"""
+#include <cstdint>
+#include <cstdio>
+#include <random>
+#include "ring.cuh"
+using nvfp4::gemm::wait_turn;
+
+// One CTA of the fused cluster kernel as a model: the producer loads blocks in order, loads land in any order, kGroups groups
+// take blocks in turn, the tensor core takes them in order.  Roles step in a random order, a role that waits stays where it is.
+// `uses` counts a barrier's completed uses; a wait sees their parity only.  Returns false when a wait passed too early.
+template <uint32_t kDepth, uint32_t kGroups, uint32_t kBlocks> bool run(std::mt19937& rng)
+{
+    uint32_t a_full[kDepth] = {}, a_empty[kDepth] = {}, share_full[kDepth] = {}, p_empty[kDepth] = {};
+    bool landed[kBlocks] = {}, issued[kBlocks] = {};
+    uint32_t next_load = 0, next_mma = 0, at[kGroups], stage[kGroups] = {};
+    bool early = false;
+    auto passes = [&](uint32_t uses, uint32_t parity) { return ((uses - 1u) & 1u) == parity; };
+    for (uint32_t g = 0; g < kGroups; ++g) at[g] = g;
+    for (uint32_t steps = 0; steps < 400000 && next_mma < kBlocks; ++steps) {
+        const uint32_t who = rng() % (kGroups + 3);
+        if (who < kGroups) {
+            const uint32_t it = at[who], slot = it % kDepth, use = it / kDepth;
+            if (it >= kBlocks) continue;
+            if (stage[who] == 0) {                               // wait for the tile, then hand its slot back
+                if (!wait_turn<kDepth, kGroups>(it, [&](uint32_t i, uint32_t p) { return passes(share_full[i], p); },
+                                                [&](uint32_t i, uint32_t p) { return passes(a_full[i], p); })) continue;
+                if (a_full[slot] != use + 1) early = true;
+                ++a_empty[slot];
+                stage[who] = 1;
+            } else {                                             // wait for the slot of the products, then write them
+                if (!passes(p_empty[slot], (use & 1u) ^ 1u)) continue;
+                if (p_empty[slot] != use) early = true;
+                ++share_full[slot];
+                stage[who] = 0;
+                at[who] += kGroups;
+            }
+        } else if (who == kGroups) {                             // producer
+            if (next_load < kBlocks && a_empty[next_load % kDepth] == next_load / kDepth) issued[next_load++] = true;
+        } else if (who == kGroups + 1) {                         // some load lands
+            const uint32_t b = next_load == 0 ? 0 : next_load - 1 - rng() % (next_load < kDepth ? next_load : kDepth);
+            if (issued[b] && !landed[b] && rng() % 8 == 0) { landed[b] = true; ++a_full[b % kDepth]; }
+        } else if (share_full[next_mma % kDepth] == next_mma / kDepth + 1) {
+            ++p_empty[next_mma % kDepth];
+            ++next_mma;
+        }
+        if (early) return false;
+    }
+    return next_mma == kBlocks;
+}
+int main()
+{
+    std::mt19937 rng(1);
+    for (int i = 0; i < 3000; ++i)
+        if (!run<5, 3, 64>(rng) || !run<4, 1, 64>(rng) || !run<3, 2, 48>(rng) || !run<5, 4, 64>(rng)) { std::printf("run %d\n", i); return 1; }
+    return 0;
+}
+"""
+
+
+def test_groups_in_turn_never_pass_a_wait_early(tmp_path):
+    program = tmp_path / "turn.cpp"
+    program.write_text(TURN_CHECK)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-Wall", "-I", CSRC, str(program), "-o", str(tmp_path / "turn")], check=True)
+    assert subprocess.run([str(tmp_path / "turn")], capture_output=True, text=True).stdout == ""
+    text = source("gemm_cluster.cu")                                   # the only kernel whose roles take blocks in turn
+    assert re.search(r"wait_turn<C::kDepthA, C::kGroups>\(\s*it,.*?share_full \+ i,.*?a_full \+ i,", text, re.S)
+    assert not any("% C::kGroups" in source(k) for k in KERNELS if k != "gemm_cluster.cu")
