@@ -67,7 +67,9 @@ NVFP4_API int nvfp4_set_num_sms(int device, int value);
  *   sfb  (E*K/64, N) int32, byte j = E4M3 scale of 16-block j of the 64-element atom
  *   gw   (E,) float
  * K must be a multiple of 64 (NVFP4_E_INVALID_ARGUMENT otherwise, where the
- * reference raises ValueError). */
+ * reference raises ValueError).
+ * Blocks of the kernel wait for an expert's maximum with a limit of about a second.  Should a wait ever run out, the kernel
+ * ends, some codes are not written and EVERY gw is NaN: nothing that is computed with these weights passes for a result. */
 NVFP4_API int nvfp4_quantize_weight(const void* w, int w_dtype, int E, int N, int K,
                           void* b, void* sfb, float* gw, void* stream);
 
@@ -327,6 +329,11 @@ NVFP4_API int nvfp4_debug_split_workspace(const void* a, int64_t lda_elems, int 
  * signals, while the CTA holds tensor memory.  The wait runs out, the kernel ORs bit 0 into *device_status, unwinds
  * the way the GEMM kernels do (every role leaves, tensor memory is freed) and returns: the context stays usable. */
 NVFP4_API int nvfp4_debug_wait_timeout(int64_t budget_cycles, int32_t* device_status, void* stream);
+
+/* Test hook: nvfp4_quantize_weight in which the waits for an expert's maximum can only run out, after budget_cycles clock
+ * cycles (at most 2e9).  The kernel ends by itself; every gw is NaN. */
+NVFP4_API int nvfp4_debug_quantize_weight_expired(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,
+                                                  int64_t budget_cycles, void* stream);
 
 /* Measurement hook: issues `iters` rounds of resident-operand block-scaled FP4 MMAs
  * (128 x 256 x 64 each) per SM with no memory traffic and returns through

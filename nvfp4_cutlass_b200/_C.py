@@ -33,7 +33,7 @@ EXPORTS = ("nvfp4_last_error", "nvfp4_version", "nvfp4_get_num_sms", "nvfp4_set_
            "nvfp4_dispatch_rows_peer", "nvfp4_dispatch_quantized_peer", "nvfp4_relayout_scales",
            "nvfp4_grouped_gemm_masked_quantized", "nvfp4_grouped_gemm_masked_quantized_swiglu", "nvfp4_grouped_gemm_masked_quantized_rows", "nvfp4_combine_rows_peer", "nvfp4_expert_histogram",
            "nvfp4_grouped_gemm_swiglu_contiguous", "nvfp4_grouped_gemm_masked", "nvfp4_load_checkpoint_weights",
-           "nvfp4_read_status", "nvfp4_debug_split_workspace", "nvfp4_debug_wait_timeout", "nvfp4_plan_peer_masked",
+           "nvfp4_read_status", "nvfp4_debug_split_workspace", "nvfp4_debug_wait_timeout", "nvfp4_debug_quantize_weight_expired", "nvfp4_plan_peer_masked",
            "nvfp4_peer_barrier")
 
 
@@ -79,6 +79,7 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_read_status.argtypes = [vp, ctypes.POINTER(ctypes.c_int32), vp]
         L.nvfp4_debug_split_workspace.argtypes = [vp, i64, i32, i32, i32, i32, i32, vp, vp, vp, vp]
         L.nvfp4_debug_wait_timeout.argtypes = [i64, vp, vp]
+        L.nvfp4_debug_quantize_weight_expired.argtypes = [vp, i32, i32, i32, i32, vp, vp, vp, i64, vp]
         L.nvfp4_debug_mma_peak.argtypes = [i32, ctypes.POINTER(ctypes.c_double), vp]
         L.nvfp4_debug_mma_peak_pair.argtypes = [i32, ctypes.POINTER(ctypes.c_double), vp]
         L.nvfp4_debug_mma_pattern.argtypes = [i32, i32, i32, i32, i32, ctypes.POINTER(ctypes.c_double), vp]
@@ -336,6 +337,19 @@ def quantize_weight(w: torch.Tensor):
     with _on(w.device):
         _check(lib().nvfp4_quantize_weight(w.data_ptr(), 0 if w.dtype == torch.bfloat16 else 1, e, n, k,
                                            b.data_ptr(), sfb.data_ptr(), gw.data_ptr(), _stream()))
+    return b, sfb, gw
+
+
+def debug_quantize_weight_expired(w: torch.Tensor, budget_cycles: int):
+    """quantize_weight whose waits run out after `budget_cycles` (test hook): returns (b, sfb, gw), gw NaN throughout."""
+    _require(w.is_cuda and w.is_contiguous() and w.dtype in (torch.bfloat16, torch.float32), "w is a contiguous BF16 or FP32 CUDA tensor")
+    e, n, k = w.shape
+    b = torch.zeros(e * n, k // 2, dtype=torch.int8, device=w.device)
+    sfb = torch.zeros(e * k // 64, n, dtype=torch.int32, device=w.device)
+    gw = torch.zeros(e, dtype=torch.float32, device=w.device)
+    with _on(w.device):
+        _check(lib().nvfp4_debug_quantize_weight_expired(w.data_ptr(), 0 if w.dtype == torch.bfloat16 else 1, e, n, k, b.data_ptr(),
+                                                         sfb.data_ptr(), gw.data_ptr(), int(budget_cycles), _stream()))
     return b, sfb, gw
 
 

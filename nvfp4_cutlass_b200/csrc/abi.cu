@@ -165,8 +165,8 @@ int nvfp4_set_num_sms(int device, int value)
     return NVFP4_OK;
 }
 
-int nvfp4_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,
-                          void* stream)
+static int quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,
+                           int64_t expire_after_cycles, void* stream)
 {
     host::clear_error();
     NVFP4_REQUIRE(E >= 0 && N >= 0 && K >= 0, "negative shape (E=%d, N=%d, K=%d)", E, N, K);
@@ -178,7 +178,21 @@ int nvfp4_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void*
     host::DeviceInfo* d;
     if (int rc = host::device_info(-1, &d)) return rc;
     if (d->cc_major != 10) return host::fail(NVFP4_E_UNSUPPORTED, "needs an sm_100 GPU, found sm_%d%d", d->cc_major, d->cc_minor);
-    return launch_quantize_weight(w, w_dtype, E, N, K, b, sfb, gw, static_cast<cudaStream_t>(stream));
+    return launch_quantize_weight(w, w_dtype, E, N, K, b, sfb, gw, static_cast<cudaStream_t>(stream), expire_after_cycles);
+}
+
+int nvfp4_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,
+                          void* stream)
+{
+    return quantize_weight(w, w_dtype, E, N, K, b, sfb, gw, 0, stream);
+}
+
+int nvfp4_debug_quantize_weight_expired(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,
+                                        int64_t budget_cycles, void* stream)
+{
+    host::clear_error();
+    NVFP4_REQUIRE(budget_cycles > 0 && budget_cycles <= 2000000000ll, "budget_cycles outside (0, 2e9]");
+    return quantize_weight(w, w_dtype, E, N, K, b, sfb, gw, budget_cycles, stream);
 }
 
 int nvfp4_quantize_weight_static(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,

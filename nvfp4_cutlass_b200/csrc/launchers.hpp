@@ -65,8 +65,9 @@ int launch_gemm_stream_quantized(const void* a0, const void* a1, const void* sca
                                  void* d, int64_t ldd, const int32_t* masked_m, int max_m, int N, int K, int E, int token_tile, void* out_a0,
                                  void* out_a1, void* out_sf, bool pdl, int num_sms, int32_t* status, cudaStream_t stream);
 
+// expire_after_cycles > 0: the waits for the maxima are made to run out after so many cycles (a test's hook)
 int launch_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,
-                           cudaStream_t stream);
+                           cudaStream_t stream, int64_t expire_after_cycles = 0);
 
 int launch_quantize_weight_static(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,
                                   cudaStream_t stream);

@@ -229,40 +229,63 @@ __device__ __forceinline__ void quantize_unit(const T* __restrict__ w, int N, in
     if (kFull || (at < K / 64 && n + 4 < N)) out[4] = static_cast<int32_t>(word_hi);
 }
 
-// The scratch words of a call, zero at its start: the next tile to draw, and per expert the maximum (FP32 bits) and the
-// number of its maximum tiles that are done, each spread over kSlots words.  (An atomic per warp on one word of either
-// kind was what the kernel waited for: some 7 ns each on one address.)
+// The scratch words of a call, zero at its start: the next tile to draw, whether a wait ran out of time, and per expert the
+// maximum (FP32 bits) and the number of its maximum tiles that are done, each spread over kSlots words.  (An atomic per
+// warp on one word of either kind was what the kernel waited for: some 7 ns each on one address.)
 constexpr int kSlots = 16;
 struct Scratch {
     uint32_t* amax_bits;
     uint32_t* done;
     uint32_t* ticket;
+    uint32_t* expired;
 };
-constexpr int64_t scratch_words(int64_t experts) { return 2 * kSlots * experts + 1; }
+constexpr int64_t scratch_words(int64_t experts) { return 2 * kSlots * experts + 2; }
 constexpr long long kDoneBudget = 2000000000ll;      // cycles, about a second; maxima are taken in microseconds
+
+// A wait for an expert's maxima that runs out of time (it does not happen in a healthy run) must not end in weights that look
+// like weights: every global scale becomes NaN.  Who stores one looks at `expired` after its store, who found the
+// time run out sets `expired` before its own; with a sequentially consistent fence between the two on either side, the
+// NaN is what remains whichever comes first.
+__device__ __forceinline__ void fence_sc() { asm volatile("fence.sc.gpu;" ::: "memory"); }
+__device__ __forceinline__ void poison(const Scratch& scratch, float* gw, int experts)
+{
+    for (int e = static_cast<int>(threadIdx.x & 31u); e < experts; e += 32) {
+        *reinterpret_cast<volatile uint32_t*>(scratch.expired) = 1u;
+        fence_sc();
+        *reinterpret_cast<volatile float*>(gw + e) = __int_as_float(0x7fffffff);
+    }
+}
+__device__ __forceinline__ void store_global_scale(const Scratch& scratch, float* gw, float g)
+{
+    *reinterpret_cast<volatile float*>(gw) = g;
+    fence_sc();
+    if (*reinterpret_cast<const volatile uint32_t*>(scratch.expired) != 0) *reinterpret_cast<volatile float*>(gw) = __int_as_float(0x7fffffff);
+}
 
 // List position i: stage 0 is the maxima of batch 0; stage s the quantisation of batch s - 1 and the maxima of batch s
 // in proportion; the last stage the quantisation of the last batch.  A stage opens with as many maxima tiles as there are
 // blocks: while they are read, the maxima that its quantisation tiles need, drawn just before them, are finished.
+// `need`: maxima tiles of an expert to wait for, `at` but in the test of the wait that runs out after `budget` cycles.
 template <typename T, bool kAligned>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
 quantize_weight_kernel(const T* __restrict__ w, int E, int N, int K, int batch, uint32_t qt, uint32_t at, Scratch scratch,
-                       uint8_t* __restrict__ b, int32_t* __restrict__ sfb, float* __restrict__ gw)
+                       uint32_t need, long long budget, uint8_t* __restrict__ b, int32_t* __restrict__ sfb, float* gw)
 {
     __shared__ uint32_t warp_max[kWarps];
-    __shared__ uint32_t drawn;
+    __shared__ uint32_t drawn, stop;
     const uint32_t kt = static_cast<uint32_t>((K + kUnitK - 1) / kUnitK), lane = threadIdx.x & 31;
     const uint32_t total = static_cast<uint32_t>(E) * (at + qt);
     uint32_t next = 0;
-    if (threadIdx.x == 0) next = atomicAdd(scratch.ticket, 1u);
+    if (threadIdx.x == 0) { next = atomicAdd(scratch.ticket, 1u); stop = 0; }
     int known = -1;                                  // expert whose global scale this thread holds
     float g = 0.0f, rg = 0.0f;
     for (;;) {
         if (threadIdx.x == 0) drawn = next;
         __syncthreads();
         uint32_t i = drawn;
+        const bool stopped = stop != 0;
         __syncthreads();
-        if (i >= total) return;
+        if (stopped || i >= total) return;
         if (threadIdx.x == 0) next = atomicAdd(scratch.ticket, 1u);      // arrives while this tile is worked on
         int first_a = 0;                             // first expert of the stage's maxima
         uint32_t na = min(batch, E) * at, nq = 0;    // tiles of either kind in the stage
@@ -292,9 +315,13 @@ quantize_weight_kernel(const T* __restrict__ w, int E, int N, int K, int batch, 
                 for (;;) {
                     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(scratch.done + slot) : "memory");
                     n = __reduce_add_sync(0xffffffffu, lane < kSlots ? n : 0u);
-                    // (running out of time does not happen in a healthy run: go on with what there is rather than wait for ever)
-                    if (n >= at || __any_sync(0xffffffffu, clock64() - t0 > kDoneBudget)) break;
+                    if (n >= need || __any_sync(0xffffffffu, clock64() - t0 > budget)) break;
                     __nanosleep(100);
+                }
+                if (n < need) {                       // the whole warp: the block ends before its next tile
+                    poison(scratch, gw, E);
+                    stop = 1;
+                    continue;
                 }
                 const uint32_t bits = __reduce_max_sync(0xffffffffu, *reinterpret_cast<const volatile uint32_t*>(scratch.amax_bits + slot));
                 g = fmaxf(__fdiv_rn(__uint_as_float(bits), 2688.0f), 1.17549435e-38f);
@@ -306,7 +333,7 @@ quantize_weight_kernel(const T* __restrict__ w, int E, int N, int K, int batch, 
             if (full && ordinary) quantize_unit<T, kAligned, true, true>(w, N, K, e, nw, k0, b, sfb, rows, g, rg);
             else if (ordinary) quantize_unit<T, kAligned, false, true>(w, N, K, e, nw, k0, b, sfb, rows, g, rg);
             else quantize_unit<T, kAligned, false, false>(w, N, K, e, nw, k0, b, sfb, rows, g, rg);
-            if (r == 0 && threadIdx.x == 0) gw[e] = g;
+            if (r == 0 && threadIdx.x == 0) store_global_scale(scratch, gw + e, g);
         } else {
             const uint32_t t = i - q_before;
             const int e = first_a + static_cast<int>(t / at);
@@ -323,7 +350,8 @@ quantize_weight_kernel(const T* __restrict__ w, int E, int N, int K, int batch, 
 }
 
 template <typename T>
-int run_batches(const T* w, int E, int N, int K, void* b, void* sfb, float* gw, const Scratch& scratch, cudaStream_t stream)
+int run_batches(const T* w, int E, int N, int K, void* b, void* sfb, float* gw, const Scratch& scratch, uint32_t need_more,
+                long long budget, cudaStream_t stream)
 {
     const int64_t per_expert = static_cast<int64_t>(N) * K;
     const int64_t fit = kBatchBytes / (per_expert * static_cast<int64_t>(sizeof(T)));
@@ -338,19 +366,21 @@ int run_batches(const T* w, int E, int N, int K, void* b, void* sfb, float* gw, 
     const bool aligned = (reinterpret_cast<uintptr_t>(w) & 31u) == 0;
     auto kernel = aligned ? quantize_weight_kernel<T, true> : quantize_weight_kernel<T, false>;
     return host::launch_kernel(kernel, dim3(static_cast<unsigned>(blocks < tiles ? blocks : tiles)), dim3(kThreads), 0, stream, false, w, E, N, K,
-                               batch, static_cast<uint32_t>(qt), static_cast<uint32_t>(at), scratch, static_cast<uint8_t*>(b),
-                               static_cast<int32_t*>(sfb), gw);
+                               batch, static_cast<uint32_t>(qt), static_cast<uint32_t>(at), scratch,
+                               static_cast<uint32_t>(at) + need_more, budget, static_cast<uint8_t*>(b), static_cast<int32_t*>(sfb), gw);
 }
 
-// `words`: scratch_words(E) words the caller provides; they are cleared here, on the call's stream.
+// `words`: scratch_words(E) words the caller provides; they are cleared here, on the call's stream.  need_more, budget: for the
+// test of a wait that runs out of time.
 int run_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw, uint32_t* words,
-                        cudaStream_t stream)
+                        cudaStream_t stream, uint32_t need_more = 0, long long budget = kDoneBudget)
 {
     NVFP4_CUDA_CHECK(cudaMemsetAsync(words, 0, sizeof(uint32_t) * scratch_words(E), stream));
     const int64_t slots = static_cast<int64_t>(kSlots) * E;
-    const Scratch scratch{words, words + slots, words + 2 * slots};
-    return w_dtype == NVFP4_DTYPE_BF16 ? run_batches(static_cast<const __nv_bfloat16*>(w), E, N, K, b, sfb, gw, scratch, stream)
-                                       : run_batches(static_cast<const float*>(w), E, N, K, b, sfb, gw, scratch, stream);
+    const Scratch scratch{words, words + slots, words + 2 * slots, words + 2 * slots + 1};
+    return w_dtype == NVFP4_DTYPE_BF16
+               ? run_batches(static_cast<const __nv_bfloat16*>(w), E, N, K, b, sfb, gw, scratch, need_more, budget, stream)
+               : run_batches(static_cast<const float*>(w), E, N, K, b, sfb, gw, scratch, need_more, budget, stream);
 }
 
 }  // namespace
@@ -358,7 +388,7 @@ int run_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b
 // The per-expert maxima live in a stream-ordered allocation from the library's memory pool: calls on
 // different streams never share it, nothing synchronises the device, and after the first call it is a pool look-up.
 int launch_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,
-                           cudaStream_t stream)
+                           cudaStream_t stream, int64_t expire_after_cycles)
 {
     if (E == 0 || N == 0 || K == 0) return NVFP4_OK;
     int dev = 0;
@@ -367,7 +397,8 @@ int launch_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void
     if (int rc = host::workspace_pool(dev, &pool)) return rc;
     uint32_t* amax_bits = nullptr;
     NVFP4_CUDA_CHECK(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&amax_bits), sizeof(uint32_t) * scratch_words(E), pool, stream));
-    const int rc = run_quantize_weight(w, w_dtype, E, N, K, b, sfb, gw, amax_bits, stream);
+    const int rc = expire_after_cycles > 0 ? run_quantize_weight(w, w_dtype, E, N, K, b, sfb, gw, amax_bits, stream, 1u, expire_after_cycles)
+                                           : run_quantize_weight(w, w_dtype, E, N, K, b, sfb, gw, amax_bits, stream);
     cudaFreeAsync(amax_bits, stream);
     return rc;
 }

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import nvfp4_gemm
+from nvfp4_cutlass_b200 import _C
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +35,14 @@ def test_every_global_scale_mantissa(oracle, dtype, scale):
     w[:, 0, 0] = 1.0 + torch.arange(128) / 128.0             # one expert per BF16 mantissa of the largest magnitude
     w = (w * scale).to(dtype)
     check(oracle, w, w.cuda())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 16, 64), (70, 64, 512), (3, 2048, 4096)])
+def test_a_wait_that_runs_out_shows(oracle, dtype, shape):
+    """Waits that can only run out (after half a millisecond): the kernel ends, and no global scale looks like one."""
+    w = (torch.randn(shape, generator=torch.Generator().manual_seed(9)) * 0.02).to(dtype)
+    wd = w.cuda()
+    gw = _C.debug_quantize_weight_expired(wd, 1_000_000)[2]
+    assert bool(torch.isnan(gw).all())
+    check(oracle, w[:2, :64], wd[:2, :64])                   # and the next call is an ordinary one

@@ -144,6 +144,7 @@ def test_new_entry_points_validate_without_gpu():
     assert lib.nvfp4_load_checkpoint_weights(9, None, None, None, None, 1, 1, 64, None, None, None, None) == 1
     assert lib.nvfp4_read_status(None, None, None) == 1
     assert lib.nvfp4_debug_wait_timeout(0, None, None) == 1
+    assert lib.nvfp4_debug_quantize_weight_expired(None, 0, 1, 64, 64, None, None, None, 0, None) == 1
     # normal orientation: alignment 128, or 256 as the caller's statement of whole row pairs; nothing else
     rc = lib.nvfp4_grouped_gemm_contiguous(None, 0, None, None, None, None, 0, None, 384, 256, 128, 1, 0, 1, 0, 256, None, None, None)
     assert rc == 1 and b"multiple of the token-tile alignment" in lib.nvfp4_last_error()
