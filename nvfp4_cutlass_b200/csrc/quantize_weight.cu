@@ -127,11 +127,17 @@ __device__ __forceinline__ float divide(float x, float d, float y)
 // (T in {1, 3, 5, 7}) that asks for X 2^a = D (T 2^b +- 1) + eps with |eps| <= 4, a >= 41 and b in {22, 23, 24}; modulo
 // 2^41 the only solution below 2^24 is D = 2^24 - 1 with T = 1 and X a power of two.  For that D the reciprocal
 // (1 + 2^-24 + 2^-48 times a power of two) is rounded up by hand; the remainder step then lands above the boundary.
+//
+// This form takes -x, which costs nothing where the halves of a word are unpacked: what comes out is then +q, with the sign of
+// a zero, and a NaN is left to the conversion, which makes it the largest positive code whatever its sign.  (Flipping the sign
+// bits of the codes of -q turned a NaN over, too; negating the quotients took 189 us on the 8 experts above, this 183.)
+template <typename T, bool kOrdinary>
+constexpr bool kNegated = kOrdinary && !std::is_same_v<T, float>;
 template <typename T, bool kOrdinary>
 __device__ __forceinline__ void quantize_block(const float (&x)[16], float d, uint32_t (&packed)[2])
 {
     float q[16];
-    if constexpr (kOrdinary && !std::is_same_v<T, float>) {
+    if constexpr (kNegated<T, kOrdinary>) {
         const float r = ptx::rcp_approx(d);
         float y = __fmaf_rn(r, __fmaf_rn(-d, r, 1.0f), r);
         if ((__float_as_uint(d) & 0x7fffffu) == 0x7fffffu) y = __uint_as_float(__float_as_uint(y) | 1u);
@@ -150,10 +156,6 @@ __device__ __forceinline__ void quantize_block(const float (&x)[16], float d, ui
     }
     packed[0] = ptx::cvt_e2m1x8(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
     packed[1] = ptx::cvt_e2m1x8(q[8], q[9], q[10], q[11], q[12], q[13], q[14], q[15]);
-    if constexpr (kOrdinary && !std::is_same_v<T, float>) {              // these are the codes of -x / d
-        packed[0] ^= 0x88888888u;
-        packed[1] ^= 0x88888888u;
-    }
 }
 
 // A warp's share of a quantisation tile: 8 weight rows x 512 K of one expert, a row at a time, a lane one 16-element block of
@@ -205,8 +207,9 @@ __device__ __forceinline__ void quantize_unit(const T* __restrict__ w, int N, in
                     if constexpr (std::is_same_v<T, float>) {
                         x[8 * c + i] = __uint_as_float(q.w[i]);
                     } else {
-                        x[2 * i] = __uint_as_float(q.w[i] << 16);
-                        x[2 * i + 1] = __uint_as_float(q.w[i] & 0xffff0000u);
+                        constexpr uint32_t kSign = kNegated<T, kOrdinary> ? 0x80000000u : 0u;
+                        x[2 * i] = __uint_as_float(q.w[i] * 65536u + kSign);
+                        x[2 * i + 1] = __uint_as_float((q.w[i] & 0xffff0000u) ^ kSign);
                     }
                 }
             }

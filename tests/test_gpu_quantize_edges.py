@@ -46,3 +46,28 @@ def test_a_wait_that_runs_out_shows(oracle, dtype, shape):
     gw = _C.debug_quantize_weight_expired(wd, 1_000_000)[2]
     assert bool(torch.isnan(gw).all())
     check(oracle, w[:2, :64], wd[:2, :64])                   # and the next call is an ordinary one
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -70])         # kept reciprocals, divisions
+def test_nan_and_infinity(oracle, dtype, scale):
+    """A NaN does not count for a maximum and gets the largest positive code whatever its sign (the conversion's rule; the oracle
+    keeps the sign); the elements around it get the codes they would get beside a zero.  Infinities make G infinite."""
+    g = torch.Generator().manual_seed(11)
+    clean = (torch.randn(2, 70, 640, generator=g) * 0.02 * scale).to(dtype)
+    at = torch.rand(clean.shape, generator=g) < 0.02
+    at[0, 3, 16:32] = True                                   # a block of nothing else
+    clean[at] = 0.0
+    nan = torch.where(torch.rand(clean.shape, generator=g) < 0.5, torch.tensor(float("nan")), -torch.tensor(float("nan"))).to(dtype)
+    w = torch.where(at, nan, clean)
+    b, sfb, gw = nvfp4_gemm.quantize_weight_nvfp4(w.cuda())
+    want_b, want_sfb, want_gw = oracle.quantize_weight(clean)
+    codes = want_b.view(torch.uint8).view(2, 70, 320)
+    codes = torch.stack((codes & 15, codes >> 4), dim=-1).view(2, 70, 640)
+    codes[at] = 7
+    want_b = (codes[..., 0::2] | codes[..., 1::2] << 4).view(140, 320)
+    assert torch.equal(b.cpu().view(torch.uint8), want_b) and torch.equal(sfb.cpu(), want_sfb) and torch.equal(gw.cpu(), want_gw)
+    w[1, 5, 7], w[1, 60, 639] = float("inf"), -float("inf")
+    b, sfb, gw = nvfp4_gemm.quantize_weight_nvfp4(w.cuda())
+    assert torch.equal(gw.cpu(), torch.stack((want_gw[0], torch.tensor(float("inf")))))
+    assert torch.equal(b.cpu().view(torch.uint8)[:70], want_b[:70])
