@@ -251,6 +251,18 @@ NVFP4_API int nvfp4_grouped_gemm_masked_quantized_rows(const void* a0, const voi
                                                        void* out_a1, void* out_scale_rows, const int32_t* masked_m, int E, int max_m,
                                                        int N, int K, int token_tile, int32_t* device_status, void* stream);
 
+/* The expert MLP over quantised rows when most groups probably have few rows: nvfp4_grouped_gemm_masked_quantized_rows for the up-
+ * (gate/up-interleaved, SwiGLU-quantised output in the h planes) and the down-projection, or, with `decide`, either those or
+ * nvfp4_relayout_scales and the 128-row forms, whichever the row counts call for: both are launched, and the ones that are not
+ * called for leave at once.  Planes and weights as in those entries: a0, a1, scale_rows (E * max_m rows of `hidden`), h_* (rows
+ * of `inter`), up (E, 2 inter, hidden), down (E, hidden, inter), d BF16 rows; scale_atoms and h_scale_atoms are scratch
+ * of the 128-row forms.  hidden and inter multiples of 256, token_tile 32 or 64.  No counterpart in the reference. */
+NVFP4_API int nvfp4_expert_mlp_few_rows(const void* a0, const void* a1, const void* scale_rows, void* scale_atoms, const void* up_b,
+                                        const void* up_sfb, const float* up_gw, void* h_a0, void* h_a1, void* h_scale_rows,
+                                        void* h_scale_atoms, const void* down_b, const void* down_sfb, const float* down_gw, void* d,
+                                        int64_t ldd_elems, const int32_t* masked_m, int E, int max_m, int hidden, int inter,
+                                        int token_tile, int decide, int32_t* device_status, void* stream);
+
 /* The same two steps over peer memory, for ranks on the GPUs of one NVLink domain.  `peers` is a device array
  * with one int64 per rank: the address, in THIS process, of that rank's copy of a symmetric buffer (rows of
  * `row_bytes`, stride dst_ld_bytes / rows_ld_elems, the same on every rank).  No counterpart in the reference.

@@ -31,7 +31,7 @@ EXPORTS = ("nvfp4_last_error", "nvfp4_version", "nvfp4_get_num_sms", "nvfp4_set_
            "nvfp4_quantize_weight", "nvfp4_quantize_weight_static", "nvfp4_grouped_gemm_contiguous", "nvfp4_debug_decompose",
            "nvfp4_debug_mma_peak", "nvfp4_debug_mma_peak_pair", "nvfp4_debug_mma_pattern", "nvfp4_permute_rows", "nvfp4_swiglu", "nvfp4_combine_rows",
            "nvfp4_dispatch_rows_peer", "nvfp4_dispatch_quantized_peer", "nvfp4_relayout_scales",
-           "nvfp4_grouped_gemm_masked_quantized", "nvfp4_grouped_gemm_masked_quantized_swiglu", "nvfp4_grouped_gemm_masked_quantized_rows", "nvfp4_combine_rows_peer", "nvfp4_expert_histogram",
+           "nvfp4_grouped_gemm_masked_quantized", "nvfp4_grouped_gemm_masked_quantized_swiglu", "nvfp4_grouped_gemm_masked_quantized_rows", "nvfp4_expert_mlp_few_rows", "nvfp4_combine_rows_peer", "nvfp4_expert_histogram",
            "nvfp4_grouped_gemm_swiglu_contiguous", "nvfp4_grouped_gemm_masked", "nvfp4_load_checkpoint_weights",
            "nvfp4_read_status", "nvfp4_debug_split_workspace", "nvfp4_debug_wait_timeout", "nvfp4_debug_quantize_weight_expired", "nvfp4_plan_peer_masked",
            "nvfp4_peer_barrier")
@@ -74,6 +74,7 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_grouped_gemm_masked_quantized.argtypes = [vp, vp, vp, vp, vp, vp, vp, i64, vp, i32, i32, i32, i32, i32, vp, vp, vp]
         L.nvfp4_grouped_gemm_masked_quantized_swiglu.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp]
         L.nvfp4_grouped_gemm_masked_quantized_rows.argtypes = [vp, vp, vp, vp, vp, vp, vp, i64, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp]
+        L.nvfp4_expert_mlp_few_rows.argtypes = [vp] * 15 + [i64, vp] + [i32] * 6 + [vp, vp]
         L.nvfp4_grouped_gemm_masked.argtypes = [vp, i64, vp, vp, vp, vp, i64, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp]
         L.nvfp4_load_checkpoint_weights.argtypes = [i32, vp, vp, vp, vp, i32, i32, i32, vp, vp, vp, vp]
         L.nvfp4_read_status.argtypes = [vp, ctypes.POINTER(ctypes.c_int32), vp]
@@ -587,6 +588,32 @@ def m_grouped_few_quantized_rows_gemm_masked(rows: "QuantizedRows", b, sfb, gw, 
         _check(lib().nvfp4_grouped_gemm_masked_quantized_rows(
             rows.a0.data_ptr(), rows.a1.data_ptr(), rows.scale_rows.data_ptr(), b.data_ptr(), sfb.data_ptr(), gw.data_ptr(),
             None if quantized else out.data_ptr(), 0 if quantized else out.stride(1), *planes, masked_m.data_ptr(), e, max_m, n, k, int(token_tile),
+            device_status.data_ptr() if device_status is not None else None, _stream()))
+
+
+def expert_mlp_few_rows(rows: "QuantizedRows", up, h: "QuantizedRows", down, out, masked_m, *, token_tile: int = 32, decide: bool = True,
+                        device_status=None) -> None:
+    """Up-projection with SwiGLU into ``h`` and down-projection into ``out`` (E, max_m, hidden) BF16, for steps in which most experts have
+    few rows: as by m_grouped_few_quantized_rows_gemm_masked, or, with ``decide`` and if the counts on the device call for it, as
+    by relayout_scales and the 128-row kernels.  ``up`` and ``down`` are (b, sfb, gw), up with gate and up rows interleaved."""
+    e, max_m, hidden, inter, index = rows.e, rows.max_m, rows.k, h.k, rows.store.get_device()
+    # as few interpreter steps as the conditions allow: this call stands between the dispatch and the first GEMM
+    _require(h.e == e and h.max_m == max_m, "h is (E, max_m, I)")
+    _require(out.dtype == torch.bfloat16 and out.shape == (e, max_m, hidden) and out.stride() == (max_m * (ldd := out.stride(1)), ldd, 1),
+             "out is (E, max_m, hidden) BF16, last dimension contiguous, groups max_m rows apart")
+    _require(masked_m.dtype == torch.int32 and masked_m.numel() == e and masked_m.is_contiguous(), "masked_m is contiguous int32, one entry per group")
+    _require(index >= 0 and index == rows.scale_atoms.get_device() == h.store.get_device() == h.scale_atoms.get_device() == out.get_device() ==
+             masked_m.get_device() and (device_status is None or device_status.get_device() == index), "all operands are CUDA tensors of one device")
+    for (b, sfb, gw), n, k in ((up, 2 * inter, hidden), (down, hidden, inter)):
+        _require(b.dtype == torch.int8 and sfb.dtype == torch.int32 and gw.dtype == torch.float32 and b.shape == (e * n, k // 2) and
+                 sfb.shape == (e * (k // 64), n) and gw.numel() == e and b.is_contiguous() and sfb.is_contiguous() and gw.is_contiguous() and
+                 index == b.get_device() == sfb.get_device() == gw.get_device(),
+                 "weights are b int8 (E * N, K / 2), sfb int32 (E * K / 64, N), gw float32 (E,), contiguous, on the operands' device")
+    with _on(index):
+        _check(lib().nvfp4_expert_mlp_few_rows(
+            rows.a0.data_ptr(), rows.a1.data_ptr(), rows.scale_rows.data_ptr(), rows.scale_atoms.data_ptr(), up[0].data_ptr(), up[1].data_ptr(),
+            up[2].data_ptr(), h.a0.data_ptr(), h.a1.data_ptr(), h.scale_rows.data_ptr(), h.scale_atoms.data_ptr(), down[0].data_ptr(),
+            down[1].data_ptr(), down[2].data_ptr(), out.data_ptr(), ldd, masked_m.data_ptr(), e, max_m, hidden, inter, token_tile, decide,
             device_status.data_ptr() if device_status is not None else None, _stream()))
 
 

@@ -34,6 +34,31 @@ struct Tile {
 //   masked:     `groups` experts with `max_m` rows reserved each, of which the first masked_m[g] (a device-side
 //               count, clamped to max_m) are real; row blocks past the count do not exist
 //               (counterpart in the reference: scheduler/grouped_gemm.cuh:139-156)
+// Two families of kernels can take a masked call whose groups may have few rows or many: the decode kernels, token tiles of
+// `tile` rows, and the 128-row kernels.  Only the device knows the counts, so both are launched and the family that is the
+// slower one for them leaves at once.  The decode kernels pass an expert's weights once per token tile, the others once
+// per block of 128 rows: the decode kernels take the call with up to two and a half tiles of 32, or one and a half of 64, to a
+// block.  Expert layer of 128 experts, 4096 / 1536, decode / 128-row kernels, tiles of 32: uniform routing, 1.1 tiles to a block,
+// 260 / 359 us; skewed, 1.5, 128 / 152; 1.8, 164 / 165; 2.4, 210 / 199; all tokens on eight experts, 4, 173 / 131; tiles of 64:
+// uniform, 1.0, 340 / 378; skewed, 1.6, 225 / 215; 1.8, 300 / 260.  64 experts of 3072 / 1536, skewed, tiles of 32: 2.1, 104 /
+// 122, where few blocks leave the 128-row kernels a last wave.  To launch both costs some 7 us.
+struct Family {
+    uint32_t tile = 0;         // 0: no choice, this kernel takes the call
+    bool few = false;          // of the decode kernels
+    // For every warp on its own, the same for all; waits for the kernel that wrote the counts.
+    __device__ __forceinline__ bool leaves(const int32_t* masked_m, uint32_t groups, uint32_t max_m) const
+    {
+        if (tile == 0) return false;
+        ptx::grid_dependency_wait();
+        int balance = 0;
+        for (uint32_t g = threadIdx.x & 31u; g < groups; g += 32) {
+            const uint32_t rows = min(static_cast<uint32_t>(max(0, __ldg(masked_m + g))), max_m);
+            balance += static_cast<int>((rows + tile - 1) / tile * 2) - static_cast<int>((rows + 127) / 128 * (tile == 32 ? 5 : 3));
+        }
+        return (__reduce_add_sync(0xffffffffu, balance) <= 0) != few;
+    }
+};
+
 // Every role of a CTA owns a walker and calls next() with the same sequence of linear tile indices.
 template <uint32_t kBM, bool kMasked>
 struct TileWalker {

@@ -175,6 +175,7 @@ struct Params {
     uint32_t m, n, k;          // m: all rows of a / d (masked: groups * max_m)
     uint32_t group_m;
     uint32_t groups, max_m;    // masked layout only
+    gemm::Family family;       // masked layout only
     // SwiGLU-quantised output (kSwigluOut kernels): the workspace of the NEXT GEMM, whose K is n / 2
     uint8_t* out_a0;
     uint8_t* out_a1;
@@ -231,6 +232,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
                   const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_sfb, const Params p)
 {
     using C = Cfg<BK, kResidual, kGroup>;
+    if constexpr (kMasked)
+        if (p.family.leaves(p.layout, p.groups, p.max_m)) return;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem - ptx::smem_u32(smem_raw));
@@ -625,6 +628,8 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
                        const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_sfb, const Params p)
 {
     using C = PairCfg<BK, kResidual>;
+    if constexpr (kMasked)
+        if (p.family.leaves(p.layout, p.groups, p.max_m)) return;             // both CTAs of the pair see the same counts
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem - ptx::smem_u32(smem_raw));
@@ -1022,13 +1027,15 @@ int launch_gemm_split(const void* a, int64_t lda, const void* b, const void* sfb
     return masked_m != nullptr ? launch_for_layout<true>(c, p, residual, block_k) : launch_for_layout<false>(c, p, residual, block_k);
 }
 
-// The GEMM alone over activations the caller holds quantised (masked layout: E groups of max_m rows).
+// The GEMM alone over activations the caller holds quantised (masked layout: E groups of max_m rows).  rival_tile: the
+// decode kernels with that token tile are launched for the same call, see gemm::Family.
 int launch_gemm_split_quantized(const void* a0, const void* a1, const void* sfa, const void* b, const void* sfb, const float* gw,
                                 void* d, int64_t ldd, const int32_t* masked_m, int max_m, int N, int K, int E, bool residual,
                                 int block_k, int group_m, bool pdl, int num_sms, bool pair, void* out_a0, void* out_a1, void* out_sf,
-                                int32_t* status, cudaStream_t stream)
+                                int32_t* status, cudaStream_t stream, int rival_tile)
 {
     Params p;
+    p.family = gemm::Family{static_cast<uint32_t>(rival_tile), false};
     p.gw = gw;
     p.layout = masked_m;
     p.sfa = nullptr;

@@ -60,6 +60,7 @@ struct Params {
     __nv_bfloat16* d;
     int64_t ldd;
     uint32_t m, n, k, groups, max_m;
+    gemm::Family family;       // masked
     // SwiGLU-quantised output (gate/up-interleaved weight rows): the next GEMM's codes (rows, n / 4) and scale rows
     uint8_t* out_a0;
     uint8_t* out_a1;
@@ -112,6 +113,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
     // contiguous: all weight tiles of a token tile are neighbours; masked: the token tiles of an expert are, per weight tile
     const uint32_t num_kb = p.k / BK;
     gemm::TileWalker<T, kMasked> walk(p.layout, p.m, p.n, BW, kMasked ? 8 : 1, p.groups, p.max_m);
+    // this family is the one that is expected to stay: it leaves by finding no tile, its prologue has run ahead
+    if constexpr (kMasked)
+        if (p.family.leaves(p.layout, p.groups, p.max_m)) walk.groups = 0;
     gemm::Tile t;
     bool ok = true;
     ptx::ProbeAcc pa;
@@ -415,7 +419,7 @@ int launch_gemm_stream(const void* a, int64_t lda, const void* b, const void* sf
         });
         if (qrc) return qrc;
         const Params p{gw, m_indices, static_cast<__nv_bfloat16*>(d), ldd, static_cast<uint32_t>(M), static_cast<uint32_t>(N),
-                       static_cast<uint32_t>(K), 0u, 1u, nullptr, nullptr, nullptr, status};
+                       static_cast<uint32_t>(K), 0u, 1u, gemm::Family{}, nullptr, nullptr, nullptr, status};
         const Call c{a0, a1, sf, b, sfb, M, N, K, E, num_sms, pdl, stream};
         switch (token_tile) {
             case 16: return residual ? launch_contiguous<16, true>(c, p) : launch_contiguous<16, false>(c, p);
@@ -428,13 +432,15 @@ int launch_gemm_stream(const void* a, int64_t lda, const void* b, const void* sf
 }
 
 // Masked layout over quantised rows (both passes), token tiles of 32 or 64.  out_a0 != nullptr: gate/up-interleaved weights,
-// the output is the quantised SwiGLU activation; else BF16 rows in d.
+// the output is the quantised SwiGLU activation; else BF16 rows in d.  has_rival: the 128-row
+// kernels are launched for the same call, see gemm::Family.
 int launch_gemm_stream_quantized(const void* a0, const void* a1, const void* scale_rows, const void* b, const void* sfb, const float* gw,
                                  void* d, int64_t ldd, const int32_t* masked_m, int max_m, int N, int K, int E, int token_tile, void* out_a0,
-                                 void* out_a1, void* out_sf, bool pdl, int num_sms, int32_t* status, cudaStream_t stream)
+                                 void* out_a1, void* out_sf, bool pdl, int num_sms, int32_t* status, cudaStream_t stream, bool has_rival)
 {
     const Params p{gw, masked_m, static_cast<__nv_bfloat16*>(d), ldd, static_cast<uint32_t>(E * max_m), static_cast<uint32_t>(N),
-                   static_cast<uint32_t>(K), static_cast<uint32_t>(E), static_cast<uint32_t>(max_m), static_cast<uint8_t*>(out_a0),
+                   static_cast<uint32_t>(K), static_cast<uint32_t>(E), static_cast<uint32_t>(max_m),
+                   gemm::Family{has_rival ? static_cast<uint32_t>(token_tile) : 0u, true}, static_cast<uint8_t*>(out_a0),
                    static_cast<uint8_t*>(out_a1), static_cast<uint8_t*>(out_sf), status};
     const Call c{a0, a1, scale_rows, b, sfb, E * max_m, N, K, E, num_sms, pdl, stream};
     const bool swiglu = out_a0 != nullptr;

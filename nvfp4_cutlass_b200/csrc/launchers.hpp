@@ -24,7 +24,7 @@ int launch_gemm_split(const void* a, int64_t lda, const void* b, const void* sfb
 int launch_gemm_split_quantized(const void* a0, const void* a1, const void* sfa, const void* b, const void* sfb, const float* gw,
                                 void* d, int64_t ldd, const int32_t* masked_m, int max_m, int N, int K, int E, bool residual,
                                 int block_k, int group_m, bool pdl, int num_sms, bool pair, void* out_a0, void* out_a1, void* out_sf,
-                                int32_t* status, cudaStream_t stream);
+                                int32_t* status, cudaStream_t stream, int rival_tile = 0);
 
 int launch_debug_split_workspace(const void* a, int64_t lda, int M, int K, int policy, bool residual, bool swiglu, void* a0,
                                  void* a1, void* sfa, cudaStream_t stream);
@@ -49,7 +49,7 @@ int launch_dispatch_quantized_peer(const void* x, int64_t x_ld_bytes, int64_t to
                                    int64_t a1_off, int64_t sf_off, const int64_t* dst_rank, const int64_t* dst_row, int world,
                                    int64_t rows_cap, int32_t* status, int num_sms, cudaStream_t stream);
 int launch_relayout_scales(const void* sf_rows, const int32_t* masked_m, int max_m, int64_t rows, int kdim, void* atoms, bool pdl,
-                           cudaStream_t stream);
+                           cudaStream_t stream, int rival_tile = 0);
 int launch_combine_rows_peer(const int64_t* peers, int64_t rows_ld_elems, const int64_t* src_rank, const int64_t* src_row,
                              const float* w, int64_t tokens, int k, int hidden, void* y, int64_t y_ld_elems, int world,
                              int64_t rows_cap, int num_sms, bool bulk, int32_t* status, cudaStream_t stream);
@@ -63,7 +63,8 @@ int launch_gemm_stream(const void* a, int64_t lda, const void* b, const void* sf
                        int32_t* status, cudaStream_t stream);
 int launch_gemm_stream_quantized(const void* a0, const void* a1, const void* scale_rows, const void* b, const void* sfb, const float* gw,
                                  void* d, int64_t ldd, const int32_t* masked_m, int max_m, int N, int K, int E, int token_tile, void* out_a0,
-                                 void* out_a1, void* out_sf, bool pdl, int num_sms, int32_t* status, cudaStream_t stream);
+                                 void* out_a1, void* out_sf, bool pdl, int num_sms, int32_t* status, cudaStream_t stream,
+                                 bool has_rival = false);
 
 // expire_after_cycles > 0: the waits for the maxima are made to run out after so many cycles (a test's hook)
 int launch_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void* b, void* sfb, float* gw,

@@ -11,6 +11,7 @@
 
 #include <cstdint>
 
+#include "gemm_common.cuh"
 #include "host_common.hpp"
 #include "launchers.hpp"
 #include "transform.cuh"
@@ -202,14 +203,14 @@ dispatch_quantized_peer_kernel(const uint4* __restrict__ x, int64_t x_ld16, uint
 constexpr uint32_t kRelayoutAtoms = 8;
 __global__ void __launch_bounds__(256)
 relayout_scales_kernel(const uint8_t* __restrict__ sf_rows, const int32_t* __restrict__ masked_m, uint32_t max_m, uint32_t kdim, bool wide,
-                       uint8_t* __restrict__ atoms)
+                       uint8_t* __restrict__ atoms, uint32_t groups, gemm::Family family)
 {
     __shared__ __align__(16) uint32_t staged[kRelayoutAtoms][2][128];
     const uint32_t k64 = kdim / 64, chunks = (k64 + kRelayoutAtoms - 1) / kRelayoutAtoms;
     const uint32_t first = blockIdx.x % chunks * kRelayoutAtoms, here = min(kRelayoutAtoms, k64 - first);
     const uint64_t row0 = static_cast<uint64_t>(blockIdx.x / chunks) * 128;
     ptx::grid_dependency_wait();
-    if (masked_m == nullptr || row0 % max_m < min(static_cast<uint32_t>(max(0, __ldg(masked_m + row0 / max_m))), max_m)) {
+    if (masked_m == nullptr || (!family.leaves(masked_m, groups, max_m) && row0 % max_m < min(static_cast<uint32_t>(max(0, __ldg(masked_m + row0 / max_m))), max_m))) {
         const uint32_t r = threadIdx.x / 2, pass = threadIdx.x % 2, word = (r % 32) * 4 + r / 32;
         const uint8_t* src = sf_rows + (row0 + r) * (kdim / 8) + pass * (kdim / 16) + first * 4;
         if (wide) {
@@ -742,7 +743,7 @@ int launch_dispatch_quantized_peer(const void* x, int64_t x_ld_bytes, int64_t to
 }
 
 int launch_relayout_scales(const void* sf_rows, const int32_t* masked_m, int max_m, int64_t rows, int kdim, void* atoms, bool pdl,
-                           cudaStream_t stream)
+                           cudaStream_t stream, int rival_tile)
 {
     if (rows == 0) return NVFP4_OK;
     // whole chunks of atoms, every row piece on a 16-byte boundary
@@ -750,7 +751,8 @@ int launch_relayout_scales(const void* sf_rows, const int32_t* masked_m, int max
     const int64_t blocks = rows / 128 * ((kdim / 64 + kRelayoutAtoms - 1) / kRelayoutAtoms);
     return host::launch_kernel(relayout_scales_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, pdl,
                                static_cast<const uint8_t*>(sf_rows), masked_m, static_cast<uint32_t>(max_m > 0 ? max_m : 1),
-                               static_cast<uint32_t>(kdim), wide, static_cast<uint8_t*>(atoms));
+                               static_cast<uint32_t>(kdim), wide, static_cast<uint8_t*>(atoms),
+                               static_cast<uint32_t>(max_m > 0 ? rows / max_m : 0), gemm::Family{static_cast<uint32_t>(rival_tile), false});
 }
 
 }  // namespace nvfp4

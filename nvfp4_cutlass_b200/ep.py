@@ -353,11 +353,12 @@ class ExpertParallelMoE:
         return y.to(torch.bfloat16)
 
     def _few_rows_tile(self, pairs: int) -> int:
-        """Token tile of the decode kernel for this step, 0 for the 128-row kernels.  With a few rows per expert the weights
-        set the pace and most of a 128-row tile would be empty.  Only the average is known here, the real counts are on the
-        device; an expert with more rows than a tile has its weights read again, out of L2.  Measured on 128 experts,
-        4096 / 1536, per step: up to 24 rows on average 330 us with tiles of 32 against 437 with 128 rows, at
-        48 rows 384 us with tiles of 64 against 444, at 64 rows 540 against 447."""
+        """Token tile of the decode kernels for this step, 0 for the 128-row kernels alone.  With a few rows per expert the weights
+        set the pace and most of a 128-row tile would be empty.  Only an average is known here, and of other ranks' tokens not
+        even that; where the counts on the device say otherwise, the 128-row kernels take the step all the same (see
+        expert_mlp_few_rows).  Checked with routing near uniform, skewed, and onto k experts alone (128 experts 4096 / 1536 and 2048
+        / 768, 64 of 2048 / 1024, 16 of 4096 / 2048, 32 of 1024 / 512; 4 to 52 rows on average; the smaller ones are bound
+        by the host at 110-120 us whatever runs)."""
         if self.inter % 256 != 0:
             return 0
         rows = pairs * self.world
@@ -366,7 +367,9 @@ class ExpertParallelMoE:
                 return tile
         return 0
 
-    FEW_ROWS = ((26, 32), (52, 64))        # (rows per expert on average up to which the tile is taken, tile)
+    # (rows per expert on average up to which the tile is taken, tile).  128 experts, 4096 / 1536, near-uniform routing, one step,
+    # 128-row kernels / this: 24 rows 366 / 276 us, 32 rows 368 / 335, 48 rows 382 / 358, 52 rows 387 / 405
+    FEW_ROWS = ((26, 32), (48, 64))
 
     def _peer_step(self, buf: "PeerBuffers", x, topk_ids, topk_w, y, marks: Optional[list] = None, gemm_gate=None,
                    pairs: Optional[int] = None) -> None:
@@ -410,10 +413,9 @@ class ExpertParallelMoE:
             # `pairs`: one size for all parts of a step, so that all of them run the same kernels
             tile = self._few_rows_tile(topk_ids.numel() if pairs is None else pairs) if buf.hq is not None else 0
             if tile:
-                _C.m_grouped_few_quantized_rows_gemm_masked(buf.q, *self.up_interleaved, buf.hq, plan.masked_m, token_tile=tile,
-                                                            device_status=buf.status)
-                _C.m_grouped_few_quantized_rows_gemm_masked(buf.hq, *self.down, buf.out, plan.masked_m, token_tile=tile,
-                                                            device_status=buf.status)
+                # one rank's tokens give an expert a row each at most: with no more tokens than two tiles there is nothing to decide
+                _C.expert_mlp_few_rows(buf.q, self.up_interleaved, buf.hq, self.down, buf.out, plan.masked_m, token_tile=tile,
+                                       decide=self.world > 1 or x.shape[0] > 2 * tile, device_status=buf.status)
             elif buf.hq is not None:
                 _C.relayout_scales(buf.q, plan.masked_m)
                 _C.m_grouped_quantized_swiglu_dual_nvfp4_gemm_masked(buf.q, *self.up_interleaved, buf.hq, plan.masked_m,
@@ -441,8 +443,9 @@ class ExpertParallelMoE:
 
     def forward_peer(self, x: torch.Tensor, topk_ids: torch.Tensor, topk_w: torch.Tensor, marks: Optional[list] = None):
         """One step over peer memory.  With micro_batches > 1 the tokens are cut into that many parts, each with buffers
-        and a stream of its own, so that the NVLink traffic of one part runs under the GEMMs of another; every token's
-        result is the same whichever part it is in.  `marks`, if given, receives a CUDA event after each phase of the
+        and a stream of its own, so that the NVLink traffic of one part runs under the GEMMs of another; a token's result
+        does not depend on the part it is in, but for the low bits in steps with few rows per expert, where every part's row
+        counts choose between two kernels that add in different orders (_few_rows_tile).  `marks`, if given, receives a CUDA event after each phase of the
         (first) part: start, plan, dispatch, experts, combine."""
         tokens = x.shape[0]
         y = torch.empty(tokens, self.hidden, dtype=torch.bfloat16, device=x.device)

@@ -77,6 +77,67 @@ def test_masked_rows_match_the_128_row_kernels(k, inter, tile):
     assert rel_l2(out.view(-1, hidden)[live], ref.view(-1, hidden)[live]) < 4e-3
 
 
+@pytest.mark.parametrize("counts,tile,few", [([1, 0, 31, 33, 5], 32, True), ([256, 200, 0, 3, 128], 32, False), ([0, 0, 0, 0, 0], 32, True),
+                                             ([160, 0, 0, 0, 0], 32, True), ([161, 0, 0, 0, 0], 32, False), ([96, 64, 0, 0, 0], 32, True),
+                                             ([65, 1, 0, 0, 0], 64, True), ([65, 65, 0, 0, 0], 64, False)])
+def test_the_counts_decide_between_the_kernels(counts, tile, few):
+    """One of the two families takes the call, by the rule of gemm::Family (up to five token tiles of 32, or three of 64, to two blocks
+    of 128 rows the decode kernels): the output has that family's bits, and of the two forms of the activation's scales
+    only the one that the family writes is written."""
+    e, max_m, hidden, inter = 5, 256, 512, 256
+    up, down = weights(e, 2 * inter, hidden, 1), weights(e, hidden, inter, 2)
+    up = (*_C.interleave_gate_up(up[0], up[1], e, inter), up[2])
+    a = torch.randn(e * max_m, hidden, generator=torch.Generator().manual_seed(3)).to(torch.bfloat16).cuda()
+    masked_m = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def planes(width):
+        return _C.QuantizedRows(torch.zeros(e * max_m * (width + width // 8), dtype=torch.uint8, device="cuda"), e, max_m, width)
+
+    def outputs(call):
+        rows, h, out = planes(hidden), planes(inter), torch.zeros(e, max_m, hidden, dtype=torch.bfloat16, device="cuda")
+        a0, a1, sfa = _C.debug_split_workspace(a)
+        rows.a0.copy_(a0), rows.a1.copy_(a1)
+        rows.scale_rows.copy_(sfa.view(e * max_m // 128, hidden // 64, 2, 32, 4, 4).permute(0, 4, 3, 2, 1, 5).reshape(rows.scale_rows.shape))
+        call(rows, h, out)
+        assert _C.read_status(status) == 0
+        return torch.cat([out[i, :c] for i, c in enumerate(counts)]), bool(h.scale_rows.any()), bool(h.scale_atoms.any())
+
+    def by_decode(rows, h, out):
+        _C.m_grouped_few_quantized_rows_gemm_masked(rows, *up, h, masked_m, token_tile=tile, device_status=status)
+        _C.m_grouped_few_quantized_rows_gemm_masked(h, *down, out, masked_m, token_tile=tile, device_status=status)
+
+    def by_128_rows(rows, h, out):
+        _C.relayout_scales(rows, masked_m)
+        _C.m_grouped_quantized_swiglu_dual_nvfp4_gemm_masked(rows, *up, h, masked_m, device_status=status)
+        _C.m_grouped_quantized_dual_nvfp4_gemm_masked(h, *down, out, masked_m, device_status=status)
+
+    either = lambda decide: lambda rows, h, out: _C.expert_mlp_few_rows(rows, up, h, down, out, masked_m, token_tile=tile, decide=decide,
+                                                                       device_status=status)
+    want, live = {True: outputs(by_decode)[0], False: outputs(by_128_rows)[0]}, sum(counts) > 0
+    y, as_rows, as_atoms = outputs(either(True))
+    assert torch.equal(y, want[few]) and (as_rows, as_atoms) == (few and live, not few and live)
+    y, as_rows, as_atoms = outputs(either(False))
+    assert torch.equal(y, want[True]) and (as_rows, as_atoms) == (live, False)
+
+
+def test_layer_with_all_tokens_on_a_few_experts_runs_the_128_row_kernels():
+    e, hidden, inter, tokens, k = 32, 1024, 256, 200, 4
+    up, down = weights(e, 2 * inter, hidden, 5), weights(e, hidden, inter, 6)
+    g = torch.Generator().manual_seed(8)
+    x = torch.randn(tokens, hidden, generator=g).to(torch.bfloat16).cuda()
+    uniform = torch.randn(tokens, e, generator=g).cuda()
+    skewed = uniform + 50.0 * (torch.arange(e, device="cuda") < k)
+    layer, other = (ExpertParallelMoE(e, hidden, inter, up, down, peer_rows_cap=256) for _ in range(2))
+    other.FEW_ROWS = ()
+    for logits, by_128_rows in ((uniform, False), (skewed, True)):
+        ids, w = route_topk(logits, k)
+        assert layer._few_rows_tile(ids.numel()) == 32
+        y, want = layer(x, ids, w), other(x, ids, w)
+        assert bool(layer.peer[0].hq.scale_atoms.any()) == by_128_rows         # only those kernels write them
+        assert torch.equal(y, want) if by_128_rows else rel_l2(y, want) < 4e-3
+
+
 def test_layer_of_few_tokens_matches_the_bf16_dispatch():
     e, hidden, inter, tokens, k = 16, 1024, 256, 40, 4
     up, down = weights(e, 2 * inter, hidden, 5), weights(e, hidden, inter, 6)
