@@ -37,6 +37,85 @@ def test_contiguous_matches_oracle(oracle, align, n, k, residual):
     assert rel_l2(d, want) < 2.5e-3
 
 
+POLICIES = ["derived_div8", "residual_amax", "derived_div4", "div4_radix8"]
+
+
+@pytest.mark.parametrize("policy", POLICIES)
+@pytest.mark.parametrize("align,n,k,residual", [(16, 256, 768, True), (32, 384, 1024, False), (64, 128, 512, True)])
+def test_policies_and_row_strides(oracle, policy, align, n, k, residual):
+    """The quantisation pass in all its scale policies, activations and output as column ranges of wider tensors."""
+    sizes = [2 * align, align, 0, align]
+    m = sum(sizes)
+    b, sfb, gw = weights(len(sizes), n, k, n + k)
+    mi = nvfp4_gemm.make_m_indices(sizes, alignment=align)
+    wide = torch.randn(m, k + 72, generator=torch.Generator().manual_seed(k)).to(torch.bfloat16)
+    a, d = wide.cuda()[:, 24:24 + k], torch.full((m, n + 40), 7.0, dtype=torch.bfloat16, device="cuda")
+    nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(a, b, sfb, gw, d[:, 16:16 + n], mi.cuda(), policy, residual, m_alignment=align,
+                                                         tune_swap_ab=1, tune_split_transform=1)
+    want = oracle.grouped_gemm(wide[:, 24:24 + k].contiguous(), b.cpu(), sfb.cpu(), gw.cpu(), mi, n, mode="dual" if residual else "single",
+                               scale_policy=policy)
+    assert rel_l2(d[:, 16:16 + n], want) < 2.5e-3                          # as above
+    assert bool((d[:, :16] == 7.0).all()) and bool((d[:, 16 + n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("align,tiles,n,k", [(16, 256, 4096, 1792), (32, 4, 6400, 4608), (64, 4, 4096, 3584), (16, 8, 640, 1024), (64, 2, 640, 1024)])
+@pytest.mark.parametrize("policy", ["derived_div8", "div4_radix8"])
+def test_the_default_is_one_of_the_two_paths(align, tiles, n, k, policy):
+    """Calls on either side of the limits from which the library takes this path by itself: both paths sum every pass in ascending K
+    and add the two at the end, so whichever it is, the bits are the same."""
+    experts = min(4, tiles)
+    b, sfb, gw = weights(experts, n, k, 3)
+    mi = nvfp4_gemm.make_m_indices([tiles // experts * align] * experts, alignment=align).cuda()
+    a = torch.randn(tiles * align, k, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).cuda()
+    d = torch.full((3, tiles * align, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    for split in range(3):
+        nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(a, b, sfb, gw, d[split], mi, policy, m_alignment=align, tune_swap_ab=1,
+                                                             tune_split_transform=split)
+    assert bool(torch.isfinite(d[0].float()).all()) and torch.equal(d[0], d[1]) and torch.equal(d[0], d[2])
+
+
+def test_workspace_under_capture_and_on_two_streams():
+    """The quantisation pass takes its workspace from a pool in stream order: inside a captured graph that is replayed with other
+    activations, and with calls in flight on two streams."""
+    align, n, k, sizes = 32, 512, 1024, [64, 32, 0, 96]
+    m = sum(sizes)
+    b, sfb, gw = weights(len(sizes), n, k, 4)
+    mi = nvfp4_gemm.make_m_indices(sizes, alignment=align).cuda()
+    inputs = [torch.randn(m, k, generator=torch.Generator().manual_seed(i)).to(torch.bfloat16).cuda() for i in range(2)]
+
+    def call(a, d, split=1):
+        nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(a, b, sfb, gw, d, mi, m_alignment=align, tune_swap_ab=1, tune_split_transform=split)
+
+    want = [torch.zeros(m, n, dtype=torch.bfloat16, device="cuda") for _ in inputs]
+    for a, d in zip(inputs, want):
+        call(a, d, split=2)                              # without a workspace
+    a, d = inputs[0].clone(), torch.zeros(m, n, dtype=torch.bfloat16, device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call(a, d)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(a, d)
+        call(a, d)
+    for i in (1, 0, 1):
+        a.copy_(inputs[i])
+        d.zero_()
+        graph.replay()
+        assert torch.equal(d, want[i])
+    streams, outs = [torch.cuda.Stream(), torch.cuda.Stream()], [torch.zeros(20, m, n, dtype=torch.bfloat16, device="cuda") for _ in inputs]
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+    for i in range(20):
+        for s, a, d in zip(streams, inputs, outs):
+            with torch.cuda.stream(s):
+                call(a, d[i])
+    torch.cuda.synchronize()
+    for d, w in zip(outs, want):
+        assert bool((d == w).all())
+
+
 @pytest.mark.parametrize("k,inter,tile", [(1024, 256, 32), (256, 512, 32), (512, 256, 64)])
 def test_masked_rows_match_the_128_row_kernels(k, inter, tile):
     e, max_m, hidden, counts = 5, 256, 512, [1, 0, tile - 1, tile + 1, 256]
@@ -68,8 +147,9 @@ def test_masked_rows_match_the_128_row_kernels(k, inter, tile):
     assert _C.read_status(status) == 0
     atoms = hw.scale_atoms.view(e * max_m // 128, inter // 64, 2, 32, 4, 4).permute(0, 4, 3, 2, 1, 5).reshape(hq.scale_rows.shape)
     for x, y in ((hq.a0, hw.a0), (hq.a1, hw.a1), (hq.scale_rows, atoms)):
-        # a gate or up value at a BF16 tie moves its product by an ulp and perhaps a code; residual codes see every ulp
-        assert float((x[live] != y[live]).float().mean()) < 0.02
+        # an FP32 sum in another order is off by some 2^-20 of its value at most, so one gate or up value in 2^12 crosses a BF16
+        # rounding boundary and moves its product by an ulp, which the residual code sees: one byte of two codes in 2^10
+        assert float((x[live] != y[live]).float().mean()) < 0.002
     out, ref = (torch.zeros(e, max_m, hidden, dtype=torch.bfloat16, device="cuda") for _ in range(2))
     _C.m_grouped_few_quantized_rows_gemm_masked(hq, *down, out, masked_m, token_tile=tile, device_status=status)
     _C.m_grouped_quantized_dual_nvfp4_gemm_masked(hw, *down, ref, masked_m, device_status=status)
