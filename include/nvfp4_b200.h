@@ -117,7 +117,8 @@ NVFP4_API int nvfp4_quantize_weight_static(const void* w, int w_dtype, int E, in
  *              [13] split_transform.  NOTE [13] means something else than in the reference (there:
  *              signal A0 early inside its one kernel): here 1 = quantise the activations once in a
  *              kernel of their own ahead of the GEMM, 2 = Algorithm 1 inside the GEMM main loop,
- *              0 = the library's choice; both orientations.  All other knobs (epilogue_threads, num_stages,
+ *              0 = the library's choice.  Normal orientation: other values are refused, and 1 unless N % 256 == 0.
+ *              Swap-AB: 1 has no effect unless K % 256 == 0 and [5] is 0, other values count as 0.  All other knobs (epilogue_threads, num_stages,
  *              swizzle_cd, epilogue_stages, l2_pin_weights, timing_probe, tail_split,
  *              shallow_stages, produced_stages, a token tile of 128) are accepted and ignored.
  *   device_status optional device int32 the kernel ORs error bits into (bit 0 =

@@ -281,8 +281,8 @@ int nvfp4_grouped_gemm_contiguous(const void* a, int64_t lda_elems, const void* 
         const int tune_block_k = tune ? tune[5] : 0;   // 0 = the largest of 512 / 256 / 128 that divides K and fits
         NVFP4_REQUIRE(tune_block_k == 0 || tune_block_k == 128 || tune_block_k == 256 || tune_block_k == 512,
                       "tune_block_k must be 0, 128, 256 or 512");
-        // tune_split_transform as in the normal orientation: 1 = activations quantised in a pass of their own, 2 = in the
-        // main loop, 0 = the library's choice
+        // tune_split_transform as in the normal orientation: 1 = activations quantised in a pass of their own (where K % 256 == 0
+        // and no K block is asked for, else it has no effect), 2 = in the main loop, anything else = the library's choice
         const int tune_split = tune ? tune[13] : 0;
         const double weight_bytes = static_cast<double>(M / tile) * N * K * (9.0 / 16.0);
         if (K % 256 == 0 && tune_block_k == 0 && tune_split != 2 && (tune_split == 1 || weight_bytes >= stream_weight_bytes(tile)))
@@ -296,7 +296,7 @@ int nvfp4_grouped_gemm_contiguous(const void* a, int64_t lda_elems, const void* 
     // tune_cluster: 2 / 4 = that many CTAs share one transformed activation tile (needs N % (256 * cluster) == 0),
     // 1 = single-CTA kernel, 0 = the library's choice
     // tune_split_transform: 1 = quantise the activations once, in a kernel of their own, ahead of a GEMM without
-    // transform warps (N % 256 == 0); 2 = decompose inside the GEMM main loop; 0 = the library's choice.  (In the
+    // transform warps (N % 256 == 0 when it is asked for; by its own choice the library also takes it for other N); 2 = decompose inside the GEMM main loop; 0 = the library's choice.  (In the
     // reference this keyword signals A0 readiness early inside its one kernel; here it chooses between the two paths.)
     const int tune_split = tune ? tune[13] : 0;
     const bool pdl = !(tune && tune[11]);                           // tune_no_pdl
@@ -309,7 +309,8 @@ int nvfp4_grouped_gemm_contiguous(const void* a, int64_t lda_elems, const void* 
     const bool fused_knobs = tune && (tune[8] != 0 || tune[1] != 0 || tune[9] != 0);
     // Where no cluster fits (N % 512 != 0) the single-CTA fused kernel transforms an activation tile per 128 or 256 columns
     // and the separate pass wins from N = 640 on, even with half a column tile of padding: 32 experts x 256
-    // rows, K = 2048: N = 640 56 / 31 us, N = 768 53 / 37; 8 x 512 rows, N = 14464, K = 4096: 939 / 207.
+    // rows, K = 2048: N = 640 56 / 31 us, N = 768 53 / 37; 8 x 512 rows, N = 14464, K = 4096: 939 / 207.  (Where both take
+    // little more than a launch it costs one launch more: N = 768, K <= 1024, up to 4k rows 13.5 / 14.5 us.)
     if (tune_split == 1 || (tune_split == 0 && !fused_knobs && (N > 1024 || (N % 512 != 0 && N > 512)))) {
         const int tune_block_k = tune ? tune[5] : 0;
         return launch_gemm_split(a, lda_elems, b, sfb, gw, d, ldd_elems, m_indices, nullptr, 0, M, N, K, E,

@@ -287,7 +287,7 @@ gemm_normal_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             if (!ptx::all_lanes(ptx::mbar_wait(tmem_full, acc_phase, abort_flag, pa, 0))) { give_up(1); break; }
             ptx::tcgen05_fence_after_sync();
             // 64 columns at a time: tensor memory -> registers -> x G_W -> BF16 -> four whole 128-byte lines per store
-            // instruction through the warp's staging area; the accumulator goes back to the MMA warp as soon as this
+            // instruction (gemm::store_rows); the accumulator goes back to the MMA warp as soon as this
             // warp's last columns are in registers, so the stores of the tail run under the next tile's main loop
             __nv_bfloat16* d_lane = p.d + static_cast<int64_t>(m_blk * BM + quad * 32 + (lane & 24u)) * p.ldd + n_blk * BN + (lane & 7u) * 8;
 #pragma unroll 1

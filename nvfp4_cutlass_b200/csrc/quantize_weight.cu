@@ -1,8 +1,9 @@
 // Offline NVFP4 weight quantisation on the GPU: w ~= dec(q) * S * G with one FP32 G
 // per expert, one E4M3 S per 16 elements and E2M1 codes, written straight into the
 // physical layouts the GEMM's tensor maps describe.  Bit-exact with the reference's
-// torch implementation (python/nvfp4_gemm/layout.py:68-127): the same three true
-// FP32 divisions, the same clamps, RNE everywhere.
+// torch implementation (python/nvfp4_gemm/layout.py:68-127): the codes and scales of
+// its three FP32 divisions (kept reciprocals where they round alike, see `divide`), the
+// same clamps, RNE everywhere.
 //
 // HBM-bound: 2 or 4 bytes read per element, 9/16 byte written.  G needs the maximum of a whole expert before any of its
 // blocks can be quantised, so the weights are read twice; the second read should come out of L2.  The experts are
@@ -12,7 +13,9 @@
 // so whatever number of blocks runs at a time, the ones that are waited for are running or done.
 // Measured (BF16): 8 experts of 4096 x 7168 (58 MB each, too large for two of them to share L2) 176 us = 1.07 GB of traffic at
 // 6.1 TB/s, before 1000 us (a scalar load per element, 40 instructions per element, an atomic per warp on one word);
-// 32 of 4096 x 1536: 128 us = 4.1 TB/s of 400 MB read and 113 MB written once, the rest is the warps' latency.
+// 32 of 4096 x 1536: 128 us = 4.1 TB/s of 400 MB read and 113 MB written once, the rest is the warps' latency.  Every tile
+// finds its stage by walking the stages before it, a batch each: with 256 batches (4096 x 2048, 2.86 ms, 1.9 TB/s) that is what
+// the kernel spends its time on; 64 (4096 x 7168) 3.3 TB/s, 1024 experts in 22 batches (256 x 1024) 4.1.
 #include <climits>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -407,8 +410,8 @@ int launch_quantize_weight(const void* w, int w_dtype, int E, int N, int K, void
 }
 
 // ---- allocation-free variant ----------------------------------------------------------
-// Same two kernels, but the per-expert maxima are staged in a fixed array that is part of
-// the library image instead of an allocation.  Every process that loads the library holds
+// The same kernel, but its scratch words are a fixed array that is part of the library
+// image instead of an allocation.  Every process that loads the library holds
 // scratch_words(NVFP4_STATIC_MAX_EXPERTS) words of it on every GPU it uses, until it exits.
 namespace {
 static __device__ __align__(256) uint32_t g_static_amax[scratch_words(NVFP4_STATIC_MAX_EXPERTS)];
@@ -437,7 +440,7 @@ int launch_quantize_weight_static(const void* w, int w_dtype, int E, int N, int 
         }
         amax_bits = scratch_addr[dev];
     }
-    // the array keeps whatever the previous call left in it: run_quantize_weight clears the maxima first
+    // the array keeps whatever the previous call left in it: run_quantize_weight clears its words first
     return run_quantize_weight(w, w_dtype, E, N, K, b, sfb, gw, amax_bits, stream);
 }
 
