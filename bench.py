@@ -59,10 +59,11 @@ WORKLOADS = {
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of ONE launch from the ncu captures summarised
 # under profiles/, on the reduced workloads c2s / c4s (the full ones exceed what a multi-pass capture should
-# hold), as (bytes measured, algorithmic bytes of that captured launch).  Both kernels stream every operand
+# hold), as (bytes measured, algorithmic bytes of that captured launch).  The kernels stream every operand
 # once, so traffic grows in proportion to the algorithmic bytes; a full launch is scaled by that ratio.
-NCU_TRAFFIC = {"normal": (246.45e6, 251.66e6, "split-path kernels (CTA-pair GEMM) on c2s, captured at commit 253fbe0"),
-               "swap_ab": (925.44e6, 911.22e6, "decode kernel on c4s, captured at commit 70bfc9c")}
+NCU_TRAFFIC = {"normal": (248.42e6, 251.66e6, "split-path kernels (CTA-pair GEMM) on c2s, captured at commit 458d43e"),
+               "swap_ab": (928.61e6, 911.22e6, "gemm_swap_kernel on c4s, captured at commit 458d43e"),
+               "swap_ab_split": (933.38e6, 911.22e6, "stream_quantize_kernel + gemm_stream_kernel on c4s, captured at commit 458d43e")}
 
 
 def scaled_traffic(orientation: str, algo_bytes: float) -> dict:
@@ -418,10 +419,13 @@ def measure_fp4_peak_sustained(seconds: float = 0.25):
 
 
 def split_default(case, extra) -> bool:
-    """Whether the dispatcher (csrc/abi.cu) sends this call to the two-kernel split path."""
+    """Whether the dispatcher (csrc/abi.cu) sends this call to a two-kernel path: activations quantised in a pass of their own."""
+    mode, N = extra.get("tune_split_transform", 0), case["N"]
+    if case["swap"]:                                       # token tiles of 16 rows: from 1 GB of weights per call
+        return case["K"] % 256 == 0 and extra.get("tune_block_k", 0) == 0 and mode != 2 and \
+            (mode == 1 or case["M"] // 16 * N * case["K"] * 9 / 16 >= 1e9)
     fused_knobs = any(extra.get(k, 0) for k in ("tune_cluster", "tune_transform_warps", "tune_direct_a"))
-    mode = extra.get("tune_split_transform", 0)
-    return (not case["swap"]) and case["N"] % 256 == 0 and (mode == 1 or (mode == 0 and not fused_knobs and case["N"] > 1024))
+    return mode == 1 or (mode == 0 and not fused_knobs and (N > 1024 or (N % 512 != 0 and N > 512)))
 
 
 def gemm_record(case, dev, steps, warmup, fp4_peak, graph=False, extra=None, sample_clocks=True, local=0):
@@ -452,7 +456,7 @@ def gemm_record(case, dev, steps, warmup, fp4_peak, graph=False, extra=None, sam
                       2 * case["real_rows"] * N + 4 * case["E"] + 4 * M)
         achieved = algo_bytes / (ms * 1e-3) / 1e9
         roofline = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
-                    "frac": achieved / pk["hbm_gbs"], **scaled_traffic("swap_ab", algo_bytes), "peak_source": pk["source"],
+                    "frac": achieved / pk["hbm_gbs"], **scaled_traffic("swap_ab_split" if split_default(case, extra) else "swap_ab", algo_bytes), "peak_source": pk["source"],
                     "algorithmic_bytes_per_launch": algo_bytes}
     else:
         achieved = 2.0 * logical / (ms * 1e-3) / 1e12       # both NVFP4 passes run on the tensor pipe
@@ -472,8 +476,7 @@ def gemm_record(case, dev, steps, warmup, fp4_peak, graph=False, extra=None, sam
 
 def north_star_record(case, dev, steps, fp4_peak, graph=False):
     """The path the project is named for -- Algorithm 1 inside the GEMM main loop, nothing quantised written to
-    global memory -- on this workload: the fused cluster kernel for the normal orientation (the decode kernel
-    always decomposes in its main loop)."""
+    global memory -- on this workload: the fused cluster kernel for the normal orientation, gemm_swap_kernel for decode."""
     rec, _, _ = gemm_record(case, dev, steps, 3, fp4_peak, graph=graph, extra=dict(tune_split_transform=2), sample_clocks=False)
     return {"ms_per_step": rec["ms_per_step"], "steps": rec["steps"], "value": rec["value"], "unit": "TFLOP/s", "frac": rec["frac"],
             "rel_l2_vs_fp32": rec["rel_l2_vs_fp32"], "cosine_vs_fp32": rec["cosine_vs_fp32"], "kernels_per_step": 1,
@@ -590,7 +593,8 @@ def single_gpu_line(workload, dev, local, steps, warmup, extra, graph=False, cpu
     pair = case["kw"].get("m_alignment") == 256 or extra.get("tune_cluster") == 2 or case["M"] // case["E"] >= 2048
     if extra.get("tune_cluster") == 1:
         pair = False
-    path = ("split: quantize_activation_kernel (Algorithm 1 once per element, into an L2-resident workspace) + " +
+    path = "decode: stream_quantize_kernel (Algorithm 1 once per element) + gemm_stream_kernel" if is_split and case["swap"] else \
+           ("split: quantize_activation_kernel (Algorithm 1 once per element, into an L2-resident workspace) + " +
             ("gemm_split_pair_kernel (block-scaled FP4 GEMM, CTA pairs: tcgen05.mma.cta_group::2 over 256 rows x 256 columns; "
              "the call states m_alignment=256)" if pair else "gemm_split_kernel (block-scaled FP4 GEMM)")) if is_split else (
             "decode: gemm_swap_kernel, Algorithm 1 in the main loop" if case["swap"] else

@@ -231,7 +231,9 @@ static bool split_gemm_as_pair(const int32_t* tune, int64_t rows, int experts, b
 // Bytes of weights per decode call (each token tile streams N x K of them) from which its activations get a pass of their own.
 // The pass costs a launch, some 3 us; what it saves is Algorithm 1 on a token tile once per 128 weight rows, which is the
 // more the larger the tile.  Measured, in the main loop / in a pass of its own: 64-token tiles, 151 MB: 79 / 40 us; 32-token
-// tiles, 302 MB: 76 / 58 us, 19 MB: 22 / 25; 16-token tiles, 264 MB: 54 / 57 us, 3.7 GB: 675 / 582.
+// tiles, 302 MB: 76 / 58 us, 19 MB: 22 / 25; 16-token tiles, 264 MB: 54 / 57 us, 3.7 GB: 675 / 582.  Checked on sixty calls of
+// 1 to 920 MB (5 to 248 experts, N up to 6656, K up to 5632, one and two passes): nowhere slower than the main loop by more than
+// 3 %.  With 16-token tiles either side wins between 60 MB and 1 GB (365 MB: 60 / 64; 329 MB: 75 / 59; 922 MB: 200 / 157).
 static double stream_weight_bytes(int token_tile) { return token_tile == 16 ? 1e9 : (token_tile == 32 ? 64e6 : 32e6); }
 
 int nvfp4_grouped_gemm_contiguous(const void* a, int64_t lda_elems, const void* b, const void* sfb, const float* gw,

@@ -11,8 +11,8 @@
 // which the quantisation of batch i - 1, which sits in L2, is interleaved with the maxima of batch i, which streams in
 // from HBM.  Blocks draw tiles from a counter in list order and a quantisation tile waits only for tiles ahead of it,
 // so whatever number of blocks runs at a time, the ones that are waited for are running or done.
-// Measured (BF16): 8 experts of 4096 x 7168 (58 MB each, too large for two of them to share L2) 176 us = 1.07 GB of traffic at
-// 6.1 TB/s, before 1000 us (a scalar load per element, 40 instructions per element, an atomic per warp on one word);
+// Measured (BF16): 8 experts of 4096 x 7168 (58 MB each, too large for two of them to share L2) 177-185 us; the
+// weights cross HBM 1.8 times, 0.94 GB of DRAM traffic in all at 5.5 TB/s; before 1000 us (a scalar load per element, 40 instructions per element, an atomic per warp on one word);
 // 32 of 4096 x 1536: 128 us = 4.1 TB/s of 400 MB read and 113 MB written once, the rest is the warps' latency.  Every tile
 // finds its stage by walking the stages before it, a batch each: with 256 batches (4096 x 2048, 2.86 ms, 1.9 TB/s) that is what
 // the kernel spends its time on; 64 (4096 x 7168) 3.3 TB/s, 1024 experts in 22 batches (256 x 1024) 4.1.
