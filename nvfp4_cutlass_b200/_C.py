@@ -11,12 +11,16 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 import torch
 
 _LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libnvfp4_b200.so")
+_BINDING_PATH = os.path.join(os.path.dirname(_LIB_PATH), "_binding.so")
 _lib = None
+_contiguous_call = None        # binding.cpp's form of the contiguous GEMM call, once the library is loaded
 
 POLICY_CODES = {"derived_div8": 0, "residual_amax": 1, "derived_div4": 2, "div4_radix8": 3}
 
@@ -43,12 +47,13 @@ def library_path() -> str:
 
 def lib() -> ctypes.CDLL:
     """The loaded shared library; raises if it has not been built."""
-    global _lib
+    global _lib, _contiguous_call
     if _lib is None:
-        if not os.path.exists(_LIB_PATH):
-            raise RuntimeError(
-                f"{_LIB_PATH} is missing: build it with `python nvfp4_cutlass_b200/csrc/build.py` "
-                "(there is no fallback path)")
+        for path in (_LIB_PATH, _BINDING_PATH):
+            if not os.path.exists(path):
+                raise RuntimeError(
+                    f"{path} is missing: build it with `python nvfp4_cutlass_b200/csrc/build.py` "
+                    "(there is no fallback path)")
         L = ctypes.CDLL(_LIB_PATH)
         vp, i32, i64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
         L.nvfp4_last_error.restype = ctypes.c_char_p
@@ -84,7 +89,11 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_debug_mma_peak.argtypes = [i32, ctypes.POINTER(ctypes.c_double), vp]
         L.nvfp4_debug_mma_peak_pair.argtypes = [i32, ctypes.POINTER(ctypes.c_double), vp]
         L.nvfp4_debug_mma_pattern.argtypes = [i32, i32, i32, i32, i32, ctypes.POINTER(ctypes.c_double), vp]
-        _lib = L
+        loader = importlib.machinery.ExtensionFileLoader("_binding", _BINDING_PATH)
+        binding = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_binding", _BINDING_PATH, loader=loader))
+        loader.exec_module(binding)
+        binding.bind(ctypes.cast(L.nvfp4_grouped_gemm_contiguous, vp).value)
+        _lib, _contiguous_call = L, binding.contiguous
     return _lib
 
 
@@ -157,19 +166,7 @@ def set_probe_buffer(t=None) -> None:
 
 
 def _contiguous_device(a, b, sfb, gw, d, m_indices, device_status) -> int:
-    """Index of the operands' device; raises if they do not fit together.  The first expression is the whole list of
-    conditions for an ordinary call (a launch-bound one spends a third of its time here); whatever fails it goes through
-    the conditions one by one, which accept a little more and name the one that does not hold."""
-    index = a.get_device()
-    if a.dtype == d.dtype == torch.bfloat16 and b.dtype == torch.int8 and sfb.dtype == m_indices.dtype == torch.int32 and \
-            gw.dtype == torch.float32 and a.dim() == d.dim() == b.dim() == sfb.dim() == 2 and m_indices.dim() == 1 and \
-            device_status is None and \
-            index == b.get_device() == sfb.get_device() == gw.get_device() == d.get_device() == m_indices.get_device() >= 0 and \
-            b.is_contiguous() and sfb.is_contiguous() and gw.is_contiguous() and m_indices.is_contiguous() and \
-            a.stride(1) == d.stride(1) == 1 and a.is_cuda:
-        (m, k), (rows, n), e = a.shape, d.shape, gw.numel()
-        if rows == m and m_indices.shape[0] == m and b.shape == (e * n, k // 2) and sfb.shape == (e * (k // 64), n):
-            return index
+    """Index of the operands' device; raises if they do not fit together."""
     _require(a.dtype == torch.bfloat16, "a.dtype == bfloat16")
     _require(d.dtype == torch.bfloat16, "d.dtype == bfloat16")
     _require(b.dtype == torch.int8, "b.dtype == int8")
@@ -201,6 +198,16 @@ def m_grouped_bf16_dual_nvfp4_gemm_contiguous(a, b, sfb, gw, d, m_indices, scale
     """d = (A0 + A1) @ W^T * gw per expert group; same contract as the reference entry
     (src/api.hpp:26-144): dtype / shape assertions first, then a silent return for
     M == 0 or N == 0, then an asynchronous launch on the current stream."""
+    # An ordinary call goes through binding.cpp, which answers None to whatever is not one.
+    if device_status is None and scale_policy in POLICY_CODES and (not tune or (len(tune) == 1 and "tune_swap_ab" in tune)):
+        if _lib is None:
+            lib()
+        rc = _contiguous_call(a, b, sfb, gw, d, m_indices, POLICY_CODES[scale_policy], 1 if enable_residual_pass else 0,
+                              1 if tune and int(tune["tune_swap_ab"]) != 0 else 0, m_alignment)
+        if rc is not None:
+            if rc:
+                _check(rc)
+            return
     for key in tune:
         if key not in TUNE_KEYS:
             raise TypeError(f"m_grouped_bf16_dual_nvfp4_gemm_contiguous() got an unexpected keyword argument {key!r}")

@@ -4,13 +4,15 @@
 
 Each .cu is compiled to an object with nvcc, then linked into one shared library
 next to the Python package (nvfp4_cutlass_b200/lib/libnvfp4_b200.so).  Objects are
-rebuilt only when a source or header is newer.
+rebuilt only when a source or header is newer.  binding.cpp becomes a CPython module
+beside it (lib/_binding.so), compiled with g++ against torch's headers.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -18,8 +20,10 @@ PKG = os.path.dirname(HERE)
 OUT_DIR = os.path.join(PKG, "lib")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(OUT_DIR, "libnvfp4_b200.so")
+BINDING = os.path.join(OUT_DIR, "_binding.so")
 SOURCES = ["abi.cu", "gemm_normal.cu", "gemm_cluster.cu", "gemm_split.cu", "gemm_swap.cu", "gemm_stream.cu", "moe_glue.cu", "quantize_weight.cu", "checkpoint_loader.cu", "debug_kernels.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+HEADER = os.path.join(os.path.dirname(PKG), "include", "nvfp4_b200.h")
 FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
          "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr",
          "-ccbin", "/usr/bin/g++"]
@@ -27,8 +31,18 @@ FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-li
 
 def _newest_header() -> float:
     hdrs = [os.path.join(HERE, f) for f in os.listdir(HERE) if f.endswith((".cuh", ".hpp"))]
-    hdrs.append(os.path.join(os.path.dirname(PKG), "include", "nvfp4_b200.h"))
+    hdrs.append(HEADER)
     return max(os.path.getmtime(h) for h in hdrs)
+
+
+def _binding_command() -> list:
+    from torch.utils import cpp_extension
+
+    include = [f"-I{d}" for d in (*cpp_extension.include_paths(), sysconfig.get_paths()["include"],
+                                  os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"))]
+    libs = [f"-L{d}" for d in cpp_extension.library_paths()]      # loaded by torch before the module is imported
+    return ["/usr/bin/g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", *include, *libs,
+            os.path.join(HERE, "binding.cpp"), "-o", BINDING, "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -42,20 +56,25 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if force or not os.path.exists(o) or os.path.getmtime(o) < max(os.path.getmtime(s), hdr_time):
             jobs.append((s, o))
 
+    link = bool(jobs) or not os.path.exists(LIB)
+    binding = os.path.join(HERE, "binding.cpp")
+    if force or not os.path.exists(BINDING) or os.path.getmtime(BINDING) < max(os.path.getmtime(binding), os.path.getmtime(HEADER)):
+        jobs.append((binding, BINDING))
+
     def compile_one(job):
         s, o = job
-        cmd = [NVCC, *FLAGS, *( ["-Xptxas", "-v"] if verbose else []), "-c", s, "-o", o]
+        cmd = _binding_command() if s.endswith(".cpp") else [NVCC, *FLAGS, *( ["-Xptxas", "-v"] if verbose else []), "-c", s, "-o", o]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError(f"nvcc failed on {s}:\n{r.stdout}\n{r.stderr}")
+            raise RuntimeError(f"{cmd[0]} failed on {s}:\n{r.stdout}\n{r.stderr}")
         return r.stderr
 
-    with ThreadPoolExecutor(max_workers=len(SOURCES)) as ex:
+    with ThreadPoolExecutor(max_workers=len(SOURCES) + 1) as ex:
         for log in ex.map(compile_one, jobs):
             if verbose and log:
                 print(log)
     objs = [os.path.join(OBJ_DIR, s.replace(".cu", ".o")) for s in SOURCES]
-    if jobs or not os.path.exists(LIB):
+    if link:
         cmd = [NVCC, "-shared", "-o", LIB, *objs, "-ccbin", "/usr/bin/g++", "-Xlinker", "--exclude-libs,ALL"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:

@@ -1,0 +1,99 @@
+"""The CPython form of the contiguous call (csrc/binding.cpp): what it does not take goes the general way, with that way's errors, and
+what it takes gives the general way's results."""
+import pytest
+import torch
+
+import nvfp4_gemm
+from nvfp4_cutlass_b200 import _C
+
+
+def operands(device, m=128, n=256, k=256, e=2):
+    g = torch.Generator().manual_seed(m + n + k)
+    w = (torch.randn(e, n, k, generator=g) * 0.05).to(torch.bfloat16)
+    b, sfb, gw = nvfp4_gemm.quantize_weight_nvfp4(w.to(device))
+    sizes = [m] + [0] * (e - 1) if m < 256 else [m // 2] * e
+    return dict(a=torch.randn(m, k, generator=g).to(torch.bfloat16).to(device), b=b, sfb=sfb, gw=gw,
+                d=torch.zeros(m, n, dtype=torch.bfloat16, device=device), m_indices=nvfp4_gemm.make_m_indices(sizes, device=device, alignment=16))
+
+
+WRONG = {
+    "a": lambda t: t.float(), "b": lambda t: t.to(torch.uint8), "sfb": lambda t: t[:-1], "gw": lambda t: t.double(), "d": lambda t: t[:-1],
+    "m_indices": lambda t: t.long(),
+}
+
+
+@pytest.mark.parametrize("name", WRONG)
+def test_it_answers_none_to_what_does_not_fit(name):
+    _C.lib()
+    t = operands("cpu")
+    t[name] = WRONG[name](t[name])
+    assert _C._contiguous_call(*t.values(), 0, 1, 0, 0) is None
+    with pytest.raises(RuntimeError, match="assertion failed"):
+        nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(**t)
+
+
+def test_it_answers_none_to_host_tensors_subclasses_and_odd_options():
+    _C.lib()
+
+    class Sub(torch.Tensor):
+        pass
+
+    t = list(operands("cpu").values())
+    assert _C._contiguous_call(*t, 0, 1, 0, 0) is None
+    assert _C._contiguous_call(t[0].as_subclass(Sub), *t[1:], 0, 1, 0, 0) is None
+    assert _C._contiguous_call(*t, 0, 1, 0, -16) is None and _C._contiguous_call(*t, 0, 1, 0, "16") is None
+    assert _C._contiguous_call(*t, 0, 1, 0, 1 << 80) is None and _C._contiguous_call(None, *t[1:], 0, 1, 0, 0) is None
+    with pytest.raises(TypeError):
+        _C._contiguous_call(*t)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("swap,align,m", [(0, 128, 256), (1, 16, 16), (1, 32, 96)])
+@pytest.mark.parametrize("residual", [True, False])
+def test_both_ways_give_the_same(swap, align, m, residual):
+    t = operands("cuda", m=m)
+    calls = []
+    fast = _C._contiguous_call
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    wide = torch.full((m, 384), 7.0, dtype=torch.bfloat16, device="cuda")
+    for kw in ({}, dict(device_status=status)):                 # a status word is not an ordinary call
+        for d in (t["d"], wide[:, :256]):
+            d.zero_()
+            _C.lib()
+            _C._contiguous_call = lambda *a: calls.append(fast(*a)) or calls[-1]
+            try:
+                nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(**{**t, "d": d}, enable_residual_pass=residual, m_alignment=align,
+                                                                     tune_swap_ab=swap, **kw)
+            finally:
+                _C._contiguous_call = fast
+            calls.append(d.clone())
+    assert calls[0] == 0 and calls[2] == 0 and len(calls) == 6          # the first two went through the binding, the others did not
+    assert float(calls[1].float().norm()) > 0
+    for other in (calls[3], calls[4], calls[5]):
+        assert torch.equal(calls[1], other)
+    assert bool((wide[:, 256:] == 7.0).all())
+
+
+@pytest.mark.gpu
+def test_errors_and_streams_are_those_of_the_general_way():
+    t = operands("cuda", m=256)
+    with pytest.raises(RuntimeError, match="m_alignment 128 or 256"):
+        nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(**t, m_alignment=64)
+    with pytest.raises(RuntimeError, match="multiples of 8 elements"):
+        odd = torch.zeros(256, 257, dtype=torch.bfloat16, device="cuda")[:, :256]
+        nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(**{**t, "d": odd})
+    with pytest.raises(RuntimeError, match="operand is a CUDA tensor|is a CUDA tensor"):
+        nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(**{**t, "gw": t["gw"].cpu()})
+    want = t["d"].clone()
+    nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(**{**t, "d": want})
+    torch.cuda.synchronize()
+    side, got = torch.cuda.Stream(), torch.zeros_like(want)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):              # captured on the stream that is current
+            nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(**{**t, "d": got})
+    assert float(got.float().norm()) == 0
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
