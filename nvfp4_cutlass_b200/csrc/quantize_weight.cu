@@ -11,11 +11,13 @@
 // which the quantisation of batch i - 1, which sits in L2, is interleaved with the maxima of batch i, which streams in
 // from HBM.  Blocks draw tiles from a counter in list order and a quantisation tile waits only for tiles ahead of it,
 // so whatever number of blocks runs at a time, the ones that are waited for are running or done.
-// Measured (BF16): 8 experts of 4096 x 7168 (58 MB each, too large for two of them to share L2) 177-185 us; the
-// weights cross HBM 1.8 times, 0.94 GB of DRAM traffic in all at 5.5 TB/s; before 1000 us (a scalar load per element, 40 instructions per element, an atomic per warp on one word);
-// 32 of 4096 x 1536: 128 us = 4.1 TB/s of 400 MB read and 113 MB written once, the rest is the warps' latency.  Every tile
-// finds its stage by walking the stages before it, a batch each: with 256 batches (4096 x 2048, 2.86 ms, 1.9 TB/s) that is what
-// the kernel spends its time on; 64 (4096 x 7168) 3.3 TB/s, 1024 experts in 22 batches (256 x 1024) 4.1.
+// Quantisation goes through a batch backwards, from what was read last: its reads end up further apart the longer the stage
+// lasts, and the early ones hit L2 where, in list order, every one would come a whole batch after its first read.
+// Measured (BF16): 8 experts of 4096 x 7168 (58 MB each, too large for two of them to share L2) 179-180 us, 184-185 in list
+// order, 92 if the weights crossed HBM once; 64 of them 1280 us, 1480 in list order;
+// 32 of 4096 x 1536: 132 us, 136 in list order = 3.9 TB/s of 400 MB read and 113 MB written once, the rest is the warps' latency.
+// A tile's stage comes from a division: all stages but the first and the last two have as many tiles.  (Walking the stages, a batch each: 256 of
+// 4096 x 2048, 256 batches, 2870 us; 1870-1940 so.)  1024 experts in 22 batches (256 x 1024) 166 us.
 #include <climits>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -281,6 +283,7 @@ quantize_weight_kernel(const T* __restrict__ w, int E, int N, int K, int batch, 
     __shared__ uint32_t drawn, stop;
     const uint32_t kt = static_cast<uint32_t>((K + kUnitK - 1) / kUnitK), lane = threadIdx.x & 31;
     const uint32_t total = static_cast<uint32_t>(E) * (at + qt);
+    const uint32_t full_stage = static_cast<uint32_t>(batch) * (at + qt), stages = static_cast<uint32_t>((E + batch - 1) / batch);
     uint32_t next = 0;
     if (threadIdx.x == 0) { next = atomicAdd(scratch.ticket, 1u); stop = 0; }
     int known = -1;                                  // expert whose global scale this thread holds
@@ -295,6 +298,11 @@ quantize_weight_kernel(const T* __restrict__ w, int E, int N, int K, int batch, 
         if (threadIdx.x == 0) next = atomicAdd(scratch.ticket, 1u);      // arrives while this tile is worked on
         int first_a = 0;                             // first expert of the stage's maxima
         uint32_t na = min(batch, E) * at, nq = 0;    // tiles of either kind in the stage
+        if (i >= na + full_stage) {                  // all stages but the first and the last two are alike
+            const uint32_t skip = min((i - na) / full_stage, stages - 2);
+            i -= skip * full_stage;
+            first_a = static_cast<int>(skip) * batch;
+        }
         while (i >= na + nq) {
             i -= na + nq;
             nq = min(batch, E - first_a) * qt;
@@ -306,8 +314,9 @@ quantize_weight_kernel(const T* __restrict__ w, int E, int N, int K, int batch, 
         const uint32_t q_before = here ? static_cast<uint32_t>(at_mix * nq / here) : 0u;
         const uint32_t q_after = here && i >= lead ? static_cast<uint32_t>((at_mix + 1) * nq / here) : q_before;
         if (q_after > q_before) {
-            const int e = first_a - batch + static_cast<int>(q_before / qt);
-            const uint32_t r = q_before % qt;
+            // last read, first quantised
+            const uint32_t back = nq - 1 - q_before, r = back % qt;
+            const int e = first_a - batch + static_cast<int>(back / qt);
             const int n0 = static_cast<int>(r / kt) * kTileRows, k0 = static_cast<int>(r % kt) * kUnitK;
             const int nw = n0 + static_cast<int>(threadIdx.x >> 5) * kUnitRows;
             const bool full = n0 + kTileRows <= N && k0 + kUnitK <= K;

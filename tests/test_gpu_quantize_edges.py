@@ -71,3 +71,11 @@ def test_nan_and_infinity(oracle, dtype, scale):
     b, sfb, gw = nvfp4_gemm.quantize_weight_nvfp4(w.cuda())
     assert torch.equal(gw.cpu(), torch.stack((want_gw[0], torch.tensor(float("inf")))))
     assert torch.equal(b.cpu().view(torch.uint8)[:70], want_b[:70])
+
+
+@pytest.mark.parametrize("shape", [(5, 2048, 4096), (7, 1000, 4160), (4, 4096, 4096)])     # batches of 24 MB: one expert each,
+def test_stages_of_several_batches(oracle, shape):                                         # 3 + 3 + 1, one each
+    w = (torch.randn(*shape, generator=torch.Generator().manual_seed(sum(shape))) * 0.02).to(torch.bfloat16)
+    w *= torch.arange(1, shape[0] + 1).reshape(-1, 1, 1)                                   # every expert a global scale of its own
+    for got, want in zip(nvfp4_gemm.quantize_weight_nvfp4(w.cuda()), oracle.quantize_weight(w)):
+        assert torch.equal(got.cpu(), want)
