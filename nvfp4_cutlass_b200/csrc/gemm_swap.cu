@@ -66,7 +66,7 @@ struct Cfg {
     static constexpr uint32_t kOffSFW = kOffP + kDepthP * kSlotP;
     static constexpr uint32_t kOffSFT = kOffSFW + kDepthW * kSlotSFW;
     static constexpr uint32_t kOffBars = kOffSFT + kDepthP * kSlotSFT;
-    static constexpr uint32_t kNumBars = 2 * kDepthW + 2 * kDepthA + kDepthP + 4 + 2;
+    static constexpr uint32_t kNumBars = 2 * kDepthW + 2 * kDepthA + 2 * kDepthP + 4 + 2;
     static constexpr uint32_t kSmemAlloc = kOffBars + kNumBars * 8 + 16 + 1024;
     static_assert(kDepthW >= 3, "weight ring too shallow");
     static_assert(kSmemAlloc <= 232448, "shared memory budget");
@@ -86,12 +86,50 @@ struct Params {
     __nv_bfloat16* d;
     int64_t ldd;
     uint32_t m, n, k;
+    uint32_t run_log2;         // consecutive weight tiles that a CTA takes with one token tile, as a power of two (1 tile unless the P ring
+                               // holds all of K)
     int32_t* status;
 };
 
 using gemm::Ring;
 
-template <uint32_t T, uint32_t BK, bool kResidual, int kPolicy>
+// Tiles in the order of a CTA.  kGeneral: runs of consecutive weight tiles of one token tile, the runs in static stride over the CTAs;
+// else a tile at a time.
+template <bool kGeneral>
+struct Walker {
+    uint32_t per, run_log2, runs;      // runs of a token tile, of all
+    uint32_t at = blockIdx.x, i = 0;
+    uint32_t m_blk = 0, n_blk = 0;
+    bool fresh = true, done = true;    // the token tile is a new one; it is no longer needed after this weight tile
+    __device__ __forceinline__ Walker(const Params& p, uint32_t token_tile)
+        : per(kGeneral ? (p.n / BW) >> p.run_log2 : p.n / BW), run_log2(p.run_log2), runs(p.m / token_tile * per) {}
+    __device__ __forceinline__ bool next()
+    {
+        if (at >= runs) return false;
+        if constexpr (!kGeneral) {
+            m_blk = at / per;
+            n_blk = at % per;
+            at += gridDim.x;
+        } else {
+            fresh = i == 0;
+            if (fresh) {
+                m_blk = at / per;
+                n_blk = (at - m_blk * per) << run_log2;
+            } else {
+                ++n_blk;
+            }
+            done = (++i >> run_log2) != 0;
+            if (done) { i = 0; at += gridDim.x; }
+        }
+        return true;
+    }
+};
+
+// kGeneral: K need not be a multiple of BK, and a CTA may take several weight tiles with one transformed token tile.  A form of its
+// own, because a decode call is over in a few microseconds and is held up by every instruction that it fetches: all of the
+// general form's in one kernel took a call of 16 tokens, 32 experts, N = 1024, K = 2048 from 6.0 to 6.8 us
+// (now 6.2).
+template <uint32_t T, uint32_t BK, bool kResidual, int kPolicy, bool kGeneral>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                  const __grid_constant__ CUtensorMap tm_sfw, const Params p)
@@ -107,7 +145,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     uint64_t* a_full = w_empty + C::kDepthW;
     uint64_t* a_empty = a_full + C::kDepthA;
     uint64_t* p_full = a_empty + C::kDepthA;
-    uint64_t* sf_full = p_full + C::kDepthP;         // [2]: scales of a K block are in tensor memory
+    uint64_t* p_empty = p_full + C::kDepthP;         // the last weight tile's MMAs over this slot have retired
+    uint64_t* sf_full = p_empty + C::kDepthP;        // [2]: scales of a K block are in tensor memory
     uint64_t* tmem_full = sf_full + 2;               // [2]
     uint64_t* tmem_empty = tmem_full + 2;            // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
@@ -120,7 +159,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             ptx::mbar_init(w_empty + i, 1);
         }
         for (uint32_t i = 0; i < C::kDepthA; ++i) { ptx::mbar_init(a_full + i, 1); ptx::mbar_init(a_empty + i, kXformWarps); }
-        for (uint32_t i = 0; i < C::kDepthP; ++i) ptx::mbar_init(p_full + i, kXformWarps);
+        for (uint32_t i = 0; i < C::kDepthP; ++i) { ptx::mbar_init(p_full + i, kXformWarps); if constexpr (kGeneral) ptx::mbar_init(p_empty + i, 1); }
         for (uint32_t i = 0; i < 2; ++i) {
             ptx::mbar_init(tmem_full + i, 1);
             ptx::mbar_init(tmem_empty + i, kNumEpiWarps);
@@ -144,8 +183,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     // tiles: all weight-row blocks of one token block are neighbours, so the CTAs of a
     // wave share that token block's activations through L2 while streaming disjoint weights
     const long long probe_start = ptx::probe_clock();
-    const uint32_t num_n = p.n / BW, num_kb = p.k / BK;
-    const uint32_t num_tiles = (p.m / T) * num_n;
+    // the general form's last K block may be a part of one: loads fill in zeros, and K atoms past the end get no MMA
+    const uint32_t num_kb = kGeneral ? (p.k + BK - 1) / BK : p.k / BK;
+    Walker<kGeneral> walk(p, T);
     bool ok = true;
     ptx::ProbeAcc pa;
     auto give_up = [&](uint32_t code) {
@@ -159,9 +199,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         if (lane == 0) {
             Ring rw;
             const uint64_t stream_once = ptx::l2_policy_evict_first();
-            for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const uint32_t m_blk = tile / num_n, n_blk = tile % num_n;
-                const int32_t e = max(0, __ldg(p.m_indices + m_blk * T));
+            while (ok && walk.next()) {
+                const uint32_t n_blk = walk.n_blk;
+                const int32_t e = max(0, __ldg(p.m_indices + walk.m_blk * T));
                 for (uint32_t kb = 0; kb < num_kb; ++kb) {
                     if (!ptx::mbar_wait(w_empty + rw.slot, rw.phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
                     ptx::mbar_arrive_expect_tx(w_full + rw.slot, C::kSlotW + C::kSlotSFW);
@@ -181,25 +221,30 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     } else if (warp == kWarpTmaA) {
         // activation producer (a separate thread, so a full A ring never holds the weights back)
         if (lane == 0) {
-            Ring ra;
-            for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const uint32_t m_blk = tile / num_n;
+            Ring ra, rp;
+            while (ok && walk.next()) {
+                if (kGeneral && !walk.fresh) continue;
                 for (uint32_t kb = 0; kb < num_kb; ++kb) {
                     if (!ptx::mbar_wait(a_empty + ra.slot, ra.phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
                     ptx::mbar_arrive_expect_tx(a_full + ra.slot, C::kSlotA);
 #pragma unroll
                     for (uint32_t box = 0; box < BK / 64; ++box)
                         ptx::tma_load_2d(smem_gen + C::kOffA + ra.slot * C::kSlotA + box * (T * 128), &tm_a,
-                                         a_full + ra.slot, kb * BK + box * 64, m_blk * T);
+                                         a_full + ra.slot, kb * BK + box * 64, walk.m_blk * T);
                     ra.advance<C::kDepthA>();
+                    rp.advance<C::kDepthP>();
                 }
             }
+            // nobody refills the last P slots, whose commits have to have arrived all the same
+            if (kGeneral && ok && !gemm::drain_ring<C::kDepthP>(rp, [&](uint32_t i, uint32_t parity) {
+                    return ptx::mbar_wait(p_empty + i, parity, abort_flag, pa, 0); })) give_up(1);
         }
     } else if (warp == kWarpMma && lane == 0) {
-        Ring rw, rp;
+        Ring rw, rp, rp0;                            // rp0: where the token tile begins
         uint32_t it = 0, cnt = 0;
         constexpr uint32_t idesc = ptx::make_idesc_nvf4(BW, C::kRowsP);
-        for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
+        for (; ok && walk.next(); ++it) {
+            if constexpr (kGeneral) { if (walk.fresh) rp0 = rp; else rp = rp0; }
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
             if (!ptx::mbar_wait(tmem_empty + acc, acc_phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
             ptx::tcgen05_fence_after_sync();
@@ -215,15 +260,22 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 const uint32_t w = smem + C::kOffW + rw.slot * C::kSlotW;
                 const uint32_t pt = smem + C::kOffP + rp.slot * C::kSlotP;
                 const uint32_t sf = tmem_base + C::kColSF + buf * C::kSfBufCols;
-#pragma unroll
-                for (uint32_t a = 0; a < C::kAtoms; ++a)
-                    ptx::tcgen05_mma_nvf4(tmem_acc,
-                                          ptx::make_smem_desc(w + (a / 4) * C::kSubW + (a % 4) * 32, C::kSBO, C::kSwizzle),
+                const uint32_t atoms = p.k / 64 - kb * C::kAtoms;
+                auto issue = [&](uint32_t a) {
+                    ptx::tcgen05_mma_nvf4(tmem_acc, ptx::make_smem_desc(w + (a / 4) * C::kSubW + (a % 4) * 32, C::kSBO, C::kSwizzle),
                                           ptx::make_smem_desc(pt + (a / 4) * C::kSubP + (a % 4) * 32, C::kSBO, C::kSwizzle), idesc,
                                           sf + C::kSfW + 4 * a, sf + C::kSfT + 4 * a, (kb | a) != 0 ? 1u : 0u);
-                // one commit per K block: the weight producer, the scale warps and the transform warps all
-                // read "the MMAs of K block i have retired" from this barrier
+                };
+                if (!kGeneral || atoms >= C::kAtoms) {
+#pragma unroll
+                    for (uint32_t a = 0; a < C::kAtoms; ++a) issue(a);
+                } else {
+#pragma unroll 1
+                    for (uint32_t a = 0; a < atoms; ++a) issue(a);
+                }
+                // the weight producer and the scale warps both read "the MMAs of K block i have retired" from this barrier
                 ptx::tcgen05_commit(w_empty + rw.slot);
+                if (kGeneral && walk.done) ptx::tcgen05_commit(p_empty + rp.slot);
                 if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full + acc);
                 rp.advance<C::kDepthP>();
                 rw.advance<C::kDepthW>();
@@ -237,9 +289,10 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         // atoms the transform wrote.  Two column buffers alternate; a buffer is rewritten once the MMAs of two K
         // blocks earlier have retired (their commit on the W-empty barrier).
         const uint32_t quad = warp & 3;
-        Ring rw, rp;
+        Ring rw, rp, rp0;
         uint32_t cnt = 0;
-        for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        while (ok && walk.next()) {
+            if constexpr (kGeneral) { if (walk.fresh) rp0 = rp; else rp = rp0; }
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++cnt) {
                 const uint32_t buf = cnt & 1u;
                 const uint32_t sf = tmem_base + ((quad * 32) << 16) + C::kColSF + buf * C::kSfBufCols;
@@ -273,9 +326,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         // fixed token the 32 lanes of a warp write 32 consecutive BF16
         const uint32_t quad = warp & 3;
         uint32_t it = 0;
-        for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
+        for (; ok && walk.next(); ++it) {
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-            const uint32_t m_blk = tile / num_n, n_blk = tile % num_n;
+            const uint32_t m_blk = walk.m_blk, n_blk = walk.n_blk;
             const int32_t e = max(0, __ldg(p.m_indices + m_blk * T));
             const float g = __ldg(p.gw + e);
             if (!ptx::all_lanes(ptx::mbar_wait(tmem_full + acc, acc_phase, abort_flag, pa, 0))) { give_up(1); break; }
@@ -325,7 +378,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         const uint32_t t = threadIdx.x - kWarpXform0 * 32;
         Ring ra, rp;
         uint32_t cnt = 0;
-        for (uint32_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        while (ok && walk.next()) {
+            if (kGeneral && !walk.fresh) continue;
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++cnt) {
                 if (!ptx::all_lanes(ptx::mbar_wait(a_full + ra.slot, ra.phase, abort_flag, pa, 0))) { give_up(1); break; }
                 bool p_ok = true;
@@ -335,10 +389,14 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     smem + C::kOffSFT + rp.slot * C::kSlotSFT + C::kSF1Bytes, t, [&] {
                         __syncwarp();
                         if (lane == 0) ptx::mbar_arrive(a_empty + ra.slot);
-                        // the slot is free once the MMAs of kDepthP K blocks ago have retired
-                        p_ok = ptx::all_lanes(cnt < C::kDepthP ||
-                                              ptx::mbar_wait(w_empty + (cnt - C::kDepthP) % C::kDepthW,
-                                                             ((cnt - C::kDepthP) / C::kDepthW) & 1u, abort_flag, pa, 1));
+                        // the slot is free once the MMAs of the last weight tile over it have retired; with one weight tile that is
+                        // what the weight ring's barrier says of kDepthP K blocks ago
+                        const uint32_t ago = cnt - C::kDepthP;
+                        if constexpr (kGeneral)
+                            p_ok = ptx::all_lanes(ptx::mbar_wait(p_empty + rp.slot, rp.phase ^ 1, abort_flag, pa, 1));
+                        else
+                            p_ok = ptx::all_lanes(cnt < C::kDepthP ||
+                                                  ptx::mbar_wait(w_empty + ago % C::kDepthW, (ago / C::kDepthW) & 1u, abort_flag, pa, 1));
                     });
                 if (!p_ok) { give_up(1); break; }
                 ptx::fence_proxy_async_smem();
@@ -365,9 +423,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     }
 }
 
-template <uint32_t T, uint32_t BK, bool kResidual, int kPolicy = 0>
-int launch_variant(const void* a, int64_t lda, const void* b, const void* sfb, int M, int N, int K, int E,
-                   const Params& p, bool pdl, int num_sms, cudaStream_t stream)
+template <uint32_t T, uint32_t BK, bool kResidual, int kPolicy, bool kGeneral>
+int launch_kernel_form(const void* a, int64_t lda, const void* b, const void* sfb, int M, int N, int K, int E,
+                       const Params& p, bool pdl, int num_sms, cudaStream_t stream)
 {
     using C = Cfg<T, BK, kResidual>;
     CUtensorMap tm_a, tm_w, tm_sfw;
@@ -381,7 +439,7 @@ int launch_variant(const void* a, int64_t lda, const void* b, const void* sfb, i
                                     static_cast<uint64_t>(E) * (K / 64), static_cast<uint64_t>(N) * 4, BW, C::kAtoms,
                                     CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
-    auto kernel = gemm_swap_kernel<T, BK, kResidual, kPolicy>;
+    auto kernel = gemm_swap_kernel<T, BK, kResidual, kPolicy, kGeneral>;
     static bool attr_set[host::kMaxDevices] = {};
     int dev = 0;
     NVFP4_CUDA_CHECK(cudaGetDevice(&dev));
@@ -389,40 +447,60 @@ int launch_variant(const void* a, int64_t lda, const void* b, const void* sfb, i
         NVFP4_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemAlloc));
         attr_set[dev] = true;
     }
-    const int num_tiles = (M / static_cast<int>(T)) * (N / static_cast<int>(BW));
-    const int grid = num_tiles < num_sms ? num_tiles : num_sms;
+    const int runs = (M / static_cast<int>(T)) * (N / static_cast<int>(BW)) >> p.run_log2;
+    const int grid = runs < num_sms ? runs : num_sms;
     return host::launch_kernel(kernel, dim3(grid), dim3(kThreads), C::kSmemAlloc, stream, pdl, tm_a, tm_w, tm_sfw, p);
+}
+
+template <uint32_t T, uint32_t BK, bool kResidual, int kPolicy>
+int launch_variant(const void* a, int64_t lda, const void* b, const void* sfb, int M, int N, int K, int E,
+                   const Params& p, bool pdl, int num_sms, cudaStream_t stream)
+{
+    using C = Cfg<T, BK, kResidual>;
+    const int num_n = N / static_cast<int>(BW), num_tiles = (M / static_cast<int>(T)) * num_n;
+    Params q = p;
+    q.run_log2 = 0;
+    if constexpr (BK >= 256) {
+        // Where the P ring holds a token tile's whole K, a CTA can transform it once for a run of weight tiles.  To transform it costs
+        // about as much as a weight tile and the general form about as much again: the run is the one with the shortest
+        // rounds * (run + 1), if that saves more than 1.  128 tokens over 32 of 256 experts, N = 2048, K = 512:
+        // 8.3 us a call, with runs of four 7.3; 192 experts' worth of routing, N = 5120, K = 1024: 17.8 / 16.4.
+        int best = (num_tiles + num_sms - 1) / num_sms * 2 - 1;
+        if ((K + static_cast<int>(BK) - 1) / static_cast<int>(BK) <= static_cast<int>(C::kDepthP))
+            for (int log2 = 1; log2 <= 2 && num_n % (1 << log2) == 0; ++log2) {
+                const int cost = ((num_tiles >> log2) + num_sms - 1) / num_sms * ((1 << log2) + 1);
+                if (cost < best) { best = cost; q.run_log2 = static_cast<uint32_t>(log2); }
+            }
+        if (q.run_log2 != 0 || K % static_cast<int>(BK) != 0)
+            return launch_kernel_form<T, BK, kResidual, kPolicy, true>(a, lda, b, sfb, M, N, K, E, q, pdl, num_sms, stream);
+    }
+    return launch_kernel_form<T, BK, kResidual, kPolicy, false>(a, lda, b, sfb, M, N, K, E, q, pdl, num_sms, stream);
 }
 
 template <uint32_t T>
 int launch_for_tile(const void* a, int64_t lda, const void* b, const void* sfb, int M, int N, int K, int E,
                     const Params& p, bool residual, int block_k, int policy, bool pdl, int num_sms, cudaStream_t stream)
 {
-    if (policy != 0)      // the other scale policies: the default K-block choice only
-        return host::with_policy(policy, [&](auto pol) {
-            constexpr int kP = decltype(pol)::value;
-            if constexpr (T <= 32) {
-                if (K % 512 == 0)
-                    return residual ? launch_variant<T, 512, true, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream)
-                                    : launch_variant<T, 512, false, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream);
-            }
-            if (K % 256 == 0)
-                return residual ? launch_variant<T, 256, true, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream)
-                                : launch_variant<T, 256, false, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream);
-            return residual ? launch_variant<T, 128, true, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream)
-                            : launch_variant<T, 128, false, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream);
-        });
-    // K blocks of 512 halve the per-block barrier traffic and commits; a 64-token tile has no room for them
-    if constexpr (T <= 32) {
-        if (K % 512 == 0 && (block_k == 0 || block_k == 512))
-            return residual ? launch_variant<T, 512, true>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream)
-                            : launch_variant<T, 512, false>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream);
-    }
-    if (K % 256 == 0 && block_k != 128)
-        return residual ? launch_variant<T, 256, true>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream)
-                        : launch_variant<T, 256, false>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream);
-    return residual ? launch_variant<T, 128, true>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream)
-                    : launch_variant<T, 128, false>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream);
+    // K blocks of 512 (256 for 64 tokens, which leave no room for more) where they divide K, else of 256 where those do; for other K from
+    // 896 on the large ones all the same, the last one in part: the rounds of barriers of seven blocks of 128 take longer than
+    // the arithmetic on zeros.  In blocks of 128 / in part: K = 896, 168 experts' share of 51 tokens 17.2 / 11.8 us; K = 1408, 96 experts 6.6 / 5.2;
+    // K = 2944, 168 experts, N = 3328 338 / 166; K = 6784, 128 experts, N = 6912 1318 / 822; K = 640, 60 tokens 4.3 / 5.0.
+    constexpr int kMost = T <= 32 ? 512 : 256;
+    const int fits = K % kMost == 0 ? kMost : (K % 256 == 0 ? 256 : (K >= 896 ? kMost : 128));
+    const int bk = block_k != 0 && K % block_k == 0 && block_k <= kMost ? block_k : fits;
+    return host::with_policy(policy, [&](auto pol) {
+        constexpr int kP = decltype(pol)::value;
+        if constexpr (T <= 32) {
+            if (bk == 512)
+                return residual ? launch_variant<T, 512, true, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream)
+                                : launch_variant<T, 512, false, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream);
+        }
+        if (bk >= 256)
+            return residual ? launch_variant<T, 256, true, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream)
+                            : launch_variant<T, 256, false, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream);
+        return residual ? launch_variant<T, 128, true, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream)
+                        : launch_variant<T, 128, false, kP>(a, lda, b, sfb, M, N, K, E, p, pdl, num_sms, stream);
+    });
 }
 
 }  // namespace
