@@ -308,6 +308,10 @@ NVFP4_API int nvfp4_combine_rows_peer(const int64_t* peers, int64_t rows_ld_elem
  * since all see the same histograms; the step's result is then incomplete and the caller repeats it another way.
  * cap_m % 128 == 0.  No counterpart in the reference.
  *
+ * nvfp4_plan_one_rank: the same plan where one rank owns all experts, straight from the pairs: expert e's rows begin at e * cap_m, no
+ * histogram is needed beforehand.  Also writes dst_rank[p] (0; for an id out of range the id divided by num_experts, rounded
+ * down, which the movers skip and report).
+ *
  * nvfp4_peer_barrier: a barrier over the ranks of one NVLink domain whose wait is bounded.  flag_peers[r] is the
  * address, in this process, of rank r's flag array: int64 [NVFP4_BARRIER_SLOTS][world] in symmetric memory, zero
  * before the first use.  Every rank calls it with the same slot and the same epoch, epochs growing by one per call
@@ -317,6 +321,8 @@ NVFP4_API int nvfp4_combine_rows_peer(const int64_t* peers, int64_t rows_ld_elem
 NVFP4_API int nvfp4_plan_peer_masked(const int64_t* all_counts, int world, int num_experts, int rank, int cap_m,
                                      const int64_t* ids, int64_t n, int64_t* base, int64_t* limit, int32_t* masked_m,
                                      int64_t* dst_row, int32_t* device_status, void* stream);
+NVFP4_API int nvfp4_plan_one_rank(const int64_t* ids, int64_t n, int num_experts, int cap_m, int32_t* masked_m, int64_t* dst_rank,
+                                  int64_t* dst_row, int32_t* device_status, void* stream);
 NVFP4_API int nvfp4_peer_barrier(const int64_t* flag_peers, int rank, int world, int slot, int64_t epoch,
                                  int64_t budget_cycles, int32_t* device_status, void* stream);
 

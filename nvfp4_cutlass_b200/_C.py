@@ -37,7 +37,7 @@ EXPORTS = ("nvfp4_last_error", "nvfp4_version", "nvfp4_get_num_sms", "nvfp4_set_
            "nvfp4_dispatch_rows_peer", "nvfp4_dispatch_quantized_peer", "nvfp4_relayout_scales",
            "nvfp4_grouped_gemm_masked_quantized", "nvfp4_grouped_gemm_masked_quantized_swiglu", "nvfp4_grouped_gemm_masked_quantized_rows", "nvfp4_expert_mlp_few_rows", "nvfp4_combine_rows_peer", "nvfp4_expert_histogram",
            "nvfp4_grouped_gemm_swiglu_contiguous", "nvfp4_grouped_gemm_masked", "nvfp4_load_checkpoint_weights",
-           "nvfp4_read_status", "nvfp4_debug_split_workspace", "nvfp4_debug_wait_timeout", "nvfp4_debug_quantize_weight_expired", "nvfp4_plan_peer_masked",
+           "nvfp4_read_status", "nvfp4_debug_split_workspace", "nvfp4_debug_wait_timeout", "nvfp4_debug_quantize_weight_expired", "nvfp4_plan_peer_masked", "nvfp4_plan_one_rank",
            "nvfp4_peer_barrier")
 
 
@@ -69,6 +69,7 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_swiglu.argtypes = [vp, i64, i64, i32, vp, i64, vp]
         L.nvfp4_dispatch_rows_peer.argtypes = [vp, i64, vp, i32, vp, vp, vp, i64, i32, i64, i32, i64, i32, vp, vp]
         L.nvfp4_plan_peer_masked.argtypes = [vp, i32, i32, i32, i32, vp, i64, vp, vp, vp, vp, vp, vp]
+        L.nvfp4_plan_one_rank.argtypes = [vp, i64, i32, i32, vp, vp, vp, vp, vp]
         L.nvfp4_peer_barrier.argtypes = [vp, i32, i32, i32, i64, i64, vp, vp]
         L.nvfp4_expert_histogram.argtypes = [vp, i64, i32, vp, vp]
         L.nvfp4_grouped_gemm_swiglu_contiguous.argtypes = [vp, i64, vp, vp, vp, vp, i64, vp, i32, i32, i32, i32, i32, vp, vp, vp]
@@ -448,6 +449,20 @@ def plan_peer_masked(all_counts: torch.Tensor, ids: torch.Tensor, world: int, ra
                                             base.data_ptr(), limit.data_ptr(), masked_m.data_ptr(), dst_row.data_ptr(),
                                             status.data_ptr(), _stream()))
     return masked_m, dst_row
+
+
+def plan_one_rank(ids: torch.Tensor, num_experts: int, cap_m: int, status: torch.Tensor = None):
+    """The plan of plan_peer_masked where one rank owns all experts, without a histogram: (masked_m int32 (E,), dst_rank int64 (pairs,),
+    dst_row int64 (pairs,))."""
+    n = ids.numel()
+    _require(_i64_ok(ids, n), "ids is a contiguous int64 CUDA tensor")
+    dev = _one_device(ids, status)
+    masked_m = torch.empty(num_experts, dtype=torch.int32, device=dev)
+    dst_rank, dst_row = torch.empty_like(ids), torch.empty_like(ids)
+    with _on(dev):
+        _check(lib().nvfp4_plan_one_rank(ids.data_ptr(), n, num_experts, cap_m, masked_m.data_ptr(), dst_rank.data_ptr(), dst_row.data_ptr(),
+                                         status.data_ptr() if status is not None else None, _stream()))
+    return masked_m, dst_rank, dst_row
 
 
 def peer_barrier(flag_peers: torch.Tensor, rank: int, world: int, slot: int, epoch: int, status: torch.Tensor,

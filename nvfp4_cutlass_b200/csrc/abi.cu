@@ -530,6 +530,16 @@ int nvfp4_plan_peer_masked(const int64_t* all_counts, int world, int num_experts
                                    static_cast<cudaStream_t>(stream));
 }
 
+int nvfp4_plan_one_rank(const int64_t* ids, int64_t n, int num_experts, int cap_m, int32_t* masked_m, int64_t* dst_rank, int64_t* dst_row,
+                        int32_t* device_status, void* stream)
+{
+    host::clear_error();
+    NVFP4_REQUIRE(num_experts >= 1 && num_experts <= 4096, "num_experts (%d) must be in [1, 4096]", num_experts);
+    NVFP4_REQUIRE(cap_m >= 128 && cap_m % 128 == 0 && n >= 0, "bad capacity / pair count");
+    NVFP4_REQUIRE(masked_m && (n == 0 || (ids && dst_rank && dst_row)), "null pointer argument");
+    return launch_plan_one_rank(ids, n, num_experts, cap_m, masked_m, dst_rank, dst_row, device_status, static_cast<cudaStream_t>(stream));
+}
+
 int nvfp4_peer_barrier(const int64_t* flag_peers, int rank, int world, int slot, int64_t epoch, int64_t budget_cycles,
                        int32_t* device_status, void* stream)
 {

@@ -40,6 +40,8 @@ int launch_expert_histogram(const int64_t* ids, int64_t n, int num_experts, int6
 int launch_plan_peer_masked(const int64_t* all_counts, int world, int num_experts, int rank, int cap_m, const int64_t* ids,
                             int64_t n, int64_t* base, int64_t* limit, int32_t* masked_m, int64_t* dst_row, int32_t* status,
                             cudaStream_t stream);
+int launch_plan_one_rank(const int64_t* ids, int64_t n, int num_experts, int cap_m, int32_t* masked_m, int64_t* dst_rank, int64_t* dst_row,
+                         int32_t* status, cudaStream_t stream);
 int launch_peer_barrier(const int64_t* flag_peers, int rank, int world, int slot, int64_t epoch, int64_t budget_cycles,
                         int32_t* status, cudaStream_t stream);
 int launch_dispatch_rows_peer(const void* src, int64_t src_ld_bytes, const int64_t* src_idx, int src_div, const int64_t* peers,

@@ -203,14 +203,16 @@ dispatch_quantized_peer_kernel(const uint4* __restrict__ x, int64_t x_ld16, uint
 constexpr uint32_t kRelayoutAtoms = 8;
 __global__ void __launch_bounds__(256)
 relayout_scales_kernel(const uint8_t* __restrict__ sf_rows, const int32_t* __restrict__ masked_m, uint32_t max_m, uint32_t kdim, bool wide,
-                       uint8_t* __restrict__ atoms, uint32_t groups, gemm::Family family)
+                       uint8_t* __restrict__ atoms, uint32_t groups, gemm::Family family, uint32_t tiles)
 {
     __shared__ __align__(16) uint32_t staged[kRelayoutAtoms][2][128];
     const uint32_t k64 = kdim / 64, chunks = (k64 + kRelayoutAtoms - 1) / kRelayoutAtoms;
-    const uint32_t first = blockIdx.x % chunks * kRelayoutAtoms, here = min(kRelayoutAtoms, k64 - first);
-    const uint64_t row0 = static_cast<uint64_t>(blockIdx.x / chunks) * 128;
     ptx::grid_dependency_wait();
-    if (masked_m == nullptr || (!family.leaves(masked_m, groups, max_m) && row0 % max_m < min(static_cast<uint32_t>(max(0, __ldg(masked_m + row0 / max_m))), max_m))) {
+    if (masked_m != nullptr && family.leaves(masked_m, groups, max_m)) { ptx::grid_launch_dependents(); return; }
+    for (uint32_t at = blockIdx.x; at < tiles; at += gridDim.x) {
+        const uint32_t first = at % chunks * kRelayoutAtoms, here = min(kRelayoutAtoms, k64 - first);
+        const uint64_t row0 = static_cast<uint64_t>(at / chunks) * 128;
+        if (masked_m != nullptr && row0 % max_m >= min(static_cast<uint32_t>(max(0, __ldg(masked_m + row0 / max_m))), max_m)) continue;
         const uint32_t r = threadIdx.x / 2, pass = threadIdx.x % 2, word = (r % 32) * 4 + r / 32;
         const uint8_t* src = sf_rows + (row0 + r) * (kdim / 8) + pass * (kdim / 16) + first * 4;
         if (wide) {
@@ -225,6 +227,7 @@ relayout_scales_kernel(const uint8_t* __restrict__ sf_rows, const int32_t* __res
         uint4* dst = reinterpret_cast<uint4*>(atoms + ((row0 / 128) * k64 + first) * 1024);
         const uint4* out = reinterpret_cast<const uint4*>(staged);
         for (uint32_t i = threadIdx.x; i < here * 64; i += 256) dst[i] = out[i];
+        __syncthreads();                             // the stage may be written again
     }
     ptx::grid_launch_dependents();
 }
@@ -423,7 +426,10 @@ expert_histogram_kernel(const int64_t* __restrict__ ids, int64_t n, int num_expe
 // Two passes over the pairs, each block on its own chunk: plan_chunk_hist_kernel counts every chunk's pairs per expert;
 // plan_rows_kernel starts each expert's counter at base[e] + (pairs of e in earlier chunks) and hands out rows chunk-locally.
 // Up to kPlanOnePass pairs one block does all of it, offsets included (plan_small_kernel): the three launches were 14 us of a
-// layer of 256 tokens, this one under 8.  (The first version gave every expert a block that scanned ALL pairs: 128
+// layer of 256 tokens, this one under 8.  On one rank every expert's rows begin where they begin, and the counts are what
+// has been handed out in the end: no histogram ahead of the plan (plan_rows_kernel and plan_one_rank_kernel), one launch in place of
+// three up to kPlanOnePass pairs and two in place of six above: layers of 256 tokens (128 experts, 4096 / 1536) 342 -> 317 us, of 34 (16 experts,
+// 1024 / 1408) 148 -> 127, of 1655 (1024 / 512) 216 -> 178, of 16384 2977 -> 2950.  (The first version gave every expert a block that scanned ALL pairs: 128
 // experts x 131072 pairs took 0.2 ms.)
 constexpr int kPlanThreads = 1024;
 __global__ void __launch_bounds__(kPlanThreads)
@@ -448,8 +454,10 @@ constexpr int64_t kPlanOnePass = 8192;               // eight rounds of 1024: ab
 // of the round take.  With more than kPlanTable experts there is no room for that table and the warps take turns instead
 // (32 block barriers a round in place of four).
 constexpr int kPlanTable = 512;
+// limit(e): end of the expert's rows.
+template <typename Limit>
 __device__ __forceinline__ void hand_out_rows(const int64_t* __restrict__ ids, int64_t lo, int64_t hi, int num_experts, long long* next_row,
-                                              unsigned short* before, const int64_t* limit, int64_t* __restrict__ dst_row)
+                                              unsigned short* before, Limit&& limit, int64_t* __restrict__ dst_row)
 {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const bool table = num_experts <= kPlanTable;
@@ -477,7 +485,7 @@ __device__ __forceinline__ void hand_out_rows(const int64_t* __restrict__ ids, i
             __syncthreads();
             if (valid) {
                 const long long row = next_row[e] + before[wid * num_experts + e] + rank_in_warp;
-                dst_row[p] = (limit == nullptr || row < limit[e]) ? row : -1;
+                dst_row[p] = row < limit(e) ? row : -1;
             }
             __syncthreads();
             if (static_cast<int>(threadIdx.x) < num_experts) {
@@ -497,7 +505,7 @@ __device__ __forceinline__ void hand_out_rows(const int64_t* __restrict__ ids, i
                 first = __shfl_sync(0xffffffffu, first, leader);
                 if (valid) {
                     const long long row = first + rank_in_warp;
-                    dst_row[p] = (limit == nullptr || row < limit[e]) ? row : -1;
+                    dst_row[p] = row < limit(e) ? row : -1;
                 }
             }
             __syncthreads();
@@ -509,18 +517,53 @@ size_t plan_smem(int num_experts)
     return num_experts * (sizeof(long long) + (num_experts <= kPlanTable ? 32 * sizeof(unsigned short) : 0));
 }
 
+// base, limit == nullptr: one rank, expert e has rows [e * cap_m, (e + 1) * cap_m); the last block then knows all counts.
+__device__ __forceinline__ void one_rank_counts(const long long* next_row, int num_experts, int cap_m, int32_t* __restrict__ masked_m,
+                                                int32_t* __restrict__ status)
+{
+    for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
+        const long long total = next_row[e] - static_cast<long long>(e) * cap_m;
+        masked_m[e] = static_cast<int32_t>(total < cap_m ? total : cap_m);
+        if (total > cap_m && status != nullptr) atomicOr(status, 4);
+    }
+}
+// The owner of every pair's expert, rounded down as a division of tensors rounds: ids out of range get ranks out of range.
+__device__ __forceinline__ void one_rank_owners(const int64_t* __restrict__ ids, int64_t lo, int64_t hi, int num_experts, int64_t* __restrict__ dst_rank)
+{
+    for (int64_t p = lo + threadIdx.x; p < hi; p += blockDim.x) {
+        const int64_t e = ids[p];
+        dst_rank[p] = e >= 0 && e < num_experts ? 0 : (e - (e < 0 ? num_experts - 1 : 0)) / num_experts;
+    }
+}
 __global__ void __launch_bounds__(kPlanThreads)
 plan_rows_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t chunk, int num_experts, const int32_t* __restrict__ chunk_hist,
-                 const int64_t* __restrict__ base, const int64_t* __restrict__ limit, int64_t* __restrict__ dst_row)
+                 const int64_t* __restrict__ base, const int64_t* __restrict__ limit, int64_t* __restrict__ dst_row, int cap_m,
+                 int32_t* __restrict__ masked_m, int64_t* __restrict__ dst_rank, int32_t* __restrict__ status)
 {
     extern __shared__ long long next_row[];          // [num_experts] next free row of every expert, for this chunk onwards
     for (int e = threadIdx.x; e < num_experts; e += blockDim.x) {
-        long long r = base[e];
+        long long r = base != nullptr ? base[e] : static_cast<long long>(e) * cap_m;
         for (int c = 0; c < static_cast<int>(blockIdx.x); ++c) r += chunk_hist[static_cast<int64_t>(c) * num_experts + e];
         next_row[e] = r;
     }
-    const int64_t lo = blockIdx.x * chunk;
-    hand_out_rows(ids, lo, min(lo + chunk, n), num_experts, next_row, reinterpret_cast<unsigned short*>(next_row + num_experts), limit, dst_row);
+    const int64_t lo = blockIdx.x * chunk, hi = min(lo + chunk, n);
+    hand_out_rows(ids, lo, hi, num_experts, next_row, reinterpret_cast<unsigned short*>(next_row + num_experts),
+                  [&](int64_t e) { return limit != nullptr ? limit[e] : (e + 1) * cap_m; }, dst_row);
+    if (base != nullptr) return;
+    one_rank_owners(ids, lo, hi, num_experts, dst_rank);
+    if (blockIdx.x == gridDim.x - 1) one_rank_counts(next_row, num_experts, cap_m, masked_m, status);
+}
+__global__ void __launch_bounds__(kPlanThreads)
+plan_one_rank_kernel(const int64_t* __restrict__ ids, int64_t n, int num_experts, int cap_m, int32_t* __restrict__ masked_m,
+                     int64_t* __restrict__ dst_rank, int64_t* __restrict__ dst_row, int32_t* __restrict__ status)
+{
+    extern __shared__ long long next_row[];
+    for (int e = threadIdx.x; e < num_experts; e += blockDim.x) next_row[e] = static_cast<long long>(e) * cap_m;
+    one_rank_owners(ids, 0, n, num_experts, dst_rank);
+    hand_out_rows(ids, 0, n, num_experts, next_row, reinterpret_cast<unsigned short*>(next_row + num_experts),
+                  [&](int64_t e) { return (e + 1) * cap_m; }, dst_row);
+    __syncthreads();
+    one_rank_counts(next_row, num_experts, cap_m, masked_m, status);
 }
 
 // Fixed-capacity plan: every local expert owns `cap_m` rows of its rank's buffer (the masked layout of the GEMM),
@@ -564,7 +607,8 @@ plan_small_kernel(const int64_t* __restrict__ all_counts, int world, int num_exp
     extern __shared__ long long next_row[];
     plan_offsets(all_counts, world, num_experts, rank, cap_m, base, limit, masked_m, status, next_row);
     __syncthreads();
-    hand_out_rows(ids, 0, n, num_experts, next_row, reinterpret_cast<unsigned short*>(next_row + num_experts), limit, dst_row);
+    hand_out_rows(ids, 0, n, num_experts, next_row, reinterpret_cast<unsigned short*>(next_row + num_experts), [&](int64_t e) { return limit[e]; },
+                  dst_row);
 }
 
 // Barrier over the GPUs of one NVLink domain with a bounded wait.  `flag_peers[r]` is the address, in this process,
@@ -644,6 +688,28 @@ int launch_expert_histogram(const int64_t* ids, int64_t n, int num_experts, int6
     return NVFP4_OK;
 }
 
+// Two passes over chunks of whole 1024-pair steps, at most 128 of them.  base, limit == nullptr: one rank.
+static int plan_in_chunks(const int64_t* ids, int64_t n, int num_experts, const int64_t* base, const int64_t* limit, int cap_m, int32_t* masked_m,
+                          int64_t* dst_rank, int64_t* dst_row, int32_t* status, cudaStream_t stream)
+{
+    int64_t chunk = (n + 127) / 128;
+    chunk = (chunk + kPlanThreads - 1) / kPlanThreads * kPlanThreads;
+    const unsigned blocks = static_cast<unsigned>((n + chunk - 1) / chunk);
+    int dev = 0;
+    NVFP4_CUDA_CHECK(cudaGetDevice(&dev));
+    cudaMemPool_t pool;
+    if (int rc = host::workspace_pool(dev, &pool)) return rc;
+    int32_t* chunk_hist = nullptr;
+    NVFP4_CUDA_CHECK(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&chunk_hist), sizeof(int32_t) * blocks * num_experts, pool, stream));
+    plan_chunk_hist_kernel<<<blocks, kPlanThreads, num_experts * sizeof(int), stream>>>(ids, n, chunk, num_experts, chunk_hist);
+    plan_rows_kernel<<<blocks, kPlanThreads, plan_smem(num_experts), stream>>>(ids, n, chunk, num_experts, chunk_hist, base, limit, dst_row, cap_m,
+                                                                              masked_m, dst_rank, status);
+    const cudaError_t err = cudaGetLastError();
+    cudaFreeAsync(chunk_hist, stream);
+    if (err != cudaSuccess) return host::fail(NVFP4_E_CUDA, "plan kernels failed to launch: %s", cudaGetErrorString(err));
+    return NVFP4_OK;
+}
+
 int launch_plan_peer_masked(const int64_t* all_counts, int world, int num_experts, int rank, int cap_m, const int64_t* ids,
                             int64_t n, int64_t* base, int64_t* limit, int32_t* masked_m, int64_t* dst_row, int32_t* status,
                             cudaStream_t stream)
@@ -656,23 +722,15 @@ int launch_plan_peer_masked(const int64_t* all_counts, int world, int num_expert
     }
     plan_offsets_masked_kernel<<<1, 1024, 0, stream>>>(all_counts, world, num_experts, rank, cap_m, base, limit, masked_m, status);
     NVFP4_CUDA_CHECK(cudaGetLastError());
-    if (n == 0) return NVFP4_OK;
-    // chunks of whole 1024-pair steps, at most 128 of them
-    int64_t chunk = (n + 127) / 128;
-    chunk = (chunk + kPlanThreads - 1) / kPlanThreads * kPlanThreads;
-    const unsigned blocks = static_cast<unsigned>((n + chunk - 1) / chunk);
-    int dev = 0;
-    NVFP4_CUDA_CHECK(cudaGetDevice(&dev));
-    cudaMemPool_t pool;
-    if (int rc = host::workspace_pool(dev, &pool)) return rc;
-    int32_t* chunk_hist = nullptr;
-    NVFP4_CUDA_CHECK(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&chunk_hist), sizeof(int32_t) * blocks * num_experts, pool, stream));
-    plan_chunk_hist_kernel<<<blocks, kPlanThreads, num_experts * sizeof(int), stream>>>(ids, n, chunk, num_experts, chunk_hist);
-    plan_rows_kernel<<<blocks, kPlanThreads, plan_smem(num_experts), stream>>>(ids, n, chunk, num_experts, chunk_hist, base, limit,
-                                                                                      dst_row);
-    const cudaError_t err = cudaGetLastError();
-    cudaFreeAsync(chunk_hist, stream);
-    if (err != cudaSuccess) return host::fail(NVFP4_E_CUDA, "plan kernels failed to launch: %s", cudaGetErrorString(err));
+    return n == 0 ? static_cast<int>(NVFP4_OK) : plan_in_chunks(ids, n, num_experts, base, limit, cap_m, nullptr, nullptr, dst_row, status, stream);
+}
+
+int launch_plan_one_rank(const int64_t* ids, int64_t n, int num_experts, int cap_m, int32_t* masked_m, int64_t* dst_rank, int64_t* dst_row,
+                         int32_t* status, cudaStream_t stream)
+{
+    if (n > kPlanOnePass) return plan_in_chunks(ids, n, num_experts, nullptr, nullptr, cap_m, masked_m, dst_rank, dst_row, status, stream);
+    plan_one_rank_kernel<<<1, kPlanThreads, plan_smem(num_experts), stream>>>(ids, n, num_experts, cap_m, masked_m, dst_rank, dst_row, status);
+    NVFP4_CUDA_CHECK(cudaGetLastError());
     return NVFP4_OK;
 }
 
@@ -748,11 +806,18 @@ int launch_relayout_scales(const void* sf_rows, const int32_t* masked_m, int max
     if (rows == 0) return NVFP4_OK;
     // whole chunks of atoms, every row piece on a 16-byte boundary
     const bool wide = kdim % 512 == 0 && (reinterpret_cast<uintptr_t>(sf_rows) & 15u) == 0;
-    const int64_t blocks = rows / 128 * ((kdim / 64 + kRelayoutAtoms - 1) / kRelayoutAtoms);
+    const int64_t tiles = rows / 128 * ((kdim / 64 + kRelayoutAtoms - 1) / kRelayoutAtoms);
+    NVFP4_REQUIRE(tiles <= INT32_MAX, "too many rows (%lld)", static_cast<long long>(rows));
+    // eight blocks to an SM: where most row blocks are empty, or the decode kernels take the step, blocks that find nothing cost
+    // their launch (a layer of 256 tokens over 128 experts, which the decode kernels take: 7.7 us with a block per tile, 5.9 so).
+    host::DeviceInfo* dev;
+    if (int rc = host::device_info(-1, &dev)) return rc;
+    const int64_t most = static_cast<int64_t>(dev->hw_sms) * 8, blocks = tiles < most ? tiles : most;
     return host::launch_kernel(relayout_scales_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, pdl,
                                static_cast<const uint8_t*>(sf_rows), masked_m, static_cast<uint32_t>(max_m > 0 ? max_m : 1),
                                static_cast<uint32_t>(kdim), wide, static_cast<uint8_t*>(atoms),
-                               static_cast<uint32_t>(max_m > 0 ? rows / max_m : 0), gemm::Family{static_cast<uint32_t>(rival_tile), false});
+                               static_cast<uint32_t>(max_m > 0 ? rows / max_m : 0), gemm::Family{static_cast<uint32_t>(rival_tile), false},
+                               static_cast<uint32_t>(tiles));
 }
 
 }  // namespace nvfp4

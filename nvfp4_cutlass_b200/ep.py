@@ -112,6 +112,9 @@ def plan_dispatch_masked(topk_ids: torch.Tensor, num_experts: int, world: int, r
     flat = topk_ids.reshape(-1).contiguous()
     if flat.is_cuda:
         from . import _C
+        if world == 1:
+            masked_m, dst_rank, dst_row = _C.plan_one_rank(flat, num_experts, cap_m, status)
+            return MaskedDispatch(dst_rank=dst_rank, dst_row=dst_row, masked_m=masked_m)
         counts = _C.expert_histogram(flat, num_experts)
     else:
         counts = torch.zeros(num_experts, dtype=torch.int64).scatter_add_(0, flat, torch.ones_like(flat))

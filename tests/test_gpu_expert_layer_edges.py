@@ -40,3 +40,22 @@ def test_scale_relay_moves_every_byte(k):
     for block in range(e * max_m // 128):
         live = block * 128 % max_m < counts[block * 128 // max_m]
         assert torch.equal(got[block], want[block] if live else torch.full_like(got[block], 0xA5)), block
+
+
+@pytest.mark.parametrize("n,experts", [(0, 3), (1, 1), (1024, 512), (1025, 513), (8192, 64), (8193, 64), (20000, 600), (131072, 128)])
+@pytest.mark.parametrize("stray", [False, True])
+def test_one_rank_plan_is_the_plan_of_the_histogram(n, experts, stray):
+    """plan_one_rank counts while it hands out rows; ids out of range get owners out of range and no row."""
+    g = torch.Generator().manual_seed(n + experts)
+    ids = (torch.rand(n, generator=g) ** 2 * experts).long()
+    if stray:
+        ids[::7] = torch.tensor([-1, -experts - 1, experts, 2 * experts + 3]).repeat(n // 28 + 1)[:ids[::7].numel()]
+    valid, cap_m = (ids >= 0) & (ids < experts), 1024 if n > 20000 else 128
+    ids = ids.cuda()
+    counts = _C.expert_histogram(ids, experts)
+    status, want_status = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(2))
+    want_m, want_row = _C.plan_peer_masked(counts, ids, 1, 0, cap_m, want_status)
+    masked_m, dst_rank, dst_row = _C.plan_one_rank(ids, experts, cap_m, status)
+    assert torch.equal(masked_m, want_m) and int(status.item()) == int(want_status.item())
+    assert torch.equal(dst_rank, torch.div(ids, experts, rounding_mode="floor"))
+    assert torch.equal(dst_row.cpu()[valid], want_row.cpu()[valid])
