@@ -143,7 +143,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const uint32_t rank = ptx::cluster_cta_rank();
 
     if (threadIdx.x == 0) {
@@ -236,25 +236,26 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         // eight of them per K block were the larger half of the tensor-side time.
         // One thread runs the whole role.  A round takes the next K block and, if its scales are already up, the one
         // after it too: the fixed cost of a round (barrier round trips, loop) is then paid once per eight MMAs.
-        if (lane == 0) {
+        {
+            const uint32_t issue = ptx::elect_one();
             Ring rp;
             uint32_t acc_phase = 0;
             int32_t pending = -1;                   // ring position whose commit is still to be issued
             constexpr uint32_t idesc = ptx::make_idesc_nvf4(BM, BN);
             constexpr uint16_t kAllCtas = static_cast<uint16_t>((1u << CL) - 1u);
             for (uint32_t st = cid; st < num_super && ok; st += ncl) {
-                if (!ptx::mbar_wait(tmem_empty, acc_phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait(tmem_empty, acc_phase ^ 1, abort_flag, pa, 0))) { give_up(1); break; }
                 ptx::tcgen05_fence_after_sync();
                 uint32_t kb = 0;
                 while (kb < num_kb) {
                     // the scale warps arrive here only after they have seen this slot's P-full (acquired at cluster
                     // scope) and B-full complete, so this one wait also covers the operand tiles in shared memory
                     NVFP4_CTRACE(12, (st - cid) / ncl * num_kb + kb);
-                    if (!ptx::mbar_wait(sf_full + rp.slot, rp.phase, abort_flag, pa, 3)) { give_up(1); break; }
+                    if (!ptx::all_lanes(ptx::mbar_wait(sf_full + rp.slot, rp.phase, abort_flag, pa, 3))) { give_up(1); break; }
                     NVFP4_CTRACE(10, (st - cid) / ncl * num_kb + kb);
                     Ring r2 = rp;
                     r2.advance<C::kDepthP>();
-                    const uint32_t blocks = (kb + 1 < num_kb && ptx::mbar_try_wait(sf_full + r2.slot, r2.phase)) ? 2u : 1u;
+                    const uint32_t blocks = (kb + 1 < num_kb && ptx::all_lanes(ptx::mbar_try_wait(sf_full + r2.slot, r2.phase))) ? 2u : 1u;
                     ptx::tcgen05_fence_after_sync();
                     for (uint32_t u = 0; u < blocks; ++u, ++kb) {
                         // the 8-row groups of the two passes alternate: the stride between the row groups of one pass
@@ -267,20 +268,20 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                         for (uint32_t a = 0; a < kKAtoms; ++a) {
                             const uint64_t desc_b = ptx::make_smem_desc(b + a * 32, 512, ptx::kSwizzle64B);
                             ptx::tcgen05_mma_nvf4(tmem_base + kColAcc, ptx::make_smem_desc(a0 + a * 32, C::kGroupStride, ptx::kSwizzle64B),
-                                                  desc_b, idesc, sf + kSfA0 + 4 * a, sf + kSfB + 8 * a, (kb | a) != 0 ? 1u : 0u);
+                                                  desc_b, idesc, sf + kSfA0 + 4 * a, sf + kSfB + 8 * a, (kb | a) != 0 ? 1u : 0u, issue);
                             // One commit per K block, to every CTA of the cluster: it frees the P slot, the weight slot
                             // and the scale columns of a ring position.  A commit holds this thread until the MMAs before
                             // it have been handed to the tensor pipe; issued at the end of its own K block it leaves the
                             // pipe with nothing queued while this thread finds the next K block, so it goes out after the
                             // first MMA of the NEXT block.
-                            if (a == 0 && pending >= 0) ptx::tcgen05_commit_cluster(p_empty + pending, kAllCtas);
+                            if (a == 0 && pending >= 0) ptx::tcgen05_commit_cluster(p_empty + pending, kAllCtas, issue);
                             if constexpr (kResidual)
                                 ptx::tcgen05_mma_nvf4(tmem_base + kColAcc, ptx::make_smem_desc(a1 + a * 32, C::kGroupStride, ptx::kSwizzle64B),
-                                                      desc_b, idesc, sf + kSfA1 + 4 * a, sf + kSfB + 8 * a, 1u);
+                                                      desc_b, idesc, sf + kSfA1 + 4 * a, sf + kSfB + 8 * a, 1u, issue);
                         }
                         if (kb == num_kb - 1) {              // nothing follows in this tile: commit now
-                            ptx::tcgen05_commit_cluster(p_empty + rp.slot, kAllCtas);
-                            ptx::tcgen05_commit(tmem_full);
+                            ptx::tcgen05_commit_cluster(p_empty + rp.slot, kAllCtas, issue);
+                            ptx::tcgen05_commit(tmem_full, issue);
                         }
                         pending = kb == num_kb - 1 ? -1 : static_cast<int32_t>(rp.slot);
                         NVFP4_CTRACE(11, (st - cid) / ncl * num_kb + kb);

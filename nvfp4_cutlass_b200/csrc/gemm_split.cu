@@ -250,7 +250,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < C::kDepth; ++i) {
             ptx::mbar_init(full + i, 1);
@@ -320,18 +320,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
             if (ok && !gemm::drain_ring<C::kDepth, kGroup>(r, [&](uint32_t i, uint32_t parity) {
                     return ptx::mbar_wait(empty + i, parity, abort_flag, pa, 0); })) give_up(1);
         }
-    } else if (warp == kWarpMma && lane == 0) {
+    } else if (warp == kWarpMma) {
         // ================= MMA issue: one wait, 2 x kAtoms (x passes) MMAs, one commit per K block =================
+        const uint32_t issue = ptx::elect_one();
         Ring r;
         uint32_t acc_phase = 0;
         int32_t pending = -1;                       // group whose commit is still to be issued
         constexpr uint32_t idesc = ptx::make_idesc_nvf4(BM, BN);
-        for (uint32_t tile = blockIdx.x; ok && walk.next(tile, t); tile += gridDim.x) {
-            if (!ptx::mbar_wait(tmem_empty, acc_phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
+        for (uint32_t tile = blockIdx.x; ok && ptx::uniform(walk.next(tile, t)) != 0; tile += gridDim.x) {
+            if (!ptx::all_lanes(ptx::mbar_wait(tmem_empty, acc_phase ^ 1, abort_flag, pa, 0))) { give_up(1); break; }
             ptx::tcgen05_fence_after_sync();
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                if (!ptx::mbar_wait(sf_full + r.slot, r.phase, abort_flag, pa, 1) ||
-                    !ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 2)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait(sf_full + r.slot, r.phase, abort_flag, pa, 1) &&
+                                    ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 2))) { give_up(1); break; }
                 NVFP4_TRACE(3, (tile - blockIdx.x) / gridDim.x * num_kb + kb);
                 ptx::tcgen05_fence_after_sync();
                 const long long pt1 = ptx::probe_clock();
@@ -343,21 +344,21 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
                     const uint64_t desc_b = ptx::make_smem_desc(b + a * 32, C::kSBO, C::kSwizzle);
                     ptx::tcgen05_mma_nvf4(tmem_base + C::kColAcc, ptx::make_smem_desc(a0 + a * 32, C::kSBO, C::kSwizzle),
                                           desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass), sf + C::kSfB + 8 * a,
-                                          (kb | a) != 0 ? 1u : 0u);
+                                          (kb | a) != 0 ? 1u : 0u, issue);
                     if constexpr (kResidual)
                         ptx::tcgen05_mma_nvf4(tmem_base + C::kColAcc, ptx::make_smem_desc(a1 + a * 32, C::kSBO, C::kSwizzle),
-                                              desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass + 1), sf + C::kSfB + 8 * a, 1u);
+                                              desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass + 1), sf + C::kSfB + 8 * a, 1u, issue);
                     // A commit holds this thread until the MMAs before it have been handed to the tensor pipe.
                     // Issued at the end of a K block it would leave the pipe with nothing queued while this
                     // thread finds the next K block; issued after the first atom of the NEXT block it costs the
                     // ring positions a few hundred cycles but the pipe keeps its queue.
-                    if (a == 0 && pending >= 0) ptx::tcgen05_commit(empty + pending);
+                    if (a == 0 && pending >= 0) ptx::tcgen05_commit(empty + pending, issue);
                 }
                 const long long pt2 = ptx::probe_clock();
                 ptx::probe_count(pa, 5, pt2 - pt1);
                 if (kb == num_kb - 1) {
-                    if (r.slot % kGroup == kGroup - 1) ptx::tcgen05_commit(empty + r.slot / kGroup);
-                    ptx::tcgen05_commit(tmem_full);
+                    if (r.slot % kGroup == kGroup - 1) ptx::tcgen05_commit(empty + r.slot / kGroup, issue);
+                    ptx::tcgen05_commit(tmem_full, issue);
                 }
                 ptx::probe_count(pa, 6, ptx::probe_clock() - pt2);
                 // a group is complete with its last ring position; at a tile end it has been committed above
@@ -647,7 +648,7 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
     uint32_t* num_units_slot = tmem_slot + 2;
     uint16_t* units = reinterpret_cast<uint16_t*>(smem_gen + C::kOffUnits);
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const uint32_t rank = ptx::cluster_cta_rank();   // 0: leader (issues the MMAs), 1: peer
     const uint32_t pair_id = ptx::cluster_id_x(), num_pairs = ptx::num_clusters_x();
     if (threadIdx.x == 0) {
@@ -730,18 +731,19 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         }
     } else if (warp == kWarpMma) {
         // ================= MMA issue (leader only) =================
-        if (rank == 0 && lane == 0) {
+        if (rank == 0) {
+            const uint32_t issue = ptx::elect_one();
             Ring r;
             uint32_t acc_phase = 0;
             int32_t pending = -1;                   // ring position whose commit is still to be issued
             constexpr uint32_t idesc = ptx::make_idesc_nvf4(2 * BM, BN);
             constexpr uint16_t kBoth = 3;
-            for (uint32_t tile = pair_id; ok && walk.next(tile, t); tile += num_pairs) {
-                if (!ptx::mbar_wait(tmem_empty, acc_phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
+            for (uint32_t tile = pair_id; ok && ptx::uniform(walk.next(tile, t)) != 0; tile += num_pairs) {
+                if (!ptx::all_lanes(ptx::mbar_wait(tmem_empty, acc_phase ^ 1, abort_flag, pa, 0))) { give_up(1); break; }
                 ptx::tcgen05_fence_after_sync();
                 for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                    if (!ptx::mbar_wait(sf_full + r.slot, r.phase, abort_flag, pa, 1) ||
-                        !ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 2)) { give_up(1); break; }
+                    if (!ptx::all_lanes(ptx::mbar_wait(sf_full + r.slot, r.phase, abort_flag, pa, 1) &&
+                                        ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 2))) { give_up(1); break; }
                     NVFP4_TRACE(3, (tile - pair_id) / num_pairs * num_kb + kb);
                     ptx::tcgen05_fence_after_sync();
                     const uint32_t a0 = smem + C::kOffA + r.slot * C::kStage, a1 = a0 + C::kSlotA;
@@ -752,17 +754,17 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
                         const uint64_t desc_b = ptx::make_smem_desc(b + a * 32, C::kSBO, C::kSwizzle);
                         ptx::tcgen05_mma_nvf4_pair(tmem_base + C::kColAcc, ptx::make_smem_desc(a0 + a * 32, C::kSBO, C::kSwizzle),
                                                    desc_b, idesc, sf + C::kSfA + 4 * (a * C::kPass), sf + C::kSfB + 8 * a,
-                                                   (kb | a) != 0 ? 1u : 0u);
+                                                   (kb | a) != 0 ? 1u : 0u, issue);
                         if constexpr (kResidual)
                             ptx::tcgen05_mma_nvf4_pair(tmem_base + C::kColAcc,
                                                        ptx::make_smem_desc(a1 + a * 32, C::kSBO, C::kSwizzle), desc_b, idesc,
-                                                       sf + C::kSfA + 4 * (a * C::kPass + 1), sf + C::kSfB + 8 * a, 1u);
+                                                       sf + C::kSfA + 4 * (a * C::kPass + 1), sf + C::kSfB + 8 * a, 1u, issue);
                         // as in the single-CTA kernel: the commit of a K block goes out after the first atom of the next
-                        if (a == 0 && pending >= 0) ptx::tcgen05_commit_pair(empty + pending, kBoth);
+                        if (a == 0 && pending >= 0) ptx::tcgen05_commit_pair(empty + pending, kBoth, issue);
                     }
                     if (kb == num_kb - 1) {
-                        ptx::tcgen05_commit_pair(empty + r.slot, kBoth);
-                        ptx::tcgen05_commit_pair(tmem_full, kBoth);
+                        ptx::tcgen05_commit_pair(empty + r.slot, kBoth, issue);
+                        ptx::tcgen05_commit_pair(tmem_full, kBoth, issue);
                     }
                     pending = kb != num_kb - 1 ? static_cast<int32_t>(r.slot) : -1;
                     NVFP4_TRACE(4, (tile - pair_id) / num_pairs * num_kb + kb);

@@ -87,7 +87,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < C::kDepth; ++i) { ptx::mbar_init(full + i, 1); ptx::mbar_init(empty + i, 1); }
         for (uint32_t i = 0; i < 2; ++i) {
@@ -157,19 +157,20 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
             if (ok && !gemm::drain_ring<C::kDepth>(r, [&](uint32_t i, uint32_t parity) {
                     return ptx::mbar_wait(empty + i, parity, abort_flag, pa, 0); })) give_up(1);
         }
-    } else if (warp == kWarpMma && lane == 0) {
+    } else if (warp == kWarpMma) {
+        const uint32_t issue = ptx::elect_one();
         Ring r;
         uint32_t it = 0, cnt = 0;
         constexpr uint32_t idesc = ptx::make_idesc_nvf4(BW, C::kRowsP);
-        for (uint32_t tile = blockIdx.x; ok && walk.next(tile, t); tile += gridDim.x, ++it) {
+        for (uint32_t tile = blockIdx.x; ok && ptx::uniform(walk.next(tile, t)) != 0; tile += gridDim.x, ++it) {
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-            if (!ptx::mbar_wait(tmem_empty + acc, acc_phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
+            if (!ptx::all_lanes(ptx::mbar_wait(tmem_empty + acc, acc_phase ^ 1, abort_flag, pa, 0))) { give_up(1); break; }
             ptx::tcgen05_fence_after_sync();
             const uint32_t tmem_acc = tmem_base + acc * C::kAccStride;
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++cnt) {
                 const uint32_t buf = cnt & 1u;
-                if (!ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 1) ||
-                    !ptx::mbar_wait(sf_full + buf, (cnt >> 1) & 1u, abort_flag, pa, 2)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait(full + r.slot, r.phase, abort_flag, pa, 1) &&
+                                    ptx::mbar_wait(sf_full + buf, (cnt >> 1) & 1u, abort_flag, pa, 2))) { give_up(1); break; }
                 ptx::tcgen05_fence_after_sync();
                 const uint32_t w = smem + C::kOffW + r.slot * C::kSlotW, a = smem + C::kOffP + r.slot * C::kSlotP;
                 const uint32_t sf = tmem_base + C::kColSF + buf * C::kSfBufCols;
@@ -177,9 +178,9 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
                 for (uint32_t i = 0; i < C::kAtoms; ++i)
                     ptx::tcgen05_mma_nvf4(tmem_acc, ptx::make_smem_desc(w + (i / 4) * C::kSubW + (i % 4) * 32, C::kSBO, ptx::kSwizzle128B),
                                           ptx::make_smem_desc(a + (i / 4) * C::kSubP + (i % 4) * 32, C::kSBO, ptx::kSwizzle128B), idesc,
-                                          sf + C::kSfW + 4 * i, sf + C::kSfT + 4 * i, (kb | i) != 0 ? 1u : 0u);
-                ptx::tcgen05_commit(empty + r.slot);       // frees the ring position and the block's scale columns
-                if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full + acc);
+                                          sf + C::kSfW + 4 * i, sf + C::kSfT + 4 * i, (kb | i) != 0 ? 1u : 0u, issue);
+                ptx::tcgen05_commit(empty + r.slot, issue);       // frees the ring position and the block's scale columns
+                if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full + acc, issue);
                 r.advance<C::kDepth>();
             }
         }

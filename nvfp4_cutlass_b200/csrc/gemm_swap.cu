@@ -152,7 +152,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (uint32_t i = 0; i < C::kDepthW; ++i) {
             ptx::mbar_init(w_full + i, 1);
@@ -239,21 +239,22 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             if (kGeneral && ok && !gemm::drain_ring<C::kDepthP>(rp, [&](uint32_t i, uint32_t parity) {
                     return ptx::mbar_wait(p_empty + i, parity, abort_flag, pa, 0); })) give_up(1);
         }
-    } else if (warp == kWarpMma && lane == 0) {
+    } else if (warp == kWarpMma) {
+        const uint32_t issue_lane = ptx::elect_one();
         Ring rw, rp, rp0;                            // rp0: where the token tile begins
         uint32_t it = 0, cnt = 0;
         constexpr uint32_t idesc = ptx::make_idesc_nvf4(BW, C::kRowsP);
         for (; ok && walk.next(); ++it) {
             if constexpr (kGeneral) { if (walk.fresh) rp0 = rp; else rp = rp0; }
             const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-            if (!ptx::mbar_wait(tmem_empty + acc, acc_phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
+            if (!ptx::all_lanes(ptx::mbar_wait(tmem_empty + acc, acc_phase ^ 1, abort_flag, pa, 0))) { give_up(1); break; }
             ptx::tcgen05_fence_after_sync();
             const uint32_t tmem_acc = tmem_base + acc * C::kAccStride;
             for (uint32_t kb = 0; kb < num_kb; ++kb, ++cnt) {
                 const uint32_t buf = cnt & 1u;
-                if (!ptx::mbar_wait(p_full + rp.slot, rp.phase, abort_flag, pa, 1) ||
-                    !ptx::mbar_wait(w_full + rw.slot, rw.phase, abort_flag, pa, 2) ||
-                    !ptx::mbar_wait(sf_full + buf, (cnt >> 1) & 1u, abort_flag, pa, 3)) { give_up(1); break; }
+                if (!ptx::all_lanes(ptx::mbar_wait(p_full + rp.slot, rp.phase, abort_flag, pa, 1) &&
+                                    ptx::mbar_wait(w_full + rw.slot, rw.phase, abort_flag, pa, 2) &&
+                                    ptx::mbar_wait(sf_full + buf, (cnt >> 1) & 1u, abort_flag, pa, 3))) { give_up(1); break; }
                 ptx::tcgen05_fence_after_sync();
                 // the scales are already in tensor memory (scale warps, tcgen05.st): a tensor-memory copy per
                 // scale atom cost this thread as much issue time as an MMA, and there were two per K atom
@@ -264,7 +265,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 auto issue = [&](uint32_t a) {
                     ptx::tcgen05_mma_nvf4(tmem_acc, ptx::make_smem_desc(w + (a / 4) * C::kSubW + (a % 4) * 32, C::kSBO, C::kSwizzle),
                                           ptx::make_smem_desc(pt + (a / 4) * C::kSubP + (a % 4) * 32, C::kSBO, C::kSwizzle), idesc,
-                                          sf + C::kSfW + 4 * a, sf + C::kSfT + 4 * a, (kb | a) != 0 ? 1u : 0u);
+                                          sf + C::kSfW + 4 * a, sf + C::kSfT + 4 * a, (kb | a) != 0 ? 1u : 0u, issue_lane);
                 };
                 if (!kGeneral || atoms >= C::kAtoms) {
 #pragma unroll
@@ -274,9 +275,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     for (uint32_t a = 0; a < atoms; ++a) issue(a);
                 }
                 // the weight producer and the scale warps both read "the MMAs of K block i have retired" from this barrier
-                ptx::tcgen05_commit(w_empty + rw.slot);
-                if (kGeneral && walk.done) ptx::tcgen05_commit(p_empty + rp.slot);
-                if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full + acc);
+                ptx::tcgen05_commit(w_empty + rw.slot, issue_lane);
+                if (kGeneral && walk.done) ptx::tcgen05_commit(p_empty + rp.slot, issue_lane);
+                if (kb == num_kb - 1) ptx::tcgen05_commit(tmem_full + acc, issue_lane);
                 rp.advance<C::kDepthP>();
                 rw.advance<C::kDepthW>();
             }

@@ -198,10 +198,27 @@ NVFP4_DEVICE void tmem_dealloc(uint32_t taddr)
 NVFP4_DEVICE void tcgen05_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 NVFP4_DEVICE void tcgen05_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// All earlier tcgen05.mma / tcgen05.cp of this thread arrive (once) on `bar` when they retire.
-NVFP4_DEVICE void tcgen05_commit(uint64_t* bar)
+// One lane of the warp, always the same; every lane calls it.
+NVFP4_DEVICE uint32_t elect_one()
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+    uint32_t r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
+}
+// The same value for the whole warp as far as the compiler is concerned: what is computed from it stays in uniform registers.
+NVFP4_DEVICE uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// All earlier tcgen05.mma / tcgen05.cp of this thread arrive (once) on `bar` when they retire.
+// `issue`: in a role that the whole warp runs, nonzero in the lane that issues (elect_one), for MMAs as for commits.  The operands of
+// tcgen05 instructions live in uniform registers; in a branch of a single lane they are kept in the lane's own and moved for every
+// MMA, and the issuing thread, not the tensor pipe, set the pace (1300 cycles of it per K block of 256 in gemm_split.cu, whose
+// MMAs take 1024; 1240 for eight MMAs of a decode K block, which take 430).  One lane / the whole warp: decode of 128 tokens (32 experts, N =
+// 2048, K = 512) 7.4 / 6.6 us, of 25 tokens of 208 experts (N = 640, K = 4480) 39.5 / 33.3, expert layer of 16384 tokens 2889 / 2793,
+// 32k zipf rows, N = 7168, K = 2048, one pass, 653 / 639.
+NVFP4_DEVICE void tcgen05_commit(uint64_t* bar, uint32_t issue = 1)
+{
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+                 " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar)), "r"(issue)
                  : "memory");
 }
 
@@ -215,15 +232,16 @@ NVFP4_DEVICE void tcgen05_cp_32x128b_warpx4(uint32_t taddr, uint64_t smem_desc)
 // D[tmem] (+)= A[smem] * B[smem] with per-16-element E4M3 block scales read from TMEM.
 // E2M1 operands, K = 64 per instruction.
 NVFP4_DEVICE void tcgen05_mma_nvf4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                   uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate)
+                                   uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate, uint32_t issue = 1)
 {
     asm volatile(
         "{\n"
-        " .reg .pred p;\n"
+        " .reg .pred p, q;\n"
         " setp.ne.b32 p, %6, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%4], [%5], p;\n"
+        " setp.ne.b32 q, %7, 0;\n"
+        " @q tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%4], [%5], p;\n"
         "}\n" ::"r"(tmem_d),
-        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate)
+        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate), "r"(issue)
         : "memory");
 }
 
@@ -480,10 +498,11 @@ NVFP4_DEVICE bool mbar_wait_sleep(uint64_t* bar, uint32_t parity, volatile uint3
 }
 // All earlier tcgen05 operations of this thread arrive, when they retire, on the barrier at
 // this offset in every CTA of the cluster named by `cta_mask`.
-NVFP4_DEVICE void tcgen05_commit_cluster(uint64_t* bar, uint16_t cta_mask)
+NVFP4_DEVICE void tcgen05_commit_cluster(uint64_t* bar, uint16_t cta_mask, uint32_t issue = 1)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"(cta_mask)
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n"
+                 " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}\n"
+                 ::"r"(smem_u32(bar)), "h"(cta_mask), "r"(issue)
                  : "memory");
 }
 // Bulk copy of `bytes` (multiple of 16, both addresses 16-byte aligned) from this CTA's shared
@@ -526,23 +545,25 @@ NVFP4_DEVICE void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint3
 // memory at the descriptor's offset), N up to 256 (each CTA holds half of the rows of B), block scales from each
 // CTA's own tensor memory (SFA of its rows, SFB of all N).  Issued by one thread of the pair's even CTA.
 NVFP4_DEVICE void tcgen05_mma_nvf4_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                        uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate)
+                                        uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate, uint32_t issue = 1)
 {
     asm volatile(
         "{\n"
-        " .reg .pred p;\n"
+        " .reg .pred p, q;\n"
         " setp.ne.b32 p, %6, 0;\n"
-        " tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%4], [%5], p;\n"
+        " setp.ne.b32 q, %7, 0;\n"
+        " @q tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%4], [%5], p;\n"
         "}\n" ::"r"(tmem_d),
-        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate)
+        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate), "r"(issue)
         : "memory");
 }
 // All earlier pair MMAs of this thread arrive, when they retire, on the barrier at this offset in the CTAs of
 // the cluster named by `cta_mask`.
-NVFP4_DEVICE void tcgen05_commit_pair(uint64_t* bar, uint16_t cta_mask)
+NVFP4_DEVICE void tcgen05_commit_pair(uint64_t* bar, uint16_t cta_mask, uint32_t issue = 1)
 {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"(cta_mask)
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n"
+                 " @q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}\n"
+                 ::"r"(smem_u32(bar)), "h"(cta_mask), "r"(issue)
                  : "memory");
 }
 
