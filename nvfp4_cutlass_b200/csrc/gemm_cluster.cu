@@ -460,6 +460,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                     w[j][0] = lo.x; w[j][1] = lo.y; w[j][2] = lo.z; w[j][3] = lo.w;
                     w[j][4] = hi.x; w[j][5] = hi.y; w[j][6] = hi.z; w[j][7] = hi.w;
                 }
+                ptx::fence_proxy_async_smem();                        // the loads are over before TMA may rewrite the slot
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(a_empty + ra.slot);   // the tile now lives in registers
                 const long long xt1 = ptx::probe_clock();

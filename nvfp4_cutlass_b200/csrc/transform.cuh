@@ -294,6 +294,7 @@ NVFP4_DEVICE void transform_tile(uint32_t a_smem, uint32_t a0_smem, uint32_t a1_
 {
     TileShare<kRows, kBK, kThreads> s;
     load_tile_smem(s, a_smem, t);
+    ptx::fence_proxy_async_smem();   // the loads are over before on_loaded hands the slot back to the TMA that rewrites it
     on_loaded();
     emit_tile<kRows, kBK, kThreads, kResidual, kSfCols, kSubRows, kPolicy>(s, a0_smem, a1_smem, sfa0_smem, sfa1_smem, t);
 }
