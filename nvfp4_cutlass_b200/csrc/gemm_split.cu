@@ -291,34 +291,35 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_consta
 
     if (warp == kWarpTma) {
         // ================= producer: every operand of a K block on one barrier =================
-        if (lane == 0) {
+        {
+            const uint32_t issue = ptx::elect_one();
             Ring r;
-            for (uint32_t tile = blockIdx.x; ok && walk.next(tile, t); tile += gridDim.x) {
-                const uint32_t n_blk = t.n_blk;
-                const int32_t e = t.expert;
-                const uint8_t* sfa_row = p.sfa + static_cast<uint64_t>(t.row0 / BM) * (p.k / 64) * (C::kPass * 512);
+            for (uint32_t tile = blockIdx.x; ok && ptx::uniform(walk.next(tile, t)) != 0; tile += gridDim.x) {
+                const uint32_t n_blk = ptx::uniform(t.n_blk), row0 = ptx::uniform(t.row0);
+                const int32_t e = static_cast<int32_t>(ptx::uniform(static_cast<uint32_t>(t.expert)));
+                const uint8_t* sfa_row = p.sfa + static_cast<uint64_t>(row0 / BM) * (p.k / 64) * (C::kPass * 512);
                 for (uint32_t kb = 0; kb < num_kb; ++kb) {
                     if (r.slot % kGroup == 0 &&
-                        !ptx::mbar_wait(empty + r.slot / kGroup, r.phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
+                        !ptx::all_lanes(ptx::mbar_wait(empty + r.slot / kGroup, r.phase ^ 1, abort_flag, pa, 0))) { give_up(1); break; }
                     NVFP4_TRACE(0, (tile - blockIdx.x) / gridDim.x * num_kb + kb);
-                    ptx::mbar_arrive_expect_tx(sf_in + r.slot, C::kSlotSFA + C::kSlotSFB);
+                    ptx::mbar_arrive_expect_tx(sf_in + r.slot, C::kSlotSFA + C::kSlotSFB, issue);
                     ptx::tma_load_2d(smem_gen + C::kOffSFB + r.slot * C::kSlotSFB, &tm_sfb, sf_in + r.slot, n_blk * BN,
-                                     e * (p.k / 64) + kb * C::kAtoms);
+                                     e * (p.k / 64) + kb * C::kAtoms, issue);
                     ptx::bulk_load(smem_gen + C::kOffSFA + r.slot * C::kSlotSFA,
-                                   sfa_row + static_cast<uint64_t>(kb) * C::kSlotSFA, C::kSlotSFA, sf_in + r.slot);
-                    ptx::mbar_arrive_expect_tx(full + r.slot, C::kPass * C::kSlotA + C::kSlotB);
+                                   sfa_row + static_cast<uint64_t>(kb) * C::kSlotSFA, C::kSlotSFA, sf_in + r.slot, issue);
+                    ptx::mbar_arrive_expect_tx(full + r.slot, C::kPass * C::kSlotA + C::kSlotB, issue);
                     uint8_t* a_dst = smem_gen + C::kOffA + r.slot * C::kPass * C::kSlotA;
-                    ptx::tma_load_2d(a_dst, &tm_a0, full + r.slot, kb * C::kRowBytes, t.row0);
+                    ptx::tma_load_2d(a_dst, &tm_a0, full + r.slot, kb * C::kRowBytes, row0, issue);
                     if constexpr (kResidual)
-                        ptx::tma_load_2d(a_dst + C::kSlotA, &tm_a1, full + r.slot, kb * C::kRowBytes, t.row0);
+                        ptx::tma_load_2d(a_dst + C::kSlotA, &tm_a1, full + r.slot, kb * C::kRowBytes, row0, issue);
                     ptx::tma_load_2d(smem_gen + C::kOffB + r.slot * C::kSlotB, &tm_b, full + r.slot, kb * C::kRowBytes,
-                                     e * p.n + n_blk * BN);
+                                     e * p.n + n_blk * BN, issue);
                     r.advance<C::kDepth>();
                 }
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
             if (ok && !gemm::drain_ring<C::kDepth, kGroup>(r, [&](uint32_t i, uint32_t parity) {
-                    return ptx::mbar_wait(empty + i, parity, abort_flag, pa, 0); })) give_up(1);
+                    return ptx::all_lanes(ptx::mbar_wait(empty + i, parity, abort_flag, pa, 0)); })) give_up(1);
         }
     } else if (warp == kWarpMma) {
         // ================= MMA issue: one wait, 2 x kAtoms (x passes) MMAs, one commit per K block =================
@@ -696,30 +697,31 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
 
     if (warp == kWarpTma) {
         // ================= producer =================
-        if (lane == 0) {
+        {
+            const uint32_t issue = ptx::elect_one();
             Ring r, rs;
             const uint32_t full_leader = ptx::map_to_cta(ptx::smem_u32(full), 0);
-            for (uint32_t tile = pair_id; ok && walk.next(tile, t); tile += num_pairs) {
-                const uint32_t row0 = my_row0(t);
+            for (uint32_t tile = pair_id; ok && ptx::uniform(walk.next(tile, t)) != 0; tile += num_pairs) {
+                const uint32_t row0 = ptx::uniform(my_row0(t)), n_blk = ptx::uniform(t.n_blk), e = ptx::uniform(static_cast<uint32_t>(t.expert));
                 const uint8_t* sfa_row = p.sfa + static_cast<uint64_t>(row0 / BM) * (p.k / 64) * (C::kPass * 512);
                 for (uint32_t kb = 0; kb < num_kb; ++kb) {
                     // the roles that run ahead sleep between polls: every poll is an instruction of the shared-memory pipe
-                    if (!ptx::mbar_wait_sleep<false>(empty + r.slot, r.phase ^ 1, abort_flag, PAIR_SLEEP_TMA, pa, 0)) { give_up(1); break; }
-                    if (!ptx::mbar_wait_sleep<false>(sf_free + rs.slot, rs.phase ^ 1, abort_flag, PAIR_SLEEP_TMA, pa, 0)) { give_up(1); break; }
+                    if (!ptx::all_lanes(ptx::mbar_wait_sleep<false>(empty + r.slot, r.phase ^ 1, abort_flag, PAIR_SLEEP_TMA, pa, 0))) { give_up(1); break; }
+                    if (!ptx::all_lanes(ptx::mbar_wait_sleep<false>(sf_free + rs.slot, rs.phase ^ 1, abort_flag, PAIR_SLEEP_TMA, pa, 0))) { give_up(1); break; }
                     NVFP4_TRACE(0, (tile - pair_id) / num_pairs * num_kb + kb);
                     uint8_t* sf_dst = smem_gen + C::kOffSf + rs.slot * C::kSfStage;
-                    ptx::mbar_arrive_expect_tx(sf_in + rs.slot, C::kSfStage);
-                    ptx::tma_load_2d(sf_dst + C::kSlotSFA, &tm_sfb, sf_in + rs.slot, t.n_blk * BN,
-                                     t.expert * (p.k / 64) + kb * C::kAtoms);
-                    ptx::bulk_load(sf_dst, sfa_row + static_cast<uint64_t>(kb) * C::kSlotSFA, C::kSlotSFA, sf_in + rs.slot);
+                    ptx::mbar_arrive_expect_tx(sf_in + rs.slot, C::kSfStage, issue);
+                    ptx::tma_load_2d(sf_dst + C::kSlotSFA, &tm_sfb, sf_in + rs.slot, n_blk * BN,
+                                     e * (p.k / 64) + kb * C::kAtoms, issue);
+                    ptx::bulk_load(sf_dst, sfa_row + static_cast<uint64_t>(kb) * C::kSlotSFA, C::kSlotSFA, sf_in + rs.slot, issue);
                     // the leader announces the operand bytes of both CTAs; the peer's bytes complete on the leader's barrier
-                    if (rank == 0) ptx::mbar_arrive_expect_tx(full + r.slot, 2 * (C::kPass * C::kSlotA + C::kSlotB));
+                    if (rank == 0) ptx::mbar_arrive_expect_tx(full + r.slot, 2 * (C::kPass * C::kSlotA + C::kSlotB), issue);
                     const uint32_t bar = full_leader + r.slot * 8;
                     uint8_t* a_dst = smem_gen + C::kOffA + r.slot * C::kStage;
-                    ptx::tma_load_2d_pair(a_dst, &tm_a0, bar, kb * C::kRowBytes, row0);
-                    if constexpr (kResidual) ptx::tma_load_2d_pair(a_dst + C::kSlotA, &tm_a1, bar, kb * C::kRowBytes, row0);
+                    ptx::tma_load_2d_pair(a_dst, &tm_a0, bar, kb * C::kRowBytes, row0, issue);
+                    if constexpr (kResidual) ptx::tma_load_2d_pair(a_dst + C::kSlotA, &tm_a1, bar, kb * C::kRowBytes, row0, issue);
                     ptx::tma_load_2d_pair(a_dst + C::kPass * C::kSlotA, &tm_b, bar, kb * C::kRowBytes,
-                                          t.expert * p.n + t.n_blk * BN + rank * (BN / 2));
+                                          e * p.n + n_blk * BN + rank * (BN / 2), issue);
                     r.advance<C::kDepth>();
                     rs.advance<C::kDepthSf>();
                 }
@@ -727,7 +729,7 @@ gemm_split_pair_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
             ptx::grid_launch_dependents();
             // the leader's commits arrive in both CTAs
             if (ok && !gemm::drain_ring<C::kDepth>(r, [&](uint32_t i, uint32_t parity) {
-                    return ptx::mbar_wait_sleep<false>(empty + i, parity, abort_flag, PAIR_SLEEP_TMA, pa, 0); })) give_up(1);
+                    return ptx::all_lanes(ptx::mbar_wait_sleep<false>(empty + i, parity, abort_flag, PAIR_SLEEP_TMA, pa, 0)); })) give_up(1);
         }
     } else if (warp == kWarpMma) {
         // ================= MMA issue (leader only) =================

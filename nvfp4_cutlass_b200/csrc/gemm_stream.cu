@@ -126,36 +126,38 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_const
     };
 
     if (warp == kWarpTma) {
-        if (lane == 0) {
+        {
+            const uint32_t issue = ptx::elect_one();
             Ring r;
             const uint64_t stream_once = ptx::l2_policy_evict_first();
-            for (uint32_t tile = blockIdx.x; ok && walk.next(tile, t); tile += gridDim.x) {
-                const uint32_t w_row = t.expert * p.n + t.n_blk * BW;
+            for (uint32_t tile = blockIdx.x; ok && ptx::uniform(walk.next(tile, t)) != 0; tile += gridDim.x) {
+                const uint32_t e = ptx::uniform(static_cast<uint32_t>(t.expert)), n_blk = ptx::uniform(t.n_blk), row0 = ptx::uniform(t.row0);
+                const uint32_t w_row = e * p.n + n_blk * BW;
                 for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                    if (!ptx::mbar_wait(empty + r.slot, r.phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
+                    if (!ptx::all_lanes(ptx::mbar_wait(empty + r.slot, r.phase ^ 1, abort_flag, pa, 0))) { give_up(1); break; }
                     uint64_t* bar = full + r.slot;
-                    ptx::mbar_arrive_expect_tx(bar, C::kSlot);
+                    ptx::mbar_arrive_expect_tx(bar, C::kSlot, issue);
                     uint8_t* w = smem_gen + C::kOffW + r.slot * C::kSlotW;
                     uint8_t* a = smem_gen + C::kOffP + r.slot * C::kSlotP;
                     uint8_t* sft = smem_gen + C::kOffSFT + r.slot * C::kSlotSFT;
-                    ptx::tma_load_2d_hint(smem_gen + C::kOffSFW + r.slot * C::kSlotSFW, &tm_sfw, bar, t.n_blk * BW,
-                                          t.expert * (p.k / 64) + kb * C::kAtoms, stream_once);
+                    ptx::tma_load_2d_hint(smem_gen + C::kOffSFW + r.slot * C::kSlotSFW, &tm_sfw, bar, n_blk * BW,
+                                          e * (p.k / 64) + kb * C::kAtoms, stream_once, issue);
 #pragma unroll
                     for (uint32_t sub = 0; sub < C::kSubs; ++sub) {
                         const uint32_t col = kb * (BK / 2) + sub * 128;
-                        ptx::tma_load_2d_hint(w + sub * C::kSubW, &tm_w, bar, col, w_row, stream_once);
-                        ptx::tma_load_2d(a + sub * C::kSubP, &tm_a0, bar, col, t.row0);
-                        if constexpr (kResidual) ptx::tma_load_2d(a + sub * C::kSubP + T * 128, &tm_a1, bar, col, t.row0);
+                        ptx::tma_load_2d_hint(w + sub * C::kSubW, &tm_w, bar, col, w_row, stream_once, issue);
+                        ptx::tma_load_2d(a + sub * C::kSubP, &tm_a0, bar, col, row0, issue);
+                        if constexpr (kResidual) ptx::tma_load_2d(a + sub * C::kSubP + T * 128, &tm_a1, bar, col, row0, issue);
                     }
 #pragma unroll
                     for (uint32_t pass = 0; pass < C::kPass; ++pass)
-                        ptx::tma_load_2d(sft + pass * T * C::kAtoms * 4, &tm_sft, bar, pass * (p.k / 64) + kb * C::kAtoms, t.row0);
+                        ptx::tma_load_2d(sft + pass * T * C::kAtoms * 4, &tm_sft, bar, pass * (p.k / 64) + kb * C::kAtoms, row0, issue);
                     r.advance<C::kDepth>();
                 }
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
             if (ok && !gemm::drain_ring<C::kDepth>(r, [&](uint32_t i, uint32_t parity) {
-                    return ptx::mbar_wait(empty + i, parity, abort_flag, pa, 0); })) give_up(1);
+                    return ptx::all_lanes(ptx::mbar_wait(empty + i, parity, abort_flag, pa, 0)); })) give_up(1);
         }
     } else if (warp == kWarpMma) {
         const uint32_t issue = ptx::elect_one();

@@ -196,48 +196,50 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 
     if (warp == kWarpTma) {
         // weight producer: runs ahead by the full depth of the W ring, whatever the transform does
-        if (lane == 0) {
+        {
+            const uint32_t issue = ptx::elect_one();
             Ring rw;
             const uint64_t stream_once = ptx::l2_policy_evict_first();
             while (ok && walk.next()) {
                 const uint32_t n_blk = walk.n_blk;
-                const int32_t e = max(0, __ldg(p.m_indices + walk.m_blk * T));
+                const uint32_t e = ptx::uniform(static_cast<uint32_t>(max(0, __ldg(p.m_indices + walk.m_blk * T))));
                 for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                    if (!ptx::mbar_wait(w_empty + rw.slot, rw.phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
-                    ptx::mbar_arrive_expect_tx(w_full + rw.slot, C::kSlotW + C::kSlotSFW);
+                    if (!ptx::all_lanes(ptx::mbar_wait(w_empty + rw.slot, rw.phase ^ 1, abort_flag, pa, 0))) { give_up(1); break; }
+                    ptx::mbar_arrive_expect_tx(w_full + rw.slot, C::kSlotW + C::kSlotSFW, issue);
 #pragma unroll
                     for (uint32_t sub = 0; sub < (BK / 2) / C::kRowBytes; ++sub)
                         ptx::tma_load_2d_hint(smem_gen + C::kOffW + rw.slot * C::kSlotW + sub * C::kSubW, &tm_w, w_full + rw.slot,
-                                              kb * (BK / 2) + sub * C::kRowBytes, e * p.n + n_blk * BW, stream_once);
+                                              kb * (BK / 2) + sub * C::kRowBytes, e * p.n + n_blk * BW, stream_once, issue);
                     ptx::tma_load_2d_hint(smem_gen + C::kOffSFW + rw.slot * C::kSlotSFW, &tm_sfw, w_full + rw.slot,
-                                          n_blk * BW, e * (p.k / 64) + kb * C::kAtoms, stream_once);
+                                          n_blk * BW, e * (p.k / 64) + kb * C::kAtoms, stream_once, issue);
                     rw.advance<C::kDepthW>();
                 }
             }
             ptx::grid_launch_dependents();          // the last loads are on their way: the next kernel may start its prologue
             if (ok && !gemm::drain_ring<C::kDepthW>(rw, [&](uint32_t i, uint32_t parity) {
-                    return ptx::mbar_wait(w_empty + i, parity, abort_flag, pa, 0); })) give_up(1);
+                    return ptx::all_lanes(ptx::mbar_wait(w_empty + i, parity, abort_flag, pa, 0)); })) give_up(1);
         }
     } else if (warp == kWarpTmaA) {
         // activation producer (a separate thread, so a full A ring never holds the weights back)
-        if (lane == 0) {
+        {
+            const uint32_t issue = ptx::elect_one();
             Ring ra, rp;
             while (ok && walk.next()) {
                 if (kGeneral && !walk.fresh) continue;
                 for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                    if (!ptx::mbar_wait(a_empty + ra.slot, ra.phase ^ 1, abort_flag, pa, 0)) { give_up(1); break; }
-                    ptx::mbar_arrive_expect_tx(a_full + ra.slot, C::kSlotA);
+                    if (!ptx::all_lanes(ptx::mbar_wait(a_empty + ra.slot, ra.phase ^ 1, abort_flag, pa, 0))) { give_up(1); break; }
+                    ptx::mbar_arrive_expect_tx(a_full + ra.slot, C::kSlotA, issue);
 #pragma unroll
                     for (uint32_t box = 0; box < BK / 64; ++box)
                         ptx::tma_load_2d(smem_gen + C::kOffA + ra.slot * C::kSlotA + box * (T * 128), &tm_a,
-                                         a_full + ra.slot, kb * BK + box * 64, walk.m_blk * T);
+                                         a_full + ra.slot, kb * BK + box * 64, walk.m_blk * T, issue);
                     ra.advance<C::kDepthA>();
                     rp.advance<C::kDepthP>();
                 }
             }
             // nobody refills the last P slots, whose commits have to have arrived all the same
             if (kGeneral && ok && !gemm::drain_ring<C::kDepthP>(rp, [&](uint32_t i, uint32_t parity) {
-                    return ptx::mbar_wait(p_empty + i, parity, abort_flag, pa, 0); })) give_up(1);
+                    return ptx::all_lanes(ptx::mbar_wait(p_empty + i, parity, abort_flag, pa, 0)); })) give_up(1);
         }
     } else if (warp == kWarpMma) {
         const uint32_t issue_lane = ptx::elect_one();

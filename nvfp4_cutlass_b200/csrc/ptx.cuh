@@ -27,9 +27,12 @@ NVFP4_DEVICE void mbar_arrive(uint64_t* bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-NVFP4_DEVICE void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes)
+// `issue`: as for tcgen05_commit, here and in the loads below, whose operands are uniform registers too.  With the decode kernels'
+// and the split GEMM's producers run by the whole warp a 16-token call takes 5.4 us (5.8 with one lane), a 128-token call 6.2 (6.5).
+NVFP4_DEVICE void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes, uint32_t issue = 1)
 {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n @q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}\n"
+                 ::"r"(smem_u32(bar)), "r"(bytes), "r"(issue)
                  : "memory");
 }
 NVFP4_DEVICE bool mbar_try_wait(uint64_t* bar, uint32_t parity)
@@ -140,29 +143,32 @@ NVFP4_DEVICE void prefetch_tensormap(const CUtensorMap* map)
 {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
-NVFP4_DEVICE void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int32_t c0, int32_t c1)
+NVFP4_DEVICE void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int32_t c0, int32_t c1, uint32_t issue = 1)
 {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
+        "{\n .reg .pred q;\n setp.ne.b32 q, %5, 0;\n"
+        " @q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n}\n"
+        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(issue)
         : "memory");
 }
 // Untiled bulk copy global -> this CTA's shared memory (both addresses 16-byte aligned, size a multiple of
 // 16); the bytes complete on `bar`.
-NVFP4_DEVICE void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar)
+NVFP4_DEVICE void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar, uint32_t issue = 1)
 {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(gmem_src)), "r"(bytes), "r"(smem_u32(bar))
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %4, 0;\n"
+                 " @q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}\n"
+                 ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(gmem_src)), "r"(bytes), "r"(smem_u32(bar)), "r"(issue)
                  : "memory");
 }
 NVFP4_DEVICE void tma_load_2d_hint(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int32_t c0, int32_t c1,
-                                   uint64_t policy)
+                                   uint64_t policy, uint32_t issue = 1)
 {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint "
-        "[%0], [%1, {%3, %4}], [%2], %5;"
+        "{\n .reg .pred q;\n setp.ne.b32 q, %6, 0;\n"
+        " @q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint "
+        "[%0], [%1, {%3, %4}], [%2], %5;\n}\n"
         ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1),
-        "l"(policy)
+        "l"(policy), "r"(issue)
         : "memory");
 }
 
@@ -534,11 +540,12 @@ NVFP4_DEVICE void tmem_dealloc_pair(uint32_t taddr)
 }
 // Tiled load into this CTA's shared memory whose bytes complete on an mbarrier that may live in the other CTA
 // of the pair (`bar_cluster_addr` from map_to_cta).  Not a multicast: every CTA fetches its own tile.
-NVFP4_DEVICE void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int32_t c0, int32_t c1)
+NVFP4_DEVICE void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int32_t c0, int32_t c1, uint32_t issue = 1)
 {
     asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
+        "{\n .reg .pred q;\n setp.ne.b32 q, %5, 0;\n"
+        " @q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n}\n"
+        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(issue)
         : "memory");
 }
 // D[tmem of both CTAs] (+)= A * B over a CTA pair: M = 256 (each CTA its own 128 rows of A, from its own shared
