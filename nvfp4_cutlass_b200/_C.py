@@ -167,7 +167,20 @@ def set_probe_buffer(t=None) -> None:
 
 
 def _contiguous_device(a, b, sfb, gw, d, m_indices, device_status) -> int:
-    """Index of the operands' device; raises if they do not fit together."""
+    """Index of the operands' device; raises if they do not fit together.  The first expression is the whole list of
+    conditions for an ordinary call, which comes here with tune arguments that binding.cpp does not take (one by one the conditions
+    take 6 us more: a decode call of 4 experts x 16 rows, N = K = 512, 17.2 against 11.1 us with tune_block_n=0, 19.8 against 13.6 with
+    tune_block_k=256); whatever fails it goes through them one by one, which accept a little more and name the one that does not hold."""
+    index = a.get_device()
+    if a.dtype == d.dtype == torch.bfloat16 and b.dtype == torch.int8 and sfb.dtype == m_indices.dtype == torch.int32 and \
+            gw.dtype == torch.float32 and a.dim() == d.dim() == b.dim() == sfb.dim() == 2 and m_indices.dim() == 1 and \
+            device_status is None and \
+            index == b.get_device() == sfb.get_device() == gw.get_device() == d.get_device() == m_indices.get_device() >= 0 and \
+            b.is_contiguous() and sfb.is_contiguous() and gw.is_contiguous() and m_indices.is_contiguous() and \
+            a.stride(1) == d.stride(1) == 1 and a.is_cuda:
+        (m, k), (rows, n), e = a.shape, d.shape, gw.numel()
+        if rows == m and m_indices.shape[0] == m and b.shape == (e * n, k // 2) and sfb.shape == (e * (k // 64), n):
+            return index
     _require(a.dtype == torch.bfloat16, "a.dtype == bfloat16")
     _require(d.dtype == torch.bfloat16, "d.dtype == bfloat16")
     _require(b.dtype == torch.int8, "b.dtype == int8")

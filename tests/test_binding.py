@@ -47,6 +47,33 @@ def test_it_answers_none_to_host_tensors_subclasses_and_odd_options():
         _C._contiguous_call(*t)
 
 
+class OnDevice:
+    """A host tensor that says of itself that it is on CUDA device 0."""
+    is_cuda = True
+
+    def __init__(self, t):
+        self._t = t
+
+    def get_device(self):
+        return 0
+
+    def __getattr__(self, name):
+        return getattr(self._t, name)
+
+
+def test_a_tuned_call_that_fits_is_judged_by_one_expression(monkeypatch):
+    """Calls with tune arguments do not go through the binding; their conditions are not taken one by one either, which took half
+    as long again as the whole call."""
+    t = {name: OnDevice(x) for name, x in operands("cpu").items()}
+    one_by_one = []
+    monkeypatch.setattr(_C, "_require", lambda cond, what: one_by_one.append((bool(cond), what)))
+    assert _C._contiguous_device(**t, device_status=None) == 0 and one_by_one == []
+    monkeypatch.setattr(_C, "_one_device", lambda *tensors: torch.device("cuda", 0))
+    t["sfb"] = OnDevice(t["sfb"]._t[:-1])
+    _C._contiguous_device(**t, device_status=None)
+    assert [what for cond, what in one_by_one if not cond] == ["sfb.size(0) == num_groups * (k / 64)"]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("swap,align,m", [(0, 128, 256), (1, 16, 16), (1, 32, 96)])
 @pytest.mark.parametrize("residual", [True, False])
