@@ -20,7 +20,13 @@ import torch
 _LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libnvfp4_b200.so")
 _BINDING_PATH = os.path.join(os.path.dirname(_LIB_PATH), "_binding.so")
 _lib = None
-_contiguous_call = None        # binding.cpp's form of the contiguous GEMM call, once the library is loaded
+
+
+def _no_binding(*args):
+    """Stands where binding.cpp's form of the contiguous GEMM call belongs: takes no call, every call goes the general way."""
+
+
+_contiguous_call = _no_binding
 
 POLICY_CODES = {"derived_div8": 0, "residual_amax": 1, "derived_div4": 2, "div4_radix8": 3}
 
@@ -94,7 +100,8 @@ def lib() -> ctypes.CDLL:
         binding = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_binding", _BINDING_PATH, loader=loader))
         loader.exec_module(binding)
         binding.bind(ctypes.cast(L.nvfp4_grouped_gemm_contiguous, vp).value)
-        _lib, _contiguous_call = L, binding.contiguous
+        _contiguous_call = binding.contiguous
+        _lib = L                                     # last: another thread that finds it set makes its call at once
     return _lib
 
 

@@ -1,7 +1,12 @@
 """The CPython form of the contiguous call (csrc/binding.cpp): what it does not take goes the general way, with that way's errors, and
 what it takes gives the general way's results."""
+import subprocess
+import sys
+
 import pytest
 import torch
+
+from conftest import ROOT
 
 import nvfp4_gemm
 from nvfp4_cutlass_b200 import _C
@@ -45,6 +50,35 @@ def test_it_answers_none_to_host_tensors_subclasses_and_odd_options():
     assert _C._contiguous_call(*t, 0, 1, 0, 1 << 80) is None and _C._contiguous_call(None, *t[1:], 0, 1, 0, 0) is None
     with pytest.raises(TypeError):
         _C._contiguous_call(*t)
+
+
+FIRST_USE = """
+import sys
+from nvfp4_cutlass_b200 import _C
+seen = 0
+def step(frame, event, arg):
+    global seen
+    seen += event == "opcode"
+    if _C._lib is not None:
+        assert callable(_C._contiguous_call), "the library is there, the call is not"
+    return step
+def enter(frame, event, arg):
+    if frame.f_code is _C.lib.__code__:
+        frame.f_trace_opcodes = True
+        return step
+sys._getframe().f_trace_opcodes = True               # Python 3.12 has opcode events only if a frame asked for them before
+sys.settrace(enter)
+_C.lib()
+sys.settrace(None)
+assert seen > 100
+assert _C._lib is not None and _C._contiguous_call(*range(10)) is None
+"""
+
+
+def test_a_thread_that_finds_the_library_loaded_can_call():
+    """At no instruction of the first use is the library visible to another thread and the call that comes with it not."""
+    r = subprocess.run([sys.executable, "-c", FIRST_USE], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
 
 
 class OnDevice:
