@@ -14,6 +14,7 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import os
+import warnings
 
 import torch
 
@@ -55,11 +56,10 @@ def lib() -> ctypes.CDLL:
     """The loaded shared library; raises if it has not been built."""
     global _lib, _contiguous_call
     if _lib is None:
-        for path in (_LIB_PATH, _BINDING_PATH):
-            if not os.path.exists(path):
-                raise RuntimeError(
-                    f"{path} is missing: build it with `python nvfp4_cutlass_b200/csrc/build.py` "
-                    "(there is no fallback path)")
+        if not os.path.exists(_LIB_PATH):
+            raise RuntimeError(
+                f"{_LIB_PATH} is missing: build it with `python nvfp4_cutlass_b200/csrc/build.py` "
+                "(there is no fallback path)")
         L = ctypes.CDLL(_LIB_PATH)
         vp, i32, i64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
         L.nvfp4_last_error.restype = ctypes.c_char_p
@@ -96,13 +96,24 @@ def lib() -> ctypes.CDLL:
         L.nvfp4_debug_mma_peak.argtypes = [i32, ctypes.POINTER(ctypes.c_double), vp]
         L.nvfp4_debug_mma_peak_pair.argtypes = [i32, ctypes.POINTER(ctypes.c_double), vp]
         L.nvfp4_debug_mma_pattern.argtypes = [i32, i32, i32, i32, i32, ctypes.POINTER(ctypes.c_double), vp]
+        _contiguous_call = _bind(L)
+        _lib = L                                     # last: another thread that finds it set makes its call at once
+    return _lib
+
+
+def _bind(library):
+    """binding.cpp's form of the contiguous GEMM call, bound to the library's entry.  It is a faster way to the same entry and nothing
+    else needs it: without it (a build without torch's headers, a torch without CUDA) every call goes the general way."""
+    try:
         loader = importlib.machinery.ExtensionFileLoader("_binding", _BINDING_PATH)
         binding = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_binding", _BINDING_PATH, loader=loader))
         loader.exec_module(binding)
-        binding.bind(ctypes.cast(L.nvfp4_grouped_gemm_contiguous, vp).value)
-        _contiguous_call = binding.contiguous
-        _lib = L                                     # last: another thread that finds it set makes its call at once
-    return _lib
+    except (ImportError, OSError) as e:
+        if torch.version.cuda is not None:
+            warnings.warn(f"{_BINDING_PATH} does not load ({e}): GEMM calls take some 6 us more on the host", RuntimeWarning, stacklevel=3)
+        return _no_binding
+    binding.bind(ctypes.cast(library.nvfp4_grouped_gemm_contiguous, ctypes.c_void_p).value)
+    return binding.contiguous
 
 
 def _check(rc: int) -> None:

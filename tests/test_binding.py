@@ -81,6 +81,21 @@ def test_a_thread_that_finds_the_library_loaded_can_call():
     assert r.returncode == 0, r.stderr
 
 
+@pytest.mark.parametrize("found", ["nothing", "something else"])
+def test_without_the_binding_everything_goes_the_general_way(monkeypatch, tmp_path, found):
+    path = tmp_path / "_binding.so"
+    if found != "nothing":
+        path.write_bytes(b"not a module")
+    for name, value in (("_BINDING_PATH", str(path)), ("_lib", None), ("_contiguous_call", _C._no_binding)):
+        monkeypatch.setattr(_C, name, value)
+    with pytest.warns(RuntimeWarning, match="does not load"):
+        assert _C.lib() is not None
+    t = operands("cpu")
+    assert _C._contiguous_call(*t.values(), 0, 1, 0, 0) is None
+    with pytest.raises(RuntimeError, match="a is a CUDA tensor"):
+        nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(**t)
+
+
 class OnDevice:
     """A host tensor that says of itself that it is on CUDA device 0."""
     is_cuda = True
