@@ -19,7 +19,8 @@ import warnings
 import torch
 
 _LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libnvfp4_b200.so")
-_BINDING_PATH = os.path.join(os.path.dirname(_LIB_PATH), "_binding.so")
+# binding.cpp's module, compiled against one torch's and one Python's C interfaces, which its name says: another finds none
+_BINDING_PATH = os.path.join(os.path.dirname(_LIB_PATH), f"_binding-torch{torch.__version__}{importlib.machinery.EXTENSION_SUFFIXES[0]}")
 _lib = None
 
 

@@ -5,10 +5,11 @@
 Each .cu is compiled to an object with nvcc, then linked into one shared library
 next to the Python package (nvfp4_cutlass_b200/lib/libnvfp4_b200.so).  Objects are
 rebuilt only when a source or header is newer.  binding.cpp becomes a CPython module
-beside it (lib/_binding.so), compiled with g++ against torch's headers.
+beside it (lib/_binding-torch<version>.<Python's ABI>.so), compiled with g++ against torch's headers.
 """
 from __future__ import annotations
 
+import importlib.machinery
 import os
 import subprocess
 import sys
@@ -20,7 +21,6 @@ PKG = os.path.dirname(HERE)
 OUT_DIR = os.path.join(PKG, "lib")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(OUT_DIR, "libnvfp4_b200.so")
-BINDING = os.path.join(OUT_DIR, "_binding.so")
 SOURCES = ["abi.cu", "gemm_normal.cu", "gemm_cluster.cu", "gemm_split.cu", "gemm_swap.cu", "gemm_stream.cu", "moe_glue.cu", "quantize_weight.cu", "checkpoint_loader.cu", "debug_kernels.cu"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 HEADER = os.path.join(os.path.dirname(PKG), "include", "nvfp4_b200.h")
@@ -35,14 +35,24 @@ def _newest_header() -> float:
     return max(os.path.getmtime(h) for h in hdrs)
 
 
+def binding_path() -> str:
+    """Where the module for this interpreter and the installed torch belongs: it reads tensors through both's C interfaces, so
+    its name says which, and after an upgrade of either there is none until the next build (_C.py looks for the same name)."""
+    import torch
+
+    return os.path.join(OUT_DIR, f"_binding-torch{torch.__version__}{importlib.machinery.EXTENSION_SUFFIXES[0]}")
+
+
 def _binding_command() -> list:
+    import torch
     from torch.utils import cpp_extension
 
     include = [f"-I{d}" for d in (*cpp_extension.include_paths(), sysconfig.get_paths()["include"],
                                   os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"))]
     libs = [f"-L{d}" for d in cpp_extension.library_paths()]      # loaded by torch before the module is imported
-    return ["/usr/bin/g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", *include, *libs,
-            os.path.join(HERE, "binding.cpp"), "-o", BINDING, "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    return ["/usr/bin/g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *include, *libs,
+            os.path.join(HERE, "binding.cpp"), "-o", binding_path(), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -58,8 +68,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
     link = bool(jobs) or not os.path.exists(LIB)
     binding = os.path.join(HERE, "binding.cpp")
-    if force or not os.path.exists(BINDING) or os.path.getmtime(BINDING) < max(os.path.getmtime(binding), os.path.getmtime(HEADER)):
-        jobs.append((binding, BINDING))
+    target = binding_path()
+    if force or not os.path.exists(target) or os.path.getmtime(target) < max(os.path.getmtime(binding), os.path.getmtime(HEADER)):
+        jobs.append((binding, target))
 
     def compile_one(job):
         s, o = job

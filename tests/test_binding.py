@@ -1,7 +1,9 @@
 """The CPython form of the contiguous call (csrc/binding.cpp): what it does not take goes the general way, with that way's errors, and
 what it takes gives the general way's results."""
+import os
 import subprocess
 import sys
+import types
 
 import pytest
 import torch
@@ -10,6 +12,7 @@ from conftest import ROOT
 
 import nvfp4_gemm
 from nvfp4_cutlass_b200 import _C
+from nvfp4_cutlass_b200.csrc import build
 
 
 def operands(device, m=128, n=256, k=256, e=2):
@@ -94,6 +97,32 @@ def test_without_the_binding_everything_goes_the_general_way(monkeypatch, tmp_pa
     assert _C._contiguous_call(*t.values(), 0, 1, 0, 0) is None
     with pytest.raises(RuntimeError, match="a is a CUDA tensor"):
         nvfp4_gemm.m_grouped_bf16_dual_nvfp4_gemm_contiguous(**t)
+
+
+@pytest.fixture
+def compiled(monkeypatch):
+    """Command lines that the build would run; nothing is run."""
+    commands = []
+    monkeypatch.setattr(build.subprocess, "run", lambda cmd, **kw: commands.append(cmd) or types.SimpleNamespace(returncode=0, stdout="", stderr=""))
+    return commands
+
+
+def binding_commands(commands):
+    return [cmd for cmd in commands if any(arg.endswith("binding.cpp") for arg in cmd)]
+
+
+def test_another_torch_gets_a_module_of_its_own(compiled, monkeypatch, tmp_path):
+    assert build.binding_path() == _C._BINDING_PATH and os.path.exists(_C._BINDING_PATH)
+    monkeypatch.setattr(build, "OUT_DIR", str(tmp_path))
+    with open(build.binding_path(), "w"):
+        pass
+    build.build()
+    assert binding_commands(compiled) == []                              # this torch has its module
+    monkeypatch.setattr(torch, "__version__", "99.0")
+    build.build()
+    (cmd,) = binding_commands(compiled)
+    assert cmd[cmd.index("-o") + 1] == build.binding_path() and "torch99.0" in build.binding_path()
+    assert f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}" in cmd
 
 
 class OnDevice:
