@@ -6,6 +6,8 @@ Each .cu is compiled to an object with nvcc, then linked into one shared library
 next to the Python package (nvfp4_cutlass_b200/lib/libnvfp4_b200.so).  Objects are
 rebuilt only when a source or header is newer.  binding.cpp becomes a CPython module
 beside it (lib/_binding-torch<version>.<Python's ABI>.so), compiled with g++ against torch's headers.
+The library itself needs the CUDA toolkit alone: where there is no torch with CUDA, or the module does not compile, the build says
+so and goes on without it (a Python caller's GEMM calls then go through ctypes).
 """
 from __future__ import annotations
 
@@ -35,11 +37,16 @@ def _newest_header() -> float:
     return max(os.path.getmtime(h) for h in hdrs)
 
 
-def binding_path() -> str:
+def binding_path():
     """Where the module for this interpreter and the installed torch belongs: it reads tensors through both's C interfaces, so
-    its name says which, and after an upgrade of either there is none until the next build (_C.py looks for the same name)."""
-    import torch
-
+    its name says which, and after an upgrade of either there is none until the next build (_C.py looks for the same name).
+    None where there is no torch with CUDA to compile it against."""
+    try:
+        import torch
+    except (ImportError, OSError):
+        return None
+    if torch.version.cuda is None:
+        return None
     return os.path.join(OUT_DIR, f"_binding-torch{torch.__version__}{importlib.machinery.EXTENSION_SUFFIXES[0]}")
 
 
@@ -69,14 +76,20 @@ def build(force: bool = False, verbose: bool = False) -> str:
     link = bool(jobs) or not os.path.exists(LIB)
     binding = os.path.join(HERE, "binding.cpp")
     target = binding_path()
-    if force or not os.path.exists(target) or os.path.getmtime(target) < max(os.path.getmtime(binding), os.path.getmtime(HEADER)):
+    if target is None:
+        print("no torch with CUDA: built without binding.cpp's module", file=sys.stderr)
+    elif force or not os.path.exists(target) or os.path.getmtime(target) < max(os.path.getmtime(binding), os.path.getmtime(HEADER)):
+        if os.path.exists(target):
+            os.remove(target)                        # one that calls the library by an older header must not outlive a failed compile
         jobs.append((binding, target))
 
     def compile_one(job):
         s, o = job
-        cmd = _binding_command() if s.endswith(".cpp") else [NVCC, *FLAGS, *( ["-Xptxas", "-v"] if verbose else []), "-c", s, "-o", o]
+        cmd = _binding_command() if s == binding else [NVCC, *FLAGS, *( ["-Xptxas", "-v"] if verbose else []), "-c", s, "-o", o]
         r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
+        if r.returncode != 0 and s == binding:
+            print(f"built without binding.cpp's module, which did not compile:\n{r.stdout}\n{r.stderr}", file=sys.stderr)
+        elif r.returncode != 0:
             raise RuntimeError(f"{cmd[0]} failed on {s}:\n{r.stdout}\n{r.stderr}")
         return r.stderr
 

@@ -125,6 +125,33 @@ def test_another_torch_gets_a_module_of_its_own(compiled, monkeypatch, tmp_path)
     assert f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}" in cmd
 
 
+@pytest.mark.parametrize("torch_is", ["missing", "without CUDA", "there, its headers do not compile"])
+def test_the_library_builds_without_the_binding(compiled, monkeypatch, tmp_path, capsys, torch_is):
+    """The C ABI's consumers need the CUDA toolkit alone."""
+    monkeypatch.setattr(build, "OUT_DIR", str(tmp_path))
+    monkeypatch.setattr(build, "OBJ_DIR", str(tmp_path))
+    if torch_is == "missing":
+        monkeypatch.setitem(sys.modules, "torch", None)
+    elif torch_is == "without CUDA":
+        monkeypatch.setattr(torch.version, "cuda", None)
+    else:
+        with open(build.binding_path(), "w"):                            # of an older header
+            pass
+        record = build.subprocess.run
+        monkeypatch.setattr(build.subprocess, "run", lambda cmd, **kw: types.SimpleNamespace(
+            returncode=int(bool(binding_commands([cmd])) and record(cmd) is not None), stdout="", stderr="no such header"))
+    build.build(force=True)
+    assert "without binding.cpp's module" in capsys.readouterr().err
+    assert len(binding_commands(compiled)) == (torch_is not in ("missing", "without CUDA")) and os.listdir(tmp_path) == []
+
+
+def test_a_kernel_that_does_not_compile_fails_the_build(monkeypatch, tmp_path):
+    monkeypatch.setattr(build, "OBJ_DIR", str(tmp_path))
+    monkeypatch.setattr(build.subprocess, "run", lambda cmd, **kw: types.SimpleNamespace(returncode=1, stdout="", stderr="bad"))
+    with pytest.raises(RuntimeError, match="failed on"):
+        build.build()
+
+
 class OnDevice:
     """A host tensor that says of itself that it is on CUDA device 0."""
     is_cuda = True
