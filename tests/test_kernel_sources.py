@@ -190,3 +190,40 @@ def test_groups_in_turn_never_pass_a_wait_early(tmp_path):
     text = source("gemm_cluster.cu")                                   # the only kernel whose roles take blocks in turn
     assert re.search(r"wait_turn<C::kDepthA, C::kGroups>\(\s*it,.*?share_full \+ i,.*?a_full \+ i,", text, re.S)
     assert not any("% C::kGroups" in source(k) for k in KERNELS if k != "gemm_cluster.cu")
+
+
+def handed_back_too_early(text):
+    """Places where a slot that a bulk or TMA load fills goes back to its producer while plain loads of it may still be under way:
+    since the last load there is neither a proxy fence nor anything that used what was loaded (scales stored to tensor memory, an
+    output row stored).  Inside transform_tile the fence is transform_tile's own."""
+    bad = []
+    for m in re.finditer(r"ptx::mbar_arrive\((?:a_empty|sf_free|empty) \+", text):
+        if text.rfind("transform_tile<", 0, m.start()) > text.rfind("ptx::lds", 0, m.start()):
+            continue
+        since = text[text.rfind("ptx::lds", 0, m.start()):m.start()]
+        if not re.search(r"fence_proxy_async_smem\(\)|tmem_st_wait\(\)|\by\[[^;]*\] = make_uint4", since):
+            bad.append(text.count(chr(10), 0, m.start()) + 1)
+    return bad
+
+
+FENCED_TRANSFORM = r"load_tile_smem\(s, a_smem, t\);\s*ptx::fence_proxy_async_smem\(\);\s*on_loaded\(\);"
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_loads_of_a_slot_end_before_it_is_handed_back(name):
+    """A plain load is ordered before the asynchronous write that refills its slot by a proxy fence between the load and the arrive
+    that lets the producer go on.  Without it rows of the next tile turned up in 7 to 11 of 40 decode calls (120 experts, N = 1280,
+    K = 3456)."""
+    assert handed_back_too_early(source(name)) == []
+
+
+def test_the_rule_on_handed_back_slots_sees_a_missing_fence():
+    assert re.search(FENCED_TRANSFORM, source("transform.cuh"))
+    assert not re.search(r"\bon_loaded\(\);", re.sub(FENCED_TRANSFORM, "", source("transform.cuh")))       # the only hand-over there
+    text = source("gemm_cluster.cu")
+    fence = re.compile(r"ptx::fence_proxy_async_smem\(\);(?=\s*__syncwarp\(\);\s*if \(lane == 0\) ptx::mbar_arrive\(a_empty)")
+    assert len(fence.findall(text)) == 1 and len(handed_back_too_early(fence.sub("", text))) == 1
+    for name, used in (("gemm_split.cu", "ptx::tmem_st_wait();"), ("moe_glue.cu", "y[t * y_ld16 + c] = make_uint4(ow[0], ow[1], ow[2], ow[3]);")):
+        assert used in source(name) and handed_back_too_early(source(name).replace(used, ""))
+    places = sum(len(re.findall(r"ptx::mbar_arrive\((?:a_empty|sf_free|empty) \+", source(k))) for k in KERNELS)
+    assert places == 5                                     # decode, fused x 2, pair, bulk combine
