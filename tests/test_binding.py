@@ -1,5 +1,6 @@
 """The CPython form of the contiguous call (csrc/binding.cpp): what it does not take goes the general way, with that way's errors, and
 what it takes gives the general way's results."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -32,6 +33,8 @@ WRONG = {
 
 @pytest.mark.parametrize("name", WRONG)
 def test_it_answers_none_to_what_does_not_fit(name):
+    """Host tensors: none of them is an ordinary call's, and the general way names what does not fit.  The binding's own
+    conditions are tried below, where the tensors could be taken."""
     _C.lib()
     t = operands("cpu")
     t[name] = WRONG[name](t[name])
@@ -204,6 +207,80 @@ def test_both_ways_give_the_same(swap, align, m, residual):
     for other in (calls[3], calls[4], calls[5]):
         assert torch.equal(calls[1], other)
     assert bool((wide[:, 256:] == 7.0).all())
+
+
+@pytest.fixture
+def entry():
+    """What the binding hands to the C entry, which is not called: nothing is launched, whatever the binding takes."""
+    _C.lib()
+    module, handed = _C._contiguous_call.__self__, []
+    vp, i32, i64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
+    fake = ctypes.CFUNCTYPE(i32, vp, i64, vp, vp, vp, vp, i64, vp, *[i32] * 8, vp, vp, vp)(lambda *args: handed.append(args) or 0)
+    module.bind(ctypes.cast(fake, vp).value)
+    yield handed
+    module.bind(ctypes.cast(_C.lib().nvfp4_grouped_gemm_contiguous, vp).value)
+
+
+def across(t):
+    """The same values, the first dimension the contiguous one."""
+    return t.t().contiguous().t()
+
+
+class Subclass(torch.Tensor):
+    pass
+
+
+NOT_ORDINARY = {
+    "a": [lambda t: t.float(), lambda t: t.half(), lambda t: t[None], lambda t: t[0], lambda t: t[:-1], lambda t: t[:, :-64].contiguous(), across],
+    "b": [lambda t: t.to(torch.uint8), lambda t: t.int(), lambda t: t[None], lambda t: t.flatten(), lambda t: t[:-1], lambda t: t[:, :-1].contiguous(),
+          lambda t: torch.cat((t, t)), across, lambda t: torch.cat((t, t), 1)[:, :t.shape[1]]],
+    "sfb": [lambda t: t.long(), lambda t: t.float(), lambda t: t[None], lambda t: t.flatten(), lambda t: t[:-1], lambda t: t[:, :-1].contiguous(),
+            lambda t: torch.cat((t, t)), across],
+    "gw": [lambda t: t.double(), lambda t: t.bfloat16(), lambda t: t[:-1], lambda t: torch.cat((t, t)), lambda t: torch.stack((t, t), 1)[:, 0]],
+    "d": [lambda t: t.float(), lambda t: t.half(), lambda t: t[None], lambda t: t[0], lambda t: t[:-1], lambda t: t[:, :-8], across],
+    "m_indices": [lambda t: t.long(), lambda t: t.float(), lambda t: t[None], lambda t: t[:-1], lambda t: torch.cat((t, t)),
+                  lambda t: t.repeat_interleave(2)[::2]],
+}
+NOT_PLAIN = [lambda t: t.cpu(), lambda t: t.to("meta"), lambda t: t.as_subclass(Subclass), lambda t: t.data_ptr(), lambda t: None]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", NOT_ORDINARY)
+def test_it_takes_no_tensor_that_does_not_fit(entry, name):
+    """Nothing behind the binding knows the sizes of the buffers: each of its conditions, by a call that fails that one."""
+    t = operands("cuda", m=256)
+    assert _C._contiguous_call(*t.values(), 0, 1, 0, 0) == 0 and len(entry) == 1
+    for i, change in enumerate(NOT_ORDINARY[name] + NOT_PLAIN):
+        assert _C._contiguous_call(*{**t, name: change(t[name])}.values(), 0, 1, 0, 0) is None, i
+    if t[name].dim() == 2:
+        assert _C._contiguous_call(*{**t, name: t[name].to_sparse()}.values(), 0, 1, 0, 0) is None
+    batched = []
+    torch.vmap(lambda x: batched.append(_C._contiguous_call(*{**t, name: x}.values(), 0, 1, 0, 0)) or x)(torch.stack((t[name], t[name])))
+    assert batched == [None] and len(entry) == 1
+
+
+@pytest.mark.gpu
+def test_what_it_hands_on(entry):
+    t = operands("cuda", m=256)
+    pointers = {name: x.data_ptr() for name, x in t.items()}
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        assert _C._contiguous_call(*t.values(), 3, 0, 1, 16) == 0
+    want = (pointers["a"], 256, pointers["b"], pointers["sfb"], pointers["gw"], pointers["d"], 256, pointers["m_indices"], 256, 256, 256, 2, 3, 0, 1, 16,
+            None, None, side.cuda_stream)
+    assert entry.pop() == want
+    for option in range(4):
+        for value in (-1, 1 << 31, 1 << 80, 1.0, "1", None):
+            options = [0, 1, 0, 0]
+            options[option] = value
+            assert _C._contiguous_call(*t.values(), *options) is None
+    wide = torch.zeros(256, 384, dtype=torch.bfloat16, device="cuda")
+    for name, at in (("a", 0), ("d", 5)):                               # a parameter whose rows are further apart
+        assert _C._contiguous_call(*{**t, name: torch.nn.Parameter(wide[:, 128:], requires_grad=False)}.values(), 0, 1, 0, 0) == 0
+        assert entry.pop()[at:at + 2] == (wide.data_ptr() + 256, 384)
+    # the stride of a single row is not one
+    one = {**t, "a": t["a"].as_strided((1, 256), (8, 1)), "d": t["d"][:1], "m_indices": t["m_indices"][:1]}
+    assert _C._contiguous_call(*one.values(), 0, 1, 0, 0) == 0 and entry.pop()[1] == 256
 
 
 @pytest.mark.gpu
