@@ -280,7 +280,8 @@ int nvfp4_grouped_gemm_contiguous(const void* a, int64_t lda_elems, const void* 
         int tile = tune_block_n > 0 ? tune_block_n : (m_alignment >= 64 ? 64 : m_alignment);
         NVFP4_REQUIRE((tile == 16 || tile == 32 || tile == 64) && m_alignment % tile == 0,
                       "token tile %d must be 16, 32 or 64 and divide m_alignment %d", tile, m_alignment);
-        const int tune_block_k = tune ? tune[5] : 0;   // 0 = the largest of 512 / 256 / 128 that divides K and fits
+        const int tune_block_k = tune ? tune[5] : 0;   // 0 = 512 (256 for 64-token tiles) where it divides K, else 256 where that does, else from K = 896 on the
+                                                       // large one with the last block in part, and 128 below (launch_for_tile)
         NVFP4_REQUIRE(tune_block_k == 0 || tune_block_k == 128 || tune_block_k == 256 || tune_block_k == 512,
                       "tune_block_k must be 0, 128, 256 or 512");
         // tune_split_transform as in the normal orientation: 1 = activations quantised in a pass of their own (where K % 256 == 0

@@ -231,10 +231,10 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     } else if (warp == kWarpMma) {
         // ================= MMA issue =================
         // The scale factors are already in tensor memory when a K block is issued (the scale warps
-        // put them there with tcgen05.st), so a K block costs this thread four MMAs and its commits:
+        // put them there with tcgen05.st), so a K block costs the issuing lane four MMAs and its commits:
         // a tensor-memory copy of one scale atom costs as much issue time as an MMA of N <= 128, and
         // eight of them per K block were the larger half of the tensor-side time.
-        // One thread runs the whole role.  A round takes the next K block and, if its scales are already up, the one
+        // The whole warp runs the role, so every statement here is run by 32 lanes; one elected lane issues.  A round takes the next K block and, if its scales are already up, the one
         // after it too: the fixed cost of a round (barrier round trips, loop) is then paid once per eight MMAs.
         {
             const uint32_t issue = ptx::elect_one();

@@ -127,8 +127,7 @@ struct Walker {
 
 // kGeneral: K need not be a multiple of BK, and a CTA may take several weight tiles with one transformed token tile.  A form of its
 // own, because a decode call is over in a few microseconds and is held up by every instruction that it fetches: all of the
-// general form's in one kernel took a call of 16 tokens, 32 experts, N = 1024, K = 2048 from 6.0 to 6.8 us
-// (now 6.2).
+// general form's in one kernel took a call of 16 tokens, 32 experts, N = 1024, K = 2048 from 6.0 to 6.8 us.
 template <uint32_t T, uint32_t BK, bool kResidual, int kPolicy, bool kGeneral>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,

@@ -217,8 +217,9 @@ NVFP4_DEVICE uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0
 // All earlier tcgen05.mma / tcgen05.cp of this thread arrive (once) on `bar` when they retire.
 // `issue`: in a role that the whole warp runs, nonzero in the lane that issues (elect_one), for MMAs as for commits.  The operands of
 // tcgen05 instructions live in uniform registers; in a branch of a single lane they are kept in the lane's own and moved for every
-// MMA, and the issuing thread, not the tensor pipe, set the pace (1300 cycles of it per K block of 256 in gemm_split.cu, whose
-// MMAs take 1024; 1240 for eight MMAs of a decode K block, which take 430).  One lane / the whole warp: decode of 128 tokens (32 experts, N =
+// MMA, and in the decode kernels the issuing thread, not the tensor pipe, set the pace (1240 cycles for the eight MMAs of a K block,
+// which take 430).  In gemm_split.cu it was 1300 cycles per K block of 256, whose MMAs take 1024, in a trace of one CTA, but the large
+// calls run at the power cap and gained 1-3 %.  One lane / the whole warp: decode of 128 tokens (32 experts, N =
 // 2048, K = 512) 7.4 / 6.6 us, of 25 tokens of 208 experts (N = 640, K = 4480) 39.5 / 33.3, expert layer of 16384 tokens 2889 / 2793,
 // 32k zipf rows, N = 7168, K = 2048, one pass, 653 / 639.
 NVFP4_DEVICE void tcgen05_commit(uint64_t* bar, uint32_t issue = 1)
