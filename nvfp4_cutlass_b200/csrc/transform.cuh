@@ -285,8 +285,9 @@ NVFP4_DEVICE void emit_tile(const TileShare<kRows, kBK, kThreads>& s, uint32_t a
     }
 }
 
-// Shared-memory tile in, products out; `on_loaded()` runs between the reads and the
-// arithmetic (the caller releases the BF16 slot there).
+// Shared-memory tile in, products out; `on_loaded()` runs between the reads and the arithmetic.  The reads have been issued by then, no
+// more: a proxy fence has to follow them before the slot may go back to the TMA that rewrites it.  Without one rows of the next tile
+// turned up in 7 to 11 of 40 decode calls (120 experts, N = 1280, K = 3456).
 template <uint32_t kRows, uint32_t kBK, uint32_t kThreads, bool kResidual, uint32_t kSfCols = 4, uint32_t kSubRows = 0,
           int kPolicy = 0, typename OnLoaded>
 NVFP4_DEVICE void transform_tile(uint32_t a_smem, uint32_t a0_smem, uint32_t a1_smem, uint32_t sfa0_smem,
@@ -294,10 +295,6 @@ NVFP4_DEVICE void transform_tile(uint32_t a_smem, uint32_t a0_smem, uint32_t a1_
 {
     TileShare<kRows, kBK, kThreads> s;
     load_tile_smem(s, a_smem, t);
-    // The loads are over before on_loaded hands the slot back to the TMA that rewrites it: without the fence rows of the next tile turned
-    // up in 7 to 11 of 40 decode calls (120 experts, N = 1280, K = 3456).  It costs up to 4 % of a decode call with 32-token
-    // tiles (160 experts x 32 rows, N = 512, K = 1024: 15.9 / 16.4 us) and less elsewhere.
-    ptx::fence_proxy_async_smem();
     on_loaded();
     emit_tile<kRows, kBK, kThreads, kResidual, kSfCols, kSubRows, kPolicy>(s, a0_smem, a1_smem, sfa0_smem, sfa1_smem, t);
 }
