@@ -389,11 +389,14 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     smem + C::kOffA + ra.slot * C::kSlotA, smem + C::kOffP + rp.slot * C::kSlotP,
                     smem + C::kOffP + rp.slot * C::kSlotP + C::kA1Bytes, smem + C::kOffSFT + rp.slot * C::kSlotSFT,
                     smem + C::kOffSFT + rp.slot * C::kSlotSFT + C::kSF1Bytes, t, [&] {
-                        // the loads are over before TMA may rewrite the slot; the fence costs up to 4 % of a decode call with 32-token tiles (160
-                        // experts x 32 rows, N = 512, K = 1024: 15.9 / 16.4 us) and less elsewhere
-                        ptx::fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(a_empty + ra.slot);
+                        // The loads of the slot have to be over before TMA may rewrite it.  A fence for that here holds the arithmetic up, by
+                        // up to 5 % of a call; the general form takes it all the same, because there the early refill is worth more (120
+                        // experts x 32 rows, N = 1280, K = 3456, one pass: slot back here 57.2 us, after the arithmetic 60.4).
+                        if constexpr (kGeneral) {
+                            ptx::fence_proxy_async_smem();
+                            __syncwarp();
+                            if (lane == 0) ptx::mbar_arrive(a_empty + ra.slot);
+                        }
                         // the slot is free once the MMAs of the last weight tile over it have retired; with one weight tile that is
                         // what the weight ring's barrier says of kDepthP K blocks ago
                         const uint32_t ago = cnt - C::kDepthP;
@@ -404,9 +407,15 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                                                   ptx::mbar_wait(w_empty + ago % C::kDepthW, (ago / C::kDepthW) & 1u, abort_flag, pa, 1));
                     });
                 if (!p_ok) { give_up(1); break; }
+                // Else one fence serves both, the products before the tensor core reads them and the loads before the slot goes back.
+                // Fence of its own / this, 32-token tiles: 160 experts, N = 512, K = 1024 16.3 / 15.4 us, 32 experts, N = 1024, K = 2048
+                // 13.2 / 12.4; 16-token tiles 10.7 / 10.4 and 8.9 / 8.6; on 260 calls nowhere slower.
                 ptx::fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(p_full + rp.slot);
+                if (lane == 0) {
+                    if constexpr (!kGeneral) ptx::mbar_arrive(a_empty + ra.slot);
+                    ptx::mbar_arrive(p_full + rp.slot);
+                }
                 ra.advance<C::kDepthA>();
                 rp.advance<C::kDepthP>();
             }

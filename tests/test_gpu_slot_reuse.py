@@ -45,12 +45,14 @@ def assert_rows_match(oracle, d, a, b, sfb, gw, mi, residual, experts, columns=1
 
 
 @pytest.mark.parametrize("tile", [16, 32, 64])
+@pytest.mark.parametrize("k", [3456, 3584])
 @pytest.mark.parametrize("residual", [True, False])
-def test_decode_rows_stay_in_their_tile(oracle, tile, residual):
-    """Eight weight tiles a block, seven K blocks (thirteen at 64 tokens) with the last one in part, a P ring of two (three)."""
-    n, k = 1280, 3456
+def test_decode_rows_stay_in_their_tile(oracle, tile, k, residual):
+    """Eight weight tiles a block, seven K blocks (fourteen at 64 tokens), of 3456 the last one in part, a P ring of two (three): the two
+    forms of the kernel, which hand the slot back at different times."""
+    n = 1280
     t = operands([tile] * 120, n, k, tile)
-    kw = dict(enable_residual_pass=residual, m_alignment=tile, tune_swap_ab=1)
+    kw = dict(enable_residual_pass=residual, m_alignment=tile, tune_swap_ab=1, tune_split_transform=2)
     (want,) = calls(*t, n, 1, tune_block_k=128, **kw)
     assert_rows_match(oracle, want, *t, residual, (0, 57, 119))
     for i, d in enumerate(calls(*t, n, CALLS, **kw)):
