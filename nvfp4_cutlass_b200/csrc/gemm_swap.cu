@@ -478,7 +478,9 @@ int launch_variant(const void* a, int64_t lda, const void* b, const void* sfb, i
         // Where the P ring holds a token tile's whole K, a CTA can transform it once for a run of weight tiles.  To transform it costs
         // about as much as a weight tile and the general form about as much again: the run is the one with the shortest
         // rounds * (run + 1), if that saves more than 1.  128 tokens over 32 of 256 experts, N = 2048, K = 512:
-        // 8.3 us a call, with runs of four 7.3; 192 experts' worth of routing, N = 5120, K = 1024: 17.8 / 16.4.
+        // 8.3 us a call, with runs of four 7.3; 192 experts' worth of routing, N = 5120, K = 1024: 17.8 / 16.4.  Checked on 1248 calls (5 to 180
+        // token tiles of 16, 32 and 64, N 256-7168, K 256-1024): with the runs this rule takes 0.93 of the time on (geometric) average,
+        // nowhere more than 0.1 us above single tiles.
         int best = (num_tiles + num_sms - 1) / num_sms * 2 - 1;
         if ((K + static_cast<int>(BK) - 1) / static_cast<int>(BK) <= static_cast<int>(C::kDepthP))
             for (int log2 = 1; log2 <= 2 && num_n % (1 << log2) == 0; ++log2) {
