@@ -61,9 +61,9 @@ WORKLOADS = {
 # under profiles/, on the reduced workloads c2s / c4s (the full ones exceed what a multi-pass capture should
 # hold), as (bytes measured, algorithmic bytes of that captured launch).  The kernels stream every operand
 # once, so traffic grows in proportion to the algorithmic bytes; a full launch is scaled by that ratio.
-NCU_TRAFFIC = {"normal": (248.42e6, 251.66e6, "split-path kernels (CTA-pair GEMM) on c2s, captured at commit 458d43e"),
-               "swap_ab": (928.61e6, 911.22e6, "gemm_swap_kernel on c4s, captured at commit 458d43e"),
-               "swap_ab_split": (933.38e6, 911.22e6, "stream_quantize_kernel + gemm_stream_kernel on c4s, captured at commit 458d43e")}
+NCU_TRAFFIC = {"normal": (248.18e6, 251.66e6, "split-path kernels (CTA-pair GEMM) on c2s, captured at commit c07c85b"),
+               "swap_ab": (925.42e6, 911.22e6, "gemm_swap_kernel on c4s, captured at commit 509f954"),
+               "swap_ab_split": (933.85e6, 911.22e6, "stream_quantize_kernel + gemm_stream_kernel on c4s, captured at commit c07c85b")}
 
 
 def scaled_traffic(orientation: str, algo_bytes: float) -> dict:
